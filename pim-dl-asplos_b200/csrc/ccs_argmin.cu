@@ -1,22 +1,35 @@
 // Step 1 of the AMM: closest-centroid search (CCS).
 //
 // Replaces index_calculation() of the reference (inference-engine/src/host/index_calc_host.cpp:8-53).
-// The result has to match that function bit for bit, which pins three things:
-//   * every fp32 operation rounds on its own (the reference is built for baseline x86-64,
-//     no FMA): __fsub_rn / __fmul_rn / __fadd_rn are never contracted by nvcc;
+// The result has to match that function bit for bit.  There
+//   * every fp32 operation rounds on its own (the reference is built for baseline x86-64, no FMA);
 //   * the squared distance accumulates in dimension order starting from 0;
-//   * the "argmin" is a sequential scan with hysteresis - centroid c replaces the running
-//     minimum only if fl(min - dist[c]) > 1e-6 - so it is order dependent and each
-//     (token, codebook) scan runs in one thread, centroids 0..CT-1 in order.  A tree or
-//     shuffle reduction gives different indices on near-ties.
+//   * the "argmin" is a sequential scan with hysteresis - centroid c replaces the running minimum only
+//     if fl(min - dist[c]) > 1e-6 - so near-ties are decided by the order of the scan.
+//
+// exact_scan() below is that statement, one (token, codebook) in one thread, ~3v + 4 instructions per centroid.
+// It runs only where it can matter.  Every (token, codebook) first goes through a FILTER that evaluates
+//     s_c = |c|^2 / 2 - x.c      (so that |x - c|^2 = |x|^2 + 2 s_c),   v fused multiply-adds per centroid,
+// and looks for centroids within a margin T of the smallest s_c.  If there is exactly one, the scan ends on it
+// whatever the order: with D_c the true squared distance, A = |x|^2, B = max |c|^2 and u = 2^-24,
+//     |s_c computed - s_c|       <= 1.01 (2v+1) u (A + B)
+//     |dist[c] computed - D_c|   <= 1.01 (v+3) u D_c,   and D of the winner <= 2 (A + B),
+// so a gap of more than T = 0.51e-6 + (8v + 16) u (A + B) in s makes fl(dist[c] - dist[winner]) > 1e-6 for
+// every other c: the scan takes the winner when it meets it and nothing after it.  Otherwise - two candidates,
+// or anything not finite - the thread runs exact_scan.  For N(0,1) data a few scans in 1e5 do at v = 2.
+//
+// What bounds it: dispatch.  Per centroid v/2 packed multiply-adds, half a packed addition (two dispatch cycles
+// each), half a three-input minimum and a funnel shift that collects the comparison's sign bit, against 3v/2 packed
+// and 4 other instructions of the scan; per (token, codebook) about 25 instructions around that.  v = 2, 16 centroids,
+// 65536 x 4096: 593 -> 484 us, the ALU pipe 53 % and the FMA pipe 45 % busy (they hardly overlap); v = 4, 64
+// centroids, 32768 x 3072: 1267 -> 492 us; v = 10, 16 centroids, 1576 x 2560: 87 -> 12 us.
 //
 // Two mappings:
-//   reg path    thread <-> codebook, centroids of that codebook live in registers, the
-//               thread walks a run of tokens; activations load as coalesced float2/float4.
-//               Used when CT*v <= 64 (all v in {2,4,8} x CT in {8,16,32} points with
-//               CT*v <= 64).
-//   smem path   thread <-> token, centroids of a block of codebooks sit in shared memory
-//               and are read as warp-wide broadcasts; any v, any CT <= 256.
+//   ccs_reg_kernel  thread <-> codebook, the codebook's centroids in registers, the thread walks a run of
+//                   tokens; activations load as coalesced float2 / float4.  Small centroid sets.
+//   ccs_tile_kernel thread <-> token (one or two), activations and centroids of a few codebooks staged in
+//                   shared memory, a centroid is read as a warp-wide broadcast.  Any v up to 32, any CT.
+//   ccs_any_kernel  any v, exact_scan alone.
 //
 // HBM traffic: 4*M*K (activations) + 4*CB*CT*v (centroids) + M*CB (uint8 indices).
 #include "kernels.h"
@@ -27,25 +40,119 @@ namespace lutamm {
 namespace {
 
 constexpr float kEps = 1e-6f;  // (double)diff > 1e-6  <=>  diff > 1e-6f for fp32 diff
+constexpr float kHuge = 1e30f;  // beyond this the filter's own arithmetic could overflow
 
+__host__ __device__ constexpr float margin_factor(int v) { return (float)(8 * v + 16) * 5.9604644775390625e-08f; }
+constexpr float kMarginBase = 0.51e-6f;
+
+// V floats of shared memory
 template <int V>
-__device__ __forceinline__ void load_x(const float* __restrict__ p, float (&f)[V]) {
+__device__ __forceinline__ void load_x(const float* p, float (&f)[V]) {
     if constexpr (V % 4 == 0) {
 #pragma unroll
         for (int i = 0; i < V / 4; ++i) {
-            float4 t = __ldg(reinterpret_cast<const float4*>(p) + i);
+            const float4 t = *reinterpret_cast<const float4*>(p + 4 * i);
             f[4 * i + 0] = t.x; f[4 * i + 1] = t.y; f[4 * i + 2] = t.z; f[4 * i + 3] = t.w;
         }
     } else if constexpr (V % 2 == 0) {
 #pragma unroll
         for (int i = 0; i < V / 2; ++i) {
-            float2 t = __ldg(reinterpret_cast<const float2*>(p) + i);
+            const float2 t = *reinterpret_cast<const float2*>(p + 2 * i);
             f[2 * i + 0] = t.x; f[2 * i + 1] = t.y;
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < V; ++i) f[i] = __ldg(p + i);
+        for (int i = 0; i < V; ++i) f[i] = p[i];
     }
+}
+
+// V floats of global memory
+template <int V>
+__device__ __forceinline__ void load_global(const float* __restrict__ p, float (&f)[V]) {
+    static_assert(V == 2 || V % 4 == 0, "vector loads");
+    if constexpr (V == 2) {
+        const float2 t = __ldg(reinterpret_cast<const float2*>(p));
+        f[0] = t.x; f[1] = t.y;
+    } else {
+#pragma unroll
+        for (int i = 0; i < V; i += 4) {
+            const float4 t = __ldg(reinterpret_cast<const float4*>(p + i));
+            f[i] = t.x; f[i + 1] = t.y; f[i + 2] = t.z; f[i + 3] = t.w;
+        }
+    }
+}
+
+template <int kBytes>
+__device__ __forceinline__ void copy_async(uint32_t dst, const void* src) {
+    if constexpr (kBytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(kBytes) : "memory");
+}
+
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// smallest of n values, as a tree of three-input minima
+template <int N>
+__device__ __forceinline__ float min_of(const float (&k)[N]) {
+    if constexpr (N == 1) {
+        return k[0];
+    } else if constexpr (N == 2) {
+        return fminf(k[0], k[1]);
+    } else {
+        float t[(N + 2) / 3];
+#pragma unroll
+        for (int i = 0; i < N / 3; ++i) t[i] = min3(k[3 * i], k[3 * i + 1], k[3 * i + 2]);
+        if constexpr (N % 3 == 1) t[N / 3] = k[N - 1];
+        if constexpr (N % 3 == 2) t[N / 3] = fminf(k[N - 2], k[N - 1]);
+        return min_of(t);
+    }
+}
+
+// One bit per key that lies below the threshold: key i at bit i.  The comparison is the sign of key - threshold;
+// NaN and overflow are excluded by the callers' check of the margin.  (Two scalar multiply-adds per key, the first
+// saturating to 0 or 1, need no integer instruction but measured 4 % slower: a scalar multiply-add holds its pipe
+// as long as a packed one.)
+template <int N>
+__device__ __forceinline__ uint32_t below(const float (&k)[N], float thr) {
+    uint32_t mask = 0;
+    const float2 neg = make_float2(-thr, -thr);
+#pragma unroll
+    for (int i = N - 2; i >= 0; i -= 2) {
+        const float2 e = __fadd2_rn(make_float2(k[i], k[i + 1]), neg);
+        mask = __funnelshift_l(__float_as_uint(e.y), mask, 1);
+        mask = __funnelshift_l(__float_as_uint(e.x), mask, 1);
+    }
+    return mask;
+}
+// position of the highest set bit
+__device__ __forceinline__ uint32_t high_bit(uint32_t v) {
+    uint32_t r;
+    asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+__device__ __forceinline__ uint32_t all_but_lowest(uint32_t mask) { return mask & (mask - 1); }
+
+// The reference's scan.  cent(c, d) returns the NEGATED component, so x - c is x + (-c): the same IEEE result.
+template <int V, typename F>
+__device__ __forceinline__ uint32_t exact_scan(const float (&x)[V], uint32_t CT, F cent) {
+    float mn = 0.f;
+    uint32_t best = 0;
+#pragma unroll 1
+    for (uint32_t c = 0; c < CT; ++c) {
+        float acc = 0.f;
+#pragma unroll
+        for (int d = 0; d < V; ++d) {
+            const float e = __fadd_rn(x[d], cent(c, d));
+            acc = __fadd_rn(acc, __fmul_rn(e, e));
+        }
+        const bool take = c == 0 || __fsub_rn(mn, acc) > kEps;  // false for NaN: keeps the earlier index
+        mn = take ? acc : mn;
+        best = take ? c : best;
+    }
+    return best;
 }
 
 __device__ __forceinline__ size_t tiled_index_offset(uint32_t m, uint32_t cb, uint32_t CB, uint32_t n_stile,
@@ -56,63 +163,60 @@ __device__ __forceinline__ size_t tiled_index_offset(uint32_t m, uint32_t cb, ui
     return (size_t)n_tile * n_stile * CB + (size_t)cb_tile * n_stile * cb_mtile + (size_t)n_in * cb_mtile + cb_in;
 }
 
-// ------------------------------------------------------------------ reg path
+// Programmatic dependent launch, both kernels: launch_dependents at entry lets the LUT kernel queued behind
+// start its prologue while the search runs (it waits for this grid before it reads the indices).  The kernel
+// is itself a programmatic dependent of whatever precedes it: it stages its centroids - weights, which no
+// preceding kernel writes - before griddepcontrol.wait, and touches activations and the index buffer, which
+// the previous LUT kernel may still be reading, only after it.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// ------------------------------------------------------------------ thread <-> codebook
 constexpr int kRegThreads = 128;
 
-// kTok tokens are in flight per thread, which gives the scheduler kTok independent dependency
-// chains per warp.
-
-// Whether an instance keeps its (negated) centroids in shared memory rather than in registers: see the kernel.
-__host__ __device__ constexpr bool cent_in_smem(int V, int CT) { return (V % 2 == 0) && (CT * V >= 64 || (V >= 4 && CT * V >= 32)); }
-
-// TOKW: the CTA takes 32 codebooks and its four warps take different tokens, so that the four share one copy of the
-// centroids in shared memory (8.7 KB per CTA instead of 34.8 KB: shared memory no longer limits how many CTAs an SM
-// holds, and the staging reads a quarter of the bytes).  Otherwise the CTA takes 128 codebooks, one per thread.
-// Measured with the centroids in shared memory: up to 8192 tokens TOKW is 3-22 % faster (BERT-large linears 29.0 ->
-// 27.0 us, 78.2 -> 76.2 us; 1024 tokens 13.7 -> 10.7 us), at 65536 tokens 3-5 % slower; the launcher chooses by
-// token count.
-template <int V, int CT, bool TILED, int kTok, bool TOKW = false>
-__global__ void __launch_bounds__(kRegThreads)
+// SHORT: a thread takes one batch of kTok tokens and no more.  The CTA takes 32 codebooks, its four warps take
+// different tokens and share one staged copy of the centroids (a quarter of the bytes), the activations load
+// straight into registers, and the scan runs as it is: a batch small enough for this is bound by a chain of
+// latencies, which the filter would lengthen (0.3 us of a 15 us call).  Otherwise the CTA takes 128 codebooks, one
+// per thread, and every thread a run of tokens.
+template <int V, int CT, bool TILED, int kTok, bool SHORT>
+__global__ void __launch_bounds__(kRegThreads, SHORT ? (CT * V >= 64 ? 6 : 8) : CT * V >= 32 ? 5 : 7)
 ccs_reg_kernel(const float* __restrict__ x, const float* __restrict__ cent, void* __restrict__ out, uint32_t M,
                uint32_t K, uint32_t CB, uint32_t tokens_per_cta, uint32_t n_stile, uint32_t cb_mtile) {
-    // Let the kernel queued behind this one (the LUT kernel) start its prologue - barrier
-    // set-up, tensor-memory allocation, the first LUT tiles - while the search runs; it
-    // waits for this grid to finish before it touches the indices.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // This kernel is itself launched as a programmatic dependent of whatever precedes it in the stream, so
-    // that its launch latency and the staging of its centroids - weights, which no preceding kernel writes -
-    // overlap that kernel's tail.  Everything else it reads or overwrites - the activations, the index buffer
-    // the previous LUT kernel may still be reading - comes after griddepcontrol.wait below, which returns
-    // once the preceding grid has completed and its writes are visible.
+    pdl_launch();
     // tokens_per_cta is the run of ONE thread: the CTA's run, or each warp's where the warps take different tokens
-    constexpr uint32_t kCbCta = TOKW ? 32u : (uint32_t)kRegThreads, kTokWarps = TOKW ? (uint32_t)kRegThreads / 32u : 1u;
+    constexpr uint32_t kCbCta = SHORT ? 32u : (uint32_t)kRegThreads, kTokWarps = SHORT ? (uint32_t)kRegThreads / 32u : 1u;
     const uint32_t col = kTokWarps > 1 ? (threadIdx.x & 31u) : threadIdx.x;   // codebook of the CTA this thread works on
     const uint32_t cb = blockIdx.x * kCbCta + col;
     const uint32_t m0 = (blockIdx.y * kTokWarps + (kTokWarps > 1 ? threadIdx.x >> 5 : 0u)) * tokens_per_cta;
     const uint32_t m1 = min(M, m0 + tokens_per_cta);
     const bool active = cb < CB && m0 < M;
 
-    float xs[kTok][V];
     const float* xp = x + (size_t)(active ? cb : 0) * V;
+    // Activations arrive through a ring of kRing batches of kTok tokens in shared memory, every thread copying and
+    // reading its own bytes only (no barrier): 12 rows ahead instead of the 4 that registers have room for.  With
+    // 4, the copies in flight (17 KB per SM) held a 12608 x 3072 search to 1.9 TB/s, its first stall reason.
+    constexpr int kRing = SHORT ? 1 : V == 2 ? 4 : 3;
+    __shared__ __align__(16) float s_ring[kRing][kTok][kRegThreads][V];
+    const uint32_t ring0 = static_cast<uint32_t>(__cvta_generic_to_shared(&s_ring[0][0][threadIdx.x][0]));
+    auto fetch = [&](uint32_t m, uint32_t slot) {   // rows past the end repeat the last one (their results are not stored)
+        const uint32_t dst = ring0 + slot * (uint32_t)sizeof(s_ring[0]);
+        if (m + kTok <= m1) {
+            const float* p = xp + (size_t)m * K;
+#pragma unroll
+            for (int t = 0; t < kTok; ++t, p += K) copy_async<V * 4>(dst + t * (uint32_t)sizeof(s_ring[0][0]), p);
+        } else if (m < m1) {
+#pragma unroll
+            for (int t = 0; t < kTok; ++t)
+                copy_async<V * 4>(dst + t * (uint32_t)sizeof(s_ring[0][0]), xp + (size_t)min(m + t, M - 1) * K);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 
-    // Centroids are kept negated (the sign is flipped while they are staged) so that x - c becomes x + (-c): the same IEEE result, and
-    // for even V two dimensions go through one packed add.rn.f32x2 / mul.rn.f32x2 (each lane
-    // of a packed operation rounds on its own, and add and mul stay separate instructions,
-    // so this is still the reference's unfused arithmetic).
-    // The CTA's 128 codebooks x CT x V centroid floats are contiguous in memory: fetch them
-    // coalesced into shared memory (row pitch CT*V + 1 floats, so both the staging stores and the
-    // per-thread reads below are bank-conflict free), instead of every lane walking its own
-    // 128-byte stretch of global memory.
-    constexpr int kRow = CT * V;
-    // With more than 32 centroid floats per codebook the negated centroids stay in shared memory and
-    // are read per centroid as 16-byte (V % 4 == 0) or 8-byte loads shared by the kTok tokens in flight:
-    // held in registers they cost CT*V registers per thread (126 in all at V = 4, CT = 16: four CTAs per
-    // SM, a fifth of the warps the SM can hold).  The row pitch keeps the loads aligned and conflict free
-    // (kRow + 4 words for 16-byte loads: the eight threads of a quarter warp land in eight different
-    // four-bank groups; kRow + 2 for 8-byte loads: the sixteen threads of a half warp in sixteen pairs).
-    constexpr int kVec = (V % 4 == 0) ? 4 : 2;   // floats per shared-memory load of a centroid
-    constexpr bool kCentInSmem = cent_in_smem(V, CT);
-    constexpr int kPitch = kCentInSmem ? kRow + kVec : kRow + 1;
+    // The CTA's codebooks are contiguous in memory: fetch them coalesced into shared memory, negated.  The row pitch
+    // keeps the per-thread reads - a word at a time, or a vector in the SHORT form - free of bank conflicts.
+    constexpr int kVec = SHORT ? (V == 2 ? 2 : 4) : 1;
+    constexpr int kRow = CT * V, kPitch = kRow + kVec;
     __shared__ __align__(16) float s_cent[kCbCta * kPitch];
     {
         const uint32_t cb0 = blockIdx.x * kCbCta;
@@ -123,110 +227,344 @@ ccs_reg_kernel(const float* __restrict__ x, const float* __restrict__ cent, void
             s_cent[r * kPitch + i] = -__ldg(gp + e);
         }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    // first batch of activations: in flight while the CTA waits at the barrier for the centroids
+    pdl_wait();
+    float cur[kTok][V];
+    if constexpr (SHORT) {
 #pragma unroll
-    for (int t = 0; t < kTok; ++t) load_x<V>(xp + (size_t)min(m0 + t, M - 1) * K, xs[t]);
+        for (int t = 0; t < kTok; ++t) load_global<V>(xp + (size_t)min(m0 + t, M - 1) * K, cur[t]);
+    } else {
+#pragma unroll
+        for (uint32_t r = 0; r + 1 < kRing; ++r) fetch(active ? m0 + r * kTok : m1, r);
+    }
     __syncthreads();
     if (!active) return;
-    float nc[kCentInSmem ? 1 : CT][V];
-    const float* my_cent = s_cent + col * kPitch;
-    if constexpr (!kCentInSmem) {
-#pragma unroll
-        for (int ct = 0; ct < CT; ++ct)
-#pragma unroll
-            for (int d = 0; d < V; ++d) nc[ct][d] = my_cent[ct * V + d];
-    }
 
-    for (uint32_t m = m0; m < m1; m += kTok) {
-        float cur[kTok][V];
+    const float* my_cent = s_cent + col * kPitch;
+    auto store = [&](uint32_t m, const uint32_t (&best)[kTok]) {
+        if constexpr (TILED) {
 #pragma unroll
-        for (int t = 0; t < kTok; ++t)
+            for (int t = 0; t < kTok; ++t)
+                if (m + t < m1) reinterpret_cast<uint16_t*>(out)[tiled_index_offset(m + t, cb, CB, n_stile, cb_mtile)] = (uint16_t)best[t];
+        } else {
+            uint8_t* o = reinterpret_cast<uint8_t*>(out) + (size_t)m * CB + cb;
+            if (m + kTok <= m1) {
 #pragma unroll
-            for (int d = 0; d < V; ++d) cur[t][d] = xs[t][d];
-        if (m + kTok < m1) {  // next batch while this one is scanned
+                for (int t = 0; t < kTok; ++t, o += CB) *o = (uint8_t)best[t];
+            } else {
 #pragma unroll
-            for (int t = 0; t < kTok; ++t) load_x<V>(xp + (size_t)min(m + kTok + t, M - 1) * K, xs[t]);
+                for (int t = 0; t < kTok; ++t, o += CB)
+                    if (m + t < m1) *o = (uint8_t)best[t];
+            }
         }
+    };
+    if constexpr (SHORT) {
         float mn[kTok];
         uint32_t best[kTok];
 #pragma unroll
-        for (int ct = 0; ct < CT; ++ct) {
-            float ncv[V];   // this centroid, negated
-            if constexpr (kCentInSmem) {
-                if constexpr (kVec == 4) {
+        for (int c = 0; c < CT; ++c) {
+            float nc[V];
+            load_x<V>(my_cent + c * V, nc);
 #pragma unroll
-                    for (int q = 0; q < V / 4; ++q) {
-                        const float4 c4 = *reinterpret_cast<const float4*>(my_cent + ct * V + 4 * q);
-                        ncv[4 * q + 0] = c4.x; ncv[4 * q + 1] = c4.y; ncv[4 * q + 2] = c4.z; ncv[4 * q + 3] = c4.w;
+            for (int t = 0; t < kTok; ++t) {
+                // two components per packed instruction; each lane of it rounds on its own, and the addition and
+                // the multiplication stay separate instructions
+                float acc = 0.f;
+#pragma unroll
+                for (int d = 0; d < V; d += 2) {
+                    const float2 e = __fadd2_rn(make_float2(cur[t][d], cur[t][d + 1]), make_float2(nc[d], nc[d + 1]));
+                    const float2 sq = __fmul2_rn(e, e);
+                    acc = d == 0 ? sq.x : __fadd_rn(acc, sq.x);  // 0 + sq.x is exact
+                    acc = __fadd_rn(acc, sq.y);
+                }
+                const bool take = c == 0 || __fsub_rn(mn[t], acc) > kEps;  // false for NaN: keeps the earlier index
+                mn[t] = take ? acc : mn[t];
+                best[t] = take ? (uint32_t)c : best[t];
+            }
+        }
+        store(m0, best);
+        return;
+    } else {
+        float2 nc[CT / 2][V], h[CT / 2];   // two centroids per pair: one packed instruction works on both
+        float t_cb = kMarginBase;
+        {
+            float top = 0.f;
+            bool fine = true;
+#pragma unroll
+            for (int j = 0; j < CT / 2; ++j) {
+                float2 cc = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int d = 0; d < V; ++d) {
+                    nc[j][d] = make_float2(my_cent[2 * j * V + d], my_cent[(2 * j + 1) * V + d]);
+                    cc = __ffma2_rn(nc[j][d], nc[j][d], cc);
+                }
+                h[j] = make_float2(0.5f * cc.x, 0.5f * cc.y);
+                fine = fine && cc.x < kHuge && cc.y < kHuge;
+                top = fmaxf(top, fmaxf(cc.x, cc.y));
+            }
+            t_cb = fine ? fmaf(margin_factor(V), top, kMarginBase) : __int_as_float(0x7f800000);
+        }
+
+        auto search = [&](uint32_t m) {
+            // one margin for the kTok tokens: that of the sum of their norms
+            float2 xx = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int t = 0; t < kTok; ++t)
+#pragma unroll
+                for (int d = 0; d < V; d += 2) {
+                    const float2 q = make_float2(cur[t][d], cur[t][d + 1]);
+                    xx = __ffma2_rn(q, q, xx);
+                }
+            const float T = fmaf(margin_factor(V), xx.x + xx.y, t_cb);
+            uint32_t mask[kTok], best[kTok], several = 0;
+#pragma unroll
+            for (int t = 0; t < kTok; ++t) {
+                float k[CT];
+#pragma unroll
+                for (int j = 0; j < CT / 2; ++j) {
+                    float2 s = h[j];
+#pragma unroll
+                    for (int d = 0; d < V; ++d) s = __ffma2_rn(make_float2(cur[t][d], cur[t][d]), nc[j][d], s);
+                    k[2 * j] = s.x;
+                    k[2 * j + 1] = s.y;
+                }
+                mask[t] = below<CT>(k, min_of(k) + T);
+                best[t] = high_bit(mask[t]);
+                several |= all_but_lowest(mask[t]);
+            }
+            if (several != 0 || !(T < kHuge)) {
+#pragma unroll
+                for (int t = 0; t < kTok; ++t)
+                    if (!(T < kHuge) || all_but_lowest(mask[t]) != 0)
+                        best[t] = exact_scan<V>(cur[t], CT, [&](uint32_t c, int d) { return my_cent[c * V + d]; });
+            }
+            store(m, best);
+        };
+        uint32_t slot = 0, ahead = kRing - 1;
+        for (uint32_t m = m0; m < m1; m += kTok) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(SHORT ? 0 : kRing - 2) : "memory");
+#pragma unroll
+            for (int t = 0; t < kTok; ++t) load_x<V>(&s_ring[slot][t][threadIdx.x][0], cur[t]);
+            fetch(m + (kRing - 1) * kTok, ahead);
+            if (++slot == kRing) slot = 0;
+            if (++ahead == kRing) ahead = 0;
+            search(m);
+        }
+    }
+}
+
+// ------------------------------------------------------------------ thread <-> token
+constexpr int kTileThreads = 128;
+
+// codebooks of one CTA: about 128 to 192 bytes of a token's row
+__host__ __device__ constexpr int tile_codebooks(int v) {
+    return v == 1 ? 16 : v == 2 ? 8 : v <= 12 ? 4 : v <= 24 ? 2 : 1;
+}
+// Row pitch of the staged activations, in floats: 4 mod 8 keeps 16-byte copies aligned and 16-byte reads of 32 rows
+// free of bank conflicts; odd lengths are read word by word, which an odd pitch serves.
+__host__ __device__ constexpr int tile_pitch(int v) {
+    const int w = tile_codebooks(v) * v;
+    return v % 2 ? (w | 1) : (w + 3) / 8 * 8 + 4;
+}
+// From 12 components on, packed instructions take two components of one centroid (one horizontal addition per
+// key); below, two centroids (the activations are duplicated into register pairs, which long vectors cannot afford).
+__host__ __device__ constexpr bool tile_pairs_components(int v) { return v >= 12 && v % 4 == 0; }
+
+// Where component d of centroid c of a codebook lies in its staged block: quads of centroids, V + 1 groups of four
+// floats each.  Pairs of centroids: group d holds component d of the four, group V their |c|^2 / 2.  Pairs of
+// components: the four centroids one after the other, then their |c|^2 / 2.
+template <int V>
+__device__ __forceinline__ uint32_t cent_at(uint32_t c, uint32_t d) {
+    const uint32_t quad = (c >> 2) * (4 * (V + 1)), in = c & 3u;
+    if constexpr (tile_pairs_components(V)) return quad + in * V + d;
+    else return quad + d * 4 + in;
+}
+
+// G: centroids whose keys are held at once.  ONE: num_centroid <= G, so there is a single group.
+template <int V, int G, bool ONE, int kTok, bool TILED>
+__global__ void __launch_bounds__(kTileThreads, V <= 5 ? 6 : 4)
+ccs_tile_kernel(const float* __restrict__ x, const float* __restrict__ cent, void* __restrict__ out, uint32_t M,
+                uint32_t K, uint32_t CB, uint32_t CT, uint32_t copy16, uint32_t words, uint32_t n_stile, uint32_t cb_mtile) {
+    constexpr int kCbs = tile_codebooks(V), kPitch = tile_pitch(V), kTokens = kTileThreads * kTok;
+    constexpr bool kPairD = tile_pairs_components(V);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_launch();
+    float* s_x = reinterpret_cast<float*>(smem_raw);                    // [kTokens][kPitch]
+    constexpr int kXFloats = (kTokens * kPitch + 3) / 4 * 4;
+    float* s_c = s_x + kXFloats;                                        // [kCbs][groups][G/4][V+1][4]
+    __shared__ uint32_t s_top[kCbs];                                    // max |c|^2 as bits (NaN and infinity sort last)
+    const uint32_t groups = ONE ? 1u : (CT + G - 1) / G, ct_pad = groups * G;
+    const uint32_t c_block = ct_pad * (V + 1);
+    const uint32_t cb0 = blockIdx.x * kCbs, cbs = min((uint32_t)kCbs, CB - cb0);
+    const uint32_t m_base = blockIdx.y * kTokens;
+
+    if (threadIdx.x < kCbs) s_top[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < cbs * ct_pad; e += kTileThreads) {
+        const uint32_t b = e / ct_pad, c = e % ct_pad;
+        float v[V], cc = 0.f;
+        if (c < CT) {
+            const float* g = cent + ((size_t)(cb0 + b) * CT + c) * V;
+#pragma unroll
+            for (int d = 0; d < V; ++d) v[d] = -__ldg(g + d);
+        } else {
+#pragma unroll
+            for (int d = 0; d < V; ++d) v[d] = 0.f;
+        }
+#pragma unroll
+        for (int d = 0; d < V; ++d) cc = fmaf(v[d], v[d], cc);
+        float* blk = s_c + b * c_block;
+#pragma unroll
+        for (int d = 0; d < V; ++d) blk[cent_at<V>(c, d)] = v[d];
+        blk[(c >> 2) * (4 * (V + 1)) + 4 * V + (c & 3u)] = c < CT ? 0.5f * cc : __int_as_float(0x7f800000);
+        atomicMax(&s_top[b], __float_as_uint(cc));
+    }
+    pdl_wait();
+    {
+        const float* xg = x + (size_t)cb0 * V;
+        const uint32_t rows = min((uint32_t)kTokens, M - m_base);
+        const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(s_x));
+        constexpr uint32_t kW = kCbs * V;
+        const uint32_t w = cbs * V;
+        if (V % 2 == 0 && kW % 4 == 0 && copy16) {
+            for (uint32_t i = threadIdx.x; i < rows * (kW / 4); i += kTileThreads) {
+                const uint32_t r = i / (kW / 4), q = i % (kW / 4);
+                if (4 * q < w) copy_async<16>(dst + (r * kPitch + 4 * q) * 4, xg + (size_t)(m_base + r) * K + 4 * q);
+            }
+        } else {
+            for (uint32_t i = threadIdx.x; i < rows * kW; i += kTileThreads) {
+                const uint32_t r = i / kW, q = i % kW;
+                if (q < w) copy_async<4>(dst + (r * kPitch + q) * 4, xg + (size_t)(m_base + r) * K + q);
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    __syncthreads();
+
+    uint32_t word[kTok] = {};
+#pragma unroll 1
+    for (uint32_t b = 0; b < cbs; ++b) {
+        const float* blk = s_c + b * c_block;
+        float xv[kTok][V], T[kTok], m1[kTok];
+        uint32_t cand[kTok], base[kTok];
+        {
+            const float top = __uint_as_float(s_top[b]);
+            const float t_cb = top < kHuge ? fmaf(margin_factor(V), top, kMarginBase) : __int_as_float(0x7f800000);
+#pragma unroll
+            for (int t = 0; t < kTok; ++t) {
+                const float* row = s_x + (threadIdx.x + t * kTileThreads) * kPitch + b * V;
+                float xx = 0.f;
+                load_x<V>(row, xv[t]);
+#pragma unroll
+                for (int d = 0; d < V; ++d) xx = fmaf(xv[t][d], xv[t][d], xx);
+                T[t] = fmaf(margin_factor(V), xx, t_cb);
+                m1[t] = __int_as_float(0x7f800000);
+                cand[t] = 0;
+                base[t] = 0;
+            }
+        }
+#pragma unroll 1
+        for (uint32_t g = 0; g < groups; ++g) {
+            float k[kTok][G];
+            const float* gp = blk + g * (G * (V + 1));
+#pragma unroll
+            for (int q = 0; q < G / 4; ++q) {
+                const float* qp = gp + q * (4 * (V + 1));
+                const float4 h = *reinterpret_cast<const float4*>(qp + 4 * V);
+                if constexpr (kPairD) {
+                    const float hs[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        float2 s[kTok];
+#pragma unroll
+                        for (int t = 0; t < kTok; ++t) s[t] = make_float2(hs[c], 0.f);
+#pragma unroll
+                        for (int d = 0; d < V; d += 4) {
+                            const float4 cv = *reinterpret_cast<const float4*>(qp + c * V + d);
+#pragma unroll
+                            for (int t = 0; t < kTok; ++t) {
+                                s[t] = __ffma2_rn(make_float2(xv[t][d], xv[t][d + 1]), make_float2(cv.x, cv.y), s[t]);
+                                s[t] = __ffma2_rn(make_float2(xv[t][d + 2], xv[t][d + 3]), make_float2(cv.z, cv.w), s[t]);
+                            }
+                        }
+#pragma unroll
+                        for (int t = 0; t < kTok; ++t) k[t][4 * q + c] = s[t].x + s[t].y;
                     }
                 } else {
+                    float2 lo[kTok], hi[kTok];
 #pragma unroll
-                    for (int q = 0; q < V / 2; ++q) {
-                        const float2 c2 = *reinterpret_cast<const float2*>(my_cent + ct * V + 2 * q);
-                        ncv[2 * q + 0] = c2.x; ncv[2 * q + 1] = c2.y;
+                    for (int t = 0; t < kTok; ++t) { lo[t] = make_float2(h.x, h.y); hi[t] = make_float2(h.z, h.w); }
+#pragma unroll
+                    for (int d = 0; d < V; ++d) {
+                        const float4 cv = *reinterpret_cast<const float4*>(qp + 4 * d);
+#pragma unroll
+                        for (int t = 0; t < kTok; ++t) {
+                            const float2 xd = make_float2(xv[t][d], xv[t][d]);
+                            lo[t] = __ffma2_rn(xd, make_float2(cv.x, cv.y), lo[t]);
+                            hi[t] = __ffma2_rn(xd, make_float2(cv.z, cv.w), hi[t]);
+                        }
+                    }
+#pragma unroll
+                    for (int t = 0; t < kTok; ++t) {
+                        k[t][4 * q] = lo[t].x; k[t][4 * q + 1] = lo[t].y; k[t][4 * q + 2] = hi[t].x; k[t][4 * q + 3] = hi[t].y;
                     }
                 }
-            } else {
-#pragma unroll
-                for (int d = 0; d < V; ++d) ncv[d] = nc[ct][d];
             }
 #pragma unroll
             for (int t = 0; t < kTok; ++t) {
-                float acc = 0.f;
-                if constexpr (V % 2 == 0) {
-#pragma unroll
-                    for (int d = 0; d < V; d += 2) {
-                        const float2 e = __fadd2_rn(make_float2(cur[t][d], cur[t][d + 1]), make_float2(ncv[d], ncv[d + 1]));
-                        const float2 sq = __fmul2_rn(e, e);
-                        acc = (d == 0) ? sq.x : __fadd_rn(acc, sq.x);  // 0 + sq.x is exact
-                        acc = __fadd_rn(acc, sq.y);
-                    }
+                const float gm = min_of(k[t]);
+                if constexpr (ONE) {
+                    cand[t] = below<G>(k[t], gm + T[t]);
                 } else {
-#pragma unroll
-                    for (int d = 0; d < V; ++d) {
-                        const float e = __fadd_rn(cur[t][d], ncv[d]);
-                        acc = __fadd_rn(acc, __fmul_rn(e, e));
+                    // Candidates so far survive if the smallest of them is still within the margin; together with
+                    // new ones they are more than one.
+                    const float now = fminf(m1[t], gm), thr = now + T[t];
+                    const uint32_t mask = below<G>(k[t], thr);
+                    const bool keep = m1[t] < thr;
+                    if (mask) {
+                        cand[t] = keep ? 0xFFFFFFFFu : mask;
+                        base[t] = g * G;
                     }
-                }
-                if (ct == 0) {
-                    mn[t] = acc;
-                    best[t] = 0;
-                } else {
-                    bool take = __fsub_rn(mn[t], acc) > kEps;  // false for NaN: keeps the earlier index
-                    mn[t] = take ? acc : mn[t];
-                    best[t] = take ? (uint32_t)ct : best[t];
+                    m1[t] = now;
                 }
             }
         }
 #pragma unroll
         for (int t = 0; t < kTok; ++t) {
-            const uint32_t mm = m + t;
-            if (mm < m1) {
-                if constexpr (TILED) {
-                    reinterpret_cast<uint16_t*>(out)[tiled_index_offset(mm, cb, CB, n_stile, cb_mtile)] = (uint16_t)best[t];
-                } else {
-                    reinterpret_cast<uint8_t*>(out)[(size_t)mm * CB + cb] = (uint8_t)best[t];
+            uint32_t best = base[t] + high_bit(cand[t]);
+            const uint32_t m = m_base + threadIdx.x + t * kTileThreads;
+            if (m < M && (!(T[t] < kHuge) || all_but_lowest(cand[t]) != 0))
+                best = exact_scan<V>(xv[t], CT, [&](uint32_t c, int d) { return blk[cent_at<V>(c, d)]; });
+            if constexpr (TILED) {
+                if (m < M) reinterpret_cast<uint16_t*>(out)[tiled_index_offset(m, cb0 + b, CB, n_stile, cb_mtile)] = (uint16_t)best;
+            } else {
+                uint8_t* o = reinterpret_cast<uint8_t*>(out) + (size_t)m * CB + cb0;
+                if (kCbs % 4 == 0 && words) {   // four codebooks per store
+                    word[t] |= best << (8 * (b & 3u));
+                    if ((b & 3u) == 3u) {
+                        if (m < M) *reinterpret_cast<uint32_t*>(o + (b & ~3u)) = word[t];
+                        word[t] = 0;
+                    }
+                } else if (m < M) {
+                    o[b] = (uint8_t)best;
                 }
             }
         }
     }
 }
 
-// ------------------------------------------------------------------ smem path
-constexpr int kSmemThreads = 128;  // tokens per CTA
+// ------------------------------------------------------------------ any sub-vector length
+constexpr int kAnyThreads = 128;  // tokens per CTA
 
-// V > 0: compile-time sub-vector length, the token's slice sits in registers.
-// V == 0: run-time length, the slice is re-read (L1 resident) per centroid.
-template <int V, bool TILED>
-__global__ void __launch_bounds__(kSmemThreads)
-ccs_smem_kernel(const float* __restrict__ x, const float* __restrict__ cent, void* __restrict__ out, uint32_t M,
-                uint32_t K, uint32_t v_rt, uint32_t CB, uint32_t CT, uint32_t cb_per_cta, uint32_t n_stile,
-                uint32_t cb_mtile) {
+// Run-time length: thread <-> token, centroids of a block of codebooks in shared memory, the token's slice is
+// re-read (L1 resident) per centroid; exact_scan's arithmetic without the filter.
+template <bool TILED>
+__global__ void __launch_bounds__(kAnyThreads)
+ccs_any_kernel(const float* __restrict__ x, const float* __restrict__ cent, void* __restrict__ out, uint32_t M,
+               uint32_t K, uint32_t v, uint32_t CB, uint32_t CT, uint32_t cb_per_cta, uint32_t n_stile,
+               uint32_t cb_mtile) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // see ccs_reg_kernel
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const uint32_t v = V > 0 ? (uint32_t)V : v_rt;
+    pdl_launch();
+    pdl_wait();
     float* s_cent = reinterpret_cast<float*>(smem_raw);                   // [cbs][CT][v]
     const uint32_t cb0 = blockIdx.x * cb_per_cta;
     const uint32_t cbs = min(cb_per_cta, CB - cb0);
@@ -234,10 +572,10 @@ ccs_smem_kernel(const float* __restrict__ x, const float* __restrict__ cent, voi
 
     const uint32_t n_c = cbs * CT * v;
     const float* gc = cent + (size_t)cb0 * CT * v;
-    for (uint32_t i = threadIdx.x; i < n_c; i += kSmemThreads) s_cent[i] = __ldg(gc + i);
+    for (uint32_t i = threadIdx.x; i < n_c; i += kAnyThreads) s_cent[i] = __ldg(gc + i);
     __syncthreads();
 
-    const uint32_t m_base = blockIdx.y * kSmemThreads;
+    const uint32_t m_base = blockIdx.y * kAnyThreads;
     const uint32_t m = m_base + threadIdx.x;
     if (m < M) {
         const float* xp = x + (size_t)m * K + (size_t)cb0 * v;
@@ -245,41 +583,24 @@ ccs_smem_kernel(const float* __restrict__ x, const float* __restrict__ cent, voi
             const float* cp = s_cent + (size_t)cl * CT * v;
             float mn = 0.f;
             uint32_t best = 0;
-            if constexpr (V > 0) {
-                float xs[V > 0 ? V : 1];
-                load_x<(V > 0 ? V : 1)>(xp, xs);
-                for (uint32_t ct = 0; ct < CT; ++ct) {
-                    float t = 0.f;
-#pragma unroll
-                    for (int d = 0; d < V; ++d) {
-                        float e = __fsub_rn(xs[d], cp[ct * V + d]);
-                        t = __fadd_rn(t, __fmul_rn(e, e));
-                    }
-                    bool take = (ct > 0) && (__fsub_rn(mn, t) > kEps);
-                    if (ct == 0) mn = t;
-                    mn = take ? t : mn;
-                    best = take ? ct : best;
+            for (uint32_t ct = 0; ct < CT; ++ct) {
+                float t = 0.f;
+                for (uint32_t d = 0; d < v; ++d) {
+                    float e = __fsub_rn(__ldg(xp + d), cp[ct * v + d]);
+                    t = __fadd_rn(t, __fmul_rn(e, e));
                 }
-            } else {
-                for (uint32_t ct = 0; ct < CT; ++ct) {
-                    float t = 0.f;
-                    for (uint32_t d = 0; d < v; ++d) {
-                        float e = __fsub_rn(__ldg(xp + d), cp[ct * v + d]);
-                        t = __fadd_rn(t, __fmul_rn(e, e));
-                    }
-                    bool take = (ct > 0) && (__fsub_rn(mn, t) > kEps);
-                    if (ct == 0) mn = t;
-                    mn = take ? t : mn;
-                    best = take ? ct : best;
-                }
+                bool take = (ct > 0) && (__fsub_rn(mn, t) > kEps);
+                if (ct == 0) mn = t;
+                mn = take ? t : mn;
+                best = take ? ct : best;
             }
             s_idx[threadIdx.x * cb_per_cta + cl] = (uint8_t)best;
         }
     }
     __syncthreads();
     // write-out: consecutive threads -> consecutive codebooks of one token
-    const uint32_t rows = min((uint32_t)kSmemThreads, M > m_base ? M - m_base : 0u);
-    for (uint32_t i = threadIdx.x; i < rows * cbs; i += kSmemThreads) {
+    const uint32_t rows = min((uint32_t)kAnyThreads, M > m_base ? M - m_base : 0u);
+    for (uint32_t i = threadIdx.x; i < rows * cbs; i += kAnyThreads) {
         uint32_t r = i / cbs, cl = i % cbs;
         uint8_t b = s_idx[r * cb_per_cta + cl];
         if constexpr (TILED) {
@@ -290,9 +611,7 @@ ccs_smem_kernel(const float* __restrict__ x, const float* __restrict__ cent, voi
     }
 }
 
-// Launch with programmatic stream serialisation allowed: the grid may be scheduled while the preceding
-// kernel of the stream is still running; the kernels above wait for it (griddepcontrol.wait) before they
-// touch memory, so the ordering is that of a plain launch and only the launch latency overlaps.
+// Launch with programmatic stream serialisation allowed: see pdl_wait.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dependent(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
@@ -308,78 +627,100 @@ cudaError_t launch_dependent(void (*k)(KArgs...), dim3 grid, dim3 block, size_t 
     return cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
 }
 
-template <int V, int CT, int kTok, bool TOKW>
-cudaError_t run_reg_tok(const CcsArgs& a, cudaStream_t s) {
-    constexpr uint32_t kCbCta = TOKW ? 32u : (uint32_t)kRegThreads, kTokWarps = TOKW ? (uint32_t)kRegThreads / 32u : 1u;
-    // Run length per thread.  The grid is sized in whole waves of what the GPU holds at once - SMs x CTAs
-    // resident per SM for this instance (registers and shared memory decide: 6 to 8) - because a last wave
-    // that is a third full costs as much as a full one: a small batch is spread over as many CTAs as it has
-    // 4-token runs (one partial wave), a large one gets runs of up to 128 tokens, which also amortise the
-    // centroid staging, in an integral number of nearly full waves.
-    uint32_t tpt = a.tokens_per_thread;
-    if (!tpt) {
-        static int resident = 0, sms = 0;   // per instance; the same for every device of one kind
-        if (!resident) {
-            int dev = 0, r = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, ccs_reg_kernel<V, CT, false, kTok, TOKW>, kRegThreads, 0) != cudaSuccess || r < 1) r = 4;
-            if (sms < 1) sms = 148;
-            resident = r;
-        }
-        const uint64_t cb_blocks = (a.CB + kCbCta - 1) / kCbCta;
-        const uint64_t wave = (uint64_t)sms * resident;
-        constexpr uint64_t kCap = 128;   // longest run of one thread
-        const uint64_t ctas_at_cap = cb_blocks * ((a.M + kCap * kTokWarps - 1) / (kCap * kTokWarps));
-        const uint64_t waves = ctas_at_cap <= wave ? 1 : (ctas_at_cap + wave - 1) / wave;
-        tpt = (uint32_t)(((uint64_t)a.M * cb_blocks + waves * wave * kTokWarps - 1) / (waves * wave * kTokWarps));
-        if (tpt < (uint32_t)kTok) tpt = kTok;
-        if (tpt > kCap) tpt = kCap;
-    }
-    tpt = (tpt + kTok - 1) / kTok * kTok;
-    dim3 grid((a.CB + kCbCta - 1) / kCbCta, (a.M + tpt * kTokWarps - 1) / (tpt * kTokWarps));
-    if (a.format == LUTAMM_INDEX_U16_TILED)
-        return launch_dependent(ccs_reg_kernel<V, CT, true, kTok, TOKW>, grid, dim3(kRegThreads), 0, s, a.x, a.centroid, a.idx_out,
-                                a.M, a.K, a.CB, tpt, a.n_stile, a.cb_mtile);
-    return launch_dependent(ccs_reg_kernel<V, CT, false, kTok, TOKW>, grid, dim3(kRegThreads), 0, s, a.x, a.centroid, a.idx_out,
-                            a.M, a.K, a.CB, tpt, a.n_stile, a.cb_mtile);
+// Number of SMs of the current device (the same for every device of one kind)
+uint32_t sm_count() {
+    static const uint32_t n = [] {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        return cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? (uint32_t)v : 148u;
+    }();
+    return n;
+}
+
+template <int V, int CT, int kTok, bool SHORT>
+uint32_t resident_ctas() {
+    static const uint32_t n = [] {
+        int r = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, ccs_reg_kernel<V, CT, false, kTok, SHORT>, kRegThreads, 0) == cudaSuccess && r > 0 ? (uint32_t)r : 4u;
+    }();
+    return n * sm_count();
+}
+
+template <int V, int CT, int kTok, bool SHORT>
+cudaError_t run_reg_grid(const CcsArgs& a, dim3 grid, uint32_t run, cudaStream_t s) {
+    auto k = a.format == LUTAMM_INDEX_U16_TILED ? ccs_reg_kernel<V, CT, true, kTok, SHORT> : ccs_reg_kernel<V, CT, false, kTok, SHORT>;
+    return launch_dependent(k, grid, dim3(kRegThreads), 0, s, a.x, a.centroid, a.idx_out, a.M, a.K, a.CB, run, a.n_stile, a.cb_mtile);
+}
+
+constexpr uint32_t kTok = 4;   // tokens whose activations a thread loads together: one round trip to memory instead of four
+
+// One batch of kTok tokens per thread, while the GPU holds all those CTAs at once.
+template <int V, int CT>
+bool short_fits(const CcsArgs& a, dim3* grid) {
+    *grid = dim3((a.CB + 31) / 32, (a.M + 4 * kTok - 1) / (4 * kTok));
+    return !a.tokens_per_thread && (uint64_t)grid->x * grid->y <= resident_ctas<V, CT, kTok, true>();
 }
 
 template <int V, int CT>
 cudaError_t run_reg(const CcsArgs& a, cudaStream_t s) {
-    // Four tokens in flight per thread: their activations are loaded together (one round trip to
-    // memory instead of four) and their scans interleave.  Two or one measured no faster.
-    // The instances with their centroids in registers gain from the shared copy only while the staging is a
-    // large part of the kernel: 512 tokens x 768 features 10.7 -> 8.6 us, 12608 tokens 33.2 -> 35.2 us.
-    if (a.M <= (cent_in_smem(V, CT) ? 16384u : 512u)) return run_reg_tok<V, CT, 4, true>(a, s);
-    return run_reg_tok<V, CT, 4, false>(a, s);
+    // One wave of equal runs of up to 2048 tokens: a last wave that is a third full costs as much as a full one,
+    // and staging the centroids costs a few microseconds per wave.
+    const uint64_t cb_blocks = (a.CB + kRegThreads - 1) / kRegThreads;
+    uint64_t run = a.tokens_per_thread;
+    if (!run) {
+        const uint64_t wave = resident_ctas<V, CT, kTok, false>();
+        constexpr uint64_t kCap = 2048;
+        const uint64_t ctas_at_cap = cb_blocks * ((a.M + kCap - 1) / kCap), waves = (ctas_at_cap + wave - 1) / wave;
+        run = ((uint64_t)a.M * cb_blocks + waves * wave - 1) / (waves * wave);
+        if (run > kCap) run = kCap;
+    }
+    const uint32_t tokens = (uint32_t)((run + kTok - 1) / kTok * kTok);
+    return run_reg_grid<V, CT, kTok, false>(a, dim3((uint32_t)cb_blocks, (a.M + tokens - 1) / tokens), tokens, s);
+}
+
+template <int V, int G, bool ONE, int kTok>
+cudaError_t run_tile_tok(const CcsArgs& a, size_t smem, cudaStream_t s) {
+    constexpr uint32_t kCbs = tile_codebooks(V);
+    const uint32_t tokens = kTileThreads * kTok;
+    const dim3 grid((a.CB + kCbs - 1) / kCbs, (a.M + tokens - 1) / tokens);
+    if (grid.y > 65535u) return cudaErrorInvalidValue;
+    const uint32_t copy16 = a.K % 4 == 0 && reinterpret_cast<uintptr_t>(a.x) % 16 == 0;
+    const uint32_t words = a.CB % 4 == 0 && reinterpret_cast<uintptr_t>(a.idx_out) % 4 == 0;
+    auto k = a.format == LUTAMM_INDEX_U16_TILED ? ccs_tile_kernel<V, G, ONE, kTok, true> : ccs_tile_kernel<V, G, ONE, kTok, false>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return launch_dependent(k, grid, dim3(kTileThreads), smem, s, a.x, a.centroid, a.idx_out, a.M, a.K, a.CB, a.CT, copy16, words,
+                            a.n_stile, a.cb_mtile);
 }
 
 template <int V>
-cudaError_t run_smem(const CcsArgs& a, cudaStream_t s) {
+cudaError_t run_tile(const CcsArgs& a, cudaStream_t s) {
+    constexpr uint32_t kCbs = tile_codebooks(V);
+    const uint32_t g = a.CT <= 8 ? 8 : 16, ct_pad = (a.CT + g - 1) / g * g;
+    auto smem = [&](uint32_t tok) { return ((size_t)(kTileThreads * tok * tile_pitch(V) + 3) / 4 * 4 + (size_t)kCbs * ct_pad * (V + 1)) * sizeof(float); };
+    // Two tokens per thread share each centroid read; one where that would leave SMs without a CTA.
+    const uint64_t ctas2 = (uint64_t)((a.CB + kCbs - 1) / kCbs) * ((a.M + 2 * kTileThreads - 1) / (2 * kTileThreads));
+    const bool two = ctas2 >= 2ull * sm_count() && smem(2) <= 112 * 1024;
+    if (g == 8) return two ? run_tile_tok<V, 8, true, 2>(a, smem(2), s) : run_tile_tok<V, 8, true, 1>(a, smem(1), s);
+    if (a.CT <= 16) return two ? run_tile_tok<V, 16, true, 2>(a, smem(2), s) : run_tile_tok<V, 16, true, 1>(a, smem(1), s);
+    return two ? run_tile_tok<V, 16, false, 2>(a, smem(2), s) : run_tile_tok<V, 16, false, 1>(a, smem(1), s);
+}
+
+cudaError_t run_any(const CcsArgs& a, cudaStream_t s) {
     // centroid tile + index tile per CTA; keep under ~96 KB so two CTAs fit an SM
-    const size_t per_cb = (size_t)a.CT * a.v * sizeof(float) + kSmemThreads;
+    const size_t per_cb = (size_t)a.CT * a.v * sizeof(float) + kAnyThreads;
     uint32_t cb_per_cta = (uint32_t)((96 * 1024) / per_cb);
     if (cb_per_cta == 0) cb_per_cta = 1;
     if (cb_per_cta > 64) cb_per_cta = 64;
     if (cb_per_cta > a.CB) cb_per_cta = a.CB;
     const size_t smem = per_cb * cb_per_cta;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    dim3 grid((a.CB + cb_per_cta - 1) / cb_per_cta, (a.M + kSmemThreads - 1) / kSmemThreads);
-    cudaError_t e;
-    if (a.format == LUTAMM_INDEX_U16_TILED) {
-        auto k = ccs_smem_kernel<V, true>;
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        return launch_dependent(k, grid, dim3(kSmemThreads), smem, s, a.x, a.centroid, a.idx_out, a.M, a.K, a.v, a.CB, a.CT,
-                                cb_per_cta, a.n_stile, a.cb_mtile);
-    } else {
-        auto k = ccs_smem_kernel<V, false>;
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        return launch_dependent(k, grid, dim3(kSmemThreads), smem, s, a.x, a.centroid, a.idx_out, a.M, a.K, a.v, a.CB, a.CT,
-                                cb_per_cta, a.n_stile, a.cb_mtile);
-    }
+    dim3 grid((a.CB + cb_per_cta - 1) / cb_per_cta, (a.M + kAnyThreads - 1) / kAnyThreads);
+    auto k = a.format == LUTAMM_INDEX_U16_TILED ? ccs_any_kernel<true> : ccs_any_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return launch_dependent(k, grid, dim3(kAnyThreads), smem, s, a.x, a.centroid, a.idx_out, a.M, a.K, a.v, a.CB, a.CT,
+                            cb_per_cta, a.n_stile, a.cb_mtile);
 }
 
 }  // namespace
@@ -392,38 +733,47 @@ cudaError_t launch_ccs(const CcsArgs& a, cudaStream_t s, const char** why) {
         return cudaErrorInvalidValue;
     }
     // vector loads need the row pitch and the base address aligned to the vector width
-    const uintptr_t xa = reinterpret_cast<uintptr_t>(a.x), ca = reinterpret_cast<uintptr_t>(a.centroid);
+    const uintptr_t xa = reinterpret_cast<uintptr_t>(a.x);
     const uint32_t vec_bytes = (a.v % 4 == 0) ? 16u : (a.v % 2 == 0) ? 8u : 4u;
-    const bool aligned = (xa % vec_bytes == 0) && (ca % vec_bytes == 0);
-    if (aligned) {
+    if (xa % vec_bytes == 0) {
+        dim3 grid;
+#define LUTAMM_CCS_SHORT(V_, CT_) \
+    if (a.v == V_ && a.CT == CT_ && short_fits<V_, CT_>(a, &grid)) return run_reg_grid<V_, CT_, kTok, true>(a, grid, kTok, s);
+        LUTAMM_CCS_SHORT(2, 8)
+        LUTAMM_CCS_SHORT(2, 16)
+        LUTAMM_CCS_SHORT(2, 32)
+        LUTAMM_CCS_SHORT(4, 8)
+        LUTAMM_CCS_SHORT(4, 16)
+        LUTAMM_CCS_SHORT(8, 8)
+        LUTAMM_CCS_SHORT(8, 16)
+#undef LUTAMM_CCS_SHORT
 #define LUTAMM_CCS_REG(V_, CT_) \
     if (a.v == V_ && a.CT == CT_) return run_reg<V_, CT_>(a, s);
         LUTAMM_CCS_REG(2, 8)
         LUTAMM_CCS_REG(2, 16)
-        LUTAMM_CCS_REG(2, 32)
         LUTAMM_CCS_REG(4, 8)
-        LUTAMM_CCS_REG(4, 16)
-        LUTAMM_CCS_REG(8, 8)
 #undef LUTAMM_CCS_REG
-        switch (a.v) {
-            case 1: return run_smem<1>(a, s);
-            case 2: return run_smem<2>(a, s);
-            case 4: return run_smem<4>(a, s);
-            case 8: return run_smem<8>(a, s);
-            case 16: return run_smem<16>(a, s);
-            case 32: return run_smem<32>(a, s);
-            // hidden sizes that are not a power of two times the codebook count (2560 / 256, 5120 / 256, ...)
-            case 3: return run_smem<3>(a, s);
-            case 5: return run_smem<5>(a, s);
-            case 6: return run_smem<6>(a, s);
-            case 10: return run_smem<10>(a, s);
-            case 12: return run_smem<12>(a, s);
-            case 20: return run_smem<20>(a, s);
-            case 24: return run_smem<24>(a, s);
-            default: break;
-        }
     }
-    return run_smem<0>(a, s);
+    switch (a.v) {
+#define LUTAMM_CCS_TILE(V_) \
+    case V_: return run_tile<V_>(a, s);
+        LUTAMM_CCS_TILE(1)
+        LUTAMM_CCS_TILE(2)
+        LUTAMM_CCS_TILE(4)
+        LUTAMM_CCS_TILE(8)
+        LUTAMM_CCS_TILE(16)
+        LUTAMM_CCS_TILE(32)
+        // hidden sizes that are not a power of two times the codebook count (2560 / 256, 5120 / 256, ...)
+        LUTAMM_CCS_TILE(3)
+        LUTAMM_CCS_TILE(5)
+        LUTAMM_CCS_TILE(6)
+        LUTAMM_CCS_TILE(10)
+        LUTAMM_CCS_TILE(12)
+        LUTAMM_CCS_TILE(20)
+        LUTAMM_CCS_TILE(24)
+#undef LUTAMM_CCS_TILE
+        default: return run_any(a, s);
+    }
 }
 
 }  // namespace lutamm
