@@ -852,8 +852,7 @@ cudaError_t umma_make_tmap(CUtensorMap* out, const int8_t* lut_t, uint32_t CB, u
     return cudaSuccess;
 }
 
-// fp32 [M][N] row-major output as 32 x 32 blocks with the 128-byte swizzle the epilogue stages them in
-static cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N, const char** why) {
+cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N, const char** why) {
     EncodeTiledFn enc = get_encode_tiled();
     if (!enc) { *why = "cuTensorMapEncodeTiled is not available from this driver"; return cudaErrorNotSupported; }
     cuuint64_t dims[2] = {N, M};

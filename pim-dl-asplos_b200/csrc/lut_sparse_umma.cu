@@ -1,0 +1,461 @@
+// Steps 2+3 of the AMM on CTA pairs with the one-hot operand in the tensor cores' 2:4 sparse form.
+//
+// The same contraction as lut_onehot_umma.cu - acc[M x N] = OneHot[M x (CB*CT)] * LUT[(CB*CT) x N], exact in int32 -
+// at twice its rate.  A one-hot row has at most one non-zero in any CT >= 8 consecutive positions, so it is 2:4
+// sparse: of every four positions the operand stores two bytes and a nibble of metadata that says which two.  Here the
+// nibble is 0x4 (positions 0, 1) or 0xE (positions 2, 3), the same for all of a codebook: with centroid i, bit 1
+// chooses the nibble and the other bits are the stored byte,  d = (i >> 2) << 1 | (i & 1).
+//
+// Why pairs.  The sparse instruction eats 256 bytes of the contraction axis a row in the time the dense one eats
+// 128, and a LUT byte is read from L2 and from shared memory once per row tile: with 128 rows a tile shared memory
+// would have to deliver 128 B/clk to the tensor core alone, beside the 128 B/clk that the copies fill.  A pair of
+// CTAs (cta_group::2) works on 256 rows and each SM loads and reads half of the LUT slab: 64 + 64 B/clk.
+//
+// Otherwise the structure of the dense kernel: persistent, one pair per two SMs walking 256-token x N_TILE items,
+// accumulators double-buffered in tensor memory, every slot of both rings with one producer and one consumer.  Per CTA:
+//   warp 0        copies its half of a LUT slab (N_TILE/2 rows x 256 bytes); bytes count on the leader's barrier
+//   warps 1-2     leader only: four tcgen05.mma.sp per slab, slab x by warp 1 + x % 2
+//   warps 3-18    four groups of four warps: the operand of the CTA's 128 rows, straight from the uint8 indices;
+//                 group k takes every fourth slab, one row per thread.  The stored bytes come from shifts, not from a
+//                 table in shared memory, whose bandwidth the slabs use up
+//   warps 19-22   epilogue: tcgen05.ld, dequantise, swizzled staging, tiled bulk stores; clears the accumulator
+#include "kernels.h"
+#include "ptx.cuh"
+#include "epilogue.cuh"
+
+namespace lutamm {
+
+namespace {
+
+constexpr uint32_t kRows = 128;                // rows of a CTA: half a tile
+constexpr uint32_t kSlab = 256;                // positions of the contraction axis per ring slot
+constexpr uint32_t kGroups = 4, kMmaWarps = 2, kEpiWarps = 4;
+constexpr uint32_t kFirstBuilder = 1 + kMmaWarps, kFirstEpi = kFirstBuilder + 4 * kGroups;
+constexpr uint32_t kThreads = (kFirstEpi + kEpiWarps) * 32;   // 736
+constexpr uint32_t kASlots = 4;                // operand slots: 32 columns of bytes and 8 of metadata each
+constexpr uint32_t kMaxBSlots = 16;
+constexpr uint32_t kStageBytes = 32 * 128;     // a 32 x 32 fp32 block
+constexpr uint32_t kStages = 2;                // per epilogue warp
+constexpr uint32_t kNumBarriers = 2 * kASlots + 2 * kMaxBSlots + 4;
+
+struct SparseParams {
+    LutArgs a;
+    uint32_t slabs, b_slots, tiles_m, tiles_n, early_trigger;
+    uint32_t* dev_err;
+};
+
+// 32-bit left shift with PTX semantics: an amount of 32 or more gives 0.
+__device__ __forceinline__ uint32_t shl_clamp(uint32_t v, uint32_t n) {
+    uint32_t r;
+    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(n));
+    return r;
+}
+
+// The stored bytes (w, 128 of them) and nibbles (m, 64) of one row's slab from its 256 / CT index bytes.  An index that
+// is out of range (they may come from a caller) stores nothing.
+//
+// CT <= 32: four codebooks at a time, as packed bytes: eight times the stored position, or a value past the codebook's
+// bytes for an index out of range; then a shift per stored word.
+template <int LG>
+__device__ __forceinline__ void build_row(const uint32_t (&raw)[LG == 3 ? 8 : 4], uint32_t (&w)[32], uint32_t (&m)[8]) {
+    if constexpr (LG == 4) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t v = raw[q];
+            // bits 5, 4, 3: index bits 3, 2, 0; bits 7, 6: set if any of the index's bits 7..4 is
+            const uint32_t n4 = ((v << 2) & 0xF0F0F0F0u) | ((v << 3) & 0x08080808u) | (v & 0xC0C0C0C0u);
+            const uint32_t hi = (v >> 1) & 0x01010101u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t n = (n4 >> (8 * j)) & 0xFFu;
+                w[8 * q + 2 * j] = shl_clamp(1u, n);
+                w[8 * q + 2 * j + 1] = shl_clamp(1u, n - 32u);
+            }
+            m[2 * q] = __byte_perm(hi, 0, 0x4140) * 0xAAAAu + 0x44444444u;
+            m[2 * q + 1] = __byte_perm(hi, 0, 0x4342) * 0xAAAAu + 0x44444444u;
+        }
+    } else if constexpr (LG == 3) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t v = raw[q];
+            // bits 4, 3: index bits 2, 0; bits 7..5: set if any of the index's bits 7..3 is
+            const uint32_t n4 = ((v << 2) & 0xF0F0F0F0u) | ((v << 3) & 0x08080808u) | (v & 0xE0E0E0E0u);
+            const uint32_t hi = (v >> 1) & 0x01010101u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w[4 * q + j] = shl_clamp(1u, (n4 >> (8 * j)) & 0xFFu);
+            m[q] = hi * 0xAAu + 0x44444444u;
+        }
+    } else {
+        // one codebook at a time: kW words of stored bytes, kM of nibbles
+        constexpr int kCbs = 256 >> LG, kW = 32 / kCbs, kM = 8 / kCbs;
+#pragma unroll
+        for (int c = 0; c < kCbs; ++c) {
+            const uint32_t i = (raw[c / 4] >> (8 * (c & 3))) & 0xFFu;
+            const uint32_t d = ((i >> 2) << 1) | (i & 1u);
+            const uint32_t n = LG < 8 && (i >> LG) ? 0x8000u : 8u * d;
+#pragma unroll
+            for (int k = 0; k < kW; ++k) w[c * kW + k] = shl_clamp(1u, n - 32u * k);
+            const uint32_t meta = i & 2u ? 0xEEEEEEEEu : 0x44444444u;
+#pragma unroll
+            for (int k = 0; k < kM; ++k) m[c * kM + k] = meta;
+        }
+    }
+}
+
+struct SparseItem {
+    uint32_t m0, n0;
+};
+__device__ __forceinline__ SparseItem sparse_item(const SparseParams& p, uint32_t item, uint32_t n_tile, uint32_t rank) {
+    return {(item % p.tiles_m) * (2 * kRows) + rank * kRows, (item / p.tiles_m) * n_tile};
+}
+
+template <uint32_t N_TILE, int LG>
+__global__ void __launch_bounds__(kThreads, 1)
+lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_constant__ CUtensorMap out_map, const SparseParams p) {
+    constexpr uint32_t kHalfN = N_TILE / 2, kBBytes = kHalfN * kSlab;
+    constexpr uint32_t kIdesc = umma_idesc_i8(2 * kRows, N_TILE, 1, 1) | kIdescSparse;
+    constexpr uint32_t kDataBase = 2 * N_TILE, kMetaBase = kDataBase + 32 * kASlots;   // tensor-memory columns
+    static_assert(kMetaBase + 8 * kASlots <= 512, "tensor memory");
+
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const uint32_t SB = p.b_slots;
+    unsigned char* s_b = smem;                                        // [SB][2][kHalfN][128]
+    unsigned char* s_stage = s_b + (size_t)SB * kBBytes;              // [4][kStages][32][128]
+    float* s_bias = reinterpret_cast<float*>(s_stage + kEpiWarps * kStages * kStageBytes);   // [4][N_TILE]
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_bias + kEpiWarps * N_TILE);
+    uint32_t* s_misc = reinterpret_cast<uint32_t*>(s_bar + kNumBarriers);                  // tmem base, abort
+    volatile uint32_t* s_abort = s_misc + 1;
+    const uint32_t a_full0 = smem_u32(s_bar), a_empty0 = a_full0 + 8 * kASlots, b_full0 = a_empty0 + 8 * kASlots,
+                   b_empty0 = b_full0 + 8 * kMaxBSlots, acc_full0 = b_empty0 + 8 * kMaxBSlots, acc_empty0 = acc_full0 + 16;
+
+    const LutArgs& a = p.a;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = cluster_rank();
+    const uint32_t n_items = p.tiles_m * p.tiles_n, n_pairs = gridDim.x >> 1, first = blockIdx.x >> 1;
+
+    if (threadIdx.x == 0) {
+        s_misc[1] = 0;
+        tma_prefetch_desc(&lut_map);
+        tma_prefetch_desc(&out_map);
+    }
+    if (threadIdx.x >= 64 && threadIdx.x < 64 + kNumBarriers) {
+        const uint32_t b = threadIdx.x - 64;
+        // a_full: the four builder warps of the slab's group in each CTA; a_empty, b_empty: one commit; b_full: the
+        // leader's expect_tx (the copies of both CTAs complete the bytes); acc_full: one commit per issuing warp;
+        // acc_empty: the epilogue warps of both CTAs.  Barriers the leader waits on are unused in the other CTA.
+        const uint32_t after = 2 * kASlots + 2 * kMaxBSlots;
+        mbar_init(a_full0 + 8 * b, b < kASlots ? 8u : b < after ? 1u : b < after + 2 ? kMmaWarps : 2 * kEpiWarps);
+        fence_barrier_init();
+    }
+    if (warp == 1) tmem_alloc_pair(smem_u32(s_misc), 512);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(s_misc);
+    const uint32_t my_lanes = ((warp & 3u) * 32u) << 16;
+    if (warp >= kFirstEpi) {   // every MMA accumulates: both accumulators start at zero
+        const uint32_t zero[32] = {};
+        for (uint32_t c = 0; c < 2 * N_TILE; c += 32) tmem_st_32x32b_x32(tmem_base + my_lanes + c, zero);
+        tmem_st_wait();
+    }
+    tc_fence_before_sync();
+    cluster_sync();   // barriers initialised and accumulators cleared in both CTAs
+    tc_fence_after_sync();
+
+    if (warp == 0) {
+        // ---------------- LUT copies (the LUT never depends on the preceding kernel)
+        if (lane == 0) {
+            uint32_t j = 0, ph = 0;
+            bool ok = true;
+            const uint32_t full_leader = map_to_rank(b_full0, 0);
+            for (uint32_t item = first; item < n_items && ok; item += n_pairs) {
+                const SparseItem it = sparse_item(p, item, N_TILE, rank);
+                for (uint32_t i = 0; i < p.slabs; ++i) {
+                    ok = mbar_wait<32>(b_empty0 + 8 * j, ph ^ 1, s_abort);
+                    if (!ok) break;
+                    if (rank == 0) mbar_arrive_expect_tx(b_full0 + 8 * j, 2 * kBBytes);
+                    tma_load_3d_pair(smem_u32(s_b + (size_t)j * kBBytes), &lut_map, full_leader + 8 * j, 0,
+                                     (int32_t)(it.n0 + rank * kHalfN), (int32_t)(2 * i));
+                    if (++j == SB) { j = 0; ph ^= 1; }
+                }
+            }
+        }
+        __syncwarp();
+        if (p.early_trigger) pdl_launch_dependents();
+    } else if (warp < kFirstBuilder) {
+        // ---------------- MMA issue, leader only.  Converged loop, one elected lane issues; whether the next slab's two
+        // slots are full is asked a turn ahead.
+        if (rank == 0) {
+            const uint32_t me = warp - 1;
+            uint32_t j = me, pb = 0, t = 0, x0 = 0;   // LUT slot and phase of this warp's next slab; slabs before the item
+            bool ok = true;
+            const uint32_t b_lo0 = (uint32_t)umma_desc_k_sw128(smem_u32(s_b));
+            const uint32_t desc_hi = (uint32_t)(umma_desc_k_sw128(0) >> 32);
+            bool ready = mbar_test2_cluster(b_full0 + 8 * j, pb, a_full0 + 8 * (me % kASlots), 0);
+            for (uint32_t item = first; item < n_items && ok; item += n_pairs, ++t) {
+                const uint32_t ab = t & 1;
+                ok = mbar_wait_cluster(acc_empty0 + 8 * ab, ((t >> 1) & 1) ^ 1, s_abort);
+                if (!ok) break;
+                tc_fence_after_sync();
+                const uint32_t d_tmem = tmem_base + ab * N_TILE;
+                for (uint32_t i = (x0 + me) & 1u; i < p.slabs; i += 2) {
+                    const uint32_t x = x0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
+                    if (!ready) {
+                        ok = mbar_wait_cluster(b_full0 + 8 * j, pb, s_abort) && mbar_wait_cluster(a_full0 + 8 * k, pa, s_abort);
+                        if (!ok) break;
+                    }
+                    uint32_t j2 = j + 2, pb2 = pb;
+                    if (j2 >= SB) { j2 -= SB; pb2 ^= 1; }
+                    const uint32_t x2 = x + 2;
+                    const bool next_ready = mbar_test2_cluster(b_full0 + 8 * j2, pb2, a_full0 + 8 * (x2 % kASlots), (x2 / kASlots) & 1u);
+                    tc_fence_after_sync();
+                    if (elect_one()) {
+                        const uint32_t b_lo = b_lo0 + j * (kBBytes >> 4);
+#pragma unroll
+                        for (uint32_t kk = 0; kk < 4; ++kk)   // 64 positions each: two per 128-byte swizzle row
+                            umma_i8_sparse_pair(d_tmem, tmem_base + kDataBase + 32 * k + 8 * kk,
+                                                ((uint64_t)desc_hi << 32) | (b_lo + (kk >> 1) * (kHalfN * 128 >> 4) + (kk & 1) * 4),
+                                                tmem_base + kMetaBase + 8 * k + 2 * kk, kIdesc);
+                        umma_commit_pair(a_empty0 + 8 * k);
+                        umma_commit_pair(b_empty0 + 8 * j);
+                    }
+                    __syncwarp();
+                    j = j2; pb = pb2;
+                    ready = next_ready;
+                }
+                x0 += p.slabs;
+                if (ok && elect_one()) umma_commit_pair(acc_full0 + 8 * ab);
+                __syncwarp();
+            }
+        }
+        __syncwarp();
+        if (p.early_trigger) pdl_launch_dependents();
+    } else if (warp < kFirstEpi) {
+        // ---------------- operand builders: slab x of the CTA's sequence by group x % 4, into slot x % 4
+        pdl_wait_prior_grid();
+        constexpr int kRaw = LG == 3 ? 8 : 4;
+        const uint32_t grp = (warp - kFirstBuilder) >> 2, r = (warp & 3u) * 32 + lane;
+        const uint32_t row_bytes = a.CB;
+        // 256 / CT index bytes; L2 (under programmatic launch this SM's L1 may hold older lines)
+        auto load_raw = [&](const uint8_t* row, uint32_t slab, uint32_t (&v)[kRaw]) {
+            const uint8_t* q = row + ((slab * kSlab) >> LG);
+            if constexpr (LG == 3) {
+                const uint4 t = __ldcg(reinterpret_cast<const uint4*>(q));
+                v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+                // an odd multiple of 16 codebooks ends in half a slab
+                uint4 u = make_uint4(~0u, ~0u, ~0u, ~0u);
+                if ((slab * kSlab >> LG) + 16 < row_bytes) u = __ldcg(reinterpret_cast<const uint4*>(q) + 1);
+                v[4] = u.x; v[5] = u.y; v[6] = u.z; v[7] = u.w;
+            } else if constexpr (LG == 4) {
+                const uint4 t = __ldcg(reinterpret_cast<const uint4*>(q));
+                v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+            } else if constexpr (LG == 5) {
+                const uint2 t = __ldcg(reinterpret_cast<const uint2*>(q));
+                v[0] = t.x; v[1] = t.y;
+            } else if constexpr (LG == 6) {
+                v[0] = __ldcg(reinterpret_cast<const uint32_t*>(q));
+            } else if constexpr (LG == 7) {
+                v[0] = __ldcg(reinterpret_cast<const uint16_t*>(q));
+            } else {
+                v[0] = __ldcg(q);
+            }
+        };
+        const uint32_t full_leader = map_to_rank(a_full0, 0);
+        uint32_t x0 = 0;
+        bool ok = true;
+        for (uint32_t item = first; item < n_items && ok; item += n_pairs) {
+            const SparseItem it = sparse_item(p, item, N_TILE, rank);
+            const uint8_t* row = a.idx + (size_t)min(it.m0 + r, a.M - 1) * a.CB;   // rows past M: clipped by the epilogue
+            uint32_t i = (grp - x0) & (kGroups - 1);
+            uint32_t raw[2][kRaw];   // index bytes are fetched two turns ahead
+            if (i < p.slabs) load_raw(row, i, raw[0]);
+            if (i + kGroups < p.slabs) load_raw(row, i + kGroups, raw[1]);
+            for (; i < p.slabs && ok; i += kGroups) {
+                const uint32_t x = x0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
+                uint32_t w[32], m[8];
+                build_row<LG>(raw[0], w, m);
+#pragma unroll
+                for (int c = 0; c < kRaw; ++c) raw[0][c] = raw[1][c];
+                if (i + 2 * kGroups < p.slabs) load_raw(row, i + 2 * kGroups, raw[1]);
+                ok = mbar_wait(a_empty0 + 8 * k, pa ^ 1, s_abort);
+                if (!ok) break;
+                tc_fence_after_sync();
+                tmem_st_32x32b_x32(tmem_base + my_lanes + kDataBase + 32 * k, w);
+                tmem_st_32x32b_x8(tmem_base + my_lanes + kMetaBase + 8 * k, m);
+                tmem_st_wait();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(full_leader + 8 * k);
+            }
+            x0 += p.slabs;
+        }
+        if (p.early_trigger) pdl_launch_dependents();
+    } else {
+        // ---------------- epilogue: each warp on the lane quadrant it may read
+        pdl_wait_prior_grid();
+        const uint32_t quad = warp & 3u;
+        const float lbcb = lut_bias_times_cb(a.lut_bias, a.CB);
+        unsigned char* stg = s_stage + (warp - kFirstEpi) * (kStages * kStageBytes);
+        float* bw = s_bias + (warp - kFirstEpi) * N_TILE;
+        const uint32_t empty_leader = map_to_rank(acc_empty0, 0);
+        uint32_t t = 0, buf = 0;
+        bool ok = true;
+        for (uint32_t item = first; item < n_items; item += n_pairs, ++t) {
+            const SparseItem it = sparse_item(p, item, N_TILE, rank);
+            const uint32_t ab = t & 1;
+            if (p.early_trigger && item + n_pairs >= n_items) pdl_launch_dependents();
+            __syncwarp();   // the previous item's reads of bw are done
+#pragma unroll
+            for (uint32_t c = 0; c < N_TILE / 32; ++c) {
+                const uint32_t n = it.n0 + c * 32 + lane;
+                bw[c * 32 + lane] = n < a.N ? __ldg(a.bias + n) : 0.f;
+            }
+            uint32_t w_ok = 1;
+            if (lane == 0) w_ok = (ok && mbar_wait<256>(acc_full0 + 8 * ab, (t >> 1) & 1, s_abort)) ? 1u : 0u;
+            ok = __shfl_sync(0xffffffffu, w_ok, 0) != 0;
+            if (!ok) continue;
+            tc_fence_after_sync();
+            for (uint32_t c = 0; c < N_TILE / 32; ++c) {
+                uint32_t v[32];
+                tmem_ld_32x32b_x32(tmem_base + my_lanes + ab * N_TILE + c * 32u, v);
+                tmem_ld_wait();
+                {   // leave the columns at zero for the next item's accumulating MMAs
+                    const uint32_t zero[32] = {};
+                    tmem_st_32x32b_x32(tmem_base + my_lanes + ab * N_TILE + c * 32u, zero);
+                }
+                if (c == N_TILE / 32 - 1) {   // accumulator fully read and cleared: hand the buffer back
+                    tmem_st_wait();
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(empty_leader + 8 * ab);
+                }
+                if (it.n0 + c * 32 >= a.N || it.m0 + quad * 32 >= a.M) continue;   // a block wholly past N or M
+                unsigned char* sg = stg + buf * kStageBytes;
+                if (lane == 0) tma_store_wait_read_1();   // the copy before last has read this buffer
+                __syncwarp();
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q) {
+                    const float4 b4 = *reinterpret_cast<const float4*>(bw + c * 32 + 4 * q);
+                    float4 o = make_float4(dequant_one((int32_t)v[4 * q], a.scale, lbcb, b4.x), dequant_one((int32_t)v[4 * q + 1], a.scale, lbcb, b4.y),
+                                           dequant_one((int32_t)v[4 * q + 2], a.scale, lbcb, b4.z), dequant_one((int32_t)v[4 * q + 3], a.scale, lbcb, b4.w));
+                    if (a.act) { o.x = activate_one(o.x, a.act); o.y = activate_one(o.y, a.act); o.z = activate_one(o.z, a.act); o.w = activate_one(o.w, a.act); }
+                    *reinterpret_cast<float4*>(sg + lane * 128 + ((q ^ (lane & 7u)) << 4)) = o;
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_2d(&out_map, smem_u32(sg), (int32_t)(it.n0 + c * 32), (int32_t)(it.m0 + quad * 32));
+                    tma_store_commit();
+                }
+                buf ^= 1;
+            }
+        }
+        if (lane == 0) tma_store_wait_all();   // shared memory and the output are settled before the CTA leaves
+        __syncwarp();
+        tc_fence_before_sync();
+    }
+
+    // ---------------- tear-down (also the way out after a wait that ran out)
+    __syncthreads();
+    if (*s_abort) {
+        if (threadIdx.x == 0) {
+            // give copies that may still be in flight a bounded time to land before the shared memory is handed back
+            const long long t0 = clock64();
+            while (clock64() - t0 < 200000) {}
+            atomicExch(p.dev_err, 2u);
+        }
+        __syncthreads();
+    }
+    cluster_sync();   // nothing of this CTA is read, written or signalled by the other one any more
+    if (warp == 1) {
+        tc_fence_after_sync();
+        tmem_dealloc_pair(tmem_base, 512);
+    }
+}
+
+constexpr size_t kSmemLimit = 227 * 1024;
+
+size_t sparse_smem(uint32_t n_tile, uint32_t b_slots) {
+    return (size_t)b_slots * (n_tile / 2) * kSlab + kEpiWarps * kStages * kStageBytes + kEpiWarps * n_tile * 4 + kNumBarriers * 8 + 16 + 1024;
+}
+
+template <uint32_t N_TILE, int LG>
+cudaError_t run(const CUtensorMap& map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
+    auto k = lut_sparse_kernel<N_TILE, LG>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * pairs);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, k, map, out_map, p);
+}
+
+template <uint32_t N_TILE>
+cudaError_t run_lg(uint32_t lg, const CUtensorMap& map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
+    switch (lg) {
+        case 3: return run<N_TILE, 3>(map, out_map, p, pairs, smem, s);
+        case 4: return run<N_TILE, 4>(map, out_map, p, pairs, smem, s);
+        case 5: return run<N_TILE, 5>(map, out_map, p, pairs, smem, s);
+        case 6: return run<N_TILE, 6>(map, out_map, p, pairs, smem, s);
+        case 7: return run<N_TILE, 7>(map, out_map, p, pairs, smem, s);
+        default: return run<N_TILE, 8>(map, out_map, p, pairs, smem, s);
+    }
+}
+
+}  // namespace
+
+// LUT^T [N][CB*CT] as slabs of 256 positions: x = position within 128, y = row, z = position / 128; a box is half a
+// tile's rows of one slab.
+cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* lut_t, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile, const char** why) {
+    *why = nullptr;
+    EncodeTiledFn enc = get_encode_tiled();
+    if (!enc) { *why = "cuTensorMapEncodeTiled is not available from this driver"; return cudaErrorNotSupported; }
+    const uint64_t Kg = (uint64_t)CB * CT;
+    cuuint64_t dims[3] = {128, N, Kg / 128};
+    cuuint64_t strides[2] = {Kg, 128};
+    cuuint32_t box[3] = {128, n_tile / 2, 2};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t*>(lut_t), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the LUT slab map"; return cudaErrorInvalidValue; }
+    return cudaSuccess;
+}
+
+cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, uint32_t n_tile, uint32_t max_ctas, uint32_t* dev_err, cudaStream_t s, const char** why) {
+    *why = nullptr;
+    if (a.M == 0 || a.N == 0) return cudaSuccess;
+    if (reinterpret_cast<uintptr_t>(a.idx) & 15u) { *why = "tcgen05 variant: the index buffer must be 16-byte aligned"; return cudaErrorInvalidValue; }
+    SparseParams p;
+    p.a = a;
+    p.slabs = (uint32_t)(((uint64_t)a.CB * a.CT + kSlab - 1) / kSlab);
+    p.tiles_m = (a.M + 2 * kRows - 1) / (2 * kRows);
+    p.tiles_n = (a.N + n_tile - 1) / n_tile;
+    p.dev_err = dev_err;
+    p.b_slots = kMaxBSlots;
+    while (p.b_slots > 2 && sparse_smem(n_tile, p.b_slots) > kSmemLimit) p.b_slots -= 2;
+    const uint64_t items = (uint64_t)p.tiles_m * p.tiles_n;
+    const uint32_t cap = max_ctas / 2, pairs = (uint32_t)(items < cap ? items : cap);
+    p.early_trigger = items <= cap;
+    uint32_t lg = 0;
+    while ((1u << lg) < a.CT) ++lg;
+    CUtensorMap om;
+    cudaError_t e = make_out_tmap(&om, a.out, a.M, a.N, why);
+    if (e != cudaSuccess) return e;
+    size_t smem = sparse_smem(n_tile, p.b_slots);
+    if (n_tile == 160) return run_lg<160>(lg, lut_map, om, p, pairs, smem, s);
+    *why = "tcgen05 variant: this tile is not built";
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace lutamm

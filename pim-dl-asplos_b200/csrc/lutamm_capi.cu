@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -248,6 +249,16 @@ int run_lut(lutamm_ctx* c, Layer& L, const uint8_t* d_idx, float* d_out, int32_t
                 return fail(c, LUTAMM_ECUDA, std::string("LUT transpose: ") + cudaGetErrorString(te));
             }
             ++c->launches;
+        }
+        static const int force = getenv("LUTAMM_SPARSE") ? atoi(getenv("LUTAMM_SPARSE")) : 0;
+        if (force && !a.n_peers && !a.acc_out && !a.layout.tiled) {
+            static std::map<const void*, CUtensorMap> maps;
+            CUtensorMap m;
+            cudaError_t e = sparse_make_tmap(&m, L.d_lut_t, L.CB, L.CT, L.N, force, &why);
+            if (e == cudaSuccess) e = launch_sparse(a, m, force, c->sm_count, c->d_err, c->stream, &why);
+            if (e != cudaSuccess) return fail(c, LUTAMM_ECUDA, why ? why : cudaGetErrorString(e));
+            ++c->launches;
+            return LUTAMM_OK;
         }
         const int slot = umma_tile_slot(up.n_tile);
         if (!L.umma_map_ok[slot]) {
