@@ -82,7 +82,9 @@ uint32_t umma_auto_split(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, uint3
 cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N, const char** why);
 
 // The same contraction on CTA pairs with the one-hot operand 2:4 sparse (row-major fp32 output).
-cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* lut_t, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile,
+size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N);
+cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t N, cudaStream_t s);
+cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile,
                              const char** why);
 cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, uint32_t n_tile, uint32_t max_ctas, uint32_t* dev_err,
                           cudaStream_t s, const char** why);

@@ -1,10 +1,8 @@
 // Steps 2+3 of the AMM on CTA pairs with the one-hot operand in the tensor cores' 2:4 sparse form.
 //
 // The same contraction as lut_onehot_umma.cu - acc[M x N] = OneHot[M x (CB*CT)] * LUT[(CB*CT) x N], exact in int32 -
-// at twice its rate.  A one-hot row has at most one non-zero in any CT >= 8 consecutive positions, so it is 2:4
-// sparse: of every four positions the operand stores two bytes and a nibble of metadata that says which two.  Here the
-// nibble is 0x4 (positions 0, 1) or 0xE (positions 2, 3), the same for all of a codebook: with centroid i, bit 1
-// chooses the nibble and the other bits are the stored byte,  d = (i >> 2) << 1 | (i & 1).
+// at twice its rate.  A one-hot row has at most one non-zero per codebook, so it is 2:4 sparse: of every four positions
+// the operand stores two bytes and a nibble of metadata that says which two positions they stand for (build_row).
 //
 // Why pairs.  The sparse instruction eats 256 bytes of the contraction axis a row in the time the dense one eats
 // 128, and a LUT byte is read from L2 and from shared memory once per row tile: with 128 rows a tile shared memory
@@ -14,11 +12,11 @@
 // Otherwise the structure of the dense kernel: persistent, one pair per two SMs walking 256-token x N_TILE items,
 // accumulators double-buffered in tensor memory, every slot of both rings with one producer and one consumer.  Per CTA:
 //   warp 0        copies its half of a LUT slab (N_TILE/2 rows x 256 bytes); bytes count on the leader's barrier
-//   warps 1-2     leader only: four tcgen05.mma.sp per slab, slab x by warp 1 + x % 2
-//   warps 3-18    four groups of four warps: the operand of the CTA's 128 rows, straight from the uint8 indices;
+//   warps 1-4     leader only: four tcgen05.mma.sp per slab, slab x by warp 1 + x % 4
+//   warps 5-20    four groups of four warps: the operand of the CTA's 128 rows, straight from the uint8 indices;
 //                 group k takes every fourth slab, one row per thread.  The stored bytes come from shifts, not from a
 //                 table in shared memory, whose bandwidth the slabs use up
-//   warps 19-22   epilogue: tcgen05.ld, dequantise, swizzled staging, tiled bulk stores; clears the accumulator
+//   warps 21-24   epilogue: tcgen05.ld, dequantise, swizzled staging, tiled bulk stores; clears the accumulator
 #include "kernels.h"
 #include "ptx.cuh"
 #include "epilogue.cuh"
@@ -29,13 +27,13 @@ namespace {
 
 constexpr uint32_t kRows = 128;                // rows of a CTA: half a tile
 constexpr uint32_t kSlab = 256;                // positions of the contraction axis per ring slot
-constexpr uint32_t kGroups = 4, kMmaWarps = 2, kEpiWarps = 4;
-constexpr uint32_t kFirstBuilder = 1 + kMmaWarps, kFirstEpi = kFirstBuilder + 4 * kGroups;
-constexpr uint32_t kThreads = (kFirstEpi + kEpiWarps) * 32;   // 736
-constexpr uint32_t kASlots = 4;                // operand slots: 32 columns of bytes and 8 of metadata each
+constexpr uint32_t kGroups = 4, kCopyWarps = 2, kMmaWarps = 4, kEpiWarps = 4;
+constexpr uint32_t kFirstMma = kCopyWarps, kFirstBuilder = kFirstMma + kMmaWarps, kFirstEpi = kFirstBuilder + 4 * kGroups;
+constexpr uint32_t kThreads = (kFirstEpi + kEpiWarps) * 32;   // 832
+constexpr uint32_t kASlots = 4;                // operand slots: 32 columns of bytes and 2 of metadata each
 constexpr uint32_t kMaxBSlots = 16;
 constexpr uint32_t kStageBytes = 32 * 128;     // a 32 x 32 fp32 block
-constexpr uint32_t kStages = 2;                // per epilogue warp
+constexpr uint32_t kStages = 1;                // per epilogue warp
 constexpr uint32_t kNumBarriers = 2 * kASlots + 2 * kMaxBSlots + 4;
 
 struct SparseParams {
@@ -44,62 +42,100 @@ struct SparseParams {
     uint32_t* dev_err;
 };
 
-// 32-bit left shift with PTX semantics: an amount of 32 or more gives 0.
-__device__ __forceinline__ uint32_t shl_clamp(uint32_t v, uint32_t n) {
-    uint32_t r;
-    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(n));
-    return r;
+// Out = one word per combination of the index bits in BITS (highest first): in & (bit or its complement), two bits per
+// three-input operation.  A word holds bytes of several codebooks; `in` carries at most bit 0 of each, so what else the
+// shifted indices hold does not matter.
+template <int N>
+__device__ __forceinline__ void split1(const uint32_t (&in)[N], uint32_t b, uint32_t (&out)[2 * N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) { out[2 * i] = in[i] & ~b; out[2 * i + 1] = in[i] & b; }
+}
+template <int N>
+__device__ __forceinline__ void split2(const uint32_t (&in)[N], uint32_t b1, uint32_t b0, uint32_t (&out)[4 * N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        out[4 * i] = in[i] & ~b1 & ~b0; out[4 * i + 1] = in[i] & ~b1 & b0;
+        out[4 * i + 2] = in[i] & b1 & ~b0; out[4 * i + 3] = in[i] & b1 & b0;
+    }
 }
 
-// The stored bytes (w, 128 of them) and nibbles (m, 64) of one row's slab from its 256 / CT index bytes.  An index that
-// is out of range (they may come from a caller) stores nothing.
+// The operand of one row's slab from its 256 / CT index bytes: 128 stored bytes (w) and the metadata of 64 positions of
+// the axis (m), which repeats for all four instructions of the slab.
 //
-// CT <= 32: four codebooks at a time, as packed bytes: eight times the stored position, or a value past the codebook's
-// bytes for an index out of range; then a shift per stored word.
+// Stored byte p = d * codebooks + codebook, d being the centroid index without its bit 1: bytes of four codebooks share
+// a word, so a word is the AND of a few (complemented) bits of four packed indices - one three-input operation - where
+// codebook-major bytes would take two shifts and an extraction per codebook.  Positions 2p and 2p + 1 of the axis belong
+// to byte p: the index's bit 1 chooses, through the metadata nibble of the pair of bytes (2g, 2g + 1): the first stands
+// for position 0 or 1 of four, the second for 2 or 3.  The table is laid out to match (launch_sparse_table).
+//
+// An index that is out of range (they may come from a caller) stores nothing.
 template <int LG>
-__device__ __forceinline__ void build_row(const uint32_t (&raw)[LG == 3 ? 8 : 4], uint32_t (&w)[32], uint32_t (&m)[8]) {
-    if constexpr (LG == 4) {
+__device__ __forceinline__ void build_row(const uint32_t (&raw)[LG == 3 ? 8 : 4], uint32_t (&w)[32], uint32_t (&m)[2]) {
+    constexpr int kCbs = 256 >> LG, kQ = kCbs >= 4 ? kCbs / 4 : 1;   // codebooks, words of packed indices
+    constexpr uint32_t kOnes = 0x01010101u, kBeyond = LG == 8 ? 0u : ((0xFFu << LG) & 0xFFu) * kOnes;
+    uint32_t v[kQ], valid[kQ], top[kQ], any = 0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint32_t v = raw[q];
-            // bits 5, 4, 3: index bits 3, 2, 0; bits 7, 6: set if any of the index's bits 7..4 is
-            const uint32_t n4 = ((v << 2) & 0xF0F0F0F0u) | ((v << 3) & 0x08080808u) | (v & 0xC0C0C0C0u);
-            const uint32_t hi = (v >> 1) & 0x01010101u;
+    for (int q = 0; q < kQ; ++q) {
+        if constexpr (LG == 8) v[q] = (raw[0] & 0xFFu) * kOnes;
+        else if constexpr (LG == 7) v[q] = __byte_perm(raw[0], 0, 0x1010);
+        else v[q] = raw[q];
+        any |= v[q] & kBeyond;
+        valid[q] = kOnes;
+        // bits 0, 2, 4, 6 of the top byte: bit 1 of the four indices
+        top[q] = ((v[q] >> 1) & kOnes) * 0x01041040u;
+    }
+    if (LG < 8 && any) {
+        constexpr uint32_t kRange = 1u << (8 - LG);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t n = (n4 >> (8 * j)) & 0xFFu;
-                w[8 * q + 2 * j] = shl_clamp(1u, n);
-                w[8 * q + 2 * j + 1] = shl_clamp(1u, n - 32u);
-            }
-            m[2 * q] = __byte_perm(hi, 0, 0x4140) * 0xAAAAu + 0x44444444u;
-            m[2 * q + 1] = __byte_perm(hi, 0, 0x4342) * 0xAAAAu + 0x44444444u;
-        }
-    } else if constexpr (LG == 3) {
+        for (int q = 0; q < kQ; ++q) valid[q] = ((kRange * kOnes - ((v[q] & kBeyond) >> LG)) >> (8 - LG)) & kOnes;
+    }
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const uint32_t v = raw[q];
-            // bits 4, 3: index bits 2, 0; bits 7..5: set if any of the index's bits 7..3 is
-            const uint32_t n4 = ((v << 2) & 0xF0F0F0F0u) | ((v << 3) & 0x08080808u) | (v & 0xE0E0E0E0u);
-            const uint32_t hi = (v >> 1) & 0x01010101u;
+    for (int q = 0; q < kQ; ++q) {
+        const uint32_t x = v[q];
+        if constexpr (LG == 3) {
+            uint32_t in[1] = {valid[q]}, o[4];
+            split2(in, x >> 2, x, o);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) w[4 * q + j] = shl_clamp(1u, (n4 >> (8 * j)) & 0xFFu);
-            m[q] = hi * 0xAAu + 0x44444444u;
-        }
-    } else {
-        // one codebook at a time: kW words of stored bytes, kM of nibbles
-        constexpr int kCbs = 256 >> LG, kW = 32 / kCbs, kM = 8 / kCbs;
+            for (int d = 0; d < 4; ++d) w[d * kQ + q] = o[d];
+        } else if constexpr (LG == 4) {
+            uint32_t in[1] = {valid[q]}, t[2], o[8];
+            split1(in, x >> 3, t);
+            split2(t, x >> 2, x, o);
 #pragma unroll
-        for (int c = 0; c < kCbs; ++c) {
-            const uint32_t i = (raw[c / 4] >> (8 * (c & 3))) & 0xFFu;
-            const uint32_t d = ((i >> 2) << 1) | (i & 1u);
-            const uint32_t n = LG < 8 && (i >> LG) ? 0x8000u : 8u * d;
+            for (int d = 0; d < 8; ++d) w[d * kQ + q] = o[d];
+        } else if constexpr (LG == 5) {
+            uint32_t in[1] = {valid[q]}, t[4], o[16];
+            split2(in, x >> 4, x >> 3, t);
+            split2(t, x >> 2, x, o);
 #pragma unroll
-            for (int k = 0; k < kW; ++k) w[c * kW + k] = shl_clamp(1u, n - 32u * k);
-            const uint32_t meta = i & 2u ? 0xEEEEEEEEu : 0x44444444u;
-#pragma unroll
-            for (int k = 0; k < kM; ++k) m[c * kM + k] = meta;
+            for (int d = 0; d < 16; ++d) w[d * kQ + q] = o[d];
+        } else {
+            // 32 words of one index word: five bits; what is left of d lies within the word
+            uint32_t in[1], t[2], u[8];
+            constexpr int b = LG == 6 ? 0 : LG == 7 ? 2 : 3;   // lowest of the five bits (6: bits 5, 4, 3, 2, 0)
+            if constexpr (LG == 6) in[0] = valid[q];
+            else if constexpr (LG == 7) in[0] = valid[q] & ~(x ^ 0x01010000u);   // bytes: (d even) cb 0, 1, (d odd) cb 0, 1
+            else in[0] = 1u << (8 * (((x >> 1) & 2u) | (x & 1u)));
+            split1(in, LG == 6 ? x >> 5 : x >> (b + 4), t);
+            split2(t, LG == 6 ? x >> 4 : x >> (b + 3), LG == 6 ? x >> 3 : x >> (b + 2), u);
+            split2(u, LG == 6 ? x >> 2 : x >> (b + 1), x >> b, w);
         }
     }
+    uint32_t meta[2];
+    if constexpr (LG == 3) {
+        meta[0] = __byte_perm(__byte_perm(top[0], top[1], 0x0073), __byte_perm(top[2], top[3], 0x0073), 0x5410);
+        meta[1] = __byte_perm(__byte_perm(top[4], top[5], 0x0073), __byte_perm(top[6], top[7], 0x0073), 0x5410);
+    } else if constexpr (LG == 4) {
+        meta[0] = meta[1] = __byte_perm(__byte_perm(top[0], top[1], 0x0073), __byte_perm(top[2], top[3], 0x0073), 0x5410);
+    } else if constexpr (LG == 5) {
+        meta[0] = meta[1] = __byte_perm(top[0], top[1], 0x7373);
+    } else if constexpr (LG == 6) {
+        meta[0] = meta[1] = __byte_perm(top[0], 0, 0x3333);
+    } else {   // one nibble: (first codebook, second codebook), or the one codebook twice; the top byte holds it twice
+        meta[0] = meta[1] = __byte_perm(top[0], 0, 0x3333);
+    }
+    m[0] = meta[0] | 0x88888888u;
+    m[1] = meta[1] | 0x88888888u;
 }
 
 struct SparseItem {
@@ -115,7 +151,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     constexpr uint32_t kHalfN = N_TILE / 2, kBBytes = kHalfN * kSlab;
     constexpr uint32_t kIdesc = umma_idesc_i8(2 * kRows, N_TILE, 1, 1) | kIdescSparse;
     constexpr uint32_t kDataBase = 2 * N_TILE, kMetaBase = kDataBase + 32 * kASlots;   // tensor-memory columns
-    static_assert(kMetaBase + 8 * kASlots <= 512, "tensor memory");
+    static_assert(kMetaBase + 2 * kASlots <= 512, "tensor memory");
 
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -147,7 +183,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         mbar_init(a_full0 + 8 * b, b < kASlots ? 8u : b < after ? 1u : b < after + 2 ? kMmaWarps : 2 * kEpiWarps);
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc_pair(smem_u32(s_misc), 512);
+    if (warp == kFirstMma) tmem_alloc_pair(smem_u32(s_misc), 512);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -162,52 +198,48 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     cluster_sync();   // barriers initialised and accumulators cleared in both CTAs
     tc_fence_after_sync();
 
-    if (warp == 0) {
-        // ---------------- LUT copies (the LUT never depends on the preceding kernel)
+    if (warp < kFirstMma) {
+        // ---------------- LUT copies (the LUT never depends on the preceding kernel), slab x by warp x % kCopyWarps: a
+        // thread sustains one copy per ~ 480 cycles, of which the instruction itself holds it for 350
         if (lane == 0) {
-            uint32_t j = 0, ph = 0;
+            uint32_t j = warp, ph = 0, x0 = 0;
             bool ok = true;
             const uint32_t full_leader = map_to_rank(b_full0, 0);
             for (uint32_t item = first; item < n_items && ok; item += n_pairs) {
                 const SparseItem it = sparse_item(p, item, N_TILE, rank);
-                for (uint32_t i = 0; i < p.slabs; ++i) {
+                for (uint32_t i = (warp - x0) & (kCopyWarps - 1); i < p.slabs; i += kCopyWarps) {
                     ok = mbar_wait<32>(b_empty0 + 8 * j, ph ^ 1, s_abort);
                     if (!ok) break;
                     if (rank == 0) mbar_arrive_expect_tx(b_full0 + 8 * j, 2 * kBBytes);
                     tma_load_3d_pair(smem_u32(s_b + (size_t)j * kBBytes), &lut_map, full_leader + 8 * j, 0,
                                      (int32_t)(it.n0 + rank * kHalfN), (int32_t)(2 * i));
-                    if (++j == SB) { j = 0; ph ^= 1; }
+                    j += kCopyWarps;
+                    if (j >= SB) { j -= SB; ph ^= 1; }
                 }
+                x0 += p.slabs;
             }
         }
         __syncwarp();
         if (p.early_trigger) pdl_launch_dependents();
     } else if (warp < kFirstBuilder) {
-        // ---------------- MMA issue, leader only.  Converged loop, one elected lane issues; whether the next slab's two
-        // slots are full is asked a turn ahead.
+        // ---------------- MMA issue, leader only: a warp per operand slot, so that it is waiting when the slot fills.
+        // Converged loop, one elected lane issues.
         if (rank == 0) {
-            const uint32_t me = warp - 1;
-            uint32_t j = me, pb = 0, t = 0, x0 = 0;   // LUT slot and phase of this warp's next slab; slabs before the item
+            const uint32_t me = warp - kFirstMma;
+            uint32_t j = me, pb = 0, t = 0, x0 = 0;   // LUT slot and phases of this warp's next slab; slabs before the item
             bool ok = true;
             const uint32_t b_lo0 = (uint32_t)umma_desc_k_sw128(smem_u32(s_b));
             const uint32_t desc_hi = (uint32_t)(umma_desc_k_sw128(0) >> 32);
-            bool ready = mbar_test2_cluster(b_full0 + 8 * j, pb, a_full0 + 8 * (me % kASlots), 0);
             for (uint32_t item = first; item < n_items && ok; item += n_pairs, ++t) {
                 const uint32_t ab = t & 1;
-                ok = mbar_wait_cluster(acc_empty0 + 8 * ab, ((t >> 1) & 1) ^ 1, s_abort);
+                ok = mbar_wait(acc_empty0 + 8 * ab, ((t >> 1) & 1) ^ 1, s_abort);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + ab * N_TILE;
-                for (uint32_t i = (x0 + me) & 1u; i < p.slabs; i += 2) {
+                for (uint32_t i = (me - x0) & (kMmaWarps - 1); i < p.slabs; i += kMmaWarps) {
                     const uint32_t x = x0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
-                    if (!ready) {
-                        ok = mbar_wait_cluster(b_full0 + 8 * j, pb, s_abort) && mbar_wait_cluster(a_full0 + 8 * k, pa, s_abort);
-                        if (!ok) break;
-                    }
-                    uint32_t j2 = j + 2, pb2 = pb;
-                    if (j2 >= SB) { j2 -= SB; pb2 ^= 1; }
-                    const uint32_t x2 = x + 2;
-                    const bool next_ready = mbar_test2_cluster(b_full0 + 8 * j2, pb2, a_full0 + 8 * (x2 % kASlots), (x2 / kASlots) & 1u);
+                    ok = mbar_wait(b_full0 + 8 * j, pb, s_abort) && mbar_wait(a_full0 + 8 * k, pa, s_abort);
+                    if (!ok) break;
                     tc_fence_after_sync();
                     if (elect_one()) {
                         const uint32_t b_lo = b_lo0 + j * (kBBytes >> 4);
@@ -215,13 +247,13 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                         for (uint32_t kk = 0; kk < 4; ++kk)   // 64 positions each: two per 128-byte swizzle row
                             umma_i8_sparse_pair(d_tmem, tmem_base + kDataBase + 32 * k + 8 * kk,
                                                 ((uint64_t)desc_hi << 32) | (b_lo + (kk >> 1) * (kHalfN * 128 >> 4) + (kk & 1) * 4),
-                                                tmem_base + kMetaBase + 8 * k + 2 * kk, kIdesc);
+                                                tmem_base + kMetaBase + 2 * k, kIdesc);
                         umma_commit_pair(a_empty0 + 8 * k);
                         umma_commit_pair(b_empty0 + 8 * j);
                     }
                     __syncwarp();
-                    j = j2; pb = pb2;
-                    ready = next_ready;
+                    j += kMmaWarps;
+                    if (j >= SB) { j -= SB; pb ^= 1; }
                 }
                 x0 += p.slabs;
                 if (ok && elect_one()) umma_commit_pair(acc_full0 + 8 * ab);
@@ -272,7 +304,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             if (i + kGroups < p.slabs) load_raw(row, i + kGroups, raw[1]);
             for (; i < p.slabs && ok; i += kGroups) {
                 const uint32_t x = x0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
-                uint32_t w[32], m[8];
+                uint32_t w[32], m[2];
                 build_row<LG>(raw[0], w, m);
 #pragma unroll
                 for (int c = 0; c < kRaw; ++c) raw[0][c] = raw[1][c];
@@ -281,7 +313,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                 if (!ok) break;
                 tc_fence_after_sync();
                 tmem_st_32x32b_x32(tmem_base + my_lanes + kDataBase + 32 * k, w);
-                tmem_st_32x32b_x8(tmem_base + my_lanes + kMetaBase + 8 * k, m);
+                tmem_st_32x32b_x2(tmem_base + my_lanes + kMetaBase + 2 * k, m);
                 tmem_st_wait();
                 tc_fence_before_sync();
                 __syncwarp();
@@ -293,12 +325,12 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     } else {
         // ---------------- epilogue: each warp on the lane quadrant it may read
         pdl_wait_prior_grid();
-        const uint32_t quad = warp & 3u;
+        const uint32_t quad = warp & 3u, half = 0;
         const float lbcb = lut_bias_times_cb(a.lut_bias, a.CB);
         unsigned char* stg = s_stage + (warp - kFirstEpi) * (kStages * kStageBytes);
         float* bw = s_bias + (warp - kFirstEpi) * N_TILE;
         const uint32_t empty_leader = map_to_rank(acc_empty0, 0);
-        uint32_t t = 0, buf = 0;
+        uint32_t t = 0;
         bool ok = true;
         for (uint32_t item = first; item < n_items; item += n_pairs, ++t) {
             const SparseItem it = sparse_item(p, item, N_TILE, rank);
@@ -306,7 +338,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             if (p.early_trigger && item + n_pairs >= n_items) pdl_launch_dependents();
             __syncwarp();   // the previous item's reads of bw are done
 #pragma unroll
-            for (uint32_t c = 0; c < N_TILE / 32; ++c) {
+            for (uint32_t c = 0; c < N_TILE / 32; c += 1) {
                 const uint32_t n = it.n0 + c * 32 + lane;
                 bw[c * 32 + lane] = n < a.N ? __ldg(a.bias + n) : 0.f;
             }
@@ -315,7 +347,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             ok = __shfl_sync(0xffffffffu, w_ok, 0) != 0;
             if (!ok) continue;
             tc_fence_after_sync();
-            for (uint32_t c = 0; c < N_TILE / 32; ++c) {
+            for (uint32_t c = 0; c < N_TILE / 32; c += 1) {
                 uint32_t v[32];
                 tmem_ld_32x32b_x32(tmem_base + my_lanes + ab * N_TILE + c * 32u, v);
                 tmem_ld_wait();
@@ -323,15 +355,15 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     const uint32_t zero[32] = {};
                     tmem_st_32x32b_x32(tmem_base + my_lanes + ab * N_TILE + c * 32u, zero);
                 }
-                if (c == N_TILE / 32 - 1) {   // accumulator fully read and cleared: hand the buffer back
+                if (c + 1 >= N_TILE / 32) {   // this warp's share is read and cleared
                     tmem_st_wait();
                     tc_fence_before_sync();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(empty_leader + 8 * ab);
                 }
                 if (it.n0 + c * 32 >= a.N || it.m0 + quad * 32 >= a.M) continue;   // a block wholly past N or M
-                unsigned char* sg = stg + buf * kStageBytes;
-                if (lane == 0) tma_store_wait_read_1();   // the copy before last has read this buffer
+                unsigned char* sg = stg;
+                if (lane == 0) tma_store_wait_read();   // the previous copy has read this buffer
                 __syncwarp();
 #pragma unroll
                 for (uint32_t q = 0; q < 8; ++q) {
@@ -347,7 +379,6 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     tma_store_2d(&out_map, smem_u32(sg), (int32_t)(it.n0 + c * 32), (int32_t)(it.m0 + quad * 32));
                     tma_store_commit();
                 }
-                buf ^= 1;
             }
         }
         if (lane == 0) tma_store_wait_all();   // shared memory and the output are settled before the CTA leaves
@@ -367,13 +398,15 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         __syncthreads();
     }
     cluster_sync();   // nothing of this CTA is read, written or signalled by the other one any more
-    if (warp == 1) {
+    if (warp == kFirstMma) {
         tc_fence_after_sync();
         tmem_dealloc_pair(tmem_base, 512);
     }
 }
 
 constexpr size_t kSmemLimit = 227 * 1024;
+
+uint32_t sparse_slabs(uint32_t CB, uint32_t CT) { return (uint32_t)(((uint64_t)CB * CT + kSlab - 1) / kSlab); }
 
 size_t sparse_smem(uint32_t n_tile, uint32_t b_slots) {
     return (size_t)b_slots * (n_tile / 2) * kSlab + kEpiWarps * kStages * kStageBytes + kEpiWarps * n_tile * 4 + kNumBarriers * 8 + 16 + 1024;
@@ -415,18 +448,54 @@ cudaError_t run_lg(uint32_t lg, const CUtensorMap& map, const CUtensorMap& out_m
 
 }  // namespace
 
-// LUT^T [N][CB*CT] as slabs of 256 positions: x = position within 128, y = row, z = position / 128; a box is half a
-// tile's rows of one slab.
-cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* lut_t, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile, const char** why) {
+size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N) { return (size_t)sparse_slabs(CB, CT) * kSlab * N; }
+
+// The table as the kernel above wants it: [N][slabs * 256], row n's slab s holding at position 2 (d * codebooks + c) + h
+// the entry of codebook s * codebooks + c and centroid index (d without its bit 1, h = bit 1); positions of codebooks
+// past the last one are zero.  A block turns 256 rows x 64 columns of the canonical table.
+namespace {
+__global__ void __launch_bounds__(256) sparse_table_kernel(const int8_t* __restrict__ lut, int8_t* __restrict__ out, uint32_t rows, uint32_t N,
+                                                           uint32_t lg, uint32_t slabs) {
+    constexpr uint32_t kPitch = 260;
+    __shared__ __align__(4) int8_t tile[64 * kPitch];
+    const uint32_t slab = blockIdx.x, n0 = blockIdx.y * 64, lg_cbs = 8 - lg;
+    for (uint32_t e = threadIdx.x; e < 256 * 16; e += 256) {
+        const uint32_t r = e >> 4, n = (e & 15u) * 4, i = r & ((1u << lg) - 1u), c = r >> lg;
+        const uint32_t d = ((i >> 2) << 1) | (i & 1u), pos = 2 * ((d << lg_cbs) + c) + ((i >> 1) & 1u);
+        const size_t row = (size_t)slab * 256 + r;
+        uint32_t v = 0;
+        if (row < rows && n0 + n < N) v = *reinterpret_cast<const uint32_t*>(lut + row * N + n0 + n);   // N % 16 == 0
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) tile[(n + k) * kPitch + pos] = (int8_t)(v >> (8 * k));
+    }
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < 64 * 64; e += 256) {
+        const uint32_t n = e >> 6, w = e & 63u;
+        if (n0 + n < N)
+            *reinterpret_cast<uint32_t*>(out + ((size_t)(n0 + n) * slabs + slab) * 256 + 4 * w) = *reinterpret_cast<const uint32_t*>(tile + n * kPitch + 4 * w);
+    }
+}
+}  // namespace
+
+cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t N, cudaStream_t s) {
+    uint32_t lg = 0;
+    while ((1u << lg) < CT) ++lg;
+    const uint32_t slabs = sparse_slabs(CB, CT);
+    sparse_table_kernel<<<dim3(slabs, (N + 63) / 64), 256, 0, s>>>(lut, out, CB * CT, N, lg, slabs);
+    return cudaGetLastError();
+}
+
+// That table as boxes of half a tile's rows of one slab: x = position within 128, y = row, z = half slab.
+cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile, const char** why) {
     *why = nullptr;
     EncodeTiledFn enc = get_encode_tiled();
     if (!enc) { *why = "cuTensorMapEncodeTiled is not available from this driver"; return cudaErrorNotSupported; }
-    const uint64_t Kg = (uint64_t)CB * CT;
-    cuuint64_t dims[3] = {128, N, Kg / 128};
-    cuuint64_t strides[2] = {Kg, 128};
+    const uint64_t row = (uint64_t)sparse_slabs(CB, CT) * kSlab;
+    cuuint64_t dims[3] = {128, N, row / 128};
+    cuuint64_t strides[2] = {row, 128};
     cuuint32_t box[3] = {128, n_tile / 2, 2};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t*>(lut_t), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t*>(table), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the LUT slab map"; return cudaErrorInvalidValue; }
     return cudaSuccess;
@@ -438,12 +507,12 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, uint32_t
     if (reinterpret_cast<uintptr_t>(a.idx) & 15u) { *why = "tcgen05 variant: the index buffer must be 16-byte aligned"; return cudaErrorInvalidValue; }
     SparseParams p;
     p.a = a;
-    p.slabs = (uint32_t)(((uint64_t)a.CB * a.CT + kSlab - 1) / kSlab);
+    p.slabs = sparse_slabs(a.CB, a.CT);
     p.tiles_m = (a.M + 2 * kRows - 1) / (2 * kRows);
     p.tiles_n = (a.N + n_tile - 1) / n_tile;
     p.dev_err = dev_err;
     p.b_slots = kMaxBSlots;
-    while (p.b_slots > 2 && sparse_smem(n_tile, p.b_slots) > kSmemLimit) p.b_slots -= 2;
+    while (p.b_slots > 4 && sparse_smem(n_tile, p.b_slots) > kSmemLimit) p.b_slots -= 4;
     const uint64_t items = (uint64_t)p.tiles_m * p.tiles_n;
     const uint32_t cap = max_ctas / 2, pairs = (uint32_t)(items < cap ? items : cap);
     p.early_trigger = items <= cap;

@@ -46,6 +46,7 @@ struct Layer {
     uint32_t K = 0, v = 0, CB = 0, CT = 0, N = 0;
     float* d_centroid = nullptr;
     int8_t* d_lut = nullptr;    // canonical [CB][CT][N]
+    int8_t* d_lut_s = nullptr;  // sparse_table layout, made on first use
     int8_t* d_lut_t = nullptr;  // [N][CB*CT], made on first use of the tcgen05 variant
     float* d_bias = nullptr;
     lutamm_plan plan{};
@@ -168,6 +169,7 @@ void free_layer(Layer& L) {
     cudaFree(L.d_centroid);
     cudaFree(L.d_lut);
     cudaFree(L.d_lut_t);
+    cudaFree(L.d_lut_s);
     cudaFree(L.d_bias);
     L = Layer{};
 }
@@ -252,9 +254,13 @@ int run_lut(lutamm_ctx* c, Layer& L, const uint8_t* d_idx, float* d_out, int32_t
         }
         static const int force = getenv("LUTAMM_SPARSE") ? atoi(getenv("LUTAMM_SPARSE")) : 0;
         if (force && !a.n_peers && !a.acc_out && !a.layout.tiled) {
-            static std::map<const void*, CUtensorMap> maps;
+            if (!L.d_lut_s) {
+                CU_TRY(c, cudaMalloc(&L.d_lut_s, sparse_table_bytes(L.CB, L.CT, L.N)));
+                CU_TRY(c, launch_sparse_table(L.d_lut, L.d_lut_s, L.CB, L.CT, L.N, c->stream));
+                CU_TRY(c, cudaStreamSynchronize(c->stream));
+            }
             CUtensorMap m;
-            cudaError_t e = sparse_make_tmap(&m, L.d_lut_t, L.CB, L.CT, L.N, force, &why);
+            cudaError_t e = sparse_make_tmap(&m, L.d_lut_s, L.CB, L.CT, L.N, force, &why);
             if (e == cudaSuccess) e = launch_sparse(a, m, force, c->sm_count, c->d_err, c->stream, &why);
             if (e != cudaSuccess) return fail(c, LUTAMM_ECUDA, why ? why : cudaGetErrorString(e));
             ++c->launches;

@@ -215,12 +215,9 @@ __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// 32 lanes x 8 columns
-__device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-        : "memory");
+// 32 lanes x 2 columns
+__device__ __forceinline__ void tmem_st_32x32b_x2(uint32_t taddr, const uint32_t (&r)[2]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(r[0]), "r"(r[1]) : "memory");
 }
 
 // ---------------------------------------------------------------- CTA pairs (cta_group::2)
@@ -241,41 +238,11 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
+// Arrive on a barrier of either CTA.  The scope stays .cta on purpose: what is handed over lies in tensor memory and is
+// ordered by the tcgen05 fences around the barrier; .release.cluster would make the thread wait for all its memory
+// operations (the index loads in flight), which doubled a builder's turn.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// Waits whose arrivals may come from the other CTA of the pair.
-__device__ __forceinline__ bool mbar_test_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile uint32_t* abort_word) {
-    for (uint32_t it = 0; it < kWaitLimit; ++it) {
-        if (mbar_test_cluster(bar, parity)) return true;
-        if ((it & 63u) == 0u && *abort_word) return false;
-    }
-    *abort_word = 1u;
-    return false;
-}
-__device__ __forceinline__ bool mbar_test2_cluster(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred q0, q1;\n\t"
-        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 q0, [%1], %2;\n\t"
-        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 q1, [%3], %4;\n\t"
-        "and.pred q0, q0, q1;\n\t"
-        "selp.u32 %0, 1, 0, q0;\n\t}"
-        : "=r"(ok)
-        : "r"(b0), "r"(p0), "r"(b1), "r"(p1)
-        : "memory");
-    return ok != 0;
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Tiled load into this CTA's shared memory whose bytes are counted on a barrier of either CTA of the pair.
 __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* m, uint32_t cluster_bar, int32_t x, int32_t y, int32_t z) {
@@ -293,7 +260,7 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 }
 // D += A * B with A 2:4 sparse: 32 stored bytes a row in tensor memory for 64 of the contraction axis, beside them
 // (meta) a nibble per four of the axis - row = lane, 16 nibbles = two 32-bit columns - that names the two positions
-// the stored bytes 2g, 2g+1 of group g stand for: 0x4 the first two, 0xE the last two.
+// the stored bytes 2g, 2g+1 of group g stand for: low two bits for the first, high two for the second, ascending.
 __device__ __forceinline__ void umma_i8_sparse_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t meta, uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
