@@ -27,14 +27,19 @@ namespace {
 
 constexpr uint32_t kRows = 128;                // rows of a CTA: half a tile
 constexpr uint32_t kSlab = 256;                // positions of the contraction axis per ring slot
-constexpr uint32_t kGroups = 4, kCopyWarps = 2, kMmaWarps = 4, kEpiWarps = 4;
-constexpr uint32_t kFirstMma = kCopyWarps, kFirstBuilder = kFirstMma + kMmaWarps, kFirstEpi = kFirstBuilder + 4 * kGroups;
-constexpr uint32_t kThreads = (kFirstEpi + kEpiWarps) * 32;   // 832
+constexpr uint32_t kGroups = 4, kCopyWarps = 2, kIndexWarps = 1, kMmaWarps = 4, kEpiWarps = 4;
+constexpr uint32_t kFirstMma = kCopyWarps + kIndexWarps, kFirstBuilder = kFirstMma + kMmaWarps, kFirstEpi = kFirstBuilder + 4 * kGroups;
+constexpr uint32_t kThreads = (kFirstEpi + kEpiWarps) * 32;   // 864
 constexpr uint32_t kASlots = 4;                // operand slots: 32 columns of bytes and 2 of metadata each
 constexpr uint32_t kMaxBSlots = 16;
 constexpr uint32_t kStageBytes = 32 * 128;     // a 32 x 32 fp32 block
-constexpr uint32_t kStages = 1;                // per epilogue warp
-constexpr uint32_t kNumBarriers = 2 * kASlots + 2 * kMaxBSlots + 4;
+constexpr uint32_t kStages = 2;                // per epilogue warp
+constexpr uint32_t kIdxStages = 3;
+constexpr uint32_t kNumBarriers = 2 * kASlots + 2 * kMaxBSlots + 4 + 2 * kIdxStages;
+
+// A stage of index bytes: 128 rows of `idx_width` bytes, for `idx_slabs` slabs.
+__host__ __device__ constexpr uint32_t idx_width(int lg) { return lg == 3 ? 64u : lg <= 6 ? 4u * (256u >> lg) : 16u; }
+__host__ __device__ constexpr uint32_t idx_slabs(int lg) { return (idx_width(lg) << lg) / kSlab; }
 
 struct SparseParams {
     LutArgs a;
@@ -147,23 +152,28 @@ __device__ __forceinline__ SparseItem sparse_item(const SparseParams& p, uint32_
 
 template <uint32_t N_TILE, int LG>
 __global__ void __launch_bounds__(kThreads, 1)
-lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_constant__ CUtensorMap out_map, const SparseParams p) {
+lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_constant__ CUtensorMap idx_map,
+                  const __grid_constant__ CUtensorMap out_map, const SparseParams p) {
     constexpr uint32_t kHalfN = N_TILE / 2, kBBytes = kHalfN * kSlab;
     constexpr uint32_t kIdesc = umma_idesc_i8(2 * kRows, N_TILE, 1, 1) | kIdescSparse;
     constexpr uint32_t kDataBase = 2 * N_TILE, kMetaBase = kDataBase + 32 * kASlots;   // tensor-memory columns
     static_assert(kMetaBase + 2 * kASlots <= 512, "tensor memory");
+
+    constexpr uint32_t kIdxWidth = idx_width(LG), kIdxSlabs = idx_slabs(LG), kIdxBytes = kRows * kIdxWidth;
 
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const uint32_t SB = p.b_slots;
     unsigned char* s_b = smem;                                        // [SB][2][kHalfN][128]
     unsigned char* s_stage = s_b + (size_t)SB * kBBytes;              // [4][kStages][32][128]
-    float* s_bias = reinterpret_cast<float*>(s_stage + kEpiWarps * kStages * kStageBytes);   // [4][N_TILE]
+    unsigned char* s_idx = s_stage + kEpiWarps * kStages * kStageBytes;   // [kIdxStages][128][idx_width]
+    float* s_bias = reinterpret_cast<float*>(s_idx + kIdxStages * kIdxBytes);   // [4][N_TILE]
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_bias + kEpiWarps * N_TILE);
     uint32_t* s_misc = reinterpret_cast<uint32_t*>(s_bar + kNumBarriers);                  // tmem base, abort
     volatile uint32_t* s_abort = s_misc + 1;
     const uint32_t a_full0 = smem_u32(s_bar), a_empty0 = a_full0 + 8 * kASlots, b_full0 = a_empty0 + 8 * kASlots,
-                   b_empty0 = b_full0 + 8 * kMaxBSlots, acc_full0 = b_empty0 + 8 * kMaxBSlots, acc_empty0 = acc_full0 + 16;
+                   b_empty0 = b_full0 + 8 * kMaxBSlots, acc_full0 = b_empty0 + 8 * kMaxBSlots, acc_empty0 = acc_full0 + 16,
+                   i_full0 = acc_empty0 + 16, i_empty0 = i_full0 + 8 * kIdxStages;
 
     const LutArgs& a = p.a;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = cluster_rank();
@@ -172,15 +182,17 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     if (threadIdx.x == 0) {
         s_misc[1] = 0;
         tma_prefetch_desc(&lut_map);
+        tma_prefetch_desc(&idx_map);
         tma_prefetch_desc(&out_map);
     }
     if (threadIdx.x >= 64 && threadIdx.x < 64 + kNumBarriers) {
         const uint32_t b = threadIdx.x - 64;
         // a_full: the four builder warps of the slab's group in each CTA; a_empty, b_empty: one commit; b_full: the
         // leader's expect_tx (the copies of both CTAs complete the bytes); acc_full: one commit per issuing warp;
-        // acc_empty: the epilogue warps of both CTAs.  Barriers the leader waits on are unused in the other CTA.
+        // acc_empty: the epilogue warps of both CTAs (barriers the
+        // leader waits on are unused in the other CTA); i_full: expect_tx; i_empty: the CTA's builder warps.
         const uint32_t after = 2 * kASlots + 2 * kMaxBSlots;
-        mbar_init(a_full0 + 8 * b, b < kASlots ? 8u : b < after ? 1u : b < after + 2 ? kMmaWarps : 2 * kEpiWarps);
+        mbar_init(a_full0 + 8 * b, b < kASlots ? 8u : b < after ? 1u : b < after + 2 ? kMmaWarps : b < after + 4 ? 2 * kEpiWarps : b < after + 4 + kIdxStages ? 1u : 4 * kGroups);
         fence_barrier_init();
     }
     if (warp == kFirstMma) tmem_alloc_pair(smem_u32(s_misc), 512);
@@ -198,7 +210,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     cluster_sync();   // barriers initialised and accumulators cleared in both CTAs
     tc_fence_after_sync();
 
-    if (warp < kFirstMma) {
+    if (warp < kCopyWarps) {
         // ---------------- LUT copies (the LUT never depends on the preceding kernel), slab x by warp x % kCopyWarps: a
         // thread sustains one copy per ~ 480 cycles, of which the instruction itself holds it for 350
         if (lane == 0) {
@@ -217,6 +229,26 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     if (j >= SB) { j -= SB; ph ^= 1; }
                 }
                 x0 += p.slabs;
+            }
+        }
+        __syncwarp();
+        if (p.early_trigger) pdl_launch_dependents();
+    } else if (warp < kFirstMma) {
+        // ---------------- index copies.  Straight loads by the builders, 16 bytes of a row each, were what a builder
+        // waited for: beside the slabs an L2 access takes 1.5 us and more, and half of each sector was not used.
+        pdl_wait_prior_grid();
+        if (lane == 0) {
+            uint32_t st = 0, ph = 0;
+            bool ok = true;
+            for (uint32_t item = first; item < n_items && ok; item += n_pairs) {
+                const SparseItem it = sparse_item(p, item, N_TILE, rank);
+                for (uint32_t i = 0; i < p.slabs; i += kIdxSlabs) {
+                    ok = mbar_wait<32>(i_empty0 + 8 * st, ph ^ 1, s_abort);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(i_full0 + 8 * st, kIdxBytes);
+                    tma_load_2d(smem_u32(s_idx + st * kIdxBytes), &idx_map, i_full0 + 8 * st, (int32_t)(i * (kSlab >> LG)), (int32_t)it.m0);
+                    if (++st == kIdxStages) { st = 0; ph ^= 1; }
+                }
             }
         }
         __syncwarp();
@@ -264,60 +296,58 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         if (p.early_trigger) pdl_launch_dependents();
     } else if (warp < kFirstEpi) {
         // ---------------- operand builders: slab x of the CTA's sequence by group x % 4, into slot x % 4
-        pdl_wait_prior_grid();
         constexpr int kRaw = LG == 3 ? 8 : 4;
         const uint32_t grp = (warp - kFirstBuilder) >> 2, r = (warp & 3u) * 32 + lane;
-        const uint32_t row_bytes = a.CB;
-        // 256 / CT index bytes; L2 (under programmatic launch this SM's L1 may hold older lines)
-        auto load_raw = [&](const uint8_t* row, uint32_t slab, uint32_t (&v)[kRaw]) {
-            const uint8_t* q = row + ((slab * kSlab) >> LG);
+        // the 256 / CT index bytes of slab `sub` of a stage; 64-byte rows are swizzled
+        auto load_raw = [&](const unsigned char* st, uint32_t sub, uint32_t (&v)[kRaw]) {
+            const unsigned char* row = st + r * kIdxWidth;
             if constexpr (LG == 3) {
-                const uint4 t = __ldcg(reinterpret_cast<const uint4*>(q));
-                v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-                // an odd multiple of 16 codebooks ends in half a slab
-                uint4 u = make_uint4(~0u, ~0u, ~0u, ~0u);
-                if ((slab * kSlab >> LG) + 16 < row_bytes) u = __ldcg(reinterpret_cast<const uint4*>(q) + 1);
-                v[4] = u.x; v[5] = u.y; v[6] = u.z; v[7] = u.w;
+                const uint4 t = *reinterpret_cast<const uint4*>(row + (((2 * sub) ^ ((r >> 1) & 3u)) << 4));
+                const uint4 u = *reinterpret_cast<const uint4*>(row + (((2 * sub + 1) ^ ((r >> 1) & 3u)) << 4));
+                v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w; v[4] = u.x; v[5] = u.y; v[6] = u.z; v[7] = u.w;
             } else if constexpr (LG == 4) {
-                const uint4 t = __ldcg(reinterpret_cast<const uint4*>(q));
+                const uint4 t = *reinterpret_cast<const uint4*>(row + ((sub ^ ((r >> 1) & 3u)) << 4));
                 v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
             } else if constexpr (LG == 5) {
-                const uint2 t = __ldcg(reinterpret_cast<const uint2*>(q));
+                const uint2 t = *reinterpret_cast<const uint2*>(row + 8 * sub);
                 v[0] = t.x; v[1] = t.y;
             } else if constexpr (LG == 6) {
-                v[0] = __ldcg(reinterpret_cast<const uint32_t*>(q));
+                v[0] = *reinterpret_cast<const uint32_t*>(row + 4 * sub);
             } else if constexpr (LG == 7) {
-                v[0] = __ldcg(reinterpret_cast<const uint16_t*>(q));
+                v[0] = *reinterpret_cast<const uint16_t*>(row + 2 * sub);
             } else {
-                v[0] = __ldcg(q);
+                v[0] = row[sub];
             }
         };
         const uint32_t full_leader = map_to_rank(a_full0, 0);
-        uint32_t x0 = 0;
+        uint32_t x0 = 0, st = 0, ph = 0;
         bool ok = true;
         for (uint32_t item = first; item < n_items && ok; item += n_pairs) {
-            const SparseItem it = sparse_item(p, item, N_TILE, rank);
-            const uint8_t* row = a.idx + (size_t)min(it.m0 + r, a.M - 1) * a.CB;   // rows past M: clipped by the epilogue
-            uint32_t i = (grp - x0) & (kGroups - 1);
-            uint32_t raw[2][kRaw];   // index bytes are fetched two turns ahead
-            if (i < p.slabs) load_raw(row, i, raw[0]);
-            if (i + kGroups < p.slabs) load_raw(row, i + kGroups, raw[1]);
-            for (; i < p.slabs && ok; i += kGroups) {
-                const uint32_t x = x0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
-                uint32_t w[32], m[2];
-                build_row<LG>(raw[0], w, m);
+            for (uint32_t i0 = 0; i0 < p.slabs && ok; i0 += kIdxSlabs) {
+                ok = mbar_wait(i_full0 + 8 * st, ph, s_abort);
+                for (uint32_t i = (grp - (x0 + i0)) & (kGroups - 1); i < kIdxSlabs && i0 + i < p.slabs && ok; i += kGroups) {
+                    const uint32_t x = x0 + i0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
+                    uint32_t raw[kRaw], w[32], m[2];
+                    load_raw(s_idx + st * kIdxBytes, i, raw);
+                    build_row<LG>(raw, w, m);
+                    // the row is in registers before the slot is waited for (the compiler would sink it behind the wait,
+                    // onto the slot's turn-around path)
 #pragma unroll
-                for (int c = 0; c < kRaw; ++c) raw[0][c] = raw[1][c];
-                if (i + 2 * kGroups < p.slabs) load_raw(row, i + 2 * kGroups, raw[1]);
-                ok = mbar_wait(a_empty0 + 8 * k, pa ^ 1, s_abort);
-                if (!ok) break;
-                tc_fence_after_sync();
-                tmem_st_32x32b_x32(tmem_base + my_lanes + kDataBase + 32 * k, w);
-                tmem_st_32x32b_x2(tmem_base + my_lanes + kMetaBase + 2 * k, m);
-                tmem_st_wait();
-                tc_fence_before_sync();
+                    for (int c = 0; c < 32; ++c) asm volatile("" : "+r"(w[c]));
+                    asm volatile("" : "+r"(m[0]), "+r"(m[1]));
+                    ok = mbar_wait(a_empty0 + 8 * k, pa ^ 1, s_abort);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    tmem_st_32x32b_x32(tmem_base + my_lanes + kDataBase + 32 * k, w);
+                    tmem_st_32x32b_x2(tmem_base + my_lanes + kMetaBase + 2 * k, m);
+                    tmem_st_wait();
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(full_leader + 8 * k);
+                }
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(full_leader + 8 * k);
+                if (lane == 0) mbar_arrive(i_empty0 + 8 * st);   // this warp has read its rows of the stage
+                if (++st == kIdxStages) { st = 0; ph ^= 1; }
             }
             x0 += p.slabs;
         }
@@ -325,12 +355,12 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     } else {
         // ---------------- epilogue: each warp on the lane quadrant it may read
         pdl_wait_prior_grid();
-        const uint32_t quad = warp & 3u, half = 0;
+        const uint32_t quad = warp & 3u;
         const float lbcb = lut_bias_times_cb(a.lut_bias, a.CB);
         unsigned char* stg = s_stage + (warp - kFirstEpi) * (kStages * kStageBytes);
         float* bw = s_bias + (warp - kFirstEpi) * N_TILE;
         const uint32_t empty_leader = map_to_rank(acc_empty0, 0);
-        uint32_t t = 0;
+        uint32_t t = 0, buf = 0;
         bool ok = true;
         for (uint32_t item = first; item < n_items; item += n_pairs, ++t) {
             const SparseItem it = sparse_item(p, item, N_TILE, rank);
@@ -338,7 +368,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             if (p.early_trigger && item + n_pairs >= n_items) pdl_launch_dependents();
             __syncwarp();   // the previous item's reads of bw are done
 #pragma unroll
-            for (uint32_t c = 0; c < N_TILE / 32; c += 1) {
+            for (uint32_t c = 0; c < N_TILE / 32; ++c) {
                 const uint32_t n = it.n0 + c * 32 + lane;
                 bw[c * 32 + lane] = n < a.N ? __ldg(a.bias + n) : 0.f;
             }
@@ -347,7 +377,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             ok = __shfl_sync(0xffffffffu, w_ok, 0) != 0;
             if (!ok) continue;
             tc_fence_after_sync();
-            for (uint32_t c = 0; c < N_TILE / 32; c += 1) {
+            for (uint32_t c = 0; c < N_TILE / 32; ++c) {
                 uint32_t v[32];
                 tmem_ld_32x32b_x32(tmem_base + my_lanes + ab * N_TILE + c * 32u, v);
                 tmem_ld_wait();
@@ -355,30 +385,40 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     const uint32_t zero[32] = {};
                     tmem_st_32x32b_x32(tmem_base + my_lanes + ab * N_TILE + c * 32u, zero);
                 }
-                if (c + 1 >= N_TILE / 32) {   // this warp's share is read and cleared
+                if (c == N_TILE / 32 - 1) {   // accumulator fully read and cleared: hand the buffer back
                     tmem_st_wait();
                     tc_fence_before_sync();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(empty_leader + 8 * ab);
                 }
                 if (it.n0 + c * 32 >= a.N || it.m0 + quad * 32 >= a.M) continue;   // a block wholly past N or M
-                unsigned char* sg = stg;
-                if (lane == 0) tma_store_wait_read();   // the previous copy has read this buffer
+                unsigned char* sg = stg + buf * kStageBytes;
+                if (lane == 0) tma_store_wait_read_1();   // the copy before last has read this buffer
                 __syncwarp();
+                // straight-line code for all 32 columns: a branch per value leaves every latency of a lone warp exposed
+                float o[32];
 #pragma unroll
                 for (uint32_t q = 0; q < 8; ++q) {
                     const float4 b4 = *reinterpret_cast<const float4*>(bw + c * 32 + 4 * q);
-                    float4 o = make_float4(dequant_one((int32_t)v[4 * q], a.scale, lbcb, b4.x), dequant_one((int32_t)v[4 * q + 1], a.scale, lbcb, b4.y),
-                                           dequant_one((int32_t)v[4 * q + 2], a.scale, lbcb, b4.z), dequant_one((int32_t)v[4 * q + 3], a.scale, lbcb, b4.w));
-                    if (a.act) { o.x = activate_one(o.x, a.act); o.y = activate_one(o.y, a.act); o.z = activate_one(o.z, a.act); o.w = activate_one(o.w, a.act); }
-                    *reinterpret_cast<float4*>(sg + lane * 128 + ((q ^ (lane & 7u)) << 4)) = o;
+                    o[4 * q] = dequant_one((int32_t)v[4 * q], a.scale, lbcb, b4.x);
+                    o[4 * q + 1] = dequant_one((int32_t)v[4 * q + 1], a.scale, lbcb, b4.y);
+                    o[4 * q + 2] = dequant_one((int32_t)v[4 * q + 2], a.scale, lbcb, b4.z);
+                    o[4 * q + 3] = dequant_one((int32_t)v[4 * q + 3], a.scale, lbcb, b4.w);
                 }
+                if (a.act) {
+#pragma unroll
+                    for (uint32_t q = 0; q < 32; ++q) o[q] = activate_one(o[q], a.act);
+                }
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)
+                    *reinterpret_cast<float4*>(sg + lane * 128 + ((q ^ (lane & 7u)) << 4)) = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
                     tma_store_2d(&out_map, smem_u32(sg), (int32_t)(it.n0 + c * 32), (int32_t)(it.m0 + quad * 32));
                     tma_store_commit();
                 }
+                buf ^= 1;
             }
         }
         if (lane == 0) tma_store_wait_all();   // shared memory and the output are settled before the CTA leaves
@@ -408,12 +448,13 @@ constexpr size_t kSmemLimit = 227 * 1024;
 
 uint32_t sparse_slabs(uint32_t CB, uint32_t CT) { return (uint32_t)(((uint64_t)CB * CT + kSlab - 1) / kSlab); }
 
-size_t sparse_smem(uint32_t n_tile, uint32_t b_slots) {
-    return (size_t)b_slots * (n_tile / 2) * kSlab + kEpiWarps * kStages * kStageBytes + kEpiWarps * n_tile * 4 + kNumBarriers * 8 + 16 + 1024;
+size_t sparse_smem(uint32_t n_tile, int lg, uint32_t b_slots) {
+    return (size_t)b_slots * (n_tile / 2) * kSlab + kEpiWarps * kStages * kStageBytes + kIdxStages * kRows * idx_width(lg) +
+           kEpiWarps * n_tile * 4 + kNumBarriers * 8 + 16 + 1024;
 }
 
 template <uint32_t N_TILE, int LG>
-cudaError_t run(const CUtensorMap& map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
+cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
     auto k = lut_sparse_kernel<N_TILE, LG>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -431,18 +472,18 @@ cudaError_t run(const CUtensorMap& map, const CUtensorMap& out_map, const Sparse
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, k, map, out_map, p);
+    return cudaLaunchKernelEx(&cfg, k, map, idx_map, out_map, p);
 }
 
 template <uint32_t N_TILE>
-cudaError_t run_lg(uint32_t lg, const CUtensorMap& map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
+cudaError_t run_lg(uint32_t lg, const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
     switch (lg) {
-        case 3: return run<N_TILE, 3>(map, out_map, p, pairs, smem, s);
-        case 4: return run<N_TILE, 4>(map, out_map, p, pairs, smem, s);
-        case 5: return run<N_TILE, 5>(map, out_map, p, pairs, smem, s);
-        case 6: return run<N_TILE, 6>(map, out_map, p, pairs, smem, s);
-        case 7: return run<N_TILE, 7>(map, out_map, p, pairs, smem, s);
-        default: return run<N_TILE, 8>(map, out_map, p, pairs, smem, s);
+        case 3: return run<N_TILE, 3>(map, idx_map, out_map, p, pairs, smem, s);
+        case 4: return run<N_TILE, 4>(map, idx_map, out_map, p, pairs, smem, s);
+        case 5: return run<N_TILE, 5>(map, idx_map, out_map, p, pairs, smem, s);
+        case 6: return run<N_TILE, 6>(map, idx_map, out_map, p, pairs, smem, s);
+        case 7: return run<N_TILE, 7>(map, idx_map, out_map, p, pairs, smem, s);
+        default: return run<N_TILE, 8>(map, idx_map, out_map, p, pairs, smem, s);
     }
 }
 
@@ -501,6 +542,21 @@ cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB,
     return cudaSuccess;
 }
 
+// uint8 indices [M][CB] as 128 rows x `width` bytes
+static cudaError_t make_idx_tmap(CUtensorMap* out, const uint8_t* idx, uint32_t M, uint32_t CB, uint32_t width, const char** why) {
+    EncodeTiledFn enc = get_encode_tiled();
+    if (!enc) { *why = "cuTensorMapEncodeTiled is not available from this driver"; return cudaErrorNotSupported; }
+    cuuint64_t dims[2] = {CB, M};
+    cuuint64_t strides[1] = {CB};
+    cuuint32_t box[2] = {width, kRows};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(idx), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     width == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                     CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the index map"; return cudaErrorInvalidValue; }
+    return cudaSuccess;
+}
+
 cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, uint32_t n_tile, uint32_t max_ctas, uint32_t* dev_err, cudaStream_t s, const char** why) {
     *why = nullptr;
     if (a.M == 0 || a.N == 0) return cudaSuccess;
@@ -511,18 +567,20 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, uint32_t
     p.tiles_m = (a.M + 2 * kRows - 1) / (2 * kRows);
     p.tiles_n = (a.N + n_tile - 1) / n_tile;
     p.dev_err = dev_err;
+    int lg = 0;
+    while ((1u << lg) < a.CT) ++lg;
     p.b_slots = kMaxBSlots;
-    while (p.b_slots > 4 && sparse_smem(n_tile, p.b_slots) > kSmemLimit) p.b_slots -= 4;
+    while (p.b_slots > 4 && sparse_smem(n_tile, lg, p.b_slots) > kSmemLimit) p.b_slots -= 4;
     const uint64_t items = (uint64_t)p.tiles_m * p.tiles_n;
     const uint32_t cap = max_ctas / 2, pairs = (uint32_t)(items < cap ? items : cap);
     p.early_trigger = items <= cap;
-    uint32_t lg = 0;
-    while ((1u << lg) < a.CT) ++lg;
-    CUtensorMap om;
+    CUtensorMap om, im;
     cudaError_t e = make_out_tmap(&om, a.out, a.M, a.N, why);
     if (e != cudaSuccess) return e;
-    size_t smem = sparse_smem(n_tile, p.b_slots);
-    if (n_tile == 160) return run_lg<160>(lg, lut_map, om, p, pairs, smem, s);
+    e = make_idx_tmap(&im, a.idx, a.M, a.CB, idx_width(lg), why);
+    if (e != cudaSuccess) return e;
+    const size_t smem = sparse_smem(n_tile, lg, p.b_slots);
+    if (n_tile == 160) return run_lg<160>(lg, lut_map, im, om, p, pairs, smem, s);
     *why = "tcgen05 variant: this tile is not built";
     return cudaErrorInvalidValue;
 }
