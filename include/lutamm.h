@@ -109,7 +109,11 @@ typedef struct lutamm_plan {
     uint32_t umma_stages;     /* tcgen05: LUT slabs in flight in shared memory (0 = as many as fit) */
     uint32_t umma_groups;     /* tcgen05 one-hot builder groups of 4 warps (0 = default)  */
     uint32_t umma_operand;    /* where the one-hot operand lives: 0 = default,
-                                 1 = shared memory, 2 = tensor memory (TMEM)             */
+                                 1 = shared memory, 2 = tensor memory (TMEM), 3 = tensor memory in the 2:4
+                                 sparse form, on CTA pairs (umma_n_tile 0, 64, 128 or 160; the other
+                                 fields below are the dense kernel's and ignored).  A plan that leaves
+                                 all umma_ fields 0 takes form 3 wherever it applies: row-major output,
+                                 no peer stores, no int32 copy                            */
     uint32_t umma_sps;        /* tcgen05: 128-byte slabs of the codebook axis a one-hot builder
                                  group takes per turn, 1 or 2 (0 = default; 4 is read as 2)  */
     uint32_t umma_epilogue;   /* tcgen05: how a finished tile leaves the SM.  LUTAMM_EPILOGUE_TRANSPOSE: through a

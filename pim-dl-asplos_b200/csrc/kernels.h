@@ -81,13 +81,17 @@ uint32_t umma_auto_split(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, uint3
 // fp32 [M][N] row-major output as 32 x 32 blocks with the 128-byte swizzle the epilogues stage them in
 cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N, const char** why);
 
-// The same contraction on CTA pairs with the one-hot operand 2:4 sparse (row-major fp32 output).
+// The same contraction on CTA pairs with the one-hot operand 2:4 sparse (row-major fp32 output): from its own layout of
+// the table (sparse_table_bytes of it), at twice the rate.
 size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N);
 cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t N, cudaStream_t s);
+uint32_t sparse_default_tile(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count);
+bool sparse_tile_ok(uint32_t n_tile);
 cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile,
                              const char** why);
-cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, uint32_t n_tile, uint32_t max_ctas, uint32_t* dev_err,
-                          cudaStream_t s, const char** why);
+cudaError_t sparse_make_idx_tmap(CUtensorMap* out, const uint8_t* idx, uint32_t M, uint32_t CB, uint32_t CT, const char** why);
+cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CUtensorMap& idx_map, const CUtensorMap& out_map, uint32_t n_tile,
+                          uint32_t max_ctas, uint32_t* dev_err, cudaStream_t s, const char** why);
 
 // LUT [CB*CT][N] -> [N][CB*CT]
 cudaError_t launch_transpose_lut(const int8_t* lut, int8_t* lut_t, uint32_t rows, uint32_t cols, cudaStream_t s);

@@ -11,12 +11,13 @@
 //
 // Otherwise the structure of the dense kernel: persistent, one pair per two SMs walking 256-token x N_TILE items,
 // accumulators double-buffered in tensor memory, every slot of both rings with one producer and one consumer.  Per CTA:
-//   warp 0        copies its half of a LUT slab (N_TILE/2 rows x 256 bytes); bytes count on the leader's barrier
-//   warps 1-4     leader only: four tcgen05.mma.sp per slab, slab x by warp 1 + x % 4
-//   warps 5-20    four groups of four warps: the operand of the CTA's 128 rows, straight from the uint8 indices;
-//                 group k takes every fourth slab, one row per thread.  The stored bytes come from shifts, not from a
-//                 table in shared memory, whose bandwidth the slabs use up
-//   warps 21-24   epilogue: tcgen05.ld, dequantise, swizzled staging, tiled bulk stores; clears the accumulator
+//   warps 0-1     copy the CTA's half of a LUT slab (N_TILE/2 rows x 256 bytes); bytes count on the leader's barrier
+//   warp 2        copies the index bytes of the CTA's rows, a few slabs at a time
+//   warps 3-6     leader only: four tcgen05.mma.sp per slab, slab x by warp 3 + x % 4
+//   warps 7-22    four groups of four warps: the operand of the CTA's 128 rows, straight from the uint8 indices;
+//                 group k takes every fourth slab, one row per thread, in registers: a table in shared memory would
+//                 compete with the slabs for its bandwidth
+//   warps 23-26   epilogue: tcgen05.ld, dequantise, swizzled staging, tiled bulk stores; clears the accumulator
 #include "kernels.h"
 #include "ptx.cuh"
 #include "epilogue.cuh"
@@ -30,12 +31,14 @@ constexpr uint32_t kSlab = 256;                // positions of the contraction a
 constexpr uint32_t kGroups = 4, kCopyWarps = 2, kIndexWarps = 1, kMmaWarps = 4, kEpiWarps = 4;
 constexpr uint32_t kFirstMma = kCopyWarps + kIndexWarps, kFirstBuilder = kFirstMma + kMmaWarps, kFirstEpi = kFirstBuilder + 4 * kGroups;
 constexpr uint32_t kThreads = (kFirstEpi + kEpiWarps) * 32;   // 864
-constexpr uint32_t kASlots = 4;                // operand slots: 32 columns of bytes and 2 of metadata each
+// operand slots, 32 columns of bytes and 2 of metadata each: what two accumulators leave, in multiples of the groups
+__host__ __device__ constexpr uint32_t operand_slots(uint32_t n_tile) { return (512 - 2 * n_tile) / 34 >= 8 ? 8 : 4; }
+constexpr uint32_t kMaxASlots = 8;
 constexpr uint32_t kMaxBSlots = 16;
 constexpr uint32_t kStageBytes = 32 * 128;     // a 32 x 32 fp32 block
 constexpr uint32_t kStages = 2;                // per epilogue warp
 constexpr uint32_t kIdxStages = 3;
-constexpr uint32_t kNumBarriers = 2 * kASlots + 2 * kMaxBSlots + 4 + 2 * kIdxStages;
+constexpr uint32_t kNumBarriers = 2 * kMaxASlots + 2 * kMaxBSlots + 4 + 2 * kIdxStages;
 
 // A stage of index bytes: 128 rows of `idx_width` bytes, for `idx_slabs` slabs.
 __host__ __device__ constexpr uint32_t idx_width(int lg) { return lg == 3 ? 64u : lg <= 6 ? 4u * (256u >> lg) : 16u; }
@@ -156,6 +159,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                   const __grid_constant__ CUtensorMap out_map, const SparseParams p) {
     constexpr uint32_t kHalfN = N_TILE / 2, kBBytes = kHalfN * kSlab;
     constexpr uint32_t kIdesc = umma_idesc_i8(2 * kRows, N_TILE, 1, 1) | kIdescSparse;
+    constexpr uint32_t kASlots = operand_slots(N_TILE);
     constexpr uint32_t kDataBase = 2 * N_TILE, kMetaBase = kDataBase + 32 * kASlots;   // tensor-memory columns
     static_assert(kMetaBase + 2 * kASlots <= 512, "tensor memory");
 
@@ -171,7 +175,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_bias + kEpiWarps * N_TILE);
     uint32_t* s_misc = reinterpret_cast<uint32_t*>(s_bar + kNumBarriers);                  // tmem base, abort
     volatile uint32_t* s_abort = s_misc + 1;
-    const uint32_t a_full0 = smem_u32(s_bar), a_empty0 = a_full0 + 8 * kASlots, b_full0 = a_empty0 + 8 * kASlots,
+    const uint32_t a_full0 = smem_u32(s_bar), a_empty0 = a_full0 + 8 * kMaxASlots, b_full0 = a_empty0 + 8 * kMaxASlots,
                    b_empty0 = b_full0 + 8 * kMaxBSlots, acc_full0 = b_empty0 + 8 * kMaxBSlots, acc_empty0 = acc_full0 + 16,
                    i_full0 = acc_empty0 + 16, i_empty0 = i_full0 + 8 * kIdxStages;
 
@@ -191,8 +195,8 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         // leader's expect_tx (the copies of both CTAs complete the bytes); acc_full: one commit per issuing warp;
         // acc_empty: the epilogue warps of both CTAs (barriers the
         // leader waits on are unused in the other CTA); i_full: expect_tx; i_empty: the CTA's builder warps.
-        const uint32_t after = 2 * kASlots + 2 * kMaxBSlots;
-        mbar_init(a_full0 + 8 * b, b < kASlots ? 8u : b < after ? 1u : b < after + 2 ? kMmaWarps : b < after + 4 ? 2 * kEpiWarps : b < after + 4 + kIdxStages ? 1u : 4 * kGroups);
+        const uint32_t after = 2 * kMaxASlots + 2 * kMaxBSlots;
+        mbar_init(a_full0 + 8 * b, b < kMaxASlots ? 8u : b < after ? 1u : b < after + 2 ? kMmaWarps : b < after + 4 ? 2 * kEpiWarps : b < after + 4 + kIdxStages ? 1u : 4 * kGroups);
         fence_barrier_init();
     }
     if (warp == kFirstMma) tmem_alloc_pair(smem_u32(s_misc), 512);
@@ -295,7 +299,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         __syncwarp();
         if (p.early_trigger) pdl_launch_dependents();
     } else if (warp < kFirstEpi) {
-        // ---------------- operand builders: slab x of the CTA's sequence by group x % 4, into slot x % 4
+        // ---------------- operand builders: slab x of the CTA's sequence by group x % 4, into slot x % kASlots
         constexpr int kRaw = LG == 3 ? 8 : 4;
         const uint32_t grp = (warp - kFirstBuilder) >> 2, r = (warp & 3u) * 32 + lane;
         // the 256 / CT index bytes of slab `sub` of a stage; 64-byte rows are swizzled
@@ -446,6 +450,11 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
 
 constexpr size_t kSmemLimit = 227 * 1024;
 
+uint32_t log2_of(uint32_t v) {
+    uint32_t lg = 0;
+    while ((1u << lg) < v) ++lg;
+    return lg;
+}
 uint32_t sparse_slabs(uint32_t CB, uint32_t CT) { return (uint32_t)(((uint64_t)CB * CT + kSlab - 1) / kSlab); }
 
 size_t sparse_smem(uint32_t n_tile, int lg, uint32_t b_slots) {
@@ -519,10 +528,8 @@ __global__ void __launch_bounds__(256) sparse_table_kernel(const int8_t* __restr
 }  // namespace
 
 cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t N, cudaStream_t s) {
-    uint32_t lg = 0;
-    while ((1u << lg) < CT) ++lg;
     const uint32_t slabs = sparse_slabs(CB, CT);
-    sparse_table_kernel<<<dim3(slabs, (N + 63) / 64), 256, 0, s>>>(lut, out, CB * CT, N, lg, slabs);
+    sparse_table_kernel<<<dim3(slabs, (N + 63) / 64), 256, 0, s>>>(lut, out, CB * CT, N, log2_of(CT), slabs);
     return cudaGetLastError();
 }
 
@@ -542,46 +549,66 @@ cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB,
     return cudaSuccess;
 }
 
-// uint8 indices [M][CB] as 128 rows x `width` bytes
-static cudaError_t make_idx_tmap(CUtensorMap* out, const uint8_t* idx, uint32_t M, uint32_t CB, uint32_t width, const char** why) {
+// uint8 indices [M][CB] as 128 rows x idx_width bytes
+cudaError_t sparse_make_idx_tmap(CUtensorMap* out, const uint8_t* idx, uint32_t M, uint32_t CB, uint32_t CT, const char** why) {
+    *why = nullptr;
     EncodeTiledFn enc = get_encode_tiled();
     if (!enc) { *why = "cuTensorMapEncodeTiled is not available from this driver"; return cudaErrorNotSupported; }
+    const uint32_t width = idx_width(log2_of(CT));
     cuuint64_t dims[2] = {CB, M};
     cuuint64_t strides[1] = {CB};
     cuuint32_t box[2] = {width, kRows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(idx), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     width == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                     CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the index map"; return cudaErrorInvalidValue; }
+                     width == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the index map (is the index buffer 16-byte aligned?)"; return cudaErrorInvalidValue; }
     return cudaSuccess;
 }
 
-cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, uint32_t n_tile, uint32_t max_ctas, uint32_t* dev_err, cudaStream_t s, const char** why) {
+// Tile width by the time the launch would take: rounds of one tile per pair, each bound by its slabs or, where the
+// codebook axis is short, by the epilogue beside them (0.93 us per 32 columns), and the last tile's epilogue.  A slab
+// takes 170 / 199 / 220 ns at 64 / 128 / 160 columns: at 64 the chain of one slot's turn-around, at 160 close to the
+// tensor pipe's 320 cycles.  (Measured at 32 to 16384 tokens; at 96 columns nothing gained.)
+uint32_t sparse_default_tile(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count) {
+    const uint32_t pairs = sm_count >= 2 ? (uint32_t)sm_count / 2 : 1, slabs = sparse_slabs(CB, CT);
+    const uint64_t tm = (M + 2 * kRows - 1) / (2 * kRows);
+    const struct { uint32_t n; float slab_us; } tiles[] = {{64, 0.170f}, {128, 0.199f}, {160, 0.220f}};
+    uint32_t best = 160;
+    float least = 3e38f;
+    for (const auto& t : tiles) {
+        const uint64_t items = tm * ((N + t.n - 1) / t.n), rounds = (items + pairs - 1) / pairs;
+        const float main = slabs * t.slab_us, epi = 0.93f * (t.n / 32);
+        const float us = (float)rounds * (rounds > 1 && epi > main ? epi : main) + 0.25f * (t.n / 32);
+        if (us < least) { least = us; best = t.n; }
+    }
+    return best;
+}
+
+bool sparse_tile_ok(uint32_t n_tile) { return n_tile == 64 || n_tile == 128 || n_tile == 160; }
+
+cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CUtensorMap& idx_map, const CUtensorMap& out_map, uint32_t n_tile,
+                          uint32_t max_ctas, uint32_t* dev_err, cudaStream_t s, const char** why) {
     *why = nullptr;
     if (a.M == 0 || a.N == 0) return cudaSuccess;
-    if (reinterpret_cast<uintptr_t>(a.idx) & 15u) { *why = "tcgen05 variant: the index buffer must be 16-byte aligned"; return cudaErrorInvalidValue; }
     SparseParams p;
     p.a = a;
     p.slabs = sparse_slabs(a.CB, a.CT);
     p.tiles_m = (a.M + 2 * kRows - 1) / (2 * kRows);
     p.tiles_n = (a.N + n_tile - 1) / n_tile;
     p.dev_err = dev_err;
-    int lg = 0;
-    while ((1u << lg) < a.CT) ++lg;
-    p.b_slots = kMaxBSlots;
-    while (p.b_slots > 4 && sparse_smem(n_tile, lg, p.b_slots) > kSmemLimit) p.b_slots -= 4;
+    const int lg = (int)log2_of(a.CT);
+    p.b_slots = kMaxBSlots;   // a multiple of the issuing warps: every slot has one of them
+    while (p.b_slots > kMmaWarps && sparse_smem(n_tile, lg, p.b_slots) > kSmemLimit) p.b_slots -= kMmaWarps;
     const uint64_t items = (uint64_t)p.tiles_m * p.tiles_n;
     const uint32_t cap = max_ctas / 2, pairs = (uint32_t)(items < cap ? items : cap);
+    // With one tile per pair all pairs reach the end of their main loops together, and the next kernel of the stream
+    // may as well be launched; with several they finish a tile apart and its early CTAs would skew it.
     p.early_trigger = items <= cap;
-    CUtensorMap om, im;
-    cudaError_t e = make_out_tmap(&om, a.out, a.M, a.N, why);
-    if (e != cudaSuccess) return e;
-    e = make_idx_tmap(&im, a.idx, a.M, a.CB, idx_width(lg), why);
-    if (e != cudaSuccess) return e;
     const size_t smem = sparse_smem(n_tile, lg, p.b_slots);
-    if (n_tile == 160) return run_lg<160>(lg, lut_map, im, om, p, pairs, smem, s);
-    *why = "tcgen05 variant: this tile is not built";
+    if (n_tile == 64) return run_lg<64>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
+    if (n_tile == 128) return run_lg<128>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
+    if (n_tile == 160) return run_lg<160>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
+    *why = "tcgen05 variant: the sparse form is built for 64-, 128- and 160-wide tiles";
     return cudaErrorInvalidValue;
 }
 

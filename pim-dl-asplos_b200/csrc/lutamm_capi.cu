@@ -8,7 +8,6 @@
 
 #include <algorithm>
 #include <cstdio>
-#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -40,14 +39,17 @@ namespace {
 constexpr int kNumUmmaTiles = 5;  // 64, 128, 160, 192, 256
 inline int umma_tile_slot(uint32_t n_tile) { return n_tile == 64 ? 0 : n_tile == 128 ? 1 : n_tile == 160 ? 2 : n_tile == 192 ? 3 : 4; }
 
+constexpr int kNumSparseTiles = 3;  // 64, 128, 160
+inline int sparse_tile_slot(uint32_t n_tile) { return n_tile == 64 ? 0 : n_tile == 128 ? 1 : 2; }
+
 struct Layer {
     lutamm_index_params ip{};
     lutamm_lut_params lp{};
     uint32_t K = 0, v = 0, CB = 0, CT = 0, N = 0;
     float* d_centroid = nullptr;
     int8_t* d_lut = nullptr;    // canonical [CB][CT][N]
-    int8_t* d_lut_s = nullptr;  // sparse_table layout, made on first use
-    int8_t* d_lut_t = nullptr;  // [N][CB*CT], made on first use of the tcgen05 variant
+    int8_t* d_lut_s = nullptr;  // the sparse tcgen05 kernel's layout, made on its first use
+    int8_t* d_lut_t = nullptr;  // [N][CB*CT], made on first use of the dense tcgen05 kernel
     float* d_bias = nullptr;
     lutamm_plan plan{};
     uint32_t act = LUTAMM_ACT_NONE;
@@ -55,6 +57,12 @@ struct Layer {
     std::vector<char> gather_map_ok;
     CUtensorMap umma_maps[kNumUmmaTiles];
     bool umma_map_ok[kNumUmmaTiles] = {false, false, false, false, false};
+    // the sparse form: tensor maps of its table per tile width, and of the last index and output buffers it was called with
+    CUtensorMap sparse_maps[kNumSparseTiles];
+    bool sparse_map_ok[kNumSparseTiles] = {false, false, false};
+    CUtensorMap sparse_idx_map, sparse_out_map;
+    const void *sparse_idx = nullptr, *sparse_out = nullptr;
+    uint32_t sparse_idx_m = 0, sparse_out_m = 0;
 };
 
 struct Buf {
@@ -203,6 +211,60 @@ int check_tiled(lutamm_ctx* c, const Layer& L, uint32_t M) {
     return LUTAMM_OK;
 }
 
+// Whether a plan leaves the tcgen05 kernel's form to the library.  What it names belongs to the dense kernel, except
+// umma_operand 3, the sparse form itself, with umma_n_tile.
+bool umma_plan_open(const lutamm_plan& p) {
+    return !p.umma_operand && !p.umma_n_tile && !p.umma_split && !p.umma_stages && !p.umma_groups && !p.umma_sps && !p.umma_epilogue;
+}
+
+// The load-time layouts of the table are made on first use.  The kernel that follows is a programmatic dependent
+// launch whose copies do not wait for the preceding grid, so they have to be complete, not merely queued.
+template <typename F>
+int make_table(lutamm_ctx* c, int8_t** table, size_t bytes, F launch) {
+    if (*table) return LUTAMM_OK;
+    CU_TRY(c, cudaMalloc(table, bytes));
+    cudaError_t e = launch(*table);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e != cudaSuccess) {
+        cudaFree(*table);
+        *table = nullptr;
+        return fail(c, LUTAMM_ECUDA, std::string("LUT layout: ") + cudaGetErrorString(e));
+    }
+    ++c->launches;
+    return LUTAMM_OK;
+}
+
+// steps 2+3 on CTA pairs with the sparse operand
+int run_sparse(lutamm_ctx* c, Layer& L, const LutArgs& a, uint32_t n_tile) {
+    const char* why = nullptr;
+    if (reinterpret_cast<uintptr_t>(a.idx) & 15u) return fail(c, LUTAMM_ECUDA, "tcgen05 variant: the index buffer must be 16-byte aligned");
+    int r = make_table(c, &L.d_lut_s, sparse_table_bytes(L.CB, L.CT, L.N),
+                       [&](int8_t* t) { return launch_sparse_table(L.d_lut, t, L.CB, L.CT, L.N, c->stream); });
+    if (r) return r;
+    if (!n_tile) n_tile = sparse_default_tile(a.M, a.CB, a.CT, a.N, c->sm_count);
+    const int slot = sparse_tile_slot(n_tile);
+    cudaError_t e = cudaSuccess;
+    if (!L.sparse_map_ok[slot]) {
+        e = sparse_make_tmap(&L.sparse_maps[slot], L.d_lut_s, L.CB, L.CT, L.N, n_tile, &why);
+        L.sparse_map_ok[slot] = e == cudaSuccess;
+    }
+    if (e == cudaSuccess && (L.sparse_idx != a.idx || L.sparse_idx_m != a.M)) {
+        e = sparse_make_idx_tmap(&L.sparse_idx_map, a.idx, a.M, a.CB, a.CT, &why);
+        L.sparse_idx = e == cudaSuccess ? a.idx : nullptr;
+        L.sparse_idx_m = a.M;
+    }
+    if (e == cudaSuccess && (L.sparse_out != a.out || L.sparse_out_m != a.M)) {
+        e = make_out_tmap(&L.sparse_out_map, a.out, a.M, a.N, &why);
+        L.sparse_out = e == cudaSuccess ? a.out : nullptr;
+        L.sparse_out_m = a.M;
+    }
+    if (e == cudaSuccess)
+        e = launch_sparse(a, L.sparse_maps[slot], L.sparse_idx_map, L.sparse_out_map, n_tile, (uint32_t)c->sm_count, c->d_err, c->stream, &why);
+    if (e != cudaSuccess) return fail(c, LUTAMM_ECUDA, why ? why : (std::string("tcgen05 launch: ") + cudaGetErrorString(e)));
+    ++c->launches;
+    return LUTAMM_OK;
+}
+
 // step 2+3 on device buffers
 int run_lut(lutamm_ctx* c, Layer& L, const uint8_t* d_idx, float* d_out, int32_t* d_acc_out, uint32_t M,
             uint32_t flags, const lutamm_plan& plan, float* const* peer_out = nullptr, uint32_t n_peers = 0) {
@@ -226,8 +288,15 @@ int run_lut(lutamm_ctx* c, Layer& L, const uint8_t* d_idx, float* d_out, int32_t
     if (variant == LUTAMM_VARIANT_UMMA) {
         if (!umma_supported(L.CB, L.CT, L.N))
             return fail(c, LUTAMM_EUNSUPPORTED, "tcgen05 variant does not cover this shape (num_centroid a power of two in 8..256, num_codebook % 16 == 0)");
+        // The sparse form writes row-major fp32 alone; tiled output, the int32 copy and peer stores, and plans that
+        // name a dense form, take the dense kernel.
+        const bool sparse_fits = !a.n_peers && !a.acc_out && !a.layout.tiled;
+        if (plan.umma_operand == 3 && plan.umma_n_tile && !sparse_tile_ok(plan.umma_n_tile))
+            return fail(c, LUTAMM_EINVAL, "umma_n_tile must be 64, 128 or 160 for the sparse form");
+        if (sparse_fits && (plan.umma_operand == 3 || umma_plan_open(plan))) return run_sparse(c, L, a, plan.umma_n_tile);
         UmmaPlan up;
-        umma_default_plan(M, L.CB, L.CT, L.N, c->sm_count, plan.umma_operand, plan.umma_n_tile, plan.umma_sps, &up);
+        const bool dense_plan = plan.umma_operand != 3;   // else: where the sparse form does not fit, the dense default
+        umma_default_plan(M, L.CB, L.CT, L.N, c->sm_count, dense_plan ? plan.umma_operand : 0, dense_plan ? plan.umma_n_tile : 0, plan.umma_sps, &up);
         const bool a_tmem = up.a_tmem != 0;
         if (plan.umma_split) up.split = plan.umma_split;
         up.stages = plan.umma_stages;
@@ -237,35 +306,9 @@ int run_lut(lutamm_ctx* c, Layer& L, const uint8_t* d_idx, float* d_out, int32_t
         if (!umma_tile_ok(up.n_tile, a_tmem))
             return fail(c, LUTAMM_EINVAL, "umma_n_tile must be 64, 128 or 256 with the one-hot operand in shared memory, "
                                           "64, 128, 160 or 192 with it in tensor memory");
-        if (!L.d_lut_t) {
-            // First tcgen05 call for this layer: make the K-major copy of the table.  The kernel that
-            // follows is a programmatic dependent launch whose TMA producer does not wait for the
-            // preceding grid, so the copy has to be complete - not merely queued - before it starts.
-            const size_t bytes = (size_t)L.CB * L.CT * L.N;
-            CU_TRY(c, cudaMalloc(&L.d_lut_t, bytes));
-            cudaError_t te = launch_transpose_lut(L.d_lut, L.d_lut_t, L.CB * L.CT, L.N, c->stream);
-            if (te == cudaSuccess) te = cudaStreamSynchronize(c->stream);
-            if (te != cudaSuccess) {
-                cudaFree(L.d_lut_t);
-                L.d_lut_t = nullptr;
-                return fail(c, LUTAMM_ECUDA, std::string("LUT transpose: ") + cudaGetErrorString(te));
-            }
-            ++c->launches;
-        }
-        static const int force = getenv("LUTAMM_SPARSE") ? atoi(getenv("LUTAMM_SPARSE")) : 0;
-        if (force && !a.n_peers && !a.acc_out && !a.layout.tiled) {
-            if (!L.d_lut_s) {
-                CU_TRY(c, cudaMalloc(&L.d_lut_s, sparse_table_bytes(L.CB, L.CT, L.N)));
-                CU_TRY(c, launch_sparse_table(L.d_lut, L.d_lut_s, L.CB, L.CT, L.N, c->stream));
-                CU_TRY(c, cudaStreamSynchronize(c->stream));
-            }
-            CUtensorMap m;
-            cudaError_t e = sparse_make_tmap(&m, L.d_lut_s, L.CB, L.CT, L.N, force, &why);
-            if (e == cudaSuccess) e = launch_sparse(a, m, force, c->sm_count, c->d_err, c->stream, &why);
-            if (e != cudaSuccess) return fail(c, LUTAMM_ECUDA, why ? why : cudaGetErrorString(e));
-            ++c->launches;
-            return LUTAMM_OK;
-        }
+        if (int r = make_table(c, &L.d_lut_t, (size_t)L.CB * L.CT * L.N,
+                               [&](int8_t* t) { return launch_transpose_lut(L.d_lut, t, L.CB * L.CT, L.N, c->stream); }))
+            return r;
         const int slot = umma_tile_slot(up.n_tile);
         if (!L.umma_map_ok[slot]) {
             cudaError_t e = umma_make_tmap(&L.umma_maps[slot], L.d_lut_t, L.CB, L.CT, L.N, up.n_tile, &why);
@@ -742,8 +785,10 @@ int lutamm_set_plan(lutamm_ctx* c, int layer_id, const lutamm_plan* plan) {
     if (!plan) return fail(c, LUTAMM_EINVAL, "null plan");
     if (plan->variant > LUTAMM_VARIANT_UMMA) return fail(c, LUTAMM_EINVAL, "unknown kernel variant");
     if (plan->gather_cfg >= gather_num_cfgs()) return fail(c, LUTAMM_EINVAL, "unknown gather tile configuration");
-    if (plan->umma_operand > 2) return fail(c, LUTAMM_EINVAL, "umma_operand must be 0, 1 (shared memory) or 2 (tensor memory)");
-    if (plan->umma_n_tile && plan->umma_operand && !umma_tile_ok(plan->umma_n_tile, plan->umma_operand == 2))
+    if (plan->umma_operand > 3) return fail(c, LUTAMM_EINVAL, "umma_operand must be 0, 1 (shared memory), 2 (tensor memory) or 3 (2:4 sparse, CTA pairs)");
+    if (plan->umma_operand == 3) {
+        if (plan->umma_n_tile && !sparse_tile_ok(plan->umma_n_tile)) return fail(c, LUTAMM_EINVAL, "umma_n_tile must be 0, 64, 128 or 160 for the sparse form");
+    } else if (plan->umma_n_tile && plan->umma_operand && !umma_tile_ok(plan->umma_n_tile, plan->umma_operand == 2))
         return fail(c, LUTAMM_EINVAL, "umma_n_tile must be 0, 64, 128 or 256 with the one-hot operand in shared memory, "
                                       "0, 64, 128, 160 or 192 with it in tensor memory");
     if (plan->umma_sps != 0 && plan->umma_sps != 1 && plan->umma_sps != 2 && plan->umma_sps != 4)
@@ -807,6 +852,13 @@ int lutamm_tune(lutamm_ctx* c, int layer_id, uint32_t M, lutamm_plan* best_out) 
     }
     if (umma_supported(L->CB, L->CT, L->N)) {
         const uint32_t slabs = (uint32_t)(((uint64_t)L->CB * L->CT + 127) / 128);
+        for (uint32_t nt : {64u, 128u, 160u}) {
+            lutamm_plan p{};
+            p.variant = LUTAMM_VARIANT_UMMA;
+            p.umma_operand = 3;
+            p.umma_n_tile = nt;
+            cands.push_back(p);
+        }
         struct Cand { uint32_t operand, n_tile, sps; };
         for (const Cand& cd : {Cand{1, 256, 1}, Cand{2, 192, 1}, Cand{2, 160, 1}, Cand{2, 128, 2}, Cand{2, 128, 1}, Cand{1, 128, 1}, Cand{2, 64, 1}}) {
             if (cd.n_tile > 128 && L->N < cd.n_tile) continue;
@@ -921,7 +973,7 @@ int lutamm_plan_cache_load(lutamm_ctx* c, const char* path) {
         lutamm_plan p{};
         p.variant = v[0]; p.ccs_tokens = v[1]; p.gather_cfg = v[2]; p.umma_n_tile = v[3]; p.umma_split = v[4];
         p.umma_stages = v[5]; p.umma_groups = v[6]; p.umma_operand = v[7]; p.umma_sps = v[8];
-        if (p.variant > LUTAMM_VARIANT_UMMA || p.gather_cfg >= gather_num_cfgs() || p.umma_operand > 2) continue;  // not a plan of this build
+        if (p.variant > LUTAMM_VARIANT_UMMA || p.gather_cfg >= gather_num_cfgs() || p.umma_operand > 3) continue;  // not a plan of this build
         c->plan_cache[{k[0], k[1], k[2], k[3], k[4], k[5]}] = p;
     }
     std::fclose(f);
