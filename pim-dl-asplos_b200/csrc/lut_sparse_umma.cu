@@ -18,6 +18,13 @@
 //                 group k takes every fourth slab, one row per thread, in registers: a table in shared memory would
 //                 compete with the slabs for its bandwidth
 //   warps 23-26   epilogue: tcgen05.ld, dequantise, swizzled staging, tiled bulk stores; clears the accumulator
+//
+// What bounds it.  With a long codebook axis (16384 x 2048 codebooks of 16 -> 4096) a slab takes 220 ns, 340-380 cycles
+// at the 1.55-1.7 GHz that the power cap leaves, against 320 of the tensor pipe: 1254 -> 648 us, 6.8 P operations/s of the
+// dense contraction (4.57 is the dense pipe's peak).  With a short one (BERT-base QKV, 24 slabs a tile, 12608 tokens:
+// 118 -> 65 us) it is the epilogue of the tile before, 0.93 us per 32 columns, beside the main loop.  Steps on the way, at
+// 12608 x 384 -> 3072 (dense 160 us): arrivals with .release.cluster, which waits for the builder's loads, 160; default
+// scope 108; two copying threads 105; an issuing warp per operand slot 99; index tiles through the copy engine 84.
 #include "kernels.h"
 #include "ptx.cuh"
 #include "epilogue.cuh"
