@@ -687,7 +687,8 @@ cudaError_t run_tile_tok(const CcsArgs& a, size_t smem, cudaStream_t s) {
     const uint32_t copy16 = a.K % 4 == 0 && reinterpret_cast<uintptr_t>(a.x) % 16 == 0;
     const uint32_t words = a.CB % 4 == 0 && reinterpret_cast<uintptr_t>(a.idx_out) % 4 == 0;
     auto k = a.format == LUTAMM_INDEX_U16_TILED ? ccs_tile_kernel<V, G, ONE, kTok, true> : ccs_tile_kernel<V, G, ONE, kTok, false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemOptIn memo[2];
+    cudaError_t e = allow_smem(memo[a.format == LUTAMM_INDEX_U16_TILED], k, (int)smem);
     if (e != cudaSuccess) return e;
     return launch_dependent(k, grid, dim3(kTileThreads), smem, s, a.x, a.centroid, a.idx_out, a.M, a.K, a.CB, a.CT, copy16, words,
                             a.n_stile, a.cb_mtile);
@@ -717,7 +718,8 @@ cudaError_t run_any(const CcsArgs& a, cudaStream_t s) {
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
     dim3 grid((a.CB + cb_per_cta - 1) / cb_per_cta, (a.M + kAnyThreads - 1) / kAnyThreads);
     auto k = a.format == LUTAMM_INDEX_U16_TILED ? ccs_any_kernel<true> : ccs_any_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemOptIn memo[2];
+    cudaError_t e = allow_smem(memo[a.format == LUTAMM_INDEX_U16_TILED], k, (int)smem);
     if (e != cudaSuccess) return e;
     return launch_dependent(k, grid, dim3(kAnyThreads), smem, s, a.x, a.centroid, a.idx_out, a.M, a.K, a.v, a.CB, a.CT,
                             cb_per_cta, a.n_stile, a.cb_mtile);

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kPeakWarps * 32, 1) int8_peak_kernel(uint32_t 
         long long e = s_end[0];
         for (uint32_t w = 1; w < kPeakWarps; ++w) e = s_end[w] > e ? s_end[w] : e;
         if (blockIdx.x == 0) *cycles_out = (unsigned long long)(e - t0);
-        if (s_abort) atomicExch(dev_err, 3u);
+        if (s_abort) report_error(dev_err, 3u);
     }
     if (threadIdx.x < 32) { tc_fence_after_sync(); tmem_dealloc(tmem, 512); }
 }
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(128, 1) stalled_wait_kernel(uint32_t polls, ui
     volatile uint32_t* abort_word = &s_abort;
     if (threadIdx.x == 32) (void)mbar_wait_limited(smem_u32(&s_bar), 0, abort_word, polls);   // phase 0 never completes
     __syncthreads();
-    if (*abort_word && threadIdx.x == 0) atomicExch(dev_err, 4u);
+    if (*abort_word && threadIdx.x == 0) report_error(dev_err, 4u);
     __syncthreads();
     if (threadIdx.x < 32) { tc_fence_after_sync(); tmem_dealloc(s_tmem, 32); }
 }

@@ -1,5 +1,6 @@
 // Internal launcher interface between the C ABI (lutamm_capi.cu) and the kernels.
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -121,11 +122,30 @@ cudaError_t launch_int8_peak(uint32_t n_tile, uint32_t slabs, uint32_t grid, uns
 // Self-test: a bounded wait on a barrier nobody arrives at; the kernel reports through *dev_err and returns.
 cudaError_t launch_stalled_wait(uint32_t polls, uint32_t* dev_err, cudaStream_t s);
 
+// The opt-in to more than 48 KB of dynamic shared memory, asked for once per kernel, device and size (the call takes a
+// good part of a microsecond): remembers, per kernel, the largest size asked for on each device.
+struct SmemOptIn {
+    std::atomic<int> granted[64] = {};
+};
+template <typename K>
+cudaError_t allow_smem(SmemOptIn& memo, K kernel, int bytes) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 64 && memo.granted[dev].load(std::memory_order_relaxed) >= bytes) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < 64) memo.granted[dev].store(bytes, std::memory_order_relaxed);
+    return e;
+}
+
 // Driver entry point for tensor-map encoding, resolved through the runtime so the library
 // carries no link-time dependency on the driver and loads on machines without one.
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn get_encode_tiled();
+
+// Ordinal of the device whose (or managed) memory this is, -1 for host memory and for what CUDA does not know.
+int pointer_device(const void* p);
 
 }  // namespace lutamm

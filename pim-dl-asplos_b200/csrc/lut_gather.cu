@@ -193,7 +193,7 @@ lut_gather_kernel(const __grid_constant__ CUtensorMap lut_map, LutArgs a, uint32
             for (uint32_t blk = (issued > (uint32_t)kStages ? issued - kStages : 0u); blk < issued; ++blk)
                 for (uint32_t it = 0; it < kWaitLimit; ++it)
                     if (mbar_try_wait(full0 + 8 * (blk % kStages), (blk / kStages) & 1)) break;
-            atomicExch(dev_err, 1u);
+            report_error(dev_err, 1u);
         }
         __syncthreads();
         return;
@@ -244,7 +244,8 @@ cudaError_t run(const LutArgs& a, const CUtensorMap& map, uint32_t* dev_err, cud
     const uint32_t stage_pitch = (stage_bytes + 127u) & ~127u;
     const size_t smem = (size_t)kStages * stage_pitch + WARPS * TOK * kMaxCbBlk + 2 * kStages * 8 + 16 + 1024;
     auto k = lut_gather_kernel<COLS, WARPS, TOK>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemOptIn memo;
+    cudaError_t e = allow_smem(memo, k, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((a.N + N_TILE - 1) / N_TILE, (a.M + M_TILE - 1) / M_TILE);

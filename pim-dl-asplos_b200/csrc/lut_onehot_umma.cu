@@ -700,7 +700,7 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
             // handed back: a TMA tile arrives within microseconds; wait a bounded ~100 us.
             const long long t0 = clock64();
             while (clock64() - t0 < 200000) {}
-            atomicExch(p.dev_err, 2u);
+            report_error(p.dev_err, 2u);
         }
         __syncthreads();
     }
@@ -726,7 +726,8 @@ cudaError_t run(const CUtensorMap& map, const UmmaParams& p, uint32_t grid, size
     // (programmatic dependent launch) the block scheduler doubles CTAs up wherever two fit - which a
     // shallow ring with a single builder group does.  More than half an SM's shared memory rules it out.
     if (smem < kSmemOneCtaPerSm) smem = kSmemOneCtaPerSm;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemOptIn memo;
+    cudaError_t e = allow_smem(memo, k, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);

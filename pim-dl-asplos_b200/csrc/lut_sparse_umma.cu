@@ -444,7 +444,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             // give copies that may still be in flight a bounded time to land before the shared memory is handed back
             const long long t0 = clock64();
             while (clock64() - t0 < 200000) {}
-            atomicExch(p.dev_err, 2u);
+            report_error(p.dev_err, 2u);
         }
         __syncthreads();
     }
@@ -472,7 +472,8 @@ size_t sparse_smem(uint32_t n_tile, int lg, uint32_t b_slots) {
 template <uint32_t N_TILE, int LG>
 cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
     auto k = lut_sparse_kernel<N_TILE, LG>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemOptIn memo;
+    cudaError_t e = allow_smem(memo, k, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);

@@ -32,6 +32,31 @@ EncodeTiledFn get_encode_tiled() {
     return fn;
 }
 
+// Asked of the driver in one query: the runtime's cudaPointerGetAttributes gathers more and takes several times as long,
+// on a path where a small call is bound by the host.
+int pointer_device(const void* p) {
+    typedef CUresult (*QueryFn)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+    static const QueryFn query = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
+                   ? reinterpret_cast<QueryFn>(f) : nullptr;
+    }();
+    if (query) {
+        unsigned long long type = 0, managed = 0, device = 0;   // stay 0 for memory CUDA does not know
+        CUpointer_attribute attr[3] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL};
+        void* data[3] = {&type, &managed, &device};
+        if (query(3, attr, data, (CUdeviceptr)reinterpret_cast<uintptr_t>(p)) == CUDA_SUCCESS)
+            return (unsigned)type == CU_MEMORYTYPE_DEVICE || (managed & 0xFFu) != 0 ? (int)(unsigned)device : -1;
+    }
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return -1;
+    }
+    return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged ? at.device : -1;
+}
+
 }  // namespace lutamm
 
 namespace {
@@ -91,8 +116,8 @@ struct lutamm_ctx {
     Buf p_in[kHostSlots], p_out[kHostSlots];
     cudaEvent_t ev_in[kHostSlots] = {}, ev_comp[kHostSlots] = {}, ev_out[kHostSlots] = {};
     uint32_t slot = 0;
-    uint32_t* d_err = nullptr;
-    uint32_t* h_err = nullptr;  // pinned
+    uint32_t* h_err = nullptr;  // the kernels' error word: pinned host memory, mapped
+    uint32_t* d_err = nullptr;  // its device address
     bool timing = false;
     cudaEvent_t ev[6] = {};
     lutamm_timings last{};
@@ -128,12 +153,12 @@ int fail(lutamm_ctx* c, int code, const std::string& msg) {
 
 struct DeviceGuard {
     int prev = -1;
-    bool ok = false;
     explicit DeviceGuard(int dev) {
-        if (cudaGetDevice(&prev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) ok = true;
+        int cur = -1;
+        if (cudaGetDevice(&cur) == cudaSuccess && cur != dev && cudaSetDevice(dev) == cudaSuccess) prev = cur;
     }
     ~DeviceGuard() {
-        if (ok && prev >= 0) cudaSetDevice(prev);
+        if (prev >= 0) cudaSetDevice(prev);
     }
 };
 
@@ -159,14 +184,7 @@ int ensure(lutamm_ctx* c, Buf& b, size_t bytes, bool zero = false) {
     return LUTAMM_OK;
 }
 
-bool is_device_ptr(const void* p) {
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
-}
+bool is_device_ptr(const void* p) { return pointer_device(p) >= 0; }
 
 Layer* find_layer(lutamm_ctx* c, int id) {
     auto it = c->layers.find(id);
@@ -368,12 +386,10 @@ int run_ccs(lutamm_ctx* c, Layer& L, const float* d_x, void* d_idx, uint32_t M, 
 // read back the device error word after a synchronisation
 int check_dev_err(lutamm_ctx* c) {
     if (c->s_in) CU_TRY(c, cudaStreamSynchronize(c->s_in));
-    CU_TRY(c, cudaMemcpyAsync(c->h_err, c->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
     CU_TRY(c, cudaStreamSynchronize(c->stream));
     if (c->s_out) CU_TRY(c, cudaStreamSynchronize(c->s_out));
-    if (*c->h_err) {
-        const uint32_t code = *c->h_err;
-        cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), c->stream);
+    if (const uint32_t code = *static_cast<volatile uint32_t*>(c->h_err)) {
+        *static_cast<volatile uint32_t*>(c->h_err) = 0;
         // a kernel that gave up may have left split-K tile counters half counted
         if (c->d_counters.p) cudaMemsetAsync(c->d_counters.p, 0, c->d_counters.cap, c->stream);
         return fail(c, LUTAMM_EDEVICE, "a kernel gave up on a bounded wait (code " + std::to_string(code) + "); output is not valid");
@@ -518,9 +534,8 @@ int lutamm_create(lutamm_ctx** out, int device) {
     c->sm_count = prop.multiProcessorCount;
     DeviceGuard g(device);
     if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&c->d_err, sizeof(uint32_t)) != cudaSuccess ||
-        cudaMemset(c->d_err, 0, sizeof(uint32_t)) != cudaSuccess ||
-        cudaMallocHost(&c->h_err, sizeof(uint32_t)) != cudaSuccess) {
+        cudaHostAlloc(&c->h_err, sizeof(uint32_t), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(&c->d_err, c->h_err, 0) != cudaSuccess) {
         std::string m = std::string("context set-up failed: ") + cudaGetErrorString(cudaGetLastError());
         delete c;
         return fail(nullptr, LUTAMM_ECUDA, m);
@@ -566,7 +581,6 @@ int lutamm_destroy(lutamm_ctx* c) {
     for (Buf* b : {&c->d_in, &c->d_out, &c->d_idx, &c->d_idx16, &c->d_acc_dbg, &c->d_acc_scratch, &c->d_counters,
                    &c->d_build})
         cudaFree(b->p);
-    cudaFree(c->d_err);
     cudaFreeHost(c->h_err);
     for (auto& ev : c->ev)
         if (ev) cudaEventDestroy(ev);

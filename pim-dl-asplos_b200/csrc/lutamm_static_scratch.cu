@@ -11,23 +11,25 @@
 //
 // How.  The only intermediate of the operator is the closest-centroid index buffer,
 // uint8 [n_tokens][num_codebook], written by the search kernel and read by the
-// gather-accumulate kernel.  Here it lives in a file-scope __device__ array of fixed size
-// (plus one error word).  Every GPU that loads this library therefore holds
+// gather-accumulate kernel.  Here it lives in a file-scope __device__ array of fixed size.  The
+// kernels' error word is host memory, a static page that the first call on any device maps into
+// the devices: a call then clears and reads it without a copy (the memset, the copy back to
+// pageable memory and their gaps were 30 us of a 170 us call).  Every GPU that loads this library therefore holds
 // LUTAMM_STATIC_SCRATCH_BYTES + 256 bytes of device memory from module load until the
 // process exits, whether or not the entry point is ever called.
 //
 // Rules that follow from one shared array:
 //   * n_tokens * num_codebook must not exceed LUTAMM_STATIC_SCRATCH_BYTES; larger problems
 //     are rejected with LUTAMM_EINVAL (split the batch);
-//   * the array keeps whatever the previous call left in it; the one word that has to
-//     start at zero (the kernels' error flag) is cleared at the start of every call, and
-//     the index region is fully rewritten by the search kernel before it is read;
+//   * the array keeps whatever the previous call left in it; the error word is cleared at the
+//     start of every call, and the index region is fully rewritten by the search kernel before
+//     it is read;
 //   * two calls that overlap on the GPU (different streams, different threads, different
 //     contexts of one process on one device) race on the array.  Serialise them.
 //
 // Set-up.  A __device__ array's name is only a host-side handle; the device address comes
 // from cudaGetSymbolAddress, per device, with that device current.  The first call on a
-// device does this (and sets the kernels' shared-memory attribute); make that first call
+// device does this (and maps the error words and sets the kernels' shared-memory attribute); make that first call
 // before any stream capture begins, because these set-up calls are not stream operations.
 //
 // No counterpart in the reference, whose amm_host() allocates (and leaks) its index buffer
@@ -46,20 +48,15 @@ static __device__ __align__(256) unsigned char g_static_scratch[kHeaderBytes + L
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 unsigned char* g_scratch_ptr[kMaxDevices] = {};  // device address of g_static_scratch, per device
+// Error words, one per device, 64 bytes apart, and their addresses as the devices see them.
+alignas(4096) volatile uint32_t g_err_words[kMaxDevices * 16];
+uint32_t* g_err_ptr[kMaxDevices] = {};
+bool g_err_mapped = false;
 thread_local std::string g_err;
 
 int fail(int code, const std::string& msg) {
     g_err = msg;
     return code;
-}
-
-bool on_device(const void* p, int device) {
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged) && at.device == device;
 }
 
 }  // namespace
@@ -97,7 +94,7 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
     } restore{prev};
 
     for (const void* p : {(const void*)input, (const void*)centroid, (const void*)lut, (const void*)bias, (const void*)output})
-        if (!on_device(p, device))
+        if (lutamm::pointer_device(p) != device)
             return fail(LUTAMM_EINVAL, "every buffer must be device memory of the selected GPU: this entry point stages nothing");
     if ((reinterpret_cast<uintptr_t>(output) & 15u) || (reinterpret_cast<uintptr_t>(input) & 3u))
         return fail(LUTAMM_EINVAL, "output must be 16-byte aligned, input 4-byte aligned");
@@ -111,24 +108,32 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
             const cudaError_t e = cudaGetSymbolAddress(&p, g_static_scratch);
             if (e != cudaSuccess || !p)
                 return fail(LUTAMM_ECUDA, std::string("cudaGetSymbolAddress(static scratch): ") + cudaGetErrorString(e));
+            void* words = const_cast<uint32_t*>(g_err_words);
+            if (!g_err_mapped) {
+                const cudaError_t re = cudaHostRegister(words, sizeof g_err_words, cudaHostRegisterMapped | cudaHostRegisterPortable);
+                if (re != cudaSuccess) return fail(LUTAMM_ECUDA, std::string("cudaHostRegister(error words): ") + cudaGetErrorString(re));
+                g_err_mapped = true;
+            }
+            void* dp = nullptr;
+            const cudaError_t pe = cudaHostGetDevicePointer(&dp, words, 0);
+            if (pe != cudaSuccess) return fail(LUTAMM_ECUDA, std::string("cudaHostGetDevicePointer: ") + cudaGetErrorString(pe));
+            g_err_ptr[device] = static_cast<uint32_t*>(dp) + 16 * device;
             g_scratch_ptr[device] = static_cast<unsigned char*>(p);
         }
         scratch = g_scratch_ptr[device];
     }
-    uint32_t* d_err = reinterpret_cast<uint32_t*>(scratch);
+    uint32_t* d_err = g_err_ptr[device];
+    volatile uint32_t& err_word = g_err_words[16 * device];
     uint8_t* d_idx = scratch + kHeaderBytes;
     cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
 
-    // the one word that must start at zero
-    cudaError_t e = cudaMemsetAsync(d_err, 0, sizeof(uint32_t), s);
-    if (e != cudaSuccess) return fail(LUTAMM_ECUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-
+    err_word = 0;
     const char* why = nullptr;
     CcsArgs ca{};
     ca.x = input; ca.centroid = centroid; ca.idx_out = d_idx;
     ca.M = M; ca.K = K; ca.v = K / CB; ca.CB = CB; ca.CT = CT;
     ca.format = LUTAMM_INDEX_U8_ROWMAJOR;
-    e = launch_ccs(ca, s, &why);
+    cudaError_t e = launch_ccs(ca, s, &why);
     if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : (std::string("search launch: ") + cudaGetErrorString(e)));
 
     // The gather-accumulate kernel reads the LUT in its canonical layout through a tensor map
@@ -144,13 +149,8 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
     e = launch_gather(la, map, cfg, d_err, s, &why);
     if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : (std::string("gather launch: ") + cudaGetErrorString(e)));
 
-    // The error word comes back on the caller's stream, behind the kernels; the legacy default stream
-    // (which would serialise against every blocking stream of the process) is not touched.
-    uint32_t h_err = 0;
-    e = cudaMemcpyAsync(&h_err, d_err, sizeof h_err, cudaMemcpyDeviceToHost, s);
-    if (e != cudaSuccess) return fail(LUTAMM_ECUDA, std::string("cudaMemcpyAsync(error word): ") + cudaGetErrorString(e));
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(LUTAMM_ECUDA, std::string("cudaStreamSynchronize: ") + cudaGetErrorString(e));
-    if (h_err) return fail(LUTAMM_EDEVICE, "a kernel gave up on a bounded wait; output is not valid");
+    if (err_word) return fail(LUTAMM_EDEVICE, "a kernel gave up on a bounded wait; output is not valid");
     return LUTAMM_OK;
 }

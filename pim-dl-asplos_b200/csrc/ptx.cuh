@@ -88,6 +88,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return mbar_wait_limited<kSleepNs>(bar, parity, abort_word, kWaitLimit);
 }
 
+// The error word is host memory mapped into the device: a kernel touches it only when it gives up.
+__device__ __forceinline__ void report_error(uint32_t* word, uint32_t code) {
+    *reinterpret_cast<volatile uint32_t*>(word) = code;
+    __threadfence_system();
+}
+
 // generic-proxy writes to shared memory -> visible to the async proxy (TMA, tcgen05.mma)
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
