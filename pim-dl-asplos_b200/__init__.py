@@ -9,6 +9,7 @@ operator here, and importing the compute entry points without the built library 
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 from dataclasses import dataclass, field
 
@@ -91,6 +92,11 @@ class Timings(ctypes.Structure):
 
 
 _lib = None
+_fast = None   # the operator call as a CPython function (csrc/python/fastcall.c), where it has been built
+if os.path.exists(os.path.join(_HERE, "_fastcall.so")):
+    _spec = importlib.util.spec_from_file_location("_fastcall", os.path.join(_HERE, "_fastcall.so"))
+    _fast = importlib.util.module_from_spec(_spec)
+    _spec.loader.exec_module(_fast)
 
 
 def load_library() -> ctypes.CDLL:
@@ -215,6 +221,7 @@ class LutAmmContext:
         if rc != OK:
             raise LutAmmError(rc, self._L.lutamm_last_error(None).decode())
         self._h = h
+        self._amm_address = ctypes.cast(self._L.lutamm_amm, ctypes.c_void_p).value
         self.device = device
         self.layers: dict[int, _LayerInfo] = {}
 
@@ -287,6 +294,10 @@ class LutAmmContext:
     # -- the operator (names follow the reference)
     def amm_host(self, layer_id: int, input_tensor, output_tensor, n_tokens: int | None = None, flags: int = 0):
         """amm_host() of the reference (src/host/amm_host.cpp:10-30)."""
+        if _fast is not None and self._h:
+            rc = _fast.amm(self._amm_address, self._h.value, layer_id, input_tensor, output_tensor, n_tokens, flags)
+            if rc is not NotImplemented:
+                return None if rc == OK else self._check(rc)
         M = int(n_tokens if n_tokens is not None else input_tensor.shape[0])
         self._check(self._L.lutamm_amm(self._h, layer_id, _ptr(input_tensor), _ptr(output_tensor), M, flags))
 

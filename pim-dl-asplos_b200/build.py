@@ -10,11 +10,13 @@ import glob
 import os
 import shutil
 import subprocess
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libpimdl_b200.so")
 HOST_LIB = os.path.join(HERE, "libpimdl_host.so")
+FASTCALL = os.path.join(HERE, "_fastcall.so")
 TEST_AMM = os.path.join(HERE, "bin", "test_amm")
 TUNER = os.path.join(HERE, "bin", "tuner")
 TEST_LAYER = os.path.join(HERE, "bin", "test_transformer_layer")
@@ -88,9 +90,19 @@ def build_host(force: bool = False) -> None:
                            check=True)
 
 
+def build_fastcall(force: bool = False) -> None:
+    """The operator call as a CPython extension (the ctypes binding serves where Python's headers are missing)."""
+    src, inc = os.path.join(CSRC, "python", "fastcall.c"), sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(inc, "Python.h")):
+        return
+    if force or _stale(FASTCALL, [src]):
+        subprocess.run(["gcc", "-O2", "-Wall", "-fPIC", "-shared", "-I", inc, "-o", FASTCALL, src], check=True)
+
+
 def build_all(force: bool = False, verbose: bool = False) -> None:
     build_cuda(force, verbose)
     build_host(force)
+    build_fastcall(force)
 
 
 if __name__ == "__main__":
