@@ -110,8 +110,9 @@ typedef struct lutamm_plan {
     uint32_t umma_groups;     /* tcgen05 one-hot builder groups of 4 warps (0 = default)  */
     uint32_t umma_operand;    /* where the one-hot operand lives: 0 = default,
                                  1 = shared memory, 2 = tensor memory (TMEM), 3 = tensor memory in the 2:4
-                                 sparse form, on CTA pairs (umma_n_tile 0, 64, 128 or 160; the other
-                                 fields below are the dense kernel's and ignored).  A plan that leaves
+                                 sparse form, on CTA pairs (umma_n_tile 0, 64, 128 or 160, and
+                                 umma_split where every slice gets a pair of its own; the other umma_
+                                 fields are the dense kernel's and ignored).  A plan that leaves
                                  all umma_ fields 0 takes form 3 wherever it applies: row-major output,
                                  no peer stores, no int32 copy                            */
     uint32_t umma_sps;        /* tcgen05: 128-byte slabs of the codebook axis a one-hot builder
@@ -359,6 +360,11 @@ int lutamm_measure_int8_peak(lutamm_ctx* ctx, double* tops, double* mac_per_clk_
  * usable afterwards (error word cleared, split-tile counters re-armed).  The reference has no counterpart: a
  * DPU fault aborts its process (DPU_ASSERT, src/host/dpu_common.h:13). */
 int lutamm_selftest_bounded_wait(lutamm_ctx* ctx, uint32_t polls);
+
+/* A number that changes whenever something changes that a call captured into a CUDA graph has fixed: weights, plans,
+ * activations, the stream, timing, or the address of a scratch buffer that had to grow.  A caller that replays
+ * captured calls compares it with the value it captured under. */
+uint64_t lutamm_generation(const lutamm_ctx* ctx);
 
 /* Kernels of this library launched on this context since creation. */
 uint64_t lutamm_launch_count(const lutamm_ctx* ctx);

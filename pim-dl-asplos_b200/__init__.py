@@ -31,7 +31,7 @@ ABI_SYMBOLS = [
     "lutamm_create", "lutamm_destroy", "lutamm_set_stream", "lutamm_sync", "lutamm_last_error",
     "lutamm_version", "lutamm_load_weights", "lutamm_unload_weights", "lutamm_amm", "lutamm_amm_debug",
     "lutamm_index_calculation", "lutamm_pim_lut", "lutamm_set_plan", "lutamm_get_plan", "lutamm_set_activation", "lutamm_tune",
-    "lutamm_enable_timing", "lutamm_get_timings", "lutamm_launch_count",
+    "lutamm_enable_timing", "lutamm_get_timings", "lutamm_launch_count", "lutamm_generation",
     "lutamm_amm_static_scratch", "lutamm_static_scratch_last_error", "lutamm_build_lut",
     "lutamm_load_weights_layout", "lutamm_measure_int8_peak",
     "lutamm_shard_unique_id", "lutamm_shard_init", "lutamm_shard_finalize", "lutamm_amm_column_sharded",
@@ -150,12 +150,14 @@ def load_library() -> ctypes.CDLL:
     L.lutamm_measure_int8_peak.argtypes = [vp, dp, dp, dp]
     L.lutamm_launch_count.argtypes = [vp]
     L.lutamm_launch_count.restype = ctypes.c_uint64
+    L.lutamm_generation.argtypes = [vp]
+    L.lutamm_generation.restype = ctypes.c_uint64
     L.lutamm_amm_static_scratch.argtypes = [i32, vp, vp, vp, vp, vp, vp, ctypes.POINTER(IndexCalcParams),
                                             ctypes.POINTER(LUTParams)]
     L.lutamm_static_scratch_last_error.argtypes = []
     L.lutamm_static_scratch_last_error.restype = ctypes.c_char_p
     for name in ABI_SYMBOLS:
-        if name not in ("lutamm_version", "lutamm_last_error", "lutamm_launch_count", "lutamm_static_scratch_last_error"):
+        if name not in ("lutamm_version", "lutamm_last_error", "lutamm_launch_count", "lutamm_generation", "lutamm_static_scratch_last_error"):
             getattr(L, name).restype = i32
     _lib = L
     return L
@@ -223,6 +225,7 @@ class LutAmmContext:
         self._h = h
         self._amm_address = ctypes.cast(self._L.lutamm_amm, ctypes.c_void_p).value
         self.device = device
+        self.stream: int | None = None   # the caller's stream, None while the context runs on its own
         self.layers: dict[int, _LayerInfo] = {}
 
     # -- plumbing
@@ -249,6 +252,7 @@ class LutAmmContext:
 
     def set_stream(self, cuda_stream: int | None):
         self._check(self._L.lutamm_set_stream(self._h, cuda_stream or None))
+        self.stream = cuda_stream or None
 
     def sync(self):
         self._check(self._L.lutamm_sync(self._h))
@@ -256,6 +260,11 @@ class LutAmmContext:
     @property
     def launch_count(self) -> int:
         return int(self._L.lutamm_launch_count(self._h))
+
+    @property
+    def generation(self) -> int:
+        """Changes with anything a captured call has fixed (lutamm_generation)."""
+        return self._L.lutamm_generation(self._h)
 
     # -- weights
     def load_weights(self, layer_id: int, centroid, lut, bias, scale: float, lut_bias: float = 0.0,

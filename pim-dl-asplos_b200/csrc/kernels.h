@@ -86,13 +86,15 @@ cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N,
 // the table (sparse_table_bytes of it), at twice the rate.
 size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N);
 cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t N, cudaStream_t s);
-uint32_t sparse_default_tile(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count);
+void sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split);
+void sparse_split_scratch(uint32_t M, uint32_t N, uint32_t n_tile, uint32_t split, size_t* partial_bytes, size_t* counter_bytes);
 bool sparse_tile_ok(uint32_t n_tile);
 cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile,
                              const char** why);
 cudaError_t sparse_make_idx_tmap(CUtensorMap* out, const uint8_t* idx, uint32_t M, uint32_t CB, uint32_t CT, const char** why);
 cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CUtensorMap& idx_map, const CUtensorMap& out_map, uint32_t n_tile,
-                          uint32_t max_ctas, uint32_t* dev_err, cudaStream_t s, const char** why);
+                          uint32_t split, void* partial, uint32_t* counters /* zero between launches */, uint32_t max_ctas,
+                          uint32_t* dev_err, cudaStream_t s, const char** why);
 
 // LUT [CB*CT][N] -> [N][CB*CT]
 cudaError_t launch_transpose_lut(const int8_t* lut, int8_t* lut_t, uint32_t rows, uint32_t cols, cudaStream_t s);

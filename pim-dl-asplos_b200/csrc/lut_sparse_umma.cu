@@ -53,7 +53,11 @@ __host__ __device__ constexpr uint32_t idx_slabs(int lg) { return (idx_width(lg)
 
 struct SparseParams {
     LutArgs a;
-    uint32_t slabs, b_slots, tiles_m, tiles_n, early_trigger;
+    uint32_t slabs;          // of the whole codebook axis
+    uint32_t split, per;     // slices of it, slabs of a slice
+    uint32_t b_slots, tiles_m, tiles_n, early_trigger;
+    uint4* partial;          // split > 1: [tile][CTA][quadrant][slice][chunk of 32 columns][4 columns][row] int32
+    uint32_t* counters;      // split > 1: [tile][CTA][quadrant] x (slices arrived, slices done), zero between launches
     uint32_t* dev_err;
 };
 
@@ -153,14 +157,18 @@ __device__ __forceinline__ void build_row(const uint32_t (&raw)[LG == 3 ? 8 : 4]
     m[1] = meta[1] | 0x88888888u;
 }
 
+// A work item: a tile, or a slice of its codebook axis.
 struct SparseItem {
-    uint32_t m0, n0;
+    uint32_t m0, n0, tile, z, begin, slabs;
 };
+template <bool SPLIT>
 __device__ __forceinline__ SparseItem sparse_item(const SparseParams& p, uint32_t item, uint32_t n_tile, uint32_t rank) {
-    return {(item % p.tiles_m) * (2 * kRows) + rank * kRows, (item / p.tiles_m) * n_tile};
+    const uint32_t tile = SPLIT ? item / p.split : item, z = SPLIT ? item % p.split : 0u, begin = SPLIT ? z * p.per : 0u;
+    return {(tile % p.tiles_m) * (2 * kRows) + rank * kRows, (tile / p.tiles_m) * n_tile, tile, z, begin, SPLIT ? min(p.per, p.slabs - begin) : p.slabs};
 }
 
-template <uint32_t N_TILE, int LG>
+// SPLIT: items are slices of a tile's codebook axis, one per pair.
+template <uint32_t N_TILE, int LG, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_constant__ CUtensorMap idx_map,
                   const __grid_constant__ CUtensorMap out_map, const SparseParams p) {
@@ -188,7 +196,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
 
     const LutArgs& a = p.a;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = cluster_rank();
-    const uint32_t n_items = p.tiles_m * p.tiles_n, n_pairs = gridDim.x >> 1, first = blockIdx.x >> 1;
+    const uint32_t n_items = p.tiles_m * p.tiles_n * (SPLIT ? p.split : 1u), n_pairs = gridDim.x >> 1, first = blockIdx.x >> 1;
 
     if (threadIdx.x == 0) {
         s_misc[1] = 0;
@@ -229,17 +237,17 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             bool ok = true;
             const uint32_t full_leader = map_to_rank(b_full0, 0);
             for (uint32_t item = first; item < n_items && ok; item += n_pairs) {
-                const SparseItem it = sparse_item(p, item, N_TILE, rank);
-                for (uint32_t i = (warp - x0) & (kCopyWarps - 1); i < p.slabs; i += kCopyWarps) {
+                const SparseItem it = sparse_item<SPLIT>(p, item, N_TILE, rank);
+                for (uint32_t i = (warp - x0) & (kCopyWarps - 1); i < it.slabs; i += kCopyWarps) {
                     ok = mbar_wait<32>(b_empty0 + 8 * j, ph ^ 1, s_abort);
                     if (!ok) break;
                     if (rank == 0) mbar_arrive_expect_tx(b_full0 + 8 * j, 2 * kBBytes);
                     tma_load_3d_pair(smem_u32(s_b + (size_t)j * kBBytes), &lut_map, full_leader + 8 * j, 0,
-                                     (int32_t)(it.n0 + rank * kHalfN), (int32_t)(2 * i));
+                                     (int32_t)(it.n0 + rank * kHalfN), (int32_t)(2 * (it.begin + i)));
                     j += kCopyWarps;
                     if (j >= SB) { j -= SB; ph ^= 1; }
                 }
-                x0 += p.slabs;
+                x0 += it.slabs;
             }
         }
         __syncwarp();
@@ -252,12 +260,12 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             uint32_t st = 0, ph = 0;
             bool ok = true;
             for (uint32_t item = first; item < n_items && ok; item += n_pairs) {
-                const SparseItem it = sparse_item(p, item, N_TILE, rank);
-                for (uint32_t i = 0; i < p.slabs; i += kIdxSlabs) {
+                const SparseItem it = sparse_item<SPLIT>(p, item, N_TILE, rank);
+                for (uint32_t i = 0; i < it.slabs; i += kIdxSlabs) {
                     ok = mbar_wait<32>(i_empty0 + 8 * st, ph ^ 1, s_abort);
                     if (!ok) break;
                     mbar_arrive_expect_tx(i_full0 + 8 * st, kIdxBytes);
-                    tma_load_2d(smem_u32(s_idx + st * kIdxBytes), &idx_map, i_full0 + 8 * st, (int32_t)(i * (kSlab >> LG)), (int32_t)it.m0);
+                    tma_load_2d(smem_u32(s_idx + st * kIdxBytes), &idx_map, i_full0 + 8 * st, (int32_t)((it.begin + i) * (kSlab >> LG)), (int32_t)it.m0);
                     if (++st == kIdxStages) { st = 0; ph ^= 1; }
                 }
             }
@@ -274,12 +282,12 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             const uint32_t b_lo0 = (uint32_t)umma_desc_k_sw128(smem_u32(s_b));
             const uint32_t desc_hi = (uint32_t)(umma_desc_k_sw128(0) >> 32);
             for (uint32_t item = first; item < n_items && ok; item += n_pairs, ++t) {
-                const uint32_t ab = t & 1;
+                const uint32_t ab = t & 1, slabs = sparse_item<SPLIT>(p, item, N_TILE, rank).slabs;
                 ok = mbar_wait(acc_empty0 + 8 * ab, ((t >> 1) & 1) ^ 1, s_abort);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + ab * N_TILE;
-                for (uint32_t i = (me - x0) & (kMmaWarps - 1); i < p.slabs; i += kMmaWarps) {
+                for (uint32_t i = (me - x0) & (kMmaWarps - 1); i < slabs; i += kMmaWarps) {
                     const uint32_t x = x0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
                     ok = mbar_wait(b_full0 + 8 * j, pb, s_abort) && mbar_wait(a_full0 + 8 * k, pa, s_abort);
                     if (!ok) break;
@@ -298,7 +306,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     j += kMmaWarps;
                     if (j >= SB) { j -= SB; pb ^= 1; }
                 }
-                x0 += p.slabs;
+                x0 += slabs;
                 if (ok && elect_one()) umma_commit_pair(acc_full0 + 8 * ab);
                 __syncwarp();
             }
@@ -334,9 +342,10 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         uint32_t x0 = 0, st = 0, ph = 0;
         bool ok = true;
         for (uint32_t item = first; item < n_items && ok; item += n_pairs) {
-            for (uint32_t i0 = 0; i0 < p.slabs && ok; i0 += kIdxSlabs) {
+            const uint32_t slabs = sparse_item<SPLIT>(p, item, N_TILE, rank).slabs;
+            for (uint32_t i0 = 0; i0 < slabs && ok; i0 += kIdxSlabs) {
                 ok = mbar_wait(i_full0 + 8 * st, ph, s_abort);
-                for (uint32_t i = (grp - (x0 + i0)) & (kGroups - 1); i < kIdxSlabs && i0 + i < p.slabs && ok; i += kGroups) {
+                for (uint32_t i = (grp - (x0 + i0)) & (kGroups - 1); i < kIdxSlabs && i0 + i < slabs && ok; i += kGroups) {
                     const uint32_t x = x0 + i0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
                     uint32_t raw[kRaw], w[32], m[2];
                     load_raw(s_idx + st * kIdxBytes, i, raw);
@@ -360,7 +369,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                 if (lane == 0) mbar_arrive(i_empty0 + 8 * st);   // this warp has read its rows of the stage
                 if (++st == kIdxStages) { st = 0; ph ^= 1; }
             }
-            x0 += p.slabs;
+            x0 += slabs;
         }
         if (p.early_trigger) pdl_launch_dependents();
     } else {
@@ -374,7 +383,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         uint32_t t = 0, buf = 0;
         bool ok = true;
         for (uint32_t item = first; item < n_items; item += n_pairs, ++t) {
-            const SparseItem it = sparse_item(p, item, N_TILE, rank);
+            const SparseItem it = sparse_item<SPLIT>(p, item, N_TILE, rank);
             const uint32_t ab = t & 1;
             if (p.early_trigger && item + n_pairs >= n_items) pdl_launch_dependents();
             __syncwarp();   // the previous item's reads of bw are done
@@ -388,21 +397,9 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             ok = __shfl_sync(0xffffffffu, w_ok, 0) != 0;
             if (!ok) continue;
             tc_fence_after_sync();
-            for (uint32_t c = 0; c < N_TILE / 32; ++c) {
-                uint32_t v[32];
-                tmem_ld_32x32b_x32(tmem_base + my_lanes + ab * N_TILE + c * 32u, v);
-                tmem_ld_wait();
-                {   // leave the columns at zero for the next item's accumulating MMAs
-                    const uint32_t zero[32] = {};
-                    tmem_st_32x32b_x32(tmem_base + my_lanes + ab * N_TILE + c * 32u, zero);
-                }
-                if (c == N_TILE / 32 - 1) {   // accumulator fully read and cleared: hand the buffer back
-                    tmem_st_wait();
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(empty_leader + 8 * ab);
-                }
-                if (it.n0 + c * 32 >= a.N || it.m0 + quad * 32 >= a.M) continue;   // a block wholly past N or M
+            // v: 32 columns of this thread's row, into the output through the staging buffer and the copy engine
+            auto finish = [&](uint32_t c, const uint32_t (&v)[32]) {
+                if (it.n0 + c * 32 >= a.N || it.m0 + quad * 32 >= a.M) return;   // a block wholly past N or M
                 unsigned char* sg = stg + buf * kStageBytes;
                 if (lane == 0) tma_store_wait_read_1();   // the copy before last has read this buffer
                 __syncwarp();
@@ -430,6 +427,72 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     tma_store_commit();
                 }
                 buf ^= 1;
+            };
+            constexpr uint32_t kChunks = N_TILE / 32;
+            // a slice's place in the partial sums: 256 groups of four columns x 32 rows per chunk, coalesced both ways
+            const uint32_t corner = (it.tile * 2 + rank) * 4 + quad;
+            auto part = [&](uint32_t z, uint32_t c) { return p.partial + (((size_t)corner * p.split + z) * kChunks + c) * 256 + lane; };
+            for (uint32_t c = 0; c < kChunks; ++c) {
+                uint32_t v[32];
+                tmem_ld_32x32b_x32(tmem_base + my_lanes + ab * N_TILE + c * 32u, v);
+                tmem_ld_wait();
+                {   // leave the columns at zero for the next item's accumulating MMAs
+                    const uint32_t zero[32] = {};
+                    tmem_st_32x32b_x32(tmem_base + my_lanes + ab * N_TILE + c * 32u, zero);
+                }
+                if (c == kChunks - 1) {   // accumulator fully read and cleared: hand the buffer back
+                    tmem_st_wait();
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(empty_leader + 8 * ab);
+                }
+                if constexpr (!SPLIT) {
+                    finish(c, v);
+                } else {
+                    uint4* to = part(it.z, c);
+#pragma unroll
+                    for (uint32_t q = 0; q < 8; ++q) __stcg(to + 32 * q, make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+                }
+            }
+            if constexpr (SPLIT) {
+                // The slices of a tile are in progress together (the grid is one item per pair), and their warps for one
+                // quadrant meet here: each waits, bounded, until all have stored, then sums and finishes the chunks
+                // c = slice, slice + split, ...  The last one re-arms the counters.
+                uint32_t* ctr = p.counters + 2 * corner;
+                __threadfence();
+                __syncwarp();
+                uint32_t go = 0;
+                if (lane == 0) {
+                    atomicAdd(ctr, 1u);
+                    for (uint32_t spin = 0; spin < kWaitLimit; ++spin) {
+                        if (*reinterpret_cast<volatile uint32_t*>(ctr) >= p.split) { go = 1; break; }
+                        if ((spin & 63u) == 63u && *s_abort) break;
+                        __nanosleep(32);
+                    }
+                    if (!go) *s_abort = 1u;
+                }
+                ok = __shfl_sync(0xffffffffu, go, 0) != 0;
+                if (!ok) continue;
+                __threadfence();
+                for (uint32_t c = it.z; c < kChunks; c += p.split) {
+                    uint32_t v[32] = {};
+                    for (uint32_t z = 0; z < p.split; ++z) {   // integer sums: the order is immaterial
+                        const uint4* from = part(z, c);
+#pragma unroll
+                        for (uint32_t h = 0; h < 8; h += 4) {   // four loads in flight: registers
+                            uint4 t4[4];
+#pragma unroll
+                            for (uint32_t q = 0; q < 4; ++q) t4[q] = __ldcg(from + 32 * (h + q));
+#pragma unroll
+                            for (uint32_t q = 0; q < 4; ++q) {
+                                v[4 * (h + q)] += t4[q].x; v[4 * (h + q) + 1] += t4[q].y; v[4 * (h + q) + 2] += t4[q].z; v[4 * (h + q) + 3] += t4[q].w;
+                            }
+                        }
+                    }
+                    finish(c, v);
+                }
+                __syncwarp();
+                if (lane == 0 && atomicAdd(ctr + 1, 1u) == p.split - 1) { ctr[0] = 0u; ctr[1] = 0u; }
             }
         }
         if (lane == 0) tma_store_wait_all();   // shared memory and the output are settled before the CTA leaves
@@ -469,9 +532,9 @@ size_t sparse_smem(uint32_t n_tile, int lg, uint32_t b_slots) {
            kEpiWarps * n_tile * 4 + kNumBarriers * 8 + 16 + 1024;
 }
 
-template <uint32_t N_TILE, int LG>
+template <uint32_t N_TILE, int LG, bool SPLIT>
 cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
-    auto k = lut_sparse_kernel<N_TILE, LG>;
+    auto k = lut_sparse_kernel<N_TILE, LG, SPLIT>;
     static SmemOptIn memo;
     cudaError_t e = allow_smem(memo, k, (int)smem);
     if (e != cudaSuccess) return e;
@@ -492,15 +555,15 @@ cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtens
     return cudaLaunchKernelEx(&cfg, k, map, idx_map, out_map, p);
 }
 
-template <uint32_t N_TILE>
+template <uint32_t N_TILE, bool SPLIT>
 cudaError_t run_lg(uint32_t lg, const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
     switch (lg) {
-        case 3: return run<N_TILE, 3>(map, idx_map, out_map, p, pairs, smem, s);
-        case 4: return run<N_TILE, 4>(map, idx_map, out_map, p, pairs, smem, s);
-        case 5: return run<N_TILE, 5>(map, idx_map, out_map, p, pairs, smem, s);
-        case 6: return run<N_TILE, 6>(map, idx_map, out_map, p, pairs, smem, s);
-        case 7: return run<N_TILE, 7>(map, idx_map, out_map, p, pairs, smem, s);
-        default: return run<N_TILE, 8>(map, idx_map, out_map, p, pairs, smem, s);
+        case 3: return run<N_TILE, 3, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        case 4: return run<N_TILE, 4, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        case 5: return run<N_TILE, 5, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        case 6: return run<N_TILE, 6, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        case 7: return run<N_TILE, 7, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        default: return run<N_TILE, 8, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
     }
 }
 
@@ -573,29 +636,46 @@ cudaError_t sparse_make_idx_tmap(CUtensorMap* out, const uint8_t* idx, uint32_t 
     return cudaSuccess;
 }
 
-// Tile width by the time the launch would take: rounds of one tile per pair, each bound by its slabs or, where the
-// codebook axis is short, by the epilogue beside them (0.93 us per 32 columns), and the last tile's epilogue.  A slab
-// takes 170 / 199 / 220 ns at 64 / 128 / 160 columns: at 64 the chain of one slot's turn-around, at 160 close to the
-// tensor pipe's 320 cycles.  (Measured at 32 to 16384 tokens; at 96 columns nothing gained.)
-uint32_t sparse_default_tile(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count) {
-    const uint32_t pairs = sm_count >= 2 ? (uint32_t)sm_count / 2 : 1, slabs = sparse_slabs(CB, CT);
+// slabs whose index bytes fill the 16 bytes a copy must start on: a slice begins at a multiple
+static uint32_t slice_unit(uint32_t CT) { return CT > 16 ? CT / 16 : 1; }
+
+// Tile width and split of the codebook axis by the time the launch would take.  Rounds of one tile per pair, each bound by
+// its slabs or, where the codebook axis is short, by the epilogue beside them (0.93 us per 32 columns), and the last
+// tile's epilogue.  A slab takes 170 / 199 / 220 ns at 64 / 128 / 160 columns: at 64 the chain of one slot's
+// turn-around, at 160 close to the tensor pipe's 320 cycles.  (Measured at 32 to 16384 tokens; at 96 columns nothing
+// gained.)  Where the tiles leave pairs idle the axis is split over them, one item per pair, which costs about 3 us for
+// the partial sums' way through L2.
+void sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split) {
+    const uint32_t pairs = sm_count >= 2 ? (uint32_t)sm_count / 2 : 1, slabs = sparse_slabs(CB, CT), unit = slice_unit(CT);
     const uint64_t tm = (M + 2 * kRows - 1) / (2 * kRows);
     const struct { uint32_t n; float slab_us; } tiles[] = {{64, 0.170f}, {128, 0.199f}, {160, 0.220f}};
-    uint32_t best = 160;
+    *n_tile = 160;
+    *split = 1;
     float least = 3e38f;
     for (const auto& t : tiles) {
         const uint64_t items = tm * ((N + t.n - 1) / t.n), rounds = (items + pairs - 1) / pairs;
-        const float main = slabs * t.slab_us, epi = 0.93f * (t.n / 32);
-        const float us = (float)rounds * (rounds > 1 && epi > main ? epi : main) + 0.25f * (t.n / 32);
-        if (us < least) { least = us; best = t.n; }
+        const uint32_t most = items < pairs ? (uint32_t)(pairs / items) : 1;
+        for (uint32_t s = 1; s <= most && s <= (t.n == 160 ? 1u : 16u) && (s == 1 || s * unit <= slabs); ++s) {
+            const uint32_t per = ((slabs + s - 1) / s + unit - 1) / unit * unit;
+            const float main = per * t.slab_us, epi = 0.93f * (t.n / 32);
+            const float us = (float)rounds * (rounds > 1 && epi > main ? epi : main) + 0.25f * (t.n / 32) + (s > 1 ? 3.0f : 0.f);
+            if (us < least) { least = us; *n_tile = t.n; *split = (slabs + per - 1) / per; }
+        }
     }
-    return best;
 }
 
 bool sparse_tile_ok(uint32_t n_tile) { return n_tile == 64 || n_tile == 128 || n_tile == 160; }
 
+// Scratch of a split launch: partial sums and counter words.
+void sparse_split_scratch(uint32_t M, uint32_t N, uint32_t n_tile, uint32_t split, size_t* partial_bytes, size_t* counter_bytes) {
+    const size_t tiles = (size_t)((M + 2 * kRows - 1) / (2 * kRows)) * ((N + n_tile - 1) / n_tile);
+    *partial_bytes = split > 1 ? tiles * split * 2 * kRows * n_tile * sizeof(int32_t) : 0;
+    *counter_bytes = split > 1 ? tiles * 8 * 2 * sizeof(uint32_t) : 0;
+}
+
 cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CUtensorMap& idx_map, const CUtensorMap& out_map, uint32_t n_tile,
-                          uint32_t max_ctas, uint32_t* dev_err, cudaStream_t s, const char** why) {
+                          uint32_t split, void* partial, uint32_t* counters, uint32_t max_ctas, uint32_t* dev_err, cudaStream_t s,
+                          const char** why) {
     *why = nullptr;
     if (a.M == 0 || a.N == 0) return cudaSuccess;
     SparseParams p;
@@ -603,19 +683,31 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
     p.slabs = sparse_slabs(a.CB, a.CT);
     p.tiles_m = (a.M + 2 * kRows - 1) / (2 * kRows);
     p.tiles_n = (a.N + n_tile - 1) / n_tile;
+    const uint32_t cap = max_ctas / 2, unit = slice_unit(a.CT);
+    // the slices of a tile wait for one another: only where every item has a pair of its own
+    if (!split || n_tile == 160 || (uint64_t)p.tiles_m * p.tiles_n * split > cap || !partial || !counters) split = 1;
+    p.per = ((p.slabs + split - 1) / split + unit - 1) / unit * unit;
+    p.split = (p.slabs + p.per - 1) / p.per;   // no empty slices
+    p.partial = static_cast<uint4*>(partial);
+    p.counters = counters;
     p.dev_err = dev_err;
     const int lg = (int)log2_of(a.CT);
     p.b_slots = kMaxBSlots;   // a multiple of the issuing warps: every slot has one of them
     while (p.b_slots > kMmaWarps && sparse_smem(n_tile, lg, p.b_slots) > kSmemLimit) p.b_slots -= kMmaWarps;
-    const uint64_t items = (uint64_t)p.tiles_m * p.tiles_n;
-    const uint32_t cap = max_ctas / 2, pairs = (uint32_t)(items < cap ? items : cap);
+    const uint64_t items = (uint64_t)p.tiles_m * p.tiles_n * p.split;
+    const uint32_t pairs = (uint32_t)(items < cap ? items : cap);
     // With one tile per pair all pairs reach the end of their main loops together, and the next kernel of the stream
     // may as well be launched; with several they finish a tile apart and its early CTAs would skew it.
     p.early_trigger = items <= cap;
     const size_t smem = sparse_smem(n_tile, lg, p.b_slots);
-    if (n_tile == 64) return run_lg<64>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
-    if (n_tile == 128) return run_lg<128>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
-    if (n_tile == 160) return run_lg<160>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
+#define LUTAMM_SPARSE_CASE(NT, SP) \
+    if (n_tile == NT && (p.split > 1) == SP) return run_lg<NT, SP>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
+    LUTAMM_SPARSE_CASE(64, false)
+    LUTAMM_SPARSE_CASE(64, true)
+    LUTAMM_SPARSE_CASE(128, false)
+    LUTAMM_SPARSE_CASE(128, true)
+    LUTAMM_SPARSE_CASE(160, false)
+#undef LUTAMM_SPARSE_CASE
     *why = "tcgen05 variant: the sparse form is built for 64-, 128- and 160-wide tiles";
     return cudaErrorInvalidValue;
 }

@@ -123,6 +123,7 @@ struct lutamm_ctx {
     lutamm_timings last{};
     bool last_valid = false;
     uint64_t launches = 0;
+    uint64_t generation = 0;  // see lutamm_generation
     std::string err;
     // plans found by lutamm_tune, by shape: (n_tokens, K, N, CB, CT, SM count) -> plan
     std::map<std::vector<uint32_t>, lutamm_plan> plan_cache;
@@ -165,6 +166,7 @@ struct DeviceGuard {
 // grow-only device buffer; `zero` clears newly allocated memory
 int ensure(lutamm_ctx* c, Buf& b, size_t bytes, bool zero = false) {
     if (bytes <= b.cap) return LUTAMM_OK;
+    ++c->generation;
     // Stream order: everything queued so far may still use the old block.
     if (c->s_in) CU_TRY(c, cudaStreamSynchronize(c->s_in));
     CU_TRY(c, cudaStreamSynchronize(c->stream));
@@ -253,13 +255,23 @@ int make_table(lutamm_ctx* c, int8_t** table, size_t bytes, F launch) {
 }
 
 // steps 2+3 on CTA pairs with the sparse operand
-int run_sparse(lutamm_ctx* c, Layer& L, const LutArgs& a, uint32_t n_tile) {
+int run_sparse(lutamm_ctx* c, Layer& L, const LutArgs& a, uint32_t n_tile, uint32_t split) {
     const char* why = nullptr;
     if (reinterpret_cast<uintptr_t>(a.idx) & 15u) return fail(c, LUTAMM_ECUDA, "tcgen05 variant: the index buffer must be 16-byte aligned");
     int r = make_table(c, &L.d_lut_s, sparse_table_bytes(L.CB, L.CT, L.N),
                        [&](int8_t* t) { return launch_sparse_table(L.d_lut, t, L.CB, L.CT, L.N, c->stream); });
     if (r) return r;
-    if (!n_tile) n_tile = sparse_default_tile(a.M, a.CB, a.CT, a.N, c->sm_count);
+    if (!n_tile) {
+        uint32_t s;
+        sparse_default_plan(a.M, a.CB, a.CT, a.N, c->sm_count, &n_tile, &s);
+        if (!split) split = s;
+    }
+    if (split > 1 && (uint64_t)((a.M + 255) / 256) * ((a.N + n_tile - 1) / n_tile) * split > (uint64_t)c->sm_count / 2) split = 1;
+    size_t partial = 0, counters = 0;
+    if (split > 1) {
+        sparse_split_scratch(a.M, a.N, n_tile, split, &partial, &counters);
+        if ((r = ensure(c, c->d_acc_scratch, partial)) || (r = ensure(c, c->d_counters, counters, true))) return r;
+    }
     const int slot = sparse_tile_slot(n_tile);
     cudaError_t e = cudaSuccess;
     if (!L.sparse_map_ok[slot]) {
@@ -277,7 +289,8 @@ int run_sparse(lutamm_ctx* c, Layer& L, const LutArgs& a, uint32_t n_tile) {
         L.sparse_out_m = a.M;
     }
     if (e == cudaSuccess)
-        e = launch_sparse(a, L.sparse_maps[slot], L.sparse_idx_map, L.sparse_out_map, n_tile, (uint32_t)c->sm_count, c->d_err, c->stream, &why);
+        e = launch_sparse(a, L.sparse_maps[slot], L.sparse_idx_map, L.sparse_out_map, n_tile, split, c->d_acc_scratch.p,
+                          static_cast<uint32_t*>(c->d_counters.p), (uint32_t)c->sm_count, c->d_err, c->stream, &why);
     if (e != cudaSuccess) return fail(c, LUTAMM_ECUDA, why ? why : (std::string("tcgen05 launch: ") + cudaGetErrorString(e)));
     ++c->launches;
     return LUTAMM_OK;
@@ -311,7 +324,7 @@ int run_lut(lutamm_ctx* c, Layer& L, const uint8_t* d_idx, float* d_out, int32_t
         const bool sparse_fits = !a.n_peers && !a.acc_out && !a.layout.tiled;
         if (plan.umma_operand == 3 && plan.umma_n_tile && !sparse_tile_ok(plan.umma_n_tile))
             return fail(c, LUTAMM_EINVAL, "umma_n_tile must be 64, 128 or 160 for the sparse form");
-        if (sparse_fits && (plan.umma_operand == 3 || umma_plan_open(plan))) return run_sparse(c, L, a, plan.umma_n_tile);
+        if (sparse_fits && (plan.umma_operand == 3 || umma_plan_open(plan))) return run_sparse(c, L, a, plan.umma_n_tile, plan.umma_split);
         UmmaPlan up;
         const bool dense_plan = plan.umma_operand != 3;   // else: where the sparse form does not fit, the dense default
         umma_default_plan(M, L.CB, L.CT, L.N, c->sm_count, dense_plan ? plan.umma_operand : 0, dense_plan ? plan.umma_n_tile : 0, plan.umma_sps, &up);
@@ -594,6 +607,7 @@ int lutamm_set_stream(lutamm_ctx* c, void* cuda_stream) {
     DeviceGuard g(c->device);
     CU_TRY(c, cudaStreamSynchronize(c->stream));
     c->stream = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : c->own_stream;
+    ++c->generation;
     return LUTAMM_OK;
 }
 
@@ -628,6 +642,7 @@ int lutamm_load_weights_layout(lutamm_ctx* c, int layer_id, const float* centroi
     if ((uint64_t)CB * CT * N >= (1ull << 40)) return fail(c, LUTAMM_EINVAL, "LUT too large");
     DeviceGuard g(c->device);
     CU_TRY(c, cudaStreamSynchronize(c->stream));
+    ++c->generation;
     Layer* old = find_layer(c, layer_id);
     if (old) free_layer(*old);
     Layer& L = c->layers[layer_id];
@@ -714,6 +729,7 @@ int lutamm_unload_weights(lutamm_ctx* c, int layer_id) {
     CU_TRY(c, cudaStreamSynchronize(c->stream));
     free_layer(*L);
     c->layers.erase(layer_id);
+    ++c->generation;
     return LUTAMM_OK;
 }
 
@@ -811,6 +827,7 @@ int lutamm_set_plan(lutamm_ctx* c, int layer_id, const lutamm_plan* plan) {
     if (plan->variant == LUTAMM_VARIANT_UMMA && !umma_supported(L->CB, L->CT, L->N))
         return fail(c, LUTAMM_EUNSUPPORTED, "tcgen05 variant does not cover this shape");
     L->plan = *plan;
+    ++c->generation;
     return LUTAMM_OK;
 }
 
@@ -820,6 +837,7 @@ int lutamm_set_activation(lutamm_ctx* c, int layer_id, uint32_t activation) {
     if (!L) return fail(c, LUTAMM_ENOLAYER, "no weights loaded for layer " + std::to_string(layer_id));
     if (activation > LUTAMM_ACT_GELU_TANH_F16) return fail(c, LUTAMM_EINVAL, "unknown activation");
     L->act = activation;
+    ++c->generation;
     return LUTAMM_OK;
 }
 
@@ -843,6 +861,7 @@ int lutamm_tune(lutamm_ctx* c, int layer_id, uint32_t M, lutamm_plan* best_out) 
     auto hit = c->plan_cache.find(key);
     if (hit != c->plan_cache.end()) {
         L->plan = hit->second;
+        ++c->generation;
         if (best_out) *best_out = hit->second;
         return LUTAMM_OK;
     }
@@ -947,6 +966,7 @@ int lutamm_tune(lutamm_ctx* c, int layer_id, uint32_t M, lutamm_plan* best_out) 
     }
     best.ccs_tokens = best_tok;
     L->plan = best;
+    ++c->generation;
     c->plan_cache[key] = best;
     if (best_out) *best_out = best;
     return LUTAMM_OK;
@@ -997,6 +1017,7 @@ int lutamm_plan_cache_load(lutamm_ctx* c, const char* path) {
 int lutamm_enable_timing(lutamm_ctx* c, int on) {
     if (!c) return fail(nullptr, LUTAMM_EINVAL, "null context");
     c->timing = on != 0;
+    ++c->generation;
     c->last_valid = false;
     return LUTAMM_OK;
 }
@@ -1401,6 +1422,8 @@ int lutamm_selftest_bounded_wait(lutamm_ctx* c, uint32_t polls) {
     ++c->launches;
     return check_dev_err(c);   // LUTAMM_EDEVICE is the expected answer
 }
+
+uint64_t lutamm_generation(const lutamm_ctx* c) { return c ? c->generation : 0; }
 
 uint64_t lutamm_launch_count(const lutamm_ctx* c) { return c ? c->launches : 0; }
 

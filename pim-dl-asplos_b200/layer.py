@@ -30,6 +30,10 @@ import numpy as np
 
 from . import ACT_GELU_TANH, FLAG_ASYNC, LutAmmContext, synth
 
+# Up to this many tokens a forward is replayed from a CUDA graph: the Python and the launches of the layer take the host
+# about 110 us, longer than a GPU needs for a layer of this size.
+GRAPH_TOKENS = 1024
+
 LINEARS = ("qkv", "o", "ffn1", "ffn2")
 SEPARATE_LINEARS = ("q", "k", "v", "o", "ffn1", "ffn2")
 
@@ -155,6 +159,8 @@ class LutTransformerLayer:
         else:
             self.buf["qkv"] = torch.empty(self.n, 3 * self.token_dim, **f32)
         self.amm_ms = 0.0
+        self._graph = None          # (key, graph, input copy, h, f) of the captured forward
+        self._seen, self._seen_key = 0, None
 
     def tune(self):
         return {name: self.ctx.tune(self.ids[name], self.n) for name in self.linears}
@@ -166,6 +172,57 @@ class LutTransformerLayer:
     def forward(self, x):
         """x: contiguous fp32 [n, token_dim] on the context's device; runs on torch's current
         stream, which must be the stream given to ctx.set_stream()."""
+        if self.n <= GRAPH_TOKENS:
+            key = self._graph_key(x)
+            if key is not None:
+                if self._graph is not None and self._graph[0] == key:
+                    _, graph, x_in, h, f = self._graph
+                    x_in.copy_(x)
+                    graph.replay()
+                    return h + f
+                # two ordinary calls under the same key first: they size every buffer, and a caller that keeps
+                # changing something is left alone
+                self._graph = None
+                self._seen = self._seen + 1 if self._seen_key == key else 1
+                self._seen_key = key
+                if self._seen > 2:
+                    self._capture(x, key)
+        h, f = self._body(x)
+        return h + f
+
+    def _graph_key(self, x):
+        """What a captured forward depends on beyond the values in x; None where it does not apply."""
+        torch = self.torch
+        if ("_amm" in self.__dict__ or x.dtype != torch.float32 or x.shape != (self.n, self.token_dim) or x.device.index != self.ctx.device
+                or x.requires_grad or torch.is_autocast_enabled()):
+            return None
+        stream = torch.cuda.current_stream(x.device).cuda_stream
+        if not stream or stream != self.ctx.stream or torch.cuda.is_current_stream_capturing():
+            return None
+        sdp = torch.backends.cuda
+        return (stream, self.ctx.generation, self.fused_gelu, sdp.flash_sdp_enabled(), sdp.mem_efficient_sdp_enabled(), sdp.math_sdp_enabled(),
+                sdp.cudnn_sdp_enabled(), sdp.matmul.allow_tf32, tuple(t.data_ptr() for pair in self.ln.values() for t in pair))
+
+    def _capture(self, x, key):
+        """Record the layer up to its last addition on a copy of the input: 16 launches and their Python become one.
+        The last addition stays outside, so that every call returns a tensor of its own."""
+        torch = self.torch
+        graph = torch.cuda.CUDAGraph()
+        x_in = torch.empty_like(x)
+        try:
+            graph.capture_begin(capture_error_mode="thread_local")
+            try:
+                h, f = self._body(x_in)
+            finally:
+                graph.capture_end()
+        except RuntimeError:
+            self._seen = -(1 << 62)   # this set-up does not capture: ordinary calls from now on
+            return
+        if self.ctx.generation == key[1]:
+            self._graph = (key, graph, x_in, h, f)
+
+    def _body(self, x):
+        """The layer up to its last addition: y = h + f."""
         torch, F = self.torch, self.torch.nn.functional
         B, S, H, D = self.batch, self.seq_len, self.heads, self.token_dim
         hd = D // H
@@ -181,8 +238,7 @@ class LutTransformerLayer:
         f = self._amm("ffn1", h.contiguous())
         if not self.fused_gelu:
             f = F.gelu(f, approximate="tanh")
-        y = h + F.layer_norm(self._amm("ffn2", f), (D,), self.ln["ln2"][0], self.ln["ln2"][1], eps=1e-6)
-        return y
+        return h, F.layer_norm(self._amm("ffn2", f), (D,), self.ln["ln2"][0], self.ln["ln2"][1], eps=1e-6)
 
 
 class LutTransformer:
