@@ -157,6 +157,18 @@ __device__ __forceinline__ void build_row(const uint32_t (&raw)[LG == 3 ? 8 : 4]
     m[1] = meta[1] | 0x88888888u;
 }
 
+// One decision for all values: decided per value, the branches would part the code that has to overlap.
+template <int N>
+__device__ __forceinline__ void activate_all(float (&o)[N], uint32_t act) {
+    if (act == 1u) {
+#pragma unroll
+        for (int q = 0; q < N; ++q) o[q] = activate_one(o[q], 1u);
+    } else if (act) {
+#pragma unroll
+        for (int q = 0; q < N; ++q) o[q] = activate_one(o[q], 2u);
+    }
+}
+
 // A work item: a tile, or a slice of its codebook axis.
 struct SparseItem {
     uint32_t m0, n0, tile, z, begin, slabs;
@@ -413,10 +425,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     o[4 * q + 2] = dequant_one((int32_t)v[4 * q + 2], a.scale, lbcb, b4.z);
                     o[4 * q + 3] = dequant_one((int32_t)v[4 * q + 3], a.scale, lbcb, b4.w);
                 }
-                if (a.act) {
-#pragma unroll
-                    for (uint32_t q = 0; q < 32; ++q) o[q] = activate_one(o[q], a.act);
-                }
+                activate_all(o, a.act);
 #pragma unroll
                 for (uint32_t q = 0; q < 8; ++q)
                     *reinterpret_cast<float4*>(sg + lane * 128 + ((q ^ (lane & 7u)) << 4)) = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
@@ -456,8 +465,9 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             }
             if constexpr (SPLIT) {
                 // The slices of a tile are in progress together (the grid is one item per pair), and their warps for one
-                // quadrant meet here: each waits, bounded, until all have stored, then sums and finishes the chunks
-                // c = slice, slice + split, ...  The last one re-arms the counters.
+                // quadrant meet here: each waits, bounded, until all have stored, then sums and finishes the groups of
+                // four columns g = slice, slice + split, ... - the loads of all slices in flight together: one slice after
+                // the other is a chain of L2 round trips.  The last one re-arms the counters.
                 uint32_t* ctr = p.counters + 2 * corner;
                 __threadfence();
                 __syncwarp();
@@ -467,29 +477,34 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     for (uint32_t spin = 0; spin < kWaitLimit; ++spin) {
                         if (*reinterpret_cast<volatile uint32_t*>(ctr) >= p.split) { go = 1; break; }
                         if ((spin & 63u) == 63u && *s_abort) break;
-                        __nanosleep(32);
+                        __nanosleep(20);
                     }
                     if (!go) *s_abort = 1u;
                 }
                 ok = __shfl_sync(0xffffffffu, go, 0) != 0;
                 if (!ok) continue;
                 __threadfence();
-                for (uint32_t c = it.z; c < kChunks; c += p.split) {
-                    uint32_t v[32] = {};
-                    for (uint32_t z = 0; z < p.split; ++z) {   // integer sums: the order is immaterial
-                        const uint4* from = part(z, c);
+                const uint32_t row = it.m0 + quad * 32 + lane;
+                for (uint32_t g = it.z; g < 8 * kChunks; g += p.split) {
+                    const uint32_t n = it.n0 + 4 * g;
+                    if (n >= a.N) continue;   // N % 16 == 0: four columns are in or out together
+                    constexpr uint32_t kBatch = 8;
+                    uint4 sum = make_uint4(0, 0, 0, 0);
+                    for (uint32_t z0 = 0; z0 < p.split; z0 += kBatch) {   // integer sums: the order is immaterial
+                        uint4 t4[kBatch];
 #pragma unroll
-                        for (uint32_t h = 0; h < 8; h += 4) {   // four loads in flight: registers
-                            uint4 t4[4];
-#pragma unroll
-                            for (uint32_t q = 0; q < 4; ++q) t4[q] = __ldcg(from + 32 * (h + q));
-#pragma unroll
-                            for (uint32_t q = 0; q < 4; ++q) {
-                                v[4 * (h + q)] += t4[q].x; v[4 * (h + q) + 1] += t4[q].y; v[4 * (h + q) + 2] += t4[q].z; v[4 * (h + q) + 3] += t4[q].w;
-                            }
+                        for (uint32_t k = 0; k < kBatch; ++k) {
+                            t4[k] = make_uint4(0, 0, 0, 0);
+                            if (z0 + k < p.split) t4[k] = __ldcg(part(z0 + k, g >> 3) + 32 * (g & 7u));
                         }
+#pragma unroll
+                        for (uint32_t k = 0; k < kBatch; ++k) { sum.x += t4[k].x; sum.y += t4[k].y; sum.z += t4[k].z; sum.w += t4[k].w; }
                     }
-                    finish(c, v);
+                    const float4 b4 = *reinterpret_cast<const float4*>(bw + 4 * g);
+                    float o[4] = {dequant_one((int32_t)sum.x, a.scale, lbcb, b4.x), dequant_one((int32_t)sum.y, a.scale, lbcb, b4.y),
+                                  dequant_one((int32_t)sum.z, a.scale, lbcb, b4.z), dequant_one((int32_t)sum.w, a.scale, lbcb, b4.w)};
+                    activate_all(o, a.act);
+                    if (row < a.M) *reinterpret_cast<float4*>(a.out + (size_t)row * a.N + n) = make_float4(o[0], o[1], o[2], o[3]);
                 }
                 __syncwarp();
                 if (lane == 0 && atomicAdd(ctr + 1, 1u) == p.split - 1) { ctr[0] = 0u; ctr[1] = 0u; }
@@ -643,7 +658,7 @@ static uint32_t slice_unit(uint32_t CT) { return CT > 16 ? CT / 16 : 1; }
 // its slabs or, where the codebook axis is short, by the epilogue beside them (0.93 us per 32 columns), and the last
 // tile's epilogue.  A slab takes 170 / 199 / 220 ns at 64 / 128 / 160 columns: at 64 the chain of one slot's
 // turn-around, at 160 close to the tensor pipe's 320 cycles.  (Measured at 32 to 16384 tokens; at 96 columns nothing
-// gained.)  Where the tiles leave pairs idle the axis is split over them, one item per pair, which costs about 3 us for
+// gained.)  Where the tiles leave pairs idle the axis is split over them, one item per pair, which costs about 4.5 us for
 // the partial sums' way through L2.
 void sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split) {
     const uint32_t pairs = sm_count >= 2 ? (uint32_t)sm_count / 2 : 1, slabs = sparse_slabs(CB, CT), unit = slice_unit(CT);
@@ -658,7 +673,7 @@ void sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int s
         for (uint32_t s = 1; s <= most && s <= (t.n == 160 ? 1u : 16u) && (s == 1 || s * unit <= slabs); ++s) {
             const uint32_t per = ((slabs + s - 1) / s + unit - 1) / unit * unit;
             const float main = per * t.slab_us, epi = 0.93f * (t.n / 32);
-            const float us = (float)rounds * (rounds > 1 && epi > main ? epi : main) + 0.25f * (t.n / 32) + (s > 1 ? 3.0f : 0.f);
+            const float us = (float)rounds * (rounds > 1 && epi > main ? epi : main) + 0.25f * (t.n / 32) + (s > 1 ? 4.5f : 0.f);
             if (us < least) { least = us; *n_tile = t.n; *split = (slabs + per - 1) / per; }
         }
     }
