@@ -45,7 +45,7 @@ constexpr uint32_t kMaxBSlots = 16;
 constexpr uint32_t kStageBytes = 32 * 128;     // a 32 x 32 fp32 block
 constexpr uint32_t kStages = 2;                // per epilogue warp
 constexpr uint32_t kIdxStages = 3;
-constexpr uint32_t kNumBarriers = 2 * kMaxASlots + 2 * kMaxBSlots + 4 + 2 * kIdxStages;
+constexpr uint32_t kNumBarriers = 2 * kMaxASlots + 2 * kMaxBSlots + 4 + 2 * kIdxStages + 4;
 
 // A stage of index bytes: 128 rows of `idx_width` bytes, for `idx_slabs` slabs.
 __host__ __device__ constexpr uint32_t idx_width(int lg) { return lg == 3 ? 64u : lg <= 6 ? 4u * (256u >> lg) : 16u; }
@@ -179,6 +179,87 @@ __device__ __forceinline__ SparseItem sparse_item(const SparseParams& p, uint32_
     return {(tile % p.tiles_m) * (2 * kRows) + rank * kRows, (tile / p.tiles_m) * n_tile, tile, z, begin, SPLIT ? min(p.per, p.slabs - begin) : p.slabs};
 }
 
+// A slice's place in the partial sums of a quadrant (corner: tile, CTA, quadrant): per chunk of 32 columns 8 groups of four
+// columns x 32 rows, coalesced both ways.
+template <uint32_t N_TILE>
+__device__ __forceinline__ uint4* partial_sums(const SparseParams& p, uint32_t corner, uint32_t z, uint32_t c, uint32_t lane) {
+    return p.partial + (((size_t)corner * p.split + z) * (N_TILE / 32) + c) * 256 + lane;
+}
+
+// The end of a split tile.  Its slices are in progress together (the grid is one item per pair); for each quadrant of 32
+// rows the epilogue warp of every slice waits, bounded, until all slices have stored, and then shares out the groups of
+// four columns with the builder warps, who are done.  Eight loads in flight per warp: one slice or group after
+// the other is a chain of L2 round trips (768 codebook slabs in three slices, 1024 tokens: 10 us of it with one warp).
+// The last warp re-arms the counters.
+constexpr uint32_t kSumWarps = 1 + kGroups;
+template <uint32_t N_TILE>
+__device__ __forceinline__ bool split_finish(const SparseParams& p, const SparseItem& it, uint32_t rank, uint32_t quad, uint32_t share, uint32_t lane,
+                                             uint32_t sums_bar, volatile uint32_t* s_abort) {
+    const LutArgs& a = p.a;
+    const uint32_t corner = (it.tile * 2 + rank) * 4 + quad;
+    uint32_t* ctr = p.counters + 2 * corner;   // [0] slices stored, [1] warps done
+    bool go = true;
+    if (share == 0) {
+        if (lane == 0) {
+            go = false;
+            for (uint32_t spin = 0; spin < kWaitLimit && !go; ++spin) {
+                go = *reinterpret_cast<volatile uint32_t*>(ctr) >= p.split;
+                if ((spin & 63u) == 63u && *s_abort) break;
+            }
+            if (go) mbar_arrive(sums_bar + 8 * quad);
+            else *s_abort = 1u;
+        }
+        go = __shfl_sync(0xffffffffu, go, 0);
+    } else {
+        go = mbar_wait<32>(sums_bar + 8 * quad, 0, s_abort);
+    }
+    if (!go) return false;
+    __threadfence();
+    const float lbcb = lut_bias_times_cb(a.lut_bias, a.CB);
+    const uint32_t row = it.m0 + quad * 32 + lane;
+    constexpr uint32_t kUnits = N_TILE / 4;   // groups of four columns
+    const uint32_t step = p.split * kSumWarps;
+    auto store = [&](uint32_t g, const uint4& sum) {
+        const uint32_t n = it.n0 + 4 * g;
+        if (n >= a.N || row >= a.M) return;   // N % 16 == 0: four columns are in or out together
+        const float4 b4 = __ldg(reinterpret_cast<const float4*>(a.bias + n));
+        float o[4] = {dequant_one((int32_t)sum.x, a.scale, lbcb, b4.x), dequant_one((int32_t)sum.y, a.scale, lbcb, b4.y),
+                      dequant_one((int32_t)sum.z, a.scale, lbcb, b4.z), dequant_one((int32_t)sum.w, a.scale, lbcb, b4.w)};
+        activate_all(o, a.act);
+        *reinterpret_cast<float4*>(a.out + (size_t)row * a.N + n) = make_float4(o[0], o[1], o[2], o[3]);
+    };
+    auto load = [&](uint32_t g, uint32_t z) {
+        return g < kUnits && z < p.split ? __ldcg(partial_sums<N_TILE>(p, corner, z, g >> 3, lane) + 32 * (g & 7u)) : make_uint4(0, 0, 0, 0);
+    };
+    auto add = [](uint4& s, const uint4& t) { s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w; };
+    if (p.split <= 4) {   // two groups of up to four slices
+        for (uint32_t g = it.z * kSumWarps + share; g < kUnits; g += 2 * step) {
+            uint4 t0[4], t1[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) { t0[k] = load(g, k); t1[k] = load(g + step, k); }
+#pragma unroll
+            for (uint32_t k = 1; k < 4; ++k) { add(t0[0], t0[k]); add(t1[0], t1[k]); }
+            store(g, t0[0]);
+            if (g + step < kUnits) store(g + step, t1[0]);
+        }
+    } else {
+        for (uint32_t g = it.z * kSumWarps + share; g < kUnits; g += step) {
+            uint4 sum = make_uint4(0, 0, 0, 0);
+            for (uint32_t z0 = 0; z0 < p.split; z0 += 8) {   // integer sums: the order is immaterial
+                uint4 t[8];
+#pragma unroll
+                for (uint32_t k = 0; k < 8; ++k) t[k] = load(g, z0 + k);
+#pragma unroll
+                for (uint32_t k = 0; k < 8; ++k) add(sum, t[k]);
+            }
+            store(g, sum);
+        }
+    }
+    __syncwarp();
+    if (lane == 0 && atomicAdd(ctr + 1, 1u) == p.split * kSumWarps - 1) { ctr[0] = 0u; ctr[1] = 0u; }
+    return true;
+}
+
 // SPLIT: items are slices of a tile's codebook axis, one per pair.
 template <uint32_t N_TILE, int LG, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -204,7 +285,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     volatile uint32_t* s_abort = s_misc + 1;
     const uint32_t a_full0 = smem_u32(s_bar), a_empty0 = a_full0 + 8 * kMaxASlots, b_full0 = a_empty0 + 8 * kMaxASlots,
                    b_empty0 = b_full0 + 8 * kMaxBSlots, acc_full0 = b_empty0 + 8 * kMaxBSlots, acc_empty0 = acc_full0 + 16,
-                   i_full0 = acc_empty0 + 16, i_empty0 = i_full0 + 8 * kIdxStages;
+                   i_full0 = acc_empty0 + 16, i_empty0 = i_full0 + 8 * kIdxStages, sums0 = i_empty0 + 8 * kIdxStages;
 
     const LutArgs& a = p.a;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = cluster_rank();
@@ -221,9 +302,10 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         // a_full: the four builder warps of the slab's group in each CTA; a_empty, b_empty: one commit; b_full: the
         // leader's expect_tx (the copies of both CTAs complete the bytes); acc_full: one commit per issuing warp;
         // acc_empty: the epilogue warps of both CTAs (barriers the
-        // leader waits on are unused in the other CTA); i_full: expect_tx; i_empty: the CTA's builder warps.
+        // leader waits on are unused in the other CTA); i_full: expect_tx; i_empty: the CTA's builder warps;
+        // the last four: a quadrant's partial sums are complete.
         const uint32_t after = 2 * kMaxASlots + 2 * kMaxBSlots;
-        mbar_init(a_full0 + 8 * b, b < kMaxASlots ? 8u : b < after ? 1u : b < after + 2 ? kMmaWarps : b < after + 4 ? 2 * kEpiWarps : b < after + 4 + kIdxStages ? 1u : 4 * kGroups);
+        mbar_init(a_full0 + 8 * b, b < kMaxASlots ? 8u : b < after ? 1u : b < after + 2 ? kMmaWarps : b < after + 4 ? 2 * kEpiWarps : b < after + 4 + kIdxStages ? 1u : b < after + 4 + 2 * kIdxStages ? 4 * kGroups : 1u);
         fence_barrier_init();
     }
     if (warp == kFirstMma) tmem_alloc_pair(smem_u32(s_misc), 512);
@@ -384,6 +466,10 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             x0 += slabs;
         }
         if (p.early_trigger) pdl_launch_dependents();
+        if constexpr (SPLIT) {
+            pdl_wait_prior_grid();
+            if (ok && first < n_items) split_finish<N_TILE>(p, sparse_item<SPLIT>(p, first, N_TILE, rank), rank, warp & 3u, 1 + grp, lane, sums0, s_abort);
+        }
     } else {
         // ---------------- epilogue: each warp on the lane quadrant it may read
         pdl_wait_prior_grid();
@@ -438,9 +524,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                 buf ^= 1;
             };
             constexpr uint32_t kChunks = N_TILE / 32;
-            // a slice's place in the partial sums: 256 groups of four columns x 32 rows per chunk, coalesced both ways
             const uint32_t corner = (it.tile * 2 + rank) * 4 + quad;
-            auto part = [&](uint32_t z, uint32_t c) { return p.partial + (((size_t)corner * p.split + z) * kChunks + c) * 256 + lane; };
             for (uint32_t c = 0; c < kChunks; ++c) {
                 uint32_t v[32];
                 tmem_ld_32x32b_x32(tmem_base + my_lanes + ab * N_TILE + c * 32u, v);
@@ -458,56 +542,16 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                 if constexpr (!SPLIT) {
                     finish(c, v);
                 } else {
-                    uint4* to = part(it.z, c);
+                    uint4* to = partial_sums<N_TILE>(p, corner, it.z, c, lane);
 #pragma unroll
                     for (uint32_t q = 0; q < 8; ++q) __stcg(to + 32 * q, make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
                 }
             }
             if constexpr (SPLIT) {
-                // The slices of a tile are in progress together (the grid is one item per pair), and their warps for one
-                // quadrant meet here: each waits, bounded, until all have stored, then sums and finishes the groups of
-                // four columns g = slice, slice + split, ... - the loads of all slices in flight together: one slice after
-                // the other is a chain of L2 round trips.  The last one re-arms the counters.
-                uint32_t* ctr = p.counters + 2 * corner;
                 __threadfence();
                 __syncwarp();
-                uint32_t go = 0;
-                if (lane == 0) {
-                    atomicAdd(ctr, 1u);
-                    for (uint32_t spin = 0; spin < kWaitLimit; ++spin) {
-                        if (*reinterpret_cast<volatile uint32_t*>(ctr) >= p.split) { go = 1; break; }
-                        if ((spin & 63u) == 63u && *s_abort) break;
-                        __nanosleep(20);
-                    }
-                    if (!go) *s_abort = 1u;
-                }
-                ok = __shfl_sync(0xffffffffu, go, 0) != 0;
-                if (!ok) continue;
-                __threadfence();
-                const uint32_t row = it.m0 + quad * 32 + lane;
-                for (uint32_t g = it.z; g < 8 * kChunks; g += p.split) {
-                    const uint32_t n = it.n0 + 4 * g;
-                    if (n >= a.N) continue;   // N % 16 == 0: four columns are in or out together
-                    constexpr uint32_t kBatch = 8;
-                    uint4 sum = make_uint4(0, 0, 0, 0);
-                    for (uint32_t z0 = 0; z0 < p.split; z0 += kBatch) {   // integer sums: the order is immaterial
-                        uint4 t4[kBatch];
-#pragma unroll
-                        for (uint32_t k = 0; k < kBatch; ++k) {
-                            t4[k] = make_uint4(0, 0, 0, 0);
-                            if (z0 + k < p.split) t4[k] = __ldcg(part(z0 + k, g >> 3) + 32 * (g & 7u));
-                        }
-#pragma unroll
-                        for (uint32_t k = 0; k < kBatch; ++k) { sum.x += t4[k].x; sum.y += t4[k].y; sum.z += t4[k].z; sum.w += t4[k].w; }
-                    }
-                    const float4 b4 = *reinterpret_cast<const float4*>(bw + 4 * g);
-                    float o[4] = {dequant_one((int32_t)sum.x, a.scale, lbcb, b4.x), dequant_one((int32_t)sum.y, a.scale, lbcb, b4.y),
-                                  dequant_one((int32_t)sum.z, a.scale, lbcb, b4.z), dequant_one((int32_t)sum.w, a.scale, lbcb, b4.w)};
-                    activate_all(o, a.act);
-                    if (row < a.M) *reinterpret_cast<float4*>(a.out + (size_t)row * a.N + n) = make_float4(o[0], o[1], o[2], o[3]);
-                }
-                __syncwarp();
-                if (lane == 0 && atomicAdd(ctr + 1, 1u) == p.split - 1) { ctr[0] = 0u; ctr[1] = 0u; }
+                if (lane == 0) atomicAdd(p.counters + 2 * corner, 1u);
+                ok = split_finish<N_TILE>(p, it, rank, quad, 0, lane, sums0, s_abort);
             }
         }
         if (lane == 0) tma_store_wait_all();   // shared memory and the output are settled before the CTA leaves
@@ -658,12 +702,12 @@ static uint32_t slice_unit(uint32_t CT) { return CT > 16 ? CT / 16 : 1; }
 // its slabs or, where the codebook axis is short, by the epilogue beside them (0.93 us per 32 columns), and the last
 // tile's epilogue.  A slab takes 170 / 199 / 220 ns at 64 / 128 / 160 columns: at 64 the chain of one slot's
 // turn-around, at 160 close to the tensor pipe's 320 cycles.  (Measured at 32 to 16384 tokens; at 96 columns nothing
-// gained.)  Where the tiles leave pairs idle the axis is split over them, one item per pair, which costs about 4.5 us for
-// the partial sums' way through L2.
+// gained.)  Where the tiles leave pairs idle the axis is split over them, one item per pair, which costs 5 to 6 us for the
+// partial sums' way through L2 (1536 codebooks -> 768 at 128 tokens 20.7 -> 12.2 us, at 1024 tokens 21.6 -> 17.6).
 void sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split) {
     const uint32_t pairs = sm_count >= 2 ? (uint32_t)sm_count / 2 : 1, slabs = sparse_slabs(CB, CT), unit = slice_unit(CT);
     const uint64_t tm = (M + 2 * kRows - 1) / (2 * kRows);
-    const struct { uint32_t n; float slab_us; } tiles[] = {{64, 0.170f}, {128, 0.199f}, {160, 0.220f}};
+    const struct { uint32_t n; float slab_us, split_us; } tiles[] = {{64, 0.170f, 5.f}, {128, 0.199f, 6.2f}, {160, 0.220f, 0.f}};
     *n_tile = 160;
     *split = 1;
     float least = 3e38f;
@@ -673,7 +717,7 @@ void sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int s
         for (uint32_t s = 1; s <= most && s <= (t.n == 160 ? 1u : 16u) && (s == 1 || s * unit <= slabs); ++s) {
             const uint32_t per = ((slabs + s - 1) / s + unit - 1) / unit * unit;
             const float main = per * t.slab_us, epi = 0.93f * (t.n / 32);
-            const float us = (float)rounds * (rounds > 1 && epi > main ? epi : main) + 0.25f * (t.n / 32) + (s > 1 ? 4.5f : 0.f);
+            const float us = (float)rounds * (rounds > 1 && epi > main ? epi : main) + 0.25f * (t.n / 32) + (s > 1 ? t.split_us : 0.f);
             if (us < least) { least = us; *n_tile = t.n; *split = (slabs + per - 1) / per; }
         }
     }

@@ -42,3 +42,24 @@ def test_sparse_form(ctx, M, CB, CT, N, n_tile):
     ctx.pim_lut(78, idx, y)
     np.testing.assert_allclose(y, oracle.gelu_tanh(want), rtol=1e-5, atol=1e-9)
     ctx.unload_weights(78)
+
+
+@pytest.mark.parametrize("n_tile,split", [(0, 0), (64, 2), (64, 5), (64, 16), (128, 3), (128, 9)])
+@pytest.mark.parametrize("M,CB,CT,N", [(1, 512, 16, 64), (130, 1536, 16, 80), (300, 96, 64, 144), (60, 96, 256, 96), (40, 464, 8, 64)])
+def test_split_codebook_axis(ctx, M, CB, CT, N, n_tile, split):
+    """Slices of one tile on several pairs, summed through scratch; twice, so that the counters have been re-armed."""
+    rng = np.random.default_rng(M + CB + N)
+    lut = rng.integers(-128, 128, (CB, CT, N), dtype=np.int8)
+    bias = rng.standard_normal(N, dtype=np.float32)
+    idx = rng.integers(0, CT, (M, CB), dtype=np.uint8)
+    ctx.load_weights(79, rng.standard_normal((CB, CT, 1), dtype=np.float32), lut, bias, 0.013, 0.3)
+    ctx.set_plan(79, variant=P.VARIANT_UMMA, umma_operand=3 if n_tile else 0, umma_n_tile=n_tile, umma_split=split)
+    want = oracle.dequant(oracle.lut_gather(idx.astype(np.uint16), lut), bias, CB, 0.013, 0.3)
+    for _ in range(2):
+        y = np.full((M, N), np.nan, np.float32)
+        ctx.pim_lut(79, idx, y)
+        assert np.array_equal(y.view(np.uint32), want.view(np.uint32))
+    ctx.set_activation(79, P.ACT_GELU_TANH)
+    ctx.pim_lut(79, idx, y)
+    np.testing.assert_allclose(y, oracle.gelu_tanh(want), rtol=1e-5, atol=1e-9)
+    ctx.unload_weights(79)
