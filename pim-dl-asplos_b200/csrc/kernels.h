@@ -80,12 +80,14 @@ void umma_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_
 uint32_t umma_auto_split(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile, int sm_count);
 
 // fp32 [M][N] row-major output as 32 x 32 blocks with the 128-byte swizzle the epilogues stage them in
-cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N, const char** why);
+// (`pitch`: floats from row to row, 0 = N)
+cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N, const char** why, uint32_t pitch = 0);
 
 // The same contraction on CTA pairs with the one-hot operand 2:4 sparse (row-major fp32 output): from its own layout of
 // the table (sparse_table_bytes of it), at twice the rate.
 size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N);
-cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t N, cudaStream_t s);
+// ... of `n` columns of a table that has `pitch`, from column n0 on
+cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t n, uint32_t n0, uint32_t pitch, cudaStream_t s);
 void sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split);
 void sparse_split_scratch(uint32_t M, uint32_t N, uint32_t n_tile, uint32_t split, size_t* partial_bytes, size_t* counter_bytes);
 bool sparse_tile_ok(uint32_t n_tile);
@@ -94,7 +96,7 @@ cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB,
 cudaError_t sparse_make_idx_tmap(CUtensorMap* out, const uint8_t* idx, uint32_t M, uint32_t CB, uint32_t CT, const char** why);
 cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CUtensorMap& idx_map, const CUtensorMap& out_map, uint32_t n_tile,
                           uint32_t split, void* partial, uint32_t* counters /* zero between launches */, uint32_t max_ctas,
-                          uint32_t* dev_err, cudaStream_t s, const char** why);
+                          bool fresh_table /* written by the kernel before */, uint32_t* dev_err, cudaStream_t s, const char** why);
 
 // LUT [CB*CT][N] -> [N][CB*CT]
 cudaError_t launch_transpose_lut(const int8_t* lut, int8_t* lut_t, uint32_t rows, uint32_t cols, cudaStream_t s);
@@ -104,12 +106,11 @@ struct LutBuildArgs {
     const float* centroid;  // [CB][CT][v]
     const float* weight;    // [K = CB*v][N], row-major
     int8_t* lut;            // out: [CB][CT][N]
-    uint32_t* absmax_bits;  // device scratch word
-    float* scale_out;       // device, one float
-    float* lut_bias_out;    // device, one float
+    uint32_t* words;        // device scratch: maximum and block counter, zero between calls
+    float* scalars;         // mapped host memory: scale, LUT bias
     uint32_t CB, CT, v, N;
 };
-// Three launches on `s`: abs-max pass, quantising pass, scalar finish.
+// Two launches on `s`: abs-max pass, quantising pass.
 cudaError_t launch_lut_build(const LutBuildArgs& a, cudaStream_t s, const char** why);
 
 // LUT in the reference's DPU layout (re-tiled along the output features, tile width T) -> canonical.

@@ -853,11 +853,11 @@ cudaError_t umma_make_tmap(CUtensorMap* out, const int8_t* lut_t, uint32_t CB, u
     return cudaSuccess;
 }
 
-cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N, const char** why) {
+cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N, const char** why, uint32_t pitch) {
     EncodeTiledFn enc = get_encode_tiled();
     if (!enc) { *why = "cuTensorMapEncodeTiled is not available from this driver"; return cudaErrorNotSupported; }
     cuuint64_t dims[2] = {N, M};
-    cuuint64_t strides[1] = {(cuuint64_t)N * 4};
+    cuuint64_t strides[1] = {(cuuint64_t)(pitch ? pitch : N) * 4};
     cuuint32_t box[2] = {32, 32};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -592,7 +592,7 @@ size_t sparse_smem(uint32_t n_tile, int lg, uint32_t b_slots) {
 }
 
 template <uint32_t N_TILE, int LG, bool SPLIT>
-cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
+cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, bool plain, cudaStream_t s) {
     auto k = lut_sparse_kernel<N_TILE, LG, SPLIT>;
     static SmemOptIn memo;
     cudaError_t e = allow_smem(memo, k, (int)smem);
@@ -603,26 +603,27 @@ cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtens
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 2;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = plain ? 1 : 2;   // a programmatic launch copies table slabs before the kernel in front has finished
     return cudaLaunchKernelEx(&cfg, k, map, idx_map, out_map, p);
 }
 
 template <uint32_t N_TILE, bool SPLIT>
-cudaError_t run_lg(uint32_t lg, const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
+cudaError_t run_lg(uint32_t lg, const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, bool plain,
+                   cudaStream_t s) {
     switch (lg) {
-        case 3: return run<N_TILE, 3, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
-        case 4: return run<N_TILE, 4, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
-        case 5: return run<N_TILE, 5, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
-        case 6: return run<N_TILE, 6, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
-        case 7: return run<N_TILE, 7, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
-        default: return run<N_TILE, 8, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        case 3: return run<N_TILE, 3, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
+        case 4: return run<N_TILE, 4, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
+        case 5: return run<N_TILE, 5, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
+        case 6: return run<N_TILE, 6, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
+        case 7: return run<N_TILE, 7, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
+        default: return run<N_TILE, 8, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
     }
 }
 
@@ -635,7 +636,7 @@ size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N) { return (size_t
 // past the last one are zero.  A block turns 256 rows x 64 columns of the canonical table.
 namespace {
 __global__ void __launch_bounds__(256) sparse_table_kernel(const int8_t* __restrict__ lut, int8_t* __restrict__ out, uint32_t rows, uint32_t N,
-                                                           uint32_t lg, uint32_t slabs) {
+                                                           uint32_t first, uint32_t pitch, uint32_t lg, uint32_t slabs) {
     constexpr uint32_t kPitch = 260;
     __shared__ __align__(4) int8_t tile[64 * kPitch];
     const uint32_t slab = blockIdx.x, n0 = blockIdx.y * 64, lg_cbs = 8 - lg;
@@ -644,7 +645,7 @@ __global__ void __launch_bounds__(256) sparse_table_kernel(const int8_t* __restr
         const uint32_t d = ((i >> 2) << 1) | (i & 1u), pos = 2 * ((d << lg_cbs) + c) + ((i >> 1) & 1u);
         const size_t row = (size_t)slab * 256 + r;
         uint32_t v = 0;
-        if (row < rows && n0 + n < N) v = *reinterpret_cast<const uint32_t*>(lut + row * N + n0 + n);   // N % 16 == 0
+        if (row < rows && n0 + n < N) v = *reinterpret_cast<const uint32_t*>(lut + row * pitch + first + n0 + n);   // columns in multiples of 16
 #pragma unroll
         for (uint32_t k = 0; k < 4; ++k) tile[(n + k) * kPitch + pos] = (int8_t)(v >> (8 * k));
     }
@@ -657,9 +658,9 @@ __global__ void __launch_bounds__(256) sparse_table_kernel(const int8_t* __restr
 }
 }  // namespace
 
-cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t N, cudaStream_t s) {
+cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n0, uint32_t pitch, cudaStream_t s) {
     const uint32_t slabs = sparse_slabs(CB, CT);
-    sparse_table_kernel<<<dim3(slabs, (N + 63) / 64), 256, 0, s>>>(lut, out, CB * CT, N, log2_of(CT), slabs);
+    sparse_table_kernel<<<dim3(slabs, (N + 63) / 64), 256, 0, s>>>(lut, out, CB * CT, N, n0, pitch, log2_of(CT), slabs);
     return cudaGetLastError();
 }
 
@@ -733,8 +734,8 @@ void sparse_split_scratch(uint32_t M, uint32_t N, uint32_t n_tile, uint32_t spli
 }
 
 cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CUtensorMap& idx_map, const CUtensorMap& out_map, uint32_t n_tile,
-                          uint32_t split, void* partial, uint32_t* counters, uint32_t max_ctas, uint32_t* dev_err, cudaStream_t s,
-                          const char** why) {
+                          uint32_t split, void* partial, uint32_t* counters, uint32_t max_ctas, bool fresh_table, uint32_t* dev_err,
+                          cudaStream_t s, const char** why) {
     *why = nullptr;
     if (a.M == 0 || a.N == 0) return cudaSuccess;
     SparseParams p;
@@ -760,7 +761,7 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
     p.early_trigger = items <= cap;
     const size_t smem = sparse_smem(n_tile, lg, p.b_slots);
 #define LUTAMM_SPARSE_CASE(NT, SP) \
-    if (n_tile == NT && (p.split > 1) == SP) return run_lg<NT, SP>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
+    if (n_tile == NT && (p.split > 1) == SP) return run_lg<NT, SP>(lg, lut_map, idx_map, out_map, p, pairs, smem, fresh_table, s);
     LUTAMM_SPARSE_CASE(64, false)
     LUTAMM_SPARSE_CASE(64, true)
     LUTAMM_SPARSE_CASE(128, false)

@@ -110,7 +110,7 @@ struct lutamm_ctx {
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     std::map<int, Layer> layers;
-    Buf d_in, d_out, d_idx, d_idx16, d_acc_dbg, d_acc_scratch, d_counters, d_build;
+    Buf d_in, d_out, d_idx, d_idx16, d_acc_dbg, d_acc_scratch, d_counters, d_build, d_build_words;
     // host-buffer pipeline: copy-in and copy-out streams, kHostSlots staging slots
     cudaStream_t s_in = nullptr, s_out = nullptr;
     Buf p_in[kHostSlots], p_out[kHostSlots];
@@ -118,6 +118,7 @@ struct lutamm_ctx {
     uint32_t slot = 0;
     uint32_t* h_err = nullptr;  // the kernels' error word: pinned host memory, mapped
     uint32_t* d_err = nullptr;  // its device address
+    float* h_scalars = nullptr; // words 4 and 5 of that line: what lutamm_build_lut's kernels return
     bool timing = false;
     cudaEvent_t ev[6] = {};
     lutamm_timings last{};
@@ -259,7 +260,7 @@ int run_sparse(lutamm_ctx* c, Layer& L, const LutArgs& a, uint32_t n_tile, uint3
     const char* why = nullptr;
     if (reinterpret_cast<uintptr_t>(a.idx) & 15u) return fail(c, LUTAMM_ECUDA, "tcgen05 variant: the index buffer must be 16-byte aligned");
     int r = make_table(c, &L.d_lut_s, sparse_table_bytes(L.CB, L.CT, L.N),
-                       [&](int8_t* t) { return launch_sparse_table(L.d_lut, t, L.CB, L.CT, L.N, c->stream); });
+                       [&](int8_t* t) { return launch_sparse_table(L.d_lut, t, L.CB, L.CT, L.N, 0, L.N, c->stream); });
     if (r) return r;
     if (!n_tile) {
         uint32_t s;
@@ -290,7 +291,7 @@ int run_sparse(lutamm_ctx* c, Layer& L, const LutArgs& a, uint32_t n_tile, uint3
     }
     if (e == cudaSuccess)
         e = launch_sparse(a, L.sparse_maps[slot], L.sparse_idx_map, L.sparse_out_map, n_tile, split, c->d_acc_scratch.p,
-                          static_cast<uint32_t*>(c->d_counters.p), (uint32_t)c->sm_count, c->d_err, c->stream, &why);
+                          static_cast<uint32_t*>(c->d_counters.p), (uint32_t)c->sm_count, false, c->d_err, c->stream, &why);
     if (e != cudaSuccess) return fail(c, LUTAMM_ECUDA, why ? why : (std::string("tcgen05 launch: ") + cudaGetErrorString(e)));
     ++c->launches;
     return LUTAMM_OK;
@@ -547,13 +548,14 @@ int lutamm_create(lutamm_ctx** out, int device) {
     c->sm_count = prop.multiProcessorCount;
     DeviceGuard g(device);
     if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaHostAlloc(&c->h_err, sizeof(uint32_t), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostAlloc(&c->h_err, 64, cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(&c->d_err, c->h_err, 0) != cudaSuccess) {
         std::string m = std::string("context set-up failed: ") + cudaGetErrorString(cudaGetLastError());
         delete c;
         return fail(nullptr, LUTAMM_ECUDA, m);
     }
     *c->h_err = 0;
+    c->h_scalars = reinterpret_cast<float*>(c->h_err + 4);
     c->stream = c->own_stream;
     for (auto& ev : c->ev) cudaEventCreate(&ev);
     cudaStreamCreateWithFlags(&c->s_in, cudaStreamNonBlocking);
@@ -592,7 +594,7 @@ int lutamm_destroy(lutamm_ctx* c) {
     if (c->s_in) cudaStreamDestroy(c->s_in);
     if (c->s_out) cudaStreamDestroy(c->s_out);
     for (Buf* b : {&c->d_in, &c->d_out, &c->d_idx, &c->d_idx16, &c->d_acc_dbg, &c->d_acc_scratch, &c->d_counters,
-                   &c->d_build})
+                   &c->d_build, &c->d_build_words})
         cudaFree(b->p);
     cudaFreeHost(c->h_err);
     for (auto& ev : c->ev)
@@ -689,11 +691,12 @@ int lutamm_build_lut(lutamm_ctx* c, const float* centroid, const float* weight, 
     DeviceGuard g(c->device);
     const size_t cen_b = (size_t)CB * CT * v * sizeof(float), w_b = (size_t)CB * v * N * sizeof(float),
                  lut_b = (size_t)CB * CT * N;
-    // staging for whichever of the three tensors lives in host memory; [0..255] holds the scalars
+    // staging for whichever of the three tensors lives in host memory
     const bool cen_dev = is_device_ptr(centroid), w_dev = is_device_ptr(weight), lut_dev = is_device_ptr(lut_out);
-    const size_t off_cen = 256, off_w = off_cen + (cen_dev ? 0 : (cen_b + 255) / 256 * 256),
+    const size_t off_cen = 0, off_w = off_cen + (cen_dev ? 0 : (cen_b + 255) / 256 * 256),
                  off_lut = off_w + (w_dev ? 0 : (w_b + 255) / 256 * 256), total = off_lut + (lut_dev ? 0 : lut_b);
     if (int rc = ensure(c, c->d_build, total)) return rc;
+    if (int rc = ensure(c, c->d_build_words, 256, true)) return rc;
     char* base = static_cast<char*>(c->d_build.p);
     const float* d_cen = centroid;
     const float* d_w = weight;
@@ -707,17 +710,16 @@ int lutamm_build_lut(lutamm_ctx* c, const float* centroid, const float* weight, 
         d_w = reinterpret_cast<const float*>(base + off_w);
     }
     if (!lut_dev) d_lut = reinterpret_cast<int8_t*>(base + off_lut);
-    LutBuildArgs a{d_cen, d_w, d_lut, reinterpret_cast<uint32_t*>(base), reinterpret_cast<float*>(base + 16),
-                   reinterpret_cast<float*>(base + 32), CB, CT, v, N};
+    LutBuildArgs a{d_cen, d_w, d_lut, static_cast<uint32_t*>(c->d_build_words.p), reinterpret_cast<float*>(c->d_err + 4), CB, CT, v, N};
     const char* why = nullptr;
     cudaError_t e = launch_lut_build(a, c->stream, &why);
     if (e != cudaSuccess)
         return fail(c, why ? LUTAMM_EINVAL : LUTAMM_ECUDA, why ? std::string(why) : std::string("lut build: ") + cudaGetErrorString(e));
-    c->launches += 3;
+    c->launches += 2;
     if (!lut_dev) CU_TRY(c, cudaMemcpyAsync(lut_out, d_lut, lut_b, cudaMemcpyDeviceToHost, c->stream));
-    CU_TRY(c, cudaMemcpyAsync(scale_out, base + 16, sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-    CU_TRY(c, cudaMemcpyAsync(lut_bias_out, base + 32, sizeof(float), cudaMemcpyDeviceToHost, c->stream));
     CU_TRY(c, cudaStreamSynchronize(c->stream));
+    *scale_out = static_cast<volatile float*>(c->h_scalars)[0];
+    *lut_bias_out = static_cast<volatile float*>(c->h_scalars)[1];
     return LUTAMM_OK;
 }
 

@@ -34,6 +34,7 @@
 //
 // No counterpart in the reference, whose amm_host() allocates (and leaks) its index buffer
 // on every call (inference-engine/src/host/amm_host.cpp:19).
+#include <atomic>
 #include <mutex>
 #include <string>
 
@@ -57,6 +58,39 @@ thread_local std::string g_err;
 int fail(int code, const std::string& msg) {
     g_err = msg;
     return code;
+}
+
+uint32_t sm_count_of(int device) {
+    static std::atomic<uint32_t> known[kMaxDevices] = {};
+    uint32_t n = known[device].load(std::memory_order_relaxed);
+    if (!n) {
+        int v = 0;
+        n = cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && v > 0 ? (uint32_t)v : 148u;
+        known[device].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+// Whether to lay the table out for the tcgen05 kernel on every call, `columns` at a time in what the indices leave of
+// the array (0: the CUDA-core gather, which reads the table as it is).  By estimated time, in microseconds.
+struct TablePlan {
+    uint32_t columns;
+};
+TablePlan plan_table(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, uint32_t sms) {
+    if (!lutamm::umma_supported(CB, CT, N)) return {0};
+    const size_t per_column = lutamm::sparse_table_bytes(CB, CT, 1), used = (((size_t)M * CB + 255) / 256) * 256;
+    const size_t fit = used < LUTAMM_STATIC_SCRATCH_BYTES ? (LUTAMM_STATIC_SCRATCH_BYTES - used) / per_column : 0;
+    uint32_t columns = fit < N ? (uint32_t)(fit / 64 * 64) : N;
+    if (columns == 0) return {0};
+    const uint32_t chunks = (N + columns - 1) / columns;
+    columns = ((N + chunks - 1) / chunks + 63) / 64 * 64;   // near-equal chunks
+    if (columns > N) columns = N;
+    uint32_t n_tile, split;
+    lutamm::sparse_default_plan(M, CB, CT, columns, (int)sms, &n_tile, &split);
+    const double tiles = (double)((M + 255) / 256) * ((columns + n_tile - 1) / n_tile), rounds = (double)(uint64_t)((tiles + sms / 2 - 1) / (sms / 2));
+    const double table = chunks * (8.0 + per_column * (double)columns / 1.5e6 + rounds * per_column / 256 * 0.2);
+    const double ctas = (double)((M + 31) / 32) * ((N + 127) / 128), sum = (double)M * CB * N / 9.7e6, chain = 0.105 * CB * (ctas > sms ? 1.0 + ctas / sms / 8 : 1.0);
+    return {table < 4.0 + (sum > chain ? sum : chain) ? columns : 0u};
 }
 
 }  // namespace
@@ -136,18 +170,40 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
     cudaError_t e = launch_ccs(ca, s, &why);
     if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : (std::string("search launch: ") + cudaGetErrorString(e)));
 
-    // The gather-accumulate kernel reads the LUT in its canonical layout through a tensor map
-    // encoded on the host (no device memory involved) and the indices from the static array.
-    const uint32_t cfg = 0;
-    CUtensorMap map;
-    e = gather_make_tmap(&map, lut, CB, CT, N, cfg, &why);
-    if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : cudaGetErrorString(e));
     LutArgs la{};
     la.idx = d_idx; la.bias = bias; la.out = output; la.acc_out = nullptr;
     la.M = M; la.CB = CB; la.CT = CT; la.N = N;
     la.scale = lp->scale; la.lut_bias = lp->bias;
-    e = launch_gather(la, map, cfg, d_err, s, &why);
-    if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : (std::string("gather launch: ") + cudaGetErrorString(e)));
+    const uint32_t sms = sm_count_of(device);
+    const TablePlan plan = plan_table(M, CB, CT, N, sms);
+    if (plan.columns) {
+        // the tcgen05 kernel on as many columns at a time as the rest of the array holds of its layout of the table
+        int8_t* table = reinterpret_cast<int8_t*>(d_idx + (((size_t)M * CB + 255) / 256) * 256);
+        CUtensorMap idx_map;
+        e = sparse_make_idx_tmap(&idx_map, d_idx, M, CB, CT, &why);
+        for (uint32_t n0 = 0; n0 < N && e == cudaSuccess; n0 += plan.columns) {
+            la.N = N - n0 < plan.columns ? N - n0 : plan.columns;
+            la.bias = bias + n0;
+            la.out = output + n0;
+            uint32_t n_tile, split;
+            sparse_default_plan(M, CB, CT, la.N, (int)sms, &n_tile, &split);
+            CUtensorMap table_map, out_map;
+            e = launch_sparse_table(lut, table, CB, CT, la.N, n0, N, s);
+            if (e == cudaSuccess) e = sparse_make_tmap(&table_map, table, CB, CT, la.N, n_tile, &why);
+            if (e == cudaSuccess) e = make_out_tmap(&out_map, la.out, M, la.N, &why, N);
+            if (e == cudaSuccess) e = launch_sparse(la, table_map, idx_map, out_map, n_tile, 1, nullptr, nullptr, sms, true, d_err, s, &why);
+        }
+        if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : (std::string("tcgen05 launch: ") + cudaGetErrorString(e)));
+    } else {
+        // The gather-accumulate kernel reads the LUT in its canonical layout through a tensor map encoded on the host (no
+        // device memory involved).  Narrow tiles of few tokens where wide ones would leave SMs without a CTA.
+        const uint32_t cfg = (uint64_t)((M + 63) / 64) * ((N + 255) / 256) < sms ? 4 : 0;
+        CUtensorMap map;
+        e = gather_make_tmap(&map, lut, CB, CT, N, cfg, &why);
+        if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : cudaGetErrorString(e));
+        e = launch_gather(la, map, cfg, d_err, s, &why);
+        if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : (std::string("gather launch: ") + cudaGetErrorString(e)));
+    }
 
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(LUTAMM_ECUDA, std::string("cudaStreamSynchronize: ") + cudaGetErrorString(e));
