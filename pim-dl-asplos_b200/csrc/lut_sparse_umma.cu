@@ -55,7 +55,7 @@ struct SparseParams {
     LutArgs a;
     uint32_t slabs;          // of the whole codebook axis
     uint32_t split, per;     // slices of it, slabs of a slice
-    uint32_t b_slots, tiles_m, tiles_n, early_trigger;
+    uint32_t b_slots, tiles_m, tiles_n, group_m, early_trigger;
     uint4* partial;          // split > 1: [tile][CTA][quadrant][slice][chunk of 32 columns][4 columns][row] int32
     uint32_t* counters;      // split > 1: [tile][CTA][quadrant] x (slices arrived, slices done), zero between launches
     uint32_t* dev_err;
@@ -176,7 +176,10 @@ struct SparseItem {
 template <bool SPLIT>
 __device__ __forceinline__ SparseItem sparse_item(const SparseParams& p, uint32_t item, uint32_t n_tile, uint32_t rank) {
     const uint32_t tile = SPLIT ? item / p.split : item, z = SPLIT ? item % p.split : 0u, begin = SPLIT ? z * p.per : 0u;
-    return {(tile % p.tiles_m) * (2 * kRows) + rank * kRows, (tile / p.tiles_m) * n_tile, tile, z, begin, SPLIT ? min(p.per, p.slabs - begin) : p.slabs};
+    // row tiles in groups, column tiles within a group, row tiles of the group innermost
+    const uint32_t g = tile / (p.group_m * p.tiles_n), in = tile - g * p.group_m * p.tiles_n, rows = min(p.group_m, p.tiles_m - g * p.group_m);
+    const uint32_t tn = in / rows, tm = g * p.group_m + in - tn * rows;
+    return {tm * (2 * kRows) + rank * kRows, tn * n_tile, tile, z, begin, SPLIT ? min(p.per, p.slabs - begin) : p.slabs};
 }
 
 // A slice's place in the partial sums of a quadrant (corner: tile, CTA, quadrant): per chunk of 32 columns 8 groups of four
@@ -756,6 +759,10 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
     while (p.b_slots > kMmaWarps && sparse_smem(n_tile, lg, p.b_slots) > kSmemLimit) p.b_slots -= kMmaWarps;
     const uint64_t items = (uint64_t)p.tiles_m * p.tiles_n * p.split;
     const uint32_t pairs = (uint32_t)(items < cap ? items : cap);
+    // All pairs work on the same columns at a time and share their slabs in L2.  Where the indices of all rows would not
+    // stay there from one column tile to the next (65536 tokens x 2048 codebooks: 134 MB, read from memory 103 times),
+    // go through the columns with as many row tiles as there are pairs: 13.8 GB of reads become 1.9 GB of table.
+    p.group_m = (uint64_t)a.M * a.CB > (48ull << 20) && p.tiles_m > cap ? cap : p.tiles_m;
     // With one tile per pair all pairs reach the end of their main loops together, and the next kernel of the stream
     // may as well be launched; with several they finish a tile apart and its early CTAs would skew it.
     p.early_trigger = items <= cap;

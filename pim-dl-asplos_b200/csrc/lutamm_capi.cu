@@ -418,13 +418,15 @@ int check_dev_err(lutamm_ctx* c) {
 // and both directions of the host link are busy at once.  The reference's counterpart are the
 // serial host<->DPU transfers around dpu_launch (pim_lut_host.cpp:143-181).
 int amm_host_pipelined(lutamm_ctx* c, Layer& L, const float* input, float* output, uint32_t M, uint32_t flags) {
-    // Token slabs of at least 512 rows, at most four per call: a call's first copy-in and last copy-out overlap
-    // nothing, so halving them pays (BERT-base at 1024 tokens: 0.80 -> 0.73 ms per four-linear step through host
-    // buffers), while slabs of 256 rows or more than four slabs cost more in small copies and launches than they hide.
-    uint32_t chunks = M >= 1024 ? M / 512 : 1;
-    if (chunks > 4) chunks = 4;
-    uint32_t rows = ((M + chunks - 1) / chunks + 127) / 128 * 128;
-    if ((flags & LUTAMM_FLAG_OUTPUT_TILED) || rows >= M) { rows = M; }
+    // A call goes through whole up to 2047 tokens, from there on in slabs of at least 1024, at most four: what a call
+    // cannot overlap is its first copy-in and its last copy-out, but small copies and launches cost more than they hide
+    // (BERT-base at 1024 tokens, four linears: whole 674 us, halves 679, quarters 775).  Only when the pipeline is idle -
+    // the last result has left - does a call open with 256 rows, so that the copies out, which bound the whole, start early.
+    const uint32_t chunks = M >= 2048 ? std::min(4u, M / 1024) : 1;
+    uint32_t rows = ((M + chunks - 1) / chunks + 127) / 128 * 128, opening = 0;
+    if ((flags & LUTAMM_FLAG_OUTPUT_TILED) || rows >= M) rows = M;
+    if (!(flags & LUTAMM_FLAG_OUTPUT_TILED) && M >= 512 && cudaEventQuery(c->ev_out[(c->slot + kHostSlots - 1) % kHostSlots]) == cudaSuccess) opening = 256;
+    cudaGetLastError();   // "not ready" is an answer
     int r;
     if ((r = ensure(c, c->d_idx, (size_t)rows * L.CB))) return r;
     constexpr uint32_t n_slots = kHostSlots;
@@ -432,8 +434,8 @@ int amm_host_pipelined(lutamm_ctx* c, Layer& L, const float* input, float* outpu
         if ((r = ensure(c, c->p_in[k], (size_t)rows * L.K * sizeof(float)))) return r;
         if ((r = ensure(c, c->p_out[k], (size_t)rows * L.N * sizeof(float)))) return r;
     }
-    for (uint32_t m0 = 0; m0 < M; m0 += rows) {
-        const uint32_t m = std::min(rows, M - m0);
+    for (uint32_t m0 = 0, m; m0 < M; m0 += m) {
+        m = std::min(m0 == 0 && opening ? opening : rows, M - m0);
         const uint32_t k = c->slot++ % n_slots;
         float* d_x = static_cast<float*>(c->p_in[k].p);
         float* d_y = static_cast<float*>(c->p_out[k].p);
