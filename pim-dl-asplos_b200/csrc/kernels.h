@@ -86,8 +86,8 @@ cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N,
 // The same contraction on CTA pairs with the one-hot operand 2:4 sparse (row-major fp32 output): from its own layout of
 // the table (sparse_table_bytes of it), at twice the rate.
 size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N);
-// ... of `n` columns of a table that has `pitch`, from column n0 on
-cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t n, uint32_t n0, uint32_t pitch, cudaStream_t s);
+// ... of `n` columns of a table that has `pitch`, from column n0 on; chained: nothing the stream still runs writes `lut`
+cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t n, uint32_t n0, uint32_t pitch, bool chained, cudaStream_t s);
 void sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split);
 void sparse_split_scratch(uint32_t M, uint32_t N, uint32_t n_tile, uint32_t split, size_t* partial_bytes, size_t* counter_bytes);
 bool sparse_tile_ok(uint32_t n_tile);
@@ -96,7 +96,7 @@ cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB,
 cudaError_t sparse_make_idx_tmap(CUtensorMap* out, const uint8_t* idx, uint32_t M, uint32_t CB, uint32_t CT, const char** why);
 cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CUtensorMap& idx_map, const CUtensorMap& out_map, uint32_t n_tile,
                           uint32_t split, void* partial, uint32_t* counters /* zero between launches */, uint32_t max_ctas,
-                          bool fresh_table /* written by the kernel before */, uint32_t* dev_err, cudaStream_t s, const char** why);
+                          bool fresh_table /* written by a kernel the stream may still run */, uint32_t* dev_err, cudaStream_t s, const char** why);
 
 // LUT [CB*CT][N] -> [N][CB*CT]
 cudaError_t launch_transpose_lut(const int8_t* lut, int8_t* lut_t, uint32_t rows, uint32_t cols, cudaStream_t s);

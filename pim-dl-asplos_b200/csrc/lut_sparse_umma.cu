@@ -55,7 +55,7 @@ struct SparseParams {
     LutArgs a;
     uint32_t slabs;          // of the whole codebook axis
     uint32_t split, per;     // slices of it, slabs of a slice
-    uint32_t b_slots, tiles_m, tiles_n, group_m, early_trigger;
+    uint32_t b_slots, tiles_m, tiles_n, group_m, early_trigger, fresh_table;
     uint4* partial;          // split > 1: [tile][CTA][quadrant][slice][chunk of 32 columns][4 columns][row] int32
     uint32_t* counters;      // split > 1: [tile][CTA][quadrant] x (slices arrived, slices done), zero between launches
     uint32_t* dev_err;
@@ -327,8 +327,10 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     tc_fence_after_sync();
 
     if (warp < kCopyWarps) {
-        // ---------------- LUT copies (the LUT never depends on the preceding kernel), slab x by warp x % kCopyWarps: a
-        // thread sustains one copy per ~ 480 cycles, of which the instruction itself holds it for 350
+        // ---------------- LUT copies (unless it was laid out just now the LUT does not depend on the preceding kernel),
+        // slab x by warp x % kCopyWarps: a thread sustains one copy per ~ 480 cycles, of which the instruction itself
+        // holds it for 350
+        if (p.fresh_table) pdl_wait_prior_grid();
         if (lane == 0) {
             uint32_t j = warp, ph = 0, x0 = 0;
             bool ok = true;
@@ -595,7 +597,7 @@ size_t sparse_smem(uint32_t n_tile, int lg, uint32_t b_slots) {
 }
 
 template <uint32_t N_TILE, int LG, bool SPLIT>
-cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, bool plain, cudaStream_t s) {
+cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
     auto k = lut_sparse_kernel<N_TILE, LG, SPLIT>;
     static SmemOptIn memo;
     cudaError_t e = allow_smem(memo, k, (int)smem);
@@ -613,20 +615,19 @@ cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtens
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = plain ? 1 : 2;   // a programmatic launch copies table slabs before the kernel in front has finished
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, k, map, idx_map, out_map, p);
 }
 
 template <uint32_t N_TILE, bool SPLIT>
-cudaError_t run_lg(uint32_t lg, const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, bool plain,
-                   cudaStream_t s) {
+cudaError_t run_lg(uint32_t lg, const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
     switch (lg) {
-        case 3: return run<N_TILE, 3, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
-        case 4: return run<N_TILE, 4, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
-        case 5: return run<N_TILE, 5, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
-        case 6: return run<N_TILE, 6, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
-        case 7: return run<N_TILE, 7, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
-        default: return run<N_TILE, 8, SPLIT>(map, idx_map, out_map, p, pairs, smem, plain, s);
+        case 3: return run<N_TILE, 3, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        case 4: return run<N_TILE, 4, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        case 5: return run<N_TILE, 5, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        case 6: return run<N_TILE, 6, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        case 7: return run<N_TILE, 7, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        default: return run<N_TILE, 8, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
     }
 }
 
@@ -636,35 +637,62 @@ size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N) { return (size_t
 
 // The table as the kernel above wants it: [N][slabs * 256], row n's slab s holding at position 2 (d * codebooks + c) + h
 // the entry of codebook s * codebooks + c and centroid index (d without its bit 1, h = bit 1); positions of codebooks
-// past the last one are zero.  A block turns 256 rows x 64 columns of the canonical table.
+// past the last one are zero.  A block turns 256 rows x 64 columns of the canonical table: a thread takes the four rows
+// that make one word of the result, four columns of each, and turns the 4 x 4 bytes in registers.
+//
+// What bounds it: the latency of one round of loads, so all 16 of a thread are in flight together (one after another
+// a 1024-column table of 384 codebooks took 12 us; the call that lays out three of them in a row 88 -> 53 us).  In a chain of tables and contractions through the same memory
+// (`chained`: the canonical table was complete before the kernel in front began) they are issued while that one still
+// runs, on the SMs it leaves idle; the stores wait for it.
 namespace {
 __global__ void __launch_bounds__(256) sparse_table_kernel(const int8_t* __restrict__ lut, int8_t* __restrict__ out, uint32_t rows, uint32_t N,
-                                                           uint32_t first, uint32_t pitch, uint32_t lg, uint32_t slabs) {
-    constexpr uint32_t kPitch = 260;
-    __shared__ __align__(4) int8_t tile[64 * kPitch];
-    const uint32_t slab = blockIdx.x, n0 = blockIdx.y * 64, lg_cbs = 8 - lg;
-    for (uint32_t e = threadIdx.x; e < 256 * 16; e += 256) {
-        const uint32_t r = e >> 4, n = (e & 15u) * 4, i = r & ((1u << lg) - 1u), c = r >> lg;
-        const uint32_t d = ((i >> 2) << 1) | (i & 1u), pos = 2 * ((d << lg_cbs) + c) + ((i >> 1) & 1u);
-        const size_t row = (size_t)slab * 256 + r;
-        uint32_t v = 0;
-        if (row < rows && n0 + n < N) v = *reinterpret_cast<const uint32_t*>(lut + row * pitch + first + n0 + n);   // columns in multiples of 16
+                                                           uint32_t first, uint32_t pitch, uint32_t lg, uint32_t slabs, bool chained) {
+    constexpr uint32_t kPitch = 65;   // words
+    __shared__ uint32_t tile[64 * kPitch];
+    pdl_launch_dependents();
+    if (!chained) pdl_wait_prior_grid();
+    const uint32_t slab = blockIdx.x, n0 = blockIdx.y * 64, lg_cbs = 8 - lg, n = (threadIdx.x & 15u) * 4, w0 = threadIdx.x >> 4;
+    uint32_t v[4][4];
 #pragma unroll
-        for (uint32_t k = 0; k < 4; ++k) tile[(n + k) * kPitch + pos] = (int8_t)(v >> (8 * k));
+    for (uint32_t u = 0; u < 4; ++u) {
+#pragma unroll
+        for (uint32_t b = 0; b < 4; ++b) {
+            const uint32_t pos = 4 * (w0 + 16 * u) + b, d = (pos >> 1) >> lg_cbs, c = (pos >> 1) & ((1u << lg_cbs) - 1u);
+            const uint32_t row = slab * 256 + (c << lg) + ((d >> 1) << 2 | (pos & 1u) << 1 | (d & 1u));
+            v[u][b] = 0;
+            if (row < rows && n0 + n < N) v[u][b] = *reinterpret_cast<const uint32_t*>(lut + (size_t)row * pitch + first + n0 + n);   // columns in multiples of 16
+        }
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u) {
+        const uint32_t l0 = __byte_perm(v[u][0], v[u][1], 0x5140), l1 = __byte_perm(v[u][2], v[u][3], 0x5140);
+        const uint32_t h0 = __byte_perm(v[u][0], v[u][1], 0x7362), h1 = __byte_perm(v[u][2], v[u][3], 0x7362);
+        uint32_t* t = tile + n * kPitch + w0 + 16 * u;
+        t[0] = __byte_perm(l0, l1, 0x5410); t[kPitch] = __byte_perm(l0, l1, 0x7632);
+        t[2 * kPitch] = __byte_perm(h0, h1, 0x5410); t[3 * kPitch] = __byte_perm(h0, h1, 0x7632);
     }
     __syncthreads();
-    for (uint32_t e = threadIdx.x; e < 64 * 64; e += 256) {
-        const uint32_t n = e >> 6, w = e & 63u;
-        if (n0 + n < N)
-            *reinterpret_cast<uint32_t*>(out + ((size_t)(n0 + n) * slabs + slab) * 256 + 4 * w) = *reinterpret_cast<const uint32_t*>(tile + n * kPitch + 4 * w);
+    if (chained) pdl_wait_prior_grid();
+#pragma unroll
+    for (uint32_t k = 0; k < 16; ++k) {
+        const uint32_t r = (threadIdx.x >> 6) + 4 * k, w = threadIdx.x & 63u;
+        if (n0 + r < N) *reinterpret_cast<uint32_t*>(out + ((size_t)(n0 + r) * slabs + slab) * 256 + 4 * w) = tile[r * kPitch + w];
     }
 }
 }  // namespace
 
-cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n0, uint32_t pitch, cudaStream_t s) {
+cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n0, uint32_t pitch, bool chained, cudaStream_t s) {
     const uint32_t slabs = sparse_slabs(CB, CT);
-    sparse_table_kernel<<<dim3(slabs, (N + 63) / 64), 256, 0, s>>>(lut, out, CB * CT, N, n0, pitch, log2_of(CT), slabs);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(slabs, (N + 63) / 64);
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, sparse_table_kernel, lut, out, CB * CT, N, n0, pitch, log2_of(CT), slabs, chained);
 }
 
 // That table as boxes of half a tile's rows of one slab: x = position within 128, y = row, z = half slab.
@@ -766,9 +794,10 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
     // With one tile per pair all pairs reach the end of their main loops together, and the next kernel of the stream
     // may as well be launched; with several they finish a tile apart and its early CTAs would skew it.
     p.early_trigger = items <= cap;
+    p.fresh_table = fresh_table;
     const size_t smem = sparse_smem(n_tile, lg, p.b_slots);
 #define LUTAMM_SPARSE_CASE(NT, SP) \
-    if (n_tile == NT && (p.split > 1) == SP) return run_lg<NT, SP>(lg, lut_map, idx_map, out_map, p, pairs, smem, fresh_table, s);
+    if (n_tile == NT && (p.split > 1) == SP) return run_lg<NT, SP>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
     LUTAMM_SPARSE_CASE(64, false)
     LUTAMM_SPARSE_CASE(64, true)
     LUTAMM_SPARSE_CASE(128, false)

@@ -260,7 +260,7 @@ int run_sparse(lutamm_ctx* c, Layer& L, const LutArgs& a, uint32_t n_tile, uint3
     const char* why = nullptr;
     if (reinterpret_cast<uintptr_t>(a.idx) & 15u) return fail(c, LUTAMM_ECUDA, "tcgen05 variant: the index buffer must be 16-byte aligned");
     int r = make_table(c, &L.d_lut_s, sparse_table_bytes(L.CB, L.CT, L.N),
-                       [&](int8_t* t) { return launch_sparse_table(L.d_lut, t, L.CB, L.CT, L.N, 0, L.N, c->stream); });
+                       [&](int8_t* t) { return launch_sparse_table(L.d_lut, t, L.CB, L.CT, L.N, 0, L.N, false, c->stream); });
     if (r) return r;
     if (!n_tile) {
         uint32_t s;

@@ -88,7 +88,7 @@ TablePlan plan_table(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, uint32_t 
     uint32_t n_tile, split;
     lutamm::sparse_default_plan(M, CB, CT, columns, (int)sms, &n_tile, &split);
     const double tiles = (double)((M + 255) / 256) * ((columns + n_tile - 1) / n_tile), rounds = (double)(uint64_t)((tiles + sms / 2 - 1) / (sms / 2));
-    const double table = chunks * (8.0 + per_column * (double)columns / 1.5e6 + rounds * per_column / 256 * 0.2);
+    const double table = chunks * (5.0 + per_column * (double)columns / 2.5e6 + rounds * per_column / 256 * 0.2);
     const double ctas = (double)((M + 31) / 32) * ((N + 127) / 128), sum = (double)M * CB * N / 9.7e6, chain = 0.105 * CB * (ctas > sms ? 1.0 + ctas / sms / 8 : 1.0);
     return {table < 4.0 + (sum > chain ? sum : chain) ? columns : 0u};
 }
@@ -188,7 +188,8 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
             uint32_t n_tile, split;
             sparse_default_plan(M, CB, CT, la.N, (int)sms, &n_tile, &split);
             CUtensorMap table_map, out_map;
-            e = launch_sparse_table(lut, table, CB, CT, la.N, n0, N, s);
+            // (the second table and on: the contraction in front began when all that the caller had queued was complete)
+            e = launch_sparse_table(lut, table, CB, CT, la.N, n0, N, n0 > 0, s);
             if (e == cudaSuccess) e = sparse_make_tmap(&table_map, table, CB, CT, la.N, n_tile, &why);
             if (e == cudaSuccess) e = make_out_tmap(&out_map, la.out, M, la.N, &why, N);
             if (e == cudaSuccess) e = launch_sparse(la, table_map, idx_map, out_map, n_tile, 1, nullptr, nullptr, sms, true, d_err, s, &why);
