@@ -38,13 +38,16 @@ constexpr uint32_t kSlab = 256;                // positions of the contraction a
 constexpr uint32_t kGroups = 4, kCopyWarps = 2, kIndexWarps = 1, kMmaWarps = 4, kEpiWarps = 4;
 constexpr uint32_t kFirstMma = kCopyWarps + kIndexWarps, kFirstBuilder = kFirstMma + kMmaWarps, kFirstEpi = kFirstBuilder + 4 * kGroups;
 constexpr uint32_t kThreads = (kFirstEpi + kEpiWarps) * 32;   // 864
-// operand slots, 32 columns of bytes and 2 of metadata each: what two accumulators leave, in multiples of the groups
-__host__ __device__ constexpr uint32_t operand_slots(uint32_t n_tile) { return (512 - 2 * n_tile) / 34 >= 8 ? 8 : 4; }
+// Wider tiles than 160 columns are for launches of one tile per pair: a second accumulator would leave no room for slots.
+__host__ __device__ constexpr uint32_t accumulators(uint32_t n_tile) { return n_tile > 160 ? 1 : 2; }
+// operand slots, 32 columns of bytes and 2 of metadata each: what the accumulators leave, in multiples of the groups
+__host__ __device__ constexpr uint32_t operand_slots(uint32_t n_tile) { return (512 - accumulators(n_tile) * n_tile) / 34 >= 8 ? 8 : 4; }
 constexpr uint32_t kMaxASlots = 8;
 constexpr uint32_t kMaxBSlots = 16;
 constexpr uint32_t kStageBytes = 32 * 128;     // a 32 x 32 fp32 block
 constexpr uint32_t kStages = 2;                // per epilogue warp
 constexpr uint32_t kIdxStages = 3;
+__host__ __device__ constexpr uint32_t stage_blocks(uint32_t n_tile) { return accumulators(n_tile) == 1 ? 0 : kEpiWarps * kStages; }
 constexpr uint32_t kNumBarriers = 2 * kMaxASlots + 2 * kMaxBSlots + 4 + 2 * kIdxStages + 4;
 
 // A stage of index bytes: 128 rows of `idx_width` bytes, for `idx_slabs` slabs.
@@ -55,7 +58,7 @@ struct SparseParams {
     LutArgs a;
     uint32_t slabs;          // of the whole codebook axis
     uint32_t split, per;     // slices of it, slabs of a slice
-    uint32_t b_slots, tiles_m, tiles_n, group_m, early_trigger, fresh_table;
+    uint32_t b_slots, tiles_m, tiles_n, group_m, one_tile, early_trigger, fresh_table;
     uint4* partial;          // split > 1: [tile][CTA][quadrant][slice][chunk of 32 columns][4 columns][row] int32
     uint32_t* counters;      // split > 1: [tile][CTA][quadrant] x (slices arrived, slices done), zero between launches
     uint32_t* dev_err;
@@ -271,7 +274,8 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     constexpr uint32_t kHalfN = N_TILE / 2, kBBytes = kHalfN * kSlab;
     constexpr uint32_t kIdesc = umma_idesc_i8(2 * kRows, N_TILE, 1, 1) | kIdescSparse;
     constexpr uint32_t kASlots = operand_slots(N_TILE);
-    constexpr uint32_t kDataBase = 2 * N_TILE, kMetaBase = kDataBase + 32 * kASlots;   // tensor-memory columns
+    constexpr bool kOne = accumulators(N_TILE) == 1;
+    constexpr uint32_t kDataBase = accumulators(N_TILE) * N_TILE, kMetaBase = kDataBase + 32 * kASlots;   // tensor-memory columns
     static_assert(kMetaBase + 2 * kASlots <= 512, "tensor memory");
 
     constexpr uint32_t kIdxWidth = idx_width(LG), kIdxSlabs = idx_slabs(LG), kIdxBytes = kRows * kIdxWidth;
@@ -281,7 +285,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     const uint32_t SB = p.b_slots;
     unsigned char* s_b = smem;                                        // [SB][2][kHalfN][128]
     unsigned char* s_stage = s_b + (size_t)SB * kBBytes;              // [4][kStages][32][128]
-    unsigned char* s_idx = s_stage + kEpiWarps * kStages * kStageBytes;   // [kIdxStages][128][idx_width]
+    unsigned char* s_idx = s_stage + stage_blocks(N_TILE) * kStageBytes;   // [kIdxStages][128][idx_width]
     float* s_bias = reinterpret_cast<float*>(s_idx + kIdxStages * kIdxBytes);   // [4][N_TILE]
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_bias + kEpiWarps * N_TILE);
     uint32_t* s_misc = reinterpret_cast<uint32_t*>(s_bar + kNumBarriers);                  // tmem base, abort
@@ -317,14 +321,65 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     tc_fence_after_sync();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(s_misc);
     const uint32_t my_lanes = ((warp & 3u) * 32u) << 16;
-    if (warp >= kFirstEpi) {   // every MMA accumulates: both accumulators start at zero
-        const uint32_t zero[32] = {};
-        for (uint32_t c = 0; c < 2 * N_TILE; c += 32) tmem_st_32x32b_x32(tmem_base + my_lanes + c, zero);
+    if (warp >= kFirstEpi) {   // every MMA accumulates: the accumulators start at zero
+        const uint32_t zero[32] = {}, used = p.one_tile ? N_TILE : accumulators(N_TILE) * N_TILE;
+        for (uint32_t c = 0; c < used; c += 32) tmem_st_32x32b_x32(tmem_base + my_lanes + c, zero);
         tmem_st_wait();
     }
     tc_fence_before_sync();
     cluster_sync();   // barriers initialised and accumulators cleared in both CTAs
     tc_fence_after_sync();
+
+    // The end of a tile, columns c * 32 and up, of a warp's lane quadrant.  v: 32 columns of this thread's row, into the
+    // output through a staging block and the copy engine; bw: the block's bias values.
+    auto finish = [&](const SparseItem& it, uint32_t c, const uint32_t (&v)[32], const float* bw, unsigned char* sg) {
+        // straight-line code for all 32 columns: a branch per value leaves every latency of a lone warp exposed
+        const float lbcb = lut_bias_times_cb(a.lut_bias, a.CB);
+        float o[32];
+#pragma unroll
+        for (uint32_t q = 0; q < 8; ++q) {
+            const float4 b4 = *reinterpret_cast<const float4*>(bw + 4 * q);
+            o[4 * q] = dequant_one((int32_t)v[4 * q], a.scale, lbcb, b4.x);
+            o[4 * q + 1] = dequant_one((int32_t)v[4 * q + 1], a.scale, lbcb, b4.y);
+            o[4 * q + 2] = dequant_one((int32_t)v[4 * q + 2], a.scale, lbcb, b4.z);
+            o[4 * q + 3] = dequant_one((int32_t)v[4 * q + 3], a.scale, lbcb, b4.w);
+        }
+        activate_all(o, a.act);
+#pragma unroll
+        for (uint32_t q = 0; q < 8; ++q)
+            *reinterpret_cast<float4*>(sg + lane * 128 + ((q ^ (lane & 7u)) << 4)) = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            tma_store_2d(&out_map, smem_u32(sg), (int32_t)(it.n0 + c * 32), (int32_t)(it.m0 + (warp & 3u) * 32));
+            tma_store_commit();
+        }
+    };
+    // One wide tile per pair: its end is nobody's to hide, so the builders, who are done, take their share of the
+    // 32-column blocks, and as the slab ring is empty every block has a staging block there.  (In the narrower
+    // instances the second copy of this code cost the main loop 5 % and more than the shorter end gave.)
+    auto finish_one = [&](uint32_t helper) -> bool {
+        const SparseItem it = sparse_item<SPLIT>(p, first, N_TILE, rank);
+        const uint32_t quad = warp & 3u;
+        float* bq = s_bias + quad * N_TILE;
+        for (uint32_t c = helper; c < N_TILE / 32; c += 1 + kGroups) {
+            const uint32_t n = it.n0 + c * 32 + lane;
+            bq[c * 32 + lane] = n < a.N ? __ldg(a.bias + n) : 0.f;
+        }
+        uint32_t w_ok = 1;
+        if (lane == 0) w_ok = mbar_wait<256>(acc_full0, 0, s_abort) ? 1u : 0u;
+        if (!__shfl_sync(0xffffffffu, w_ok, 0)) return false;
+        tc_fence_after_sync();
+        for (uint32_t c = helper; c < N_TILE / 32; c += 1 + kGroups) {
+            if (it.n0 + c * 32 >= a.N || it.m0 + quad * 32 >= a.M) break;   // blocks wholly past N or M
+            uint32_t v[32];
+            tmem_ld_32x32b_x32(tmem_base + my_lanes + c * 32u, v);
+            tmem_ld_wait();
+            finish(it, c, v, bq + c * 32, s_b + (size_t)(quad * (N_TILE / 32) + c) * kStageBytes);
+        }
+        if (lane == 0) tma_store_wait_all();   // shared memory and the output are settled before the CTA leaves
+        return true;
+    };
 
     if (warp < kCopyWarps) {
         // ---------------- LUT copies (unless it was laid out just now the LUT does not depend on the preceding kernel),
@@ -474,18 +529,26 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         if constexpr (SPLIT) {
             pdl_wait_prior_grid();
             if (ok && first < n_items) split_finish<N_TILE>(p, sparse_item<SPLIT>(p, first, N_TILE, rank), rank, warp & 3u, 1 + grp, lane, sums0, s_abort);
+        } else if constexpr (kOne) {
+            pdl_wait_prior_grid();
+            if (ok && first < n_items) finish_one(1 + grp);
         }
+        __syncwarp();
+        tc_fence_before_sync();
     } else {
         // ---------------- epilogue: each warp on the lane quadrant it may read
         pdl_wait_prior_grid();
         const uint32_t quad = warp & 3u;
-        const float lbcb = lut_bias_times_cb(a.lut_bias, a.CB);
         unsigned char* stg = s_stage + (warp - kFirstEpi) * (kStages * kStageBytes);
         float* bw = s_bias + (warp - kFirstEpi) * N_TILE;
         const uint32_t empty_leader = map_to_rank(acc_empty0, 0);
         uint32_t t = 0, buf = 0;
         bool ok = true;
-        for (uint32_t item = first; item < n_items; item += n_pairs, ++t) {
+        if constexpr (kOne) {
+            if (p.early_trigger) pdl_launch_dependents();
+            if (first < n_items) finish_one(0);
+        }
+        for (uint32_t item = first; item < n_items && !kOne; item += n_pairs, ++t) {
             const SparseItem it = sparse_item<SPLIT>(p, item, N_TILE, rank);
             const uint32_t ab = t & 1;
             if (p.early_trigger && item + n_pairs >= n_items) pdl_launch_dependents();
@@ -500,34 +563,6 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             ok = __shfl_sync(0xffffffffu, w_ok, 0) != 0;
             if (!ok) continue;
             tc_fence_after_sync();
-            // v: 32 columns of this thread's row, into the output through the staging buffer and the copy engine
-            auto finish = [&](uint32_t c, const uint32_t (&v)[32]) {
-                if (it.n0 + c * 32 >= a.N || it.m0 + quad * 32 >= a.M) return;   // a block wholly past N or M
-                unsigned char* sg = stg + buf * kStageBytes;
-                if (lane == 0) tma_store_wait_read_1();   // the copy before last has read this buffer
-                __syncwarp();
-                // straight-line code for all 32 columns: a branch per value leaves every latency of a lone warp exposed
-                float o[32];
-#pragma unroll
-                for (uint32_t q = 0; q < 8; ++q) {
-                    const float4 b4 = *reinterpret_cast<const float4*>(bw + c * 32 + 4 * q);
-                    o[4 * q] = dequant_one((int32_t)v[4 * q], a.scale, lbcb, b4.x);
-                    o[4 * q + 1] = dequant_one((int32_t)v[4 * q + 1], a.scale, lbcb, b4.y);
-                    o[4 * q + 2] = dequant_one((int32_t)v[4 * q + 2], a.scale, lbcb, b4.z);
-                    o[4 * q + 3] = dequant_one((int32_t)v[4 * q + 3], a.scale, lbcb, b4.w);
-                }
-                activate_all(o, a.act);
-#pragma unroll
-                for (uint32_t q = 0; q < 8; ++q)
-                    *reinterpret_cast<float4*>(sg + lane * 128 + ((q ^ (lane & 7u)) << 4)) = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) {
-                    tma_store_2d(&out_map, smem_u32(sg), (int32_t)(it.n0 + c * 32), (int32_t)(it.m0 + quad * 32));
-                    tma_store_commit();
-                }
-                buf ^= 1;
-            };
             constexpr uint32_t kChunks = N_TILE / 32;
             const uint32_t corner = (it.tile * 2 + rank) * 4 + quad;
             for (uint32_t c = 0; c < kChunks; ++c) {
@@ -545,7 +580,12 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     if (lane == 0) mbar_arrive_cluster(empty_leader + 8 * ab);
                 }
                 if constexpr (!SPLIT) {
-                    finish(c, v);
+                    if (it.n0 + c * 32 < a.N && it.m0 + quad * 32 < a.M) {   // not wholly past N or M
+                        if (lane == 0) tma_store_wait_read_1();   // the copy before last has read this buffer
+                        __syncwarp();
+                        finish(it, c, v, bw + c * 32, stg + buf * kStageBytes);
+                        buf ^= 1;
+                    }
                 } else {
                     uint4* to = partial_sums<N_TILE>(p, corner, it.z, c, lane);
 #pragma unroll
@@ -592,7 +632,7 @@ uint32_t log2_of(uint32_t v) {
 uint32_t sparse_slabs(uint32_t CB, uint32_t CT) { return (uint32_t)(((uint64_t)CB * CT + kSlab - 1) / kSlab); }
 
 size_t sparse_smem(uint32_t n_tile, int lg, uint32_t b_slots) {
-    return (size_t)b_slots * (n_tile / 2) * kSlab + kEpiWarps * kStages * kStageBytes + kIdxStages * kRows * idx_width(lg) +
+    return (size_t)b_slots * (n_tile / 2) * kSlab + stage_blocks(n_tile) * kStageBytes + kIdxStages * kRows * idx_width(lg) +
            kEpiWarps * n_tile * 4 + kNumBarriers * 8 + 16 + 1024;
 }
 
@@ -733,20 +773,22 @@ static uint32_t slice_unit(uint32_t CT) { return CT > 16 ? CT / 16 : 1; }
 // Tile width and split of the codebook axis by the time the launch would take.  Rounds of one tile per pair, each bound by
 // its slabs or, where the codebook axis is short, by the epilogue beside them (0.93 us per 32 columns), and the last
 // tile's epilogue.  A slab takes 170 / 199 / 220 ns at 64 / 128 / 160 columns: at 64 the chain of one slot's
-// turn-around, at 160 close to the tensor pipe's 320 cycles.  (Measured at 32 to 16384 tokens; at 96 columns nothing
-// gained.)  Where the tiles leave pairs idle the axis is split over them, one item per pair, which costs 5 to 6 us for the
+// turn-around, at 160 close to the tensor pipe's 320 cycles.  192 columns only where they make one round of what would be
+// two: 384 codebooks of 16 -> 3072 at 1024 tokens 15.8 -> 12.7 us, 1024 codebooks 29.6 -> 21.3 (four LUT slots instead of
+// eight at 256 columns: 27.8 and 15.4).  (Measured at 32 to 16384 tokens; at 96 columns nothing gained.)  Where the tiles leave pairs idle the axis is split over them, one item per pair, which costs 5 to 6 us for the
 // partial sums' way through L2 (1536 codebooks -> 768 at 128 tokens 20.7 -> 12.2 us, at 1024 tokens 21.6 -> 17.6).
 void sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split) {
     const uint32_t pairs = sm_count >= 2 ? (uint32_t)sm_count / 2 : 1, slabs = sparse_slabs(CB, CT), unit = slice_unit(CT);
     const uint64_t tm = (M + 2 * kRows - 1) / (2 * kRows);
-    const struct { uint32_t n; float slab_us, split_us; } tiles[] = {{64, 0.170f, 5.f}, {128, 0.199f, 6.2f}, {160, 0.220f, 0.f}};
+    const struct { uint32_t n; float slab_us, split_us; } tiles[] = {{64, 0.170f, 5.f}, {128, 0.199f, 6.2f}, {160, 0.220f, 0.f}, {192, 0.250f, 0.f}};
     *n_tile = 160;
     *split = 1;
     float least = 3e38f;
     for (const auto& t : tiles) {
         const uint64_t items = tm * ((N + t.n - 1) / t.n), rounds = (items + pairs - 1) / pairs;
+        if (accumulators(t.n) == 1 && rounds > 1) continue;
         const uint32_t most = items < pairs ? (uint32_t)(pairs / items) : 1;
-        for (uint32_t s = 1; s <= most && s <= (t.n == 160 ? 1u : 16u) && (s == 1 || s * unit <= slabs); ++s) {
+        for (uint32_t s = 1; s <= most && s <= (t.n >= 160 ? 1u : 16u) && (s == 1 || s * unit <= slabs); ++s) {
             const uint32_t per = ((slabs + s - 1) / s + unit - 1) / unit * unit;
             const float main = per * t.slab_us, epi = 0.93f * (t.n / 32);
             const float us = (float)rounds * (rounds > 1 && epi > main ? epi : main) + 0.25f * (t.n / 32) + (s > 1 ? t.split_us : 0.f);
@@ -755,6 +797,7 @@ void sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int s
     }
 }
 
+// Tiles a plan may name; 192 columns suit only launches of one round, which sparse_default_plan() knows.
 bool sparse_tile_ok(uint32_t n_tile) { return n_tile == 64 || n_tile == 128 || n_tile == 160; }
 
 // Scratch of a split launch: partial sums and counter words.
@@ -776,7 +819,7 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
     p.tiles_n = (a.N + n_tile - 1) / n_tile;
     const uint32_t cap = max_ctas / 2, unit = slice_unit(a.CT);
     // the slices of a tile wait for one another: only where every item has a pair of its own
-    if (!split || n_tile == 160 || (uint64_t)p.tiles_m * p.tiles_n * split > cap || !partial || !counters) split = 1;
+    if (!split || n_tile >= 160 || (uint64_t)p.tiles_m * p.tiles_n * split > cap || !partial || !counters) split = 1;
     p.per = ((p.slabs + split - 1) / split + unit - 1) / unit * unit;
     p.split = (p.slabs + p.per - 1) / p.per;   // no empty slices
     p.partial = static_cast<uint4*>(partial);
@@ -791,10 +834,14 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
     // stay there from one column tile to the next (65536 tokens x 2048 codebooks: 134 MB, read from memory 103 times),
     // go through the columns with as many row tiles as there are pairs: 13.8 GB of reads become 1.9 GB of table.
     p.group_m = (uint64_t)a.M * a.CB > (48ull << 20) && p.tiles_m > cap ? cap : p.tiles_m;
+    p.one_tile = items <= cap;
     // With one tile per pair all pairs reach the end of their main loops together, and the next kernel of the stream
-    // may as well be launched; with several they finish a tile apart and its early CTAs would skew it.
-    p.early_trigger = items <= cap;
+    // may as well be launched; with several they finish a tile apart and its early CTAs, which pile up on the SMs that
+    // are free first, would skew it.  A search of many CTAs is skewed by the SMs that one tile per pair leaves idle, too:
+    // four linears of 768 at 256 tokens 53.8 us with the trigger, 55.0 without, at 1024 tokens 78.2 and 76.9.
+    p.early_trigger = p.one_tile && (uint64_t)a.M * a.CB <= 200 * 1024;
     p.fresh_table = fresh_table;
+    if (accumulators(n_tile) == 1 && !p.one_tile) { *why = "tiles wider than 160 columns of the sparse form take one tile per pair"; return cudaErrorInvalidValue; }
     const size_t smem = sparse_smem(n_tile, lg, p.b_slots);
 #define LUTAMM_SPARSE_CASE(NT, SP) \
     if (n_tile == NT && (p.split > 1) == SP) return run_lg<NT, SP>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
@@ -803,6 +850,7 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
     LUTAMM_SPARSE_CASE(128, false)
     LUTAMM_SPARSE_CASE(128, true)
     LUTAMM_SPARSE_CASE(160, false)
+    LUTAMM_SPARSE_CASE(192, false)
 #undef LUTAMM_SPARSE_CASE
     *why = "tcgen05 variant: the sparse form is built for 64-, 128- and 160-wide tiles";
     return cudaErrorInvalidValue;

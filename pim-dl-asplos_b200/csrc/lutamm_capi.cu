@@ -64,8 +64,8 @@ namespace {
 constexpr int kNumUmmaTiles = 5;  // 64, 128, 160, 192, 256
 inline int umma_tile_slot(uint32_t n_tile) { return n_tile == 64 ? 0 : n_tile == 128 ? 1 : n_tile == 160 ? 2 : n_tile == 192 ? 3 : 4; }
 
-constexpr int kNumSparseTiles = 3;  // 64, 128, 160
-inline int sparse_tile_slot(uint32_t n_tile) { return n_tile == 64 ? 0 : n_tile == 128 ? 1 : 2; }
+constexpr int kNumSparseTiles = 4;  // 64, 128, 160, 192
+inline int sparse_tile_slot(uint32_t n_tile) { return umma_tile_slot(n_tile); }
 
 struct Layer {
     lutamm_index_params ip{};
@@ -84,7 +84,7 @@ struct Layer {
     bool umma_map_ok[kNumUmmaTiles] = {false, false, false, false, false};
     // the sparse form: tensor maps of its table per tile width, and of the last index and output buffers it was called with
     CUtensorMap sparse_maps[kNumSparseTiles];
-    bool sparse_map_ok[kNumSparseTiles] = {false, false, false};
+    bool sparse_map_ok[kNumSparseTiles] = {};
     CUtensorMap sparse_idx_map, sparse_out_map;
     const void *sparse_idx = nullptr, *sparse_out = nullptr;
     uint32_t sparse_idx_m = 0, sparse_out_m = 0;

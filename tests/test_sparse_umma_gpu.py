@@ -63,3 +63,24 @@ def test_split_codebook_axis(ctx, M, CB, CT, N, n_tile, split):
     ctx.pim_lut(79, idx, y)
     np.testing.assert_allclose(y, oracle.gelu_tanh(want), rtol=1e-5, atol=1e-9)
     ctx.unload_weights(79)
+
+
+@pytest.mark.parametrize("M,CB,CT,N", [(1024, 16, 16, 3312), (1000, 48, 8, 3072), (300, 32, 32, 6160), (2049, 16, 64, 1536), (1024, 16, 256, 3280)])
+def test_one_wide_tile_per_pair(ctx, M, CB, CT, N):
+    """Where 192-column tiles make one round of what narrower ones would make two the default plan takes them; N that 192
+    and 32 do not divide, rows past M, and the fused activation."""
+    rng = np.random.default_rng(M + N)
+    cen = rng.standard_normal((CB, CT, 2), dtype=np.float32)
+    lut = rng.integers(-128, 128, (CB, CT, N), dtype=np.int8)
+    bias = rng.standard_normal(N, dtype=np.float32)
+    idx = rng.integers(0, CT, (M, CB), dtype=np.uint8)
+    ctx.load_weights(79, cen, lut, bias, 0.013, 0.3)
+    want = oracle.dequant(oracle.lut_gather(idx.astype(np.uint16), lut), bias, CB, 0.013, 0.3)
+    for _ in range(2):
+        y = np.zeros((M, N), np.float32)
+        ctx.pim_lut(79, idx, y)
+        assert np.array_equal(y.view(np.uint32), want.view(np.uint32))
+    ctx.set_activation(79, P.ACT_GELU_TANH)
+    ctx.pim_lut(79, idx, y)
+    np.testing.assert_allclose(y, oracle.gelu_tanh(want), rtol=1e-5, atol=1e-9)
+    ctx.unload_weights(79)
