@@ -299,4 +299,11 @@ cudaError_t launch_gather(const LutArgs& a, const CUtensorMap& lut_map, uint32_t
     }
 }
 
+// By the adds a full GPU sustains or, where the tiles are few, by one CTA's walk over the codebooks.
+float gather_us(uint32_t M, uint32_t CB, uint32_t N, int sm_count) {
+    const float ctas = (float)((M + 31) / 32) * ((N + 127) / 128), sum = (float)M * CB * N / 9.7e6f;
+    const float chain = 0.105f * CB * (ctas > sm_count ? 1.f + ctas / sm_count / 8 : 1.f);
+    return 4.f + (sum > chain ? sum : chain);
+}
+
 }  // namespace lutamm

@@ -297,6 +297,16 @@ int run_sparse(lutamm_ctx* c, Layer& L, const LutArgs& a, uint32_t n_tile, uint3
     return LUTAMM_OK;
 }
 
+// The library's own choice for few tokens: the used rows of the table, where reading them takes less time than the
+// contraction (or the gather, where that does not fit) takes to go through the whole table.
+bool takes_rows(const lutamm_ctx* c, const Layer& L, uint32_t M, const lutamm_plan& plan) {
+    if (plan.variant != LUTAMM_VARIANT_AUTO || plan.gather_cfg || !umma_plan_open(plan)) return false;
+    uint32_t n_tile, split;
+    const float other = umma_supported(L.CB, L.CT, L.N) ? 4.f + sparse_default_plan(M, L.CB, L.CT, L.N, c->sm_count, &n_tile, &split)
+                                                        : gather_us(M, L.CB, L.N, c->sm_count);
+    return rows_us(M, L.CB, L.N, c->sm_count) < other;
+}
+
 // step 2+3 on device buffers
 int run_lut(lutamm_ctx* c, Layer& L, const uint8_t* d_idx, float* d_out, int32_t* d_acc_out, uint32_t M,
             uint32_t flags, const lutamm_plan& plan, float* const* peer_out = nullptr, uint32_t n_peers = 0) {
@@ -316,6 +326,12 @@ int run_lut(lutamm_ctx* c, Layer& L, const uint8_t* d_idx, float* d_out, int32_t
     a.act = L.act;
     const char* why = nullptr;
     uint32_t variant = plan.variant;
+    if (takes_rows(c, L, M, plan) && !a.n_peers && !a.acc_out && !a.layout.tiled) {
+        const cudaError_t e = launch_rows(a, L.d_lut, c->sm_count, c->stream);
+        if (e != cudaSuccess) return fail(c, LUTAMM_ECUDA, std::string("row gather launch: ") + cudaGetErrorString(e));
+        ++c->launches;
+        return LUTAMM_OK;
+    }
     if (variant == LUTAMM_VARIANT_AUTO) variant = resolve_variant(c, L);
     if (variant == LUTAMM_VARIANT_UMMA) {
         if (!umma_supported(L.CB, L.CT, L.N))
@@ -887,6 +903,7 @@ int lutamm_tune(lutamm_ctx* c, int layer_id, uint32_t M, lutamm_plan* best_out) 
         p.gather_cfg = cfg;
         cands.push_back(p);
     }
+    if (takes_rows(c, *L, M, lutamm_plan{})) cands.push_back(lutamm_plan{});
     if (umma_supported(L->CB, L->CT, L->N)) {
         const uint32_t slabs = (uint32_t)(((uint64_t)L->CB * L->CT + 127) / 128);
         for (uint32_t nt : {64u, 128u, 160u}) {

@@ -71,26 +71,31 @@ uint32_t sm_count_of(int device) {
     return n;
 }
 
-// Whether to lay the table out for the tcgen05 kernel on every call, `columns` at a time in what the indices leave of
-// the array (0: the CUDA-core gather, which reads the table as it is).  By estimated time, in microseconds.
+// By estimated time: the table's used rows, for few tokens; the table laid out for the tcgen05 kernel on every call,
+// `columns` at a time in what the indices leave of the array; or the CUDA-core gather, which reads the table as it is.
 struct TablePlan {
+    bool rows;
     uint32_t columns;
 };
-TablePlan plan_table(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, uint32_t sms) {
-    if (!lutamm::umma_supported(CB, CT, N)) return {0};
-    const size_t per_column = lutamm::sparse_table_bytes(CB, CT, 1), used = (((size_t)M * CB + 255) / 256) * 256;
-    const size_t fit = used < LUTAMM_STATIC_SCRATCH_BYTES ? (LUTAMM_STATIC_SCRATCH_BYTES - used) / per_column : 0;
-    uint32_t columns = fit < N ? (uint32_t)(fit / 64 * 64) : N;
-    if (columns == 0) return {0};
-    const uint32_t chunks = (N + columns - 1) / columns;
-    columns = ((N + chunks - 1) / chunks + 63) / 64 * 64;   // near-equal chunks
-    if (columns > N) columns = N;
-    uint32_t n_tile, split;
-    lutamm::sparse_default_plan(M, CB, CT, columns, (int)sms, &n_tile, &split);
-    const double tiles = (double)((M + 255) / 256) * ((columns + n_tile - 1) / n_tile), rounds = (double)(uint64_t)((tiles + sms / 2 - 1) / (sms / 2));
-    const double table = chunks * (5.0 + per_column * (double)columns / 2.5e6 + rounds * per_column / 256 * 0.2);
-    const double ctas = (double)((M + 31) / 32) * ((N + 127) / 128), sum = (double)M * CB * N / 9.7e6, chain = 0.105 * CB * (ctas > sms ? 1.0 + ctas / sms / 8 : 1.0);
-    return {table < 4.0 + (sum > chain ? sum : chain) ? columns : 0u};
+TablePlan plan_table(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, bool aligned, uint32_t sms) {
+    const double gather = lutamm::gather_us(M, CB, N, (int)sms), rows = aligned ? lutamm::rows_us(M, CB, N, (int)sms) : 1e30;
+    double table = 1e30;
+    uint32_t columns = 0;
+    if (lutamm::umma_supported(CB, CT, N)) {
+        const size_t per_column = lutamm::sparse_table_bytes(CB, CT, 1), used = (((size_t)M * CB + 255) / 256) * 256;
+        const size_t fit = used < LUTAMM_STATIC_SCRATCH_BYTES ? (LUTAMM_STATIC_SCRATCH_BYTES - used) / per_column : 0;
+        columns = fit < N ? (uint32_t)(fit / 64 * 64) : N;
+        if (columns) {
+            const uint32_t chunks = (N + columns - 1) / columns;
+            columns = ((N + chunks - 1) / chunks + 63) / 64 * 64;   // near-equal chunks
+            if (columns > N) columns = N;
+            uint32_t n_tile, split;
+            lutamm::sparse_default_plan(M, CB, CT, columns, (int)sms, &n_tile, &split);
+            const uint64_t tiles = (uint64_t)((M + 255) / 256) * ((columns + n_tile - 1) / n_tile), rounds = (tiles + sms / 2 - 1) / (sms / 2);
+            table = chunks * (5.0 + per_column * (double)columns / 2.5e6 + rounds * per_column / 256 * 0.2);
+        }
+    }
+    return {rows < table && rows < gather, table < gather ? columns : 0u};
 }
 
 }  // namespace
@@ -175,8 +180,11 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
     la.M = M; la.CB = CB; la.CT = CT; la.N = N;
     la.scale = lp->scale; la.lut_bias = lp->bias;
     const uint32_t sms = sm_count_of(device);
-    const TablePlan plan = plan_table(M, CB, CT, N, sms);
-    if (plan.columns) {
+    const TablePlan plan = plan_table(M, CB, CT, N, !(reinterpret_cast<uintptr_t>(lut) & 15u), sms);
+    if (plan.rows) {
+        e = launch_rows(la, lut, (int)sms, s);
+        if (e != cudaSuccess) return fail(LUTAMM_ECUDA, std::string("row gather launch: ") + cudaGetErrorString(e));
+    } else if (plan.columns) {
         // the tcgen05 kernel on as many columns at a time as the rest of the array holds of its layout of the table
         int8_t* table = reinterpret_cast<int8_t*>(d_idx + (((size_t)M * CB + 255) / 256) * 256);
         CUtensorMap idx_map;
