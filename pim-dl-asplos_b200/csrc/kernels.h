@@ -103,6 +103,9 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
 
 // A few tokens: the used rows of the canonical table alone (16-byte aligned), row-major fp32 output.
 cudaError_t launch_rows(const LutArgs& a, const int8_t* lut, int sm_count, cudaStream_t s);
+// ... and the search, in one launch, where rows_search_ok()
+bool rows_search_ok(uint32_t M, uint32_t CB, uint32_t CT, uint32_t v, uint32_t N, const float* x);
+cudaError_t launch_rows_search(const LutArgs& a, const int8_t* lut, const float* x, const float* centroid, uint32_t v, int sm_count, cudaStream_t s);
 float rows_us(uint32_t M, uint32_t CB, uint32_t N, int sm_count);
 
 // LUT [CB*CT][N] -> [N][CB*CT]

@@ -1,4 +1,4 @@
-// Steps 2+3 of the AMM for a few tokens: only the table rows that are used, straight from the canonical table.
+// The AMM for a few tokens: only the table rows that are used, straight from the canonical table.
 //
 // The contraction kernels read the whole table whatever the number of tokens; M tokens use M of a codebook's CT rows at
 // most.  Up to that many bytes, M * CB * N against CB * CT * N, it is cheaper to fetch rows: 9 tokens through 3328
@@ -8,6 +8,10 @@
 // rows and every thread has 8 loads in flight.  Bytes are widened to 16 bits, two per register, offset by 128 so that
 // they cannot be negative: 256 rows of at most 255 fit, which is what a CTA reduces before it adds to int32.  The CTAs
 // of a cluster hold the shares of one token and tile and are summed through distributed shared memory.
+//
+// V > 0: the search as well, one launch for the whole operator.  A CTA searches the codebooks of its share, a thread each,
+// by the reference's scan (ccs_argmin.cu) on centroids it reads itself; every column tile of a token repeats that, which
+// costs less than a launch and the way of the indices through memory.
 //
 // What bounds it: launch and a chain of three latencies (index, row, cluster) up to about 10 MB of rows, L2 above (31 MB
 // in 11.4 us).  Against the contraction: 32 tokens, 384 codebooks of 16 -> 768 8.3 -> 5.4 us; one token, 1616 codebooks of
@@ -29,8 +33,46 @@ __device__ __forceinline__ int32_t load_cluster(uint32_t addr) {
     return v;
 }
 
-__global__ void __launch_bounds__(kThreads, 4)
-lut_rows_kernel(const int8_t* __restrict__ lut, const LutArgs a, uint32_t per) {
+struct SearchArgs {
+    const float *x, *centroid;   // [M][CB * V], [CB][CT][V], both 16-byte aligned
+};
+
+// The first 32 floats and then the rest of a codebook's centroids, 32 at a time: CT * V is a multiple of 4.
+__device__ __forceinline__ void load_centroids(float4 (&q)[8], const float* p, uint32_t left) {
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k)
+        if (4 * k < left) q[k] = __ldg(reinterpret_cast<const float4*>(p) + k);
+}
+
+// The reference's scan; q holds the first 32 floats.  32 / V centroids a batch.
+template <int V>
+__device__ __forceinline__ uint32_t scan(const float (&x)[V], const float* p, float4 (&q)[8], uint32_t CT) {
+    float mn = 0.f;
+    uint32_t best = 0;
+    for (uint32_t c0 = 0; c0 < CT; c0 += 32 / V) {
+        if (c0) load_centroids(q, p + c0 * V, (CT - c0) * V);
+        float f[32];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) { f[4 * k] = q[k].x; f[4 * k + 1] = q[k].y; f[4 * k + 2] = q[k].z; f[4 * k + 3] = q[k].w; }
+#pragma unroll
+        for (uint32_t j = 0; j < 32 / V; ++j) {
+            float acc = 0.f;
+#pragma unroll
+            for (int d = 0; d < V; ++d) {
+                const float e = __fsub_rn(x[d], f[j * V + d]);
+                acc = __fadd_rn(acc, __fmul_rn(e, e));
+            }
+            const bool take = c0 + j == 0 || (c0 + j < CT && __fsub_rn(mn, acc) > 1e-6f);   // false for NaN: keeps the earlier index
+            mn = take ? acc : mn;
+            best = take ? c0 + j : best;
+        }
+    }
+    return best;
+}
+
+template <int V>
+__global__ void __launch_bounds__(kThreads, V > 0 ? 3 : 4)
+lut_rows_kernel(const int8_t* __restrict__ lut, const LutArgs a, const SearchArgs sa, uint32_t per) {
     __shared__ uint32_t s_part[8][kTile / 2];
     __shared__ int32_t s_sum[kTile];
     __shared__ uint8_t s_idx[kChunk];
@@ -39,11 +81,34 @@ lut_rows_kernel(const int8_t* __restrict__ lut, const LutArgs a, uint32_t per) {
     const uint32_t begin = rank * per, end = min(a.CB, begin + per);
     const uint32_t group = t >> 3, n = n0 + (t & 7u) * 16;
     const float bias = t < kTile && n0 + t < a.N ? __ldg(a.bias + n0 + t) : 0.f;
-    pdl_wait_prior_grid();   // indices, and the reader of an output that may be written again
+    float4 q[8] = {};
+    if constexpr (V > 0)   // weights: nothing in the stream writes them
+        if (begin + t < end) load_centroids(q, sa.centroid + (size_t)(begin + t) * a.CT * V, a.CT * V);
+    pdl_wait_prior_grid();   // activations or indices, and the reader of an output that may be written again
     int32_t sum0 = 0, sum1 = 0;
     for (uint32_t c0 = begin; c0 < end; c0 += kChunk) {
         const uint32_t count = min(kChunk, end - c0);
-        if (t < count) s_idx[t] = __ldcg(a.idx + (size_t)m * a.CB + c0 + t);
+        if constexpr (V > 0) {
+            if (t < count) {
+                const float* p = sa.centroid + (size_t)(c0 + t) * a.CT * V;
+                float x[V];
+                const float* px = sa.x + ((size_t)m * a.CB + c0 + t) * V;
+                if constexpr (V == 2) {
+                    const float2 u = __ldcg(reinterpret_cast<const float2*>(px));
+                    x[0] = u.x; x[1] = u.y;
+                } else {
+#pragma unroll
+                    for (int d = 0; d < V; d += 4) {
+                        const float4 u = __ldcg(reinterpret_cast<const float4*>(px + d));
+                        x[d] = u.x; x[d + 1] = u.y; x[d + 2] = u.z; x[d + 3] = u.w;
+                    }
+                }
+                if (c0 != begin) load_centroids(q, p, a.CT * V);
+                s_idx[t] = (uint8_t)scan<V>(x, p, q, a.CT);
+            }
+        } else {
+            if (t < count) s_idx[t] = __ldcg(a.idx + (size_t)m * a.CB + c0 + t);
+        }
         __syncthreads();
         uint4 w[8];
 #pragma unroll
@@ -117,8 +182,18 @@ float rows_us(uint32_t M, uint32_t CB, uint32_t N, int sm_count) {
     return 4.f + 0.24e-6f * tiles * kTile * CB + (rounds > 1.f ? 1.2f * (rounds - 1.f) : 0.f);
 }
 
-cudaError_t launch_rows(const LutArgs& a, const int8_t* lut, int sm_count, cudaStream_t s) {
-    if (a.M == 0 || a.N == 0) return cudaSuccess;
+// The same with the search, for centroid sets that a thread reads in a few batches, up to 4.75 MB of them over all CTAs: a
+// lane's 16 bytes come from a line of their own, and a token's centroids are read once per column tile.  768 -> 768, v = 2,
+// 16 centroids, one launch against two: 5.0 us against 6.1 at one token, 5.4 / 6.5 at eight, 6.0 / 6.4 at 16, 7.8 / 6.7 at
+// 32.  Where the search on its own has no quick form (v = 4, 32 centroids: 800 -> 1008 at eight tokens 6.2 / 11.0,
+// 1024 -> 4096 at four 8.5 / 11.0) up to 16 MB.
+bool rows_search_ok(uint32_t M, uint32_t CB, uint32_t CT, uint32_t v, uint32_t N, const float* x) {
+    if ((v != 2 && v != 4 && v != 8) || CT * v % 4 || CT * v > 128 || (reinterpret_cast<uintptr_t>(x) & 15u) || (uint64_t)CB * v % 4) return false;
+    return (uint64_t)M * ((N + kTile - 1) / kTile) * CB * CT * v * 4 <= (CT * v > 64 ? 16000000u : 4750000u);
+}
+
+template <int V>
+static cudaError_t run_rows(const LutArgs& a, const int8_t* lut, const SearchArgs& sa, int sm_count, cudaStream_t s) {
     const uint32_t shares = rows_shares(a.M, a.CB, a.N, sm_count), per = (a.CB + shares - 1) / shares;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(shares, (a.N + kTile - 1) / kTile, a.M);
@@ -133,7 +208,18 @@ cudaError_t launch_rows(const LutArgs& a, const int8_t* lut, int sm_count, cudaS
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, lut_rows_kernel, lut, a, per);
+    return cudaLaunchKernelEx(&cfg, lut_rows_kernel<V>, lut, a, sa, per);
+}
+
+cudaError_t launch_rows(const LutArgs& a, const int8_t* lut, int sm_count, cudaStream_t s) {
+    if (a.M == 0 || a.N == 0) return cudaSuccess;
+    return run_rows<0>(a, lut, SearchArgs{}, sm_count, s);
+}
+
+cudaError_t launch_rows_search(const LutArgs& a, const int8_t* lut, const float* x, const float* centroid, uint32_t v, int sm_count, cudaStream_t s) {
+    if (a.M == 0 || a.N == 0) return cudaSuccess;
+    const SearchArgs sa{x, centroid};
+    return v == 2 ? run_rows<2>(a, lut, sa, sm_count, s) : v == 4 ? run_rows<4>(a, lut, sa, sm_count, s) : run_rows<8>(a, lut, sa, sm_count, s);
 }
 
 }  // namespace lutamm

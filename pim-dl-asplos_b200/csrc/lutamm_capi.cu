@@ -307,6 +307,21 @@ bool takes_rows(const lutamm_ctx* c, const Layer& L, uint32_t M, const lutamm_pl
     return rows_us(M, L.CB, L.N, c->sm_count) < other;
 }
 
+// All steps in one launch, for few tokens.
+int run_rows_search(lutamm_ctx* c, Layer& L, const float* d_x, float* d_y, uint32_t M) {
+    LutArgs a{};
+    a.bias = L.d_bias;
+    a.out = d_y;
+    a.M = M; a.CB = L.CB; a.CT = L.CT; a.N = L.N;
+    a.scale = L.lp.scale;
+    a.lut_bias = L.lp.bias;
+    a.act = L.act;
+    const cudaError_t e = launch_rows_search(a, L.d_lut, d_x, L.d_centroid, L.v, c->sm_count, c->stream);
+    if (e != cudaSuccess) return fail(c, LUTAMM_ECUDA, std::string("row gather launch: ") + cudaGetErrorString(e));
+    ++c->launches;
+    return LUTAMM_OK;
+}
+
 // step 2+3 on device buffers
 int run_lut(lutamm_ctx* c, Layer& L, const uint8_t* d_idx, float* d_out, int32_t* d_acc_out, uint32_t M,
             uint32_t flags, const lutamm_plan& plan, float* const* peer_out = nullptr, uint32_t n_peers = 0) {
@@ -505,6 +520,12 @@ int amm_impl(lutamm_ctx* c, int layer_id, const float* input, float* output, uin
     if (!out_dev) {
         if ((r = ensure(c, c->d_out, out_bytes))) return r;
         d_y = static_cast<float*>(c->d_out.p);
+    }
+    if (!t && !idx_out && !acc_out && !(flags & LUTAMM_FLAG_OUTPUT_TILED) && !L->plan.ccs_tokens && takes_rows(c, *L, M, L->plan) &&
+        rows_search_ok(M, L->CB, L->CT, L->v, L->N, d_x)) {
+        if ((r = run_rows_search(c, *L, d_x, d_y, M))) return r;
+        if (!out_dev) CU_TRY(c, cudaMemcpyAsync(output, d_y, out_bytes, cudaMemcpyDeviceToHost, c->stream));
+        return (flags & LUTAMM_FLAG_ASYNC) ? LUTAMM_OK : check_dev_err(c);
     }
     if ((r = ensure(c, c->d_idx, (size_t)M * L->CB))) return r;
     int32_t* d_acc = nullptr;

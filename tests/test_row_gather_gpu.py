@@ -60,3 +60,24 @@ def test_static_scratch_rows(offset):
     assert rc == P.OK
     want = oracle.amm(c.x, c.centroid, c.lut, c.bias, c.scale, c.lut_bias)[0]
     assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("M,K,N,v,CT", [(1, 768, 768, 2, 16), (3, 512, 144, 4, 8), (2, 320, 48, 8, 13), (1, 2080, 16, 2, 64), (1, 4400, 272, 8, 4), (1, 12, 32, 4, 31)])
+def test_search_and_rows_in_one_launch(ctx, M, K, N, v, CT):
+    """Ties and near-ties, which the order of the scan decides, and values that do not compare."""
+    rng = np.random.default_rng(K + N)
+    cen = (rng.integers(-3, 4, (K // v, CT, v)) * 0.5).astype(np.float32)
+    x = (rng.integers(-3, 4, (M, K)) * 0.5).astype(np.float32)
+    x[:, ::3] += rng.normal(0, 3e-7, x[:, ::3].shape).astype(np.float32)
+    x[0, -1] = np.nan
+    lut = rng.integers(-128, 128, (K // v, CT, N), dtype=np.int8)
+    bias = rng.standard_normal(N, dtype=np.float32)
+    import torch
+    ctx.load_weights(82, cen, lut, bias, 0.02, -0.4)
+    y = torch.full((M, N), float("nan"), device="cuda")
+    xd = torch.from_numpy(x).cuda()
+    torch.cuda.synchronize()
+    ctx.amm_host(82, xd, y)
+    want = oracle.amm(x, cen, lut, bias, 0.02, -0.4)[0]
+    assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    ctx.unload_weights(82)
