@@ -449,14 +449,15 @@ int check_dev_err(lutamm_ctx* c) {
 // and both directions of the host link are busy at once.  The reference's counterpart are the
 // serial host<->DPU transfers around dpu_launch (pim_lut_host.cpp:143-181).
 int amm_host_pipelined(lutamm_ctx* c, Layer& L, const float* input, float* output, uint32_t M, uint32_t flags) {
-    // A call goes through whole up to 2047 tokens, from there on in slabs of at least 1024, at most four: what a call
-    // cannot overlap is its first copy-in and its last copy-out, but small copies and launches cost more than they hide
-    // (BERT-base at 1024 tokens, four linears: whole 674 us, halves 679, quarters 775).  Only when the pipeline is idle -
-    // the last result has left - does a call open with 256 rows, so that the copies out, which bound the whole, start early.
+    // A call goes through whole up to 2047 tokens, from there on in slabs of at least 1024, at most four: small copies and
+    // launches cost more than they hide (BERT-base at 1024 tokens, four linears: whole 677 us, halves 679, quarters 775).
+    // Only when the pipeline is idle - the last result has left - does a call open with half a slab, so that the copies
+    // out, which bound the whole, start earlier: 651 us; 560 tokens 427 -> 400, 1500 tokens 968 -> 928.
     const uint32_t chunks = M >= 2048 ? std::min(4u, M / 1024) : 1;
     uint32_t rows = ((M + chunks - 1) / chunks + 127) / 128 * 128, opening = 0;
     if ((flags & LUTAMM_FLAG_OUTPUT_TILED) || rows >= M) rows = M;
-    if (!(flags & LUTAMM_FLAG_OUTPUT_TILED) && M >= 512 && cudaEventQuery(c->ev_out[(c->slot + kHostSlots - 1) % kHostSlots]) == cudaSuccess) opening = 256;
+    if (!(flags & LUTAMM_FLAG_OUTPUT_TILED) && M >= 512 && cudaEventQuery(c->ev_out[(c->slot + kHostSlots - 1) % kHostSlots]) == cudaSuccess)
+        opening = (std::min(rows, M) / 2 + 64) / 128 * 128;
     cudaGetLastError();   // "not ready" is an answer
     int r;
     if ((r = ensure(c, c->d_idx, (size_t)rows * L.CB))) return r;
