@@ -451,6 +451,7 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
                 if (lane == 0) w_ok = (ok && mbar_wait<256>(acc_full0 + 8 * ab, aph, s_abort)) ? 1u : 0u;
                 ok = __shfl_sync(0xffffffffu, w_ok, 0) != 0;
                 if (!ok) continue;
+                __syncwarp();  // all lanes' bias values, and what lane 0 waited for: a shuffle orders no memory
                 tc_fence_after_sync();
                 for (uint32_t c = 0; c < N_TILE / 32; ++c) {
                     uint32_t v[32];
@@ -509,6 +510,7 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
             if (lane == 0) w_ok = (ok && mbar_wait<256>(acc_full0 + 8 * ab, aph, s_abort)) ? 1u : 0u;
             ok = __shfl_sync(0xffffffffu, w_ok, 0) != 0;
             if (ok) {
+                __syncwarp();  // what lane 0 waited for: a shuffle orders no memory
                 tc_fence_after_sync();
                 for (uint32_t c = 0; c < N_TILE / 32; ++c) {
                     const float4 b4 = b_next;

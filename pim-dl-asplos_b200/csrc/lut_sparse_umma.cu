@@ -369,6 +369,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         uint32_t w_ok = 1;
         if (lane == 0) w_ok = mbar_wait<256>(acc_full0, 0, s_abort) ? 1u : 0u;
         if (!__shfl_sync(0xffffffffu, w_ok, 0)) return false;
+        __syncwarp();   // all lanes' bias values, and what lane 0 waited for: a shuffle orders no memory
         tc_fence_after_sync();
         for (uint32_t c = helper; c < N_TILE / 32; c += 1 + kGroups) {
             if (it.n0 + c * 32 >= a.N || it.m0 + quad * 32 >= a.M) break;   // blocks wholly past N or M
@@ -562,6 +563,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             if (lane == 0) w_ok = (ok && mbar_wait<256>(acc_full0 + 8 * ab, (t >> 1) & 1, s_abort)) ? 1u : 0u;
             ok = __shfl_sync(0xffffffffu, w_ok, 0) != 0;
             if (!ok) continue;
+            __syncwarp();   // all lanes' bias values, and what lane 0 waited for: a shuffle orders no memory
             tc_fence_after_sync();
             constexpr uint32_t kChunks = N_TILE / 32;
             const uint32_t corner = (it.tile * 2 + rank) * 4 + quad;
