@@ -13,7 +13,7 @@
 // accumulators double-buffered in tensor memory, every slot of both rings with one producer and one consumer.  Per CTA:
 //   warps 0-1     copy the CTA's half of a LUT slab (N_TILE/2 rows x 256 bytes); bytes count on the leader's barrier
 //   warp 2        copies the index bytes of the CTA's rows, a few slabs at a time
-//   warps 3-6     leader only: four tcgen05.mma.sp per slab, slab x by warp 3 + x % 4
+//   warps 3-6     leader only: four tcgen05.mma.sp per slab, slab x by warp 3 + x % 4, in turn (below)
 //   warps 7-22    four groups of four warps: the operand of the CTA's 128 rows, straight from the uint8 indices;
 //                 group k takes every fourth slab, one row per thread, in registers: a table in shared memory would
 //                 compete with the slabs for its bandwidth
@@ -48,7 +48,7 @@ constexpr uint32_t kStageBytes = 32 * 128;     // a 32 x 32 fp32 block
 constexpr uint32_t kStages = 2;                // per epilogue warp
 constexpr uint32_t kIdxStages = 3;
 __host__ __device__ constexpr uint32_t stage_blocks(uint32_t n_tile) { return accumulators(n_tile) == 1 ? 0 : kEpiWarps * kStages; }
-constexpr uint32_t kNumBarriers = 2 * kMaxASlots + 2 * kMaxBSlots + 4 + 2 * kIdxStages + 4;
+constexpr uint32_t kNumBarriers = 2 * kMaxASlots + 2 * kMaxBSlots + 4 + 2 * kIdxStages + 4 + kMmaWarps;
 
 // A stage of index bytes: 128 rows of `idx_width` bytes, for `idx_slabs` slabs.
 __host__ __device__ constexpr uint32_t idx_width(int lg) { return lg == 3 ? 64u : lg <= 6 ? 4u * (256u >> lg) : 16u; }
@@ -292,7 +292,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
     volatile uint32_t* s_abort = s_misc + 1;
     const uint32_t a_full0 = smem_u32(s_bar), a_empty0 = a_full0 + 8 * kMaxASlots, b_full0 = a_empty0 + 8 * kMaxASlots,
                    b_empty0 = b_full0 + 8 * kMaxBSlots, acc_full0 = b_empty0 + 8 * kMaxBSlots, acc_empty0 = acc_full0 + 16,
-                   i_full0 = acc_empty0 + 16, i_empty0 = i_full0 + 8 * kIdxStages, sums0 = i_empty0 + 8 * kIdxStages;
+                   i_full0 = acc_empty0 + 16, i_empty0 = i_full0 + 8 * kIdxStages, sums0 = i_empty0 + 8 * kIdxStages, turn0 = sums0 + 32;
 
     const LutArgs& a = p.a;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = cluster_rank();
@@ -310,7 +310,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         // leader's expect_tx (the copies of both CTAs complete the bytes); acc_full: one commit per issuing warp;
         // acc_empty: the epilogue warps of both CTAs (barriers the
         // leader waits on are unused in the other CTA); i_full: expect_tx; i_empty: the CTA's builder warps;
-        // the last four: a quadrant's partial sums are complete.
+        // four: a quadrant's partial sums are complete; the last kMmaWarps: an issuing warp's turn.
         const uint32_t after = 2 * kMaxASlots + 2 * kMaxBSlots;
         mbar_init(a_full0 + 8 * b, b < kMaxASlots ? 8u : b < after ? 1u : b < after + 2 ? kMmaWarps : b < after + 4 ? 2 * kEpiWarps : b < after + 4 + kIdxStages ? 1u : b < after + 4 + 2 * kIdxStages ? 4 * kGroups : 1u);
         fence_barrier_init();
@@ -428,8 +428,12 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         __syncwarp();
         if (p.early_trigger) pdl_launch_dependents();
     } else if (warp < kFirstBuilder) {
-        // ---------------- MMA issue, leader only: a warp per operand slot, so that it is waiting when the slot fills.
-        // Converged loop, one elected lane issues.
+        // ---------------- MMA issue, leader only: several warps, so that one is waiting when a slot fills.  All of them
+        // accumulate into one accumulator, and that is ordered between instructions of one thread only; between threads it takes
+        // the tcgen05 fences on either side of a barrier.  So the warps issue in turn, slab after slab, each
+        // handing over behind its four instructions (not behind their completion).  Unordered, the four linears of BERT-base at
+        // 1024 tokens take as long (76.4 and 76.8 us), 512 tokens 768 -> 3072 13.4 and 13.7 us; one warp alone, which needs no
+        // hand-over, 81.8 and 15.1 us.  Converged loop, one elected lane issues.
         if (rank == 0) {
             const uint32_t me = warp - kFirstMma;
             uint32_t j = me, pb = 0, t = 0, x0 = 0;   // LUT slot and phases of this warp's next slab; slabs before the item
@@ -444,7 +448,8 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                 const uint32_t d_tmem = tmem_base + ab * N_TILE;
                 for (uint32_t i = (me - x0) & (kMmaWarps - 1); i < slabs; i += kMmaWarps) {
                     const uint32_t x = x0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
-                    ok = mbar_wait(b_full0 + 8 * j, pb, s_abort) && mbar_wait(a_full0 + 8 * k, pa, s_abort);
+                    ok = mbar_wait(b_full0 + 8 * j, pb, s_abort) && mbar_wait(a_full0 + 8 * k, pa, s_abort) &&
+                         mbar_wait(turn0 + 8 * me, ((x / kMmaWarps) & 1u) ^ (me == 0 ? 1u : 0u), s_abort);   // slab 0 has its turn
                     if (!ok) break;
                     tc_fence_after_sync();
                     if (elect_one()) {
@@ -454,6 +459,8 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                             umma_i8_sparse_pair(d_tmem, tmem_base + kDataBase + 32 * k + 8 * kk,
                                                 ((uint64_t)desc_hi << 32) | (b_lo + (kk >> 1) * (kHalfN * 128 >> 4) + (kk & 1) * 4),
                                                 tmem_base + kMetaBase + 2 * k, kIdesc);
+                        tc_fence_before_sync();
+                        mbar_arrive(turn0 + 8 * ((me + 1) & (kMmaWarps - 1)));
                         umma_commit_pair(a_empty0 + 8 * k);
                         umma_commit_pair(b_empty0 + 8 * j);
                     }

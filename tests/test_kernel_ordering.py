@@ -23,3 +23,21 @@ def test_epilogue_warps_meet_before_they_read(name, epilogues):
         after = _source(name)[w.end():]
         until = after[:after.index("tmem_ld_32x32b_x32(")]
         assert "__syncwarp();" in until[until.index("__shfl_sync("):]
+
+
+@pytest.mark.parametrize("name", ["lut_sparse_umma.cu"])
+def test_issuing_warps_take_turns(name):
+    """Several warps issue MMAs into one accumulator.  Read-modify-writes of an accumulator are ordered between the
+    instructions of one thread; between threads it takes a fence, a barrier and a fence: before its first instruction of a
+    slab a warp waits for its turn, behind the last one it hands over."""
+    src = _source(name)
+    if int(re.search(r"\bkMmaWarps = (\d+)", src).group(1)) == 1:
+        return
+    for issue in re.finditer(r"if \(elect_one\(\)\) \{\s*const uint32_t b_lo", src):
+        before = src[src.rindex("for (uint32_t i = ", 0, issue.start()):issue.start()]
+        assert re.search(r"mbar_wait\(turn0 .*tc_fence_after_sync\(\);", before, re.S)
+        after = src[issue.start():src.index("umma_commit", issue.start())]
+        assert re.search(r"umma_i8.*tc_fence_before_sync\(\);\s*mbar_arrive\(turn0 ", after, re.S)
+        break
+    else:
+        pytest.fail("no issue loop found")
