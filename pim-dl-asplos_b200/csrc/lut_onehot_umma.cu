@@ -21,7 +21,7 @@
 //
 //   warp 0        TMA producer: B slabs = LUT^T[n0:n0+N_TILE][k:k+128] (K-major, 128-byte
 //                 swizzle) from the load-time transposed copy of the LUT
-//   warps 1-2     issue tcgen05.mma, 4 per slab, slab x by warp 1 + x % 2 (one elected lane);
+//   warps 1-2     issue tcgen05.mma, 4 per slab, slab x by warp 1 + x % 2 (one elected lane), in turn;
 //                 warp 1 also owns TMEM (alloc/dealloc)
 //   warps 3-18    build the one-hot A slab straight from the uint8 indices (it never exists in
 //                 HBM): four groups of four warps, group k taking every fourth slab, one tile
@@ -53,7 +53,7 @@ constexpr uint32_t kFirstAgenWarp = 1 + kMmaWarps;
 constexpr uint32_t kMaxThreads = (kFirstAgenWarp + 4 * kMaxAgenGroups + kEpiWarps) * 32;  // 736
 constexpr uint32_t kMaxASlots = 8;    // one-hot slabs in flight (tensor memory: 32 columns each)
 constexpr uint32_t kMaxBSlots = 16;   // LUT slabs in flight (shared memory)
-constexpr uint32_t kNumBarriers = 2 * kMaxASlots + 2 * kMaxBSlots + 4;
+constexpr uint32_t kNumBarriers = 2 * kMaxASlots + 2 * kMaxBSlots + 4 + kMmaWarps;
 constexpr uint32_t kStageWarpBytes = 32 * 128;           // epilogue transpose buffer per warp
 constexpr uint32_t kBiasWarpBytes = 256 * 4;             // a tile's bias values, one copy per epilogue warp (store-by-copy-engine epilogue)
 // One-hot table: row e (0..15) holds the 16 bytes "byte e = 1", row 16 holds zeros; a row is 128
@@ -145,7 +145,8 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
     volatile uint32_t* s_abort = s_misc + 1;
 
     const uint32_t a_full0 = smem_u32(s_bar), a_empty0 = a_full0 + 8 * kMaxASlots, b_full0 = a_empty0 + 8 * kMaxASlots,
-                   b_empty0 = b_full0 + 8 * kMaxBSlots, acc_full0 = b_empty0 + 8 * kMaxBSlots, acc_empty0 = acc_full0 + 16;
+                   b_empty0 = b_full0 + 8 * kMaxBSlots, acc_full0 = b_empty0 + 8 * kMaxBSlots, acc_empty0 = acc_full0 + 16,
+                   turn0 = acc_empty0 + 16;
 
     const LutArgs& a = p.a;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -165,8 +166,9 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
         const uint32_t b = threadIdx.x - 64;
         // a_full: the four builder warps of the group that owns the slab; a_empty, b_empty: one tcgen05.commit;
         // b_full: the producer's arrive.expect_tx (the TMA completes the bytes); acc_full: one commit per
-        // issuing warp; acc_empty: the epilogue warps
-        const uint32_t count = b < kMaxASlots ? 4u : b < 2 * kMaxASlots + 2 * kMaxBSlots ? 1u : b < 2 * kMaxASlots + 2 * kMaxBSlots + 2 ? kMmaWarps : kEpiWarps;
+        // issuing warp; acc_empty: the epilogue warps; the last two: an issuing warp's turn
+        constexpr uint32_t kRings = 2 * kMaxASlots + 2 * kMaxBSlots;
+        const uint32_t count = b < kMaxASlots ? 4u : b < kRings ? 1u : b < kRings + 2 ? kMmaWarps : b < kRings + 4 ? kEpiWarps : 1u;
         mbar_init(a_full0 + 8 * b, count);
         fence_barrier_init();
     }
@@ -182,7 +184,7 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(s_misc);
-    // Every MMA accumulates (two warps issue them, in no fixed order), so the accumulators start at
+    // Every MMA accumulates (the first of an item too), so the accumulators start at
     // zero: the epilogue warps clear both here and clear each again after reading it.
     if (warp >= kFirstEpiWarp) {
         const uint32_t zero[32] = {};
@@ -217,9 +219,10 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
         // ---------------- MMA issuers: two warps, slab x of the CTA's sequence goes to warp x % 2.
         // A slab's turn (barrier probes, fence, election, four tcgen05.mma of 32 bytes of K each, one
         // commit per ring) costs the issuing warp about 600 cycles, more than the four MMAs take to
-        // execute; two warps taking turns keep the tensor pipe fed.  All MMAs accumulate into an
-        // accumulator the epilogue left at zero, integer addition commutes, so the order in which
-        // the two warps' instructions reach the pipe does not matter.  Each warp walks its loop
+        // execute; two warps taking turns keep the tensor pipe fed.  They accumulate into one accumulator,
+        // which is ordered between instructions of one thread only: a warp waits for its turn before it issues and
+        // hands over behind its four instructions, with the tcgen05 fences on either side of the
+        // barrier.  Each warp walks its loop
         // converged (waits and descriptor arithmetic stay warp-uniform; a lone lane running the
         // loop measured 20 % slower), one elected lane issues.
         {
@@ -250,6 +253,8 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
                         ok = mbar_wait(b_full0 + 8 * j, pb, s_abort) && mbar_wait(a_full0 + 8 * k, pa, s_abort);
                         if (!ok) break;
                     }
+                    ok = mbar_wait(turn0 + 8 * me, ((x >> 1) & 1u) ^ (me == 0 ? 1u : 0u), s_abort);   // slab 0 has its turn
+                    if (!ok) break;
                     uint32_t j2 = j + 2, pb2 = pb;
                     if (j2 >= SB) { j2 -= SB; pb2 ^= 1; }
                     uint32_t k2, pa2;
@@ -271,6 +276,8 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
                                 umma_i8(d_tmem, ((uint64_t)desc_hi << 32) | (a_lo + 2 * kk),
                                         ((uint64_t)desc_hi << 32) | (b_lo + 2 * kk), kIdesc, 1u);
                         }
+                        tc_fence_before_sync();
+                        mbar_arrive(turn0 + 8 * (me ^ 1u));
                         umma_commit(a_empty0 + 8 * k);  // each slot is free once these MMAs have read it
                         umma_commit(b_empty0 + 8 * j);
                     }

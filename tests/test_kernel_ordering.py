@@ -25,7 +25,7 @@ def test_epilogue_warps_meet_before_they_read(name, epilogues):
         assert "__syncwarp();" in until[until.index("__shfl_sync("):]
 
 
-@pytest.mark.parametrize("name", ["lut_sparse_umma.cu"])
+@pytest.mark.parametrize("name", ["lut_sparse_umma.cu", "lut_onehot_umma.cu"])
 def test_issuing_warps_take_turns(name):
     """Several warps issue MMAs into one accumulator.  Read-modify-writes of an accumulator are ordered between the
     instructions of one thread; between threads it takes a fence, a barrier and a fence: before its first instruction of a
