@@ -635,13 +635,13 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
                             if ((spin & 63u) == 63u && *s_abort) break;
                             __nanosleep(64);
                         }
+                        __threadfence();  // between the counter's value and the partial sums it stands for
                         if (!go) *s_abort = 1u;
                     }
                     s_misc[2] = go;
                 }
                 named_bar_sync(1, kEpiThreads);
                 if (s_misc[2]) {
-                    __threadfence();
                     // All loads of a row first, then the stores: the loop is a chain of L2 round
                     // trips otherwise.
                     constexpr uint32_t kChunks = N_TILE / 32;

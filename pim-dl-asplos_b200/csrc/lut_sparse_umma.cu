@@ -212,15 +212,16 @@ __device__ __forceinline__ bool split_finish(const SparseParams& p, const Sparse
                 go = *reinterpret_cast<volatile uint32_t*>(ctr) >= p.split;
                 if ((spin & 63u) == 63u && *s_abort) break;
             }
+            __threadfence();   // between the counter's value and the sums that it stands for, for everybody released here
             if (go) mbar_arrive(sums_bar + 8 * quad);
             else *s_abort = 1u;
         }
         go = __shfl_sync(0xffffffffu, go, 0);
+        __syncwarp();   // ... in this warp too: a shuffle orders no memory
     } else {
         go = mbar_wait<32>(sums_bar + 8 * quad, 0, s_abort);
     }
     if (!go) return false;
-    __threadfence();
     const float lbcb = lut_bias_times_cb(a.lut_bias, a.CB);
     const uint32_t row = it.m0 + quad * 32 + lane;
     constexpr uint32_t kUnits = N_TILE / 4;   // groups of four columns

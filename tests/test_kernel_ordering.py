@@ -41,3 +41,19 @@ def test_issuing_warps_take_turns(name):
         break
     else:
         pytest.fail("no issue loop found")
+
+
+@pytest.mark.parametrize("name,poll,release", [("lut_sparse_umma.cu", "go = *reinterpret_cast<volatile uint32_t*>(ctr) >= p.split;", "mbar_arrive(sums_bar"),
+                                               ("lut_onehot_umma.cu", "*reinterpret_cast<volatile uint32_t*>(ctr) >= p.split", "s_misc[2] = go;")])
+def test_split_sums_are_read_behind_a_fence(name, poll, release):
+    """The thread that sees all slices of a tile stored releases the others, and they read what the counter stands for: the
+    fence belongs to that thread, before the release."""
+    src = _source(name)
+    seen = src.index(poll)
+    assert "__threadfence();" in src[seen:src.index(release, seen)]
+
+
+def test_the_polling_warp_meets_behind_the_fence():
+    src = _source("lut_sparse_umma.cu")
+    told = src.index("__shfl_sync(0xffffffffu, go, 0);")
+    assert "__syncwarp();" in src[told:src.index("} else {", told)]
