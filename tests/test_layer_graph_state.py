@@ -1,0 +1,59 @@
+"""When a layer's captured forward may be replayed: a set-up that changes between calls takes the ordinary path again.  On
+the CPU, with a graph that records nothing and a context that only has what the key is made of."""
+import types
+
+import pytest
+import torch
+
+from pim_dl_asplos_b200 import layer as L
+
+
+class _Graph:
+    def capture_begin(self, **kw):
+        pass
+
+    def capture_end(self):
+        pass
+
+    def replay(self):
+        self.replayed = True
+
+
+class _Torch:
+    """torch, with a stream and graphs that need no GPU."""
+    cuda = types.SimpleNamespace(current_stream=lambda device: types.SimpleNamespace(cuda_stream=7), is_current_stream_capturing=lambda: False,
+                                 CUDAGraph=_Graph)
+
+    def __getattr__(self, name):
+        return getattr(torch, name)
+
+
+class _Layer(L.LutTransformerLayer):
+    def __init__(self, n=4, dim=8):
+        self.ctx = types.SimpleNamespace(device=None, stream=7, generation=1, launch_count=0)
+        self.torch, self.n, self.token_dim, self.fused_gelu, self.ln = _Torch(), n, dim, True, {"ln1": (torch.ones(dim), torch.zeros(dim))}
+        self._graph, self._seen, self._seen_key = None, 0, None
+        self.bodies = 0
+
+    def _body(self, x):
+        self.bodies += 1
+        return x + 1, 2 * x
+
+
+def _captured(lay, x):
+    for _ in range(4):
+        lay.forward(x)
+    assert lay._graph is not None and lay._graph[1].replayed
+    lay.bodies = 0
+    return lay
+
+
+def test_a_forward_captured_in_inference_mode_is_not_replayed_outside():
+    x = torch.arange(32.0).view(4, 8)
+    with torch.inference_mode():
+        lay = _captured(_Layer(), x)
+    y = lay.forward(x)
+    assert lay.bodies == 1 and torch.equal(y, 3 * x + 1)
+    lay = _captured(_Layer(), x)
+    with torch.inference_mode():
+        assert torch.equal(lay.forward(x), 3 * x + 1)
