@@ -57,3 +57,17 @@ def test_a_forward_captured_in_inference_mode_is_not_replayed_outside():
     lay = _captured(_Layer(), x)
     with torch.inference_mode():
         assert torch.equal(lay.forward(x), 3 * x + 1)
+
+
+@pytest.mark.parametrize("owner", [torch.backends.cuda.matmul, torch.backends])
+def test_either_api_of_the_matmul_precision(owner):
+    """Reading allow_tf32 raises once a program has set fp32_precision.  The precision itself belongs to what a capture is
+    valid for: attention by two matrix products follows it."""
+    x = torch.ones(4, 8)
+    before = owner.fp32_precision
+    lay = _captured(_Layer(), x)
+    try:
+        owner.fp32_precision = "tf32"
+        assert torch.equal(lay.forward(x), 3 * x + 1) and lay.bodies == 1
+    finally:
+        owner.fp32_precision = before
