@@ -200,8 +200,9 @@ class LutTransformerLayer:
         if not stream or stream != self.ctx.stream or torch.cuda.is_current_stream_capturing():
             return None
         sdp = torch.backends.cuda
-        return (stream, self.ctx.generation, self.fused_gelu, torch.is_inference_mode_enabled(), sdp.flash_sdp_enabled(), sdp.mem_efficient_sdp_enabled(),
-                sdp.math_sdp_enabled(), sdp.cudnn_sdp_enabled(), sdp.matmul.fp32_precision, tuple(t.data_ptr() for pair in self.ln.values() for t in pair))
+        return (stream, self.ctx.generation, self.fused_gelu, torch.is_inference_mode_enabled(),
+                sdp.flash_sdp_enabled(), sdp.mem_efficient_sdp_enabled(), sdp.math_sdp_enabled(), sdp.cudnn_sdp_enabled(),
+                tuple(torch._C._get_sdp_priority_order()), sdp.matmul.fp32_precision, tuple(t.data_ptr() for pair in self.ln.values() for t in pair))
 
     def _capture(self, x, key):
         """Record the layer up to its last addition on a copy of the input: 16 launches and their Python become one.

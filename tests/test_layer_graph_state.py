@@ -71,3 +71,15 @@ def test_either_api_of_the_matmul_precision(owner):
         assert torch.equal(lay.forward(x), 3 * x + 1) and lay.bodies == 1
     finally:
         owner.fp32_precision = before
+
+
+def test_the_priority_of_the_attention_back_ends():
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+    every = [SDPBackend.MATH, SDPBackend.EFFICIENT_ATTENTION, SDPBackend.FLASH_ATTENTION, SDPBackend.CUDNN_ATTENTION]
+    x = torch.ones(4, 8)
+    lay = _Layer()
+    with sdpa_kernel(every, set_priority=True):
+        _captured(lay, x)
+    with sdpa_kernel(every[::-1], set_priority=True):
+        lay.forward(x)
+    assert lay.bodies == 1
