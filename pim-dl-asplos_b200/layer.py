@@ -193,8 +193,8 @@ class LutTransformerLayer:
     def _graph_key(self, x):
         """What a captured forward depends on beyond the values in x; None where it does not apply."""
         torch = self.torch
-        if ("_amm" in self.__dict__ or x.dtype != torch.float32 or x.shape != (self.n, self.token_dim) or x.device.index != self.ctx.device
-                or x.requires_grad or torch.is_autocast_enabled()):
+        if (x.dtype != torch.float32 or x.shape != (self.n, self.token_dim) or x.device.index != self.ctx.device or x.requires_grad
+                or torch.is_autocast_enabled()):
             return None
         stream = torch.cuda.current_stream(x.device).cuda_stream
         if not stream or stream != self.ctx.stream or torch.cuda.is_current_stream_capturing():

@@ -83,3 +83,11 @@ def test_the_priority_of_the_attention_back_ends():
     with sdpa_kernel(every[::-1], set_priority=True):
         lay.forward(x)
     assert lay.bodies == 1
+
+
+def test_no_branch_for_a_replaced_operator_call():
+    """Whether a forward may be replayed does not depend on how a test watches its linears."""
+    lay, x = _Layer(), torch.ones(4, 8)
+    key = lay._graph_key(x)
+    lay._amm = None
+    assert key is not None and lay._graph_key(x) == key
