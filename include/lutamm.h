@@ -366,7 +366,8 @@ int lutamm_selftest_bounded_wait(lutamm_ctx* ctx, uint32_t polls);
  * captured calls compares it with the value it captured under. */
 uint64_t lutamm_generation(const lutamm_ctx* ctx);
 
-/* Kernels of this library launched on this context since creation. */
+/* Kernels of this library that calls on this context have queued since creation.  A call captured into a CUDA graph
+ * counts once, when it is captured; what a replay runs the library does not see. */
 uint64_t lutamm_launch_count(const lutamm_ctx* ctx);
 
 /* ---- for callers that must not allocate -------------------------------------------- */

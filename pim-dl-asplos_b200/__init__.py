@@ -257,9 +257,13 @@ class LutAmmContext:
     def sync(self):
         self._check(self._L.lutamm_sync(self._h))
 
+    # launches of replayed graphs, which the library does not see, less those that were only recorded
+    replayed_launches = 0
+
     @property
     def launch_count(self) -> int:
-        return int(self._L.lutamm_launch_count(self._h))
+        """Kernels of this library run on this context: queued by its calls (lutamm_launch_count) or replayed by a layer."""
+        return int(self._L.lutamm_launch_count(self._h)) + self.replayed_launches
 
     @property
     def generation(self) -> int:

@@ -159,7 +159,7 @@ class LutTransformerLayer:
         else:
             self.buf["qkv"] = torch.empty(self.n, 3 * self.token_dim, **f32)
         self.amm_ms = 0.0
-        self._graph = None          # (key, graph, input copy, h, f) of the captured forward
+        self._graph = None          # (key, graph, input copy, h, f, launches) of the captured forward
         self._seen, self._seen_key = 0, None
 
     def tune(self):
@@ -176,9 +176,10 @@ class LutTransformerLayer:
             key = self._graph_key(x)
             if key is not None:
                 if self._graph is not None and self._graph[0] == key:
-                    _, graph, x_in, h, f = self._graph
+                    _, graph, x_in, h, f, launches = self._graph
                     x_in.copy_(x)
                     graph.replay()
+                    self.ctx.replayed_launches += launches
                     return h + f
                 # two ordinary calls under the same key first: they size every buffer, and a caller that keeps
                 # changing something is left alone
@@ -210,17 +211,20 @@ class LutTransformerLayer:
         torch = self.torch
         graph = torch.cuda.CUDAGraph()
         x_in = torch.empty_like(x)
+        queued = self.ctx.launch_count
         try:
             graph.capture_begin(capture_error_mode="thread_local")
             try:
                 h, f = self._body(x_in)
             finally:
+                launches = self.ctx.launch_count - queued
+                self.ctx.replayed_launches -= launches   # recorded, not run
                 graph.capture_end()
         except RuntimeError:
             self._seen = -(1 << 62)   # this set-up does not capture: ordinary calls from now on
             return
         if self.ctx.generation == key[1]:
-            self._graph = (key, graph, x_in, h, f)
+            self._graph = (key, graph, x_in, h, f, launches)
 
     def _body(self, x):
         """The layer up to its last addition: y = h + f."""

@@ -5,6 +5,7 @@ import types
 import pytest
 import torch
 
+import pim_dl_asplos_b200 as P
 from pim_dl_asplos_b200 import layer as L
 
 
@@ -28,15 +29,30 @@ class _Torch:
         return getattr(torch, name)
 
 
+class _Library:
+    queued = 0
+
+    def lutamm_launch_count(self, handle):
+        return self.queued
+
+
+class _Context(P.LutAmmContext):
+    generation = 1
+
+    def __init__(self):
+        self._L, self._h, self.device, self.stream = _Library(), None, None, 7
+
+
 class _Layer(L.LutTransformerLayer):
     def __init__(self, n=4, dim=8):
-        self.ctx = types.SimpleNamespace(device=None, stream=7, generation=1, launch_count=0)
+        self.ctx = _Context()
         self.torch, self.n, self.token_dim, self.fused_gelu, self.ln = _Torch(), n, dim, True, {"ln1": (torch.ones(dim), torch.zeros(dim))}
         self._graph, self._seen, self._seen_key = None, 0, None
         self.bodies = 0
 
     def _body(self, x):
         self.bodies += 1
+        self.ctx._L.queued += 8
         return x + 1, 2 * x
 
 
@@ -91,3 +107,12 @@ def test_no_branch_for_a_replaced_operator_call():
     key = lay._graph_key(x)
     lay._amm = None
     assert key is not None and lay._graph_key(x) == key
+
+
+def test_launches_of_a_replayed_forward_count():
+    """Each forward runs eight kernels of the library, whether it queues them or replays them; recording them runs none."""
+    lay, x = _Layer(), torch.ones(4, 8)
+    for forwards in range(1, 9):
+        lay.forward(x)
+        assert lay.ctx.launch_count == 8 * forwards
+    assert lay._graph[1].replayed
