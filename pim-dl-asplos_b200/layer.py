@@ -194,8 +194,14 @@ class LutTransformerLayer:
     def _graph_key(self, x):
         """What a captured forward depends on beyond the values in x; None where it does not apply."""
         torch = self.torch
-        if (x.dtype != torch.float32 or x.shape != (self.n, self.token_dim) or x.device.index != self.ctx.device or x.requires_grad
-                or torch.is_autocast_enabled()):
+        if (type(x) is not torch.Tensor or x.dtype != torch.float32 or x.shape != (self.n, self.token_dim) or not x.is_contiguous()
+                or x.device.index != self.ctx.device or torch.is_autocast_enabled()):
+            return None
+        # a forward that autograd follows, in either direction, is not a recorded one
+        norms = [t for pair in self.ln.values() for t in pair]
+        if torch.is_grad_enabled() and any(t.requires_grad for t in (x, *norms)):
+            return None
+        if torch.autograd.forward_ad.unpack_dual(x).tangent is not None:
             return None
         stream = torch.cuda.current_stream(x.device).cuda_stream
         if not stream or stream != self.ctx.stream or torch.cuda.is_current_stream_capturing():
@@ -203,7 +209,7 @@ class LutTransformerLayer:
         sdp = torch.backends.cuda
         return (stream, self.ctx.generation, self.fused_gelu, torch.is_inference_mode_enabled(),
                 sdp.flash_sdp_enabled(), sdp.mem_efficient_sdp_enabled(), sdp.math_sdp_enabled(), sdp.cudnn_sdp_enabled(),
-                tuple(torch._C._get_sdp_priority_order()), sdp.matmul.fp32_precision, tuple(t.data_ptr() for pair in self.ln.values() for t in pair))
+                tuple(torch._C._get_sdp_priority_order()), sdp.matmul.fp32_precision, tuple(t.data_ptr() for t in norms))
 
     def _capture(self, x, key):
         """Record the layer up to its last addition on a copy of the input: 16 launches and their Python become one.

@@ -116,3 +116,22 @@ def test_launches_of_a_replayed_forward_count():
         lay.forward(x)
         assert lay.ctx.launch_count == 8 * forwards
     assert lay._graph[1].replayed
+
+
+def test_what_the_ordinary_call_refuses_or_autograd_follows_is_not_replayed():
+    import torch.autograd.forward_ad as fw
+    x = torch.ones(4, 8)
+    lay = _captured(_Layer(), x)
+    assert lay._graph_key(torch.ones(8, 4).t()) is None           # the operator takes contiguous tensors only
+    with fw.dual_level():                                       # the addition of x carries its tangent
+        assert lay._graph_key(fw.make_dual(x, x)) is None
+        assert lay._graph_key(x) is not None
+
+    class Tensor(torch.Tensor):
+        pass
+
+    assert lay._graph_key(x.as_subclass(Tensor)) is None
+    lay.ln["ln1"][0].requires_grad_()
+    assert lay._graph_key(x) is None
+    with torch.no_grad():
+        assert lay._graph_key(x) is not None
