@@ -11,6 +11,7 @@ from __future__ import annotations
 import ctypes
 import importlib.util
 import os
+import sysconfig
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -92,11 +93,24 @@ class Timings(ctypes.Structure):
 
 
 _lib = None
-_fast = None   # the operator call as a CPython function (csrc/python/fastcall.c), where it has been built
-if os.path.exists(os.path.join(_HERE, "_fastcall.so")):
-    _spec = importlib.util.spec_from_file_location("_fastcall", os.path.join(_HERE, "_fastcall.so"))
-    _fast = importlib.util.module_from_spec(_spec)
-    _spec.loader.exec_module(_fast)
+
+
+def _load_fastcall():
+    """The operator call as a CPython function (csrc/python/fastcall.c), where it has been built for this interpreter; None
+    leaves the call to ctypes, which does the same."""
+    path = os.path.join(_HERE, "_fastcall" + sysconfig.get_config_var("EXT_SUFFIX"))
+    if not os.path.exists(path):
+        return None
+    spec = importlib.util.spec_from_file_location("_fastcall", path)
+    try:
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+    except ImportError:
+        return None
+    return module
+
+
+_fast = _load_fastcall()
 
 
 def load_library() -> ctypes.CDLL:

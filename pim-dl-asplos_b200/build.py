@@ -16,7 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libpimdl_b200.so")
 HOST_LIB = os.path.join(HERE, "libpimdl_host.so")
-FASTCALL = os.path.join(HERE, "_fastcall.so")
+FASTCALL = os.path.join(HERE, "_fastcall" + sysconfig.get_config_var("EXT_SUFFIX"))   # for this interpreter alone
 TEST_AMM = os.path.join(HERE, "bin", "test_amm")
 TUNER = os.path.join(HERE, "bin", "tuner")
 TEST_LAYER = os.path.join(HERE, "bin", "test_transformer_layer")
