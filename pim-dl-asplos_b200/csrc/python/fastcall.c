@@ -56,8 +56,11 @@ static PyObject* amm(PyObject* self, PyObject* const* args, Py_ssize_t n) {
         Py_DECREF(shape);
         if (!rows) return NULL;
     }
-    const unsigned long tokens = PyLong_AsUnsignedLongMask(rows ? rows : args[5]);
+    PyObject* count = PyNumber_Long(rows ? rows : args[5]);   /* int() of it, as in amm_host */
     Py_XDECREF(rows);
+    if (!count) return NULL;
+    const unsigned long tokens = PyLong_AsUnsignedLongMask(count);
+    Py_DECREF(count);
     const unsigned long flags = PyLong_AsUnsignedLongMask(args[6]);
     if (PyErr_Occurred()) return NULL;
     int rc;
