@@ -153,18 +153,22 @@ lut_build_kernel(const float* __restrict__ centroid, const float* __restrict__ w
 
 template <int V>
 cudaError_t launch_both(const LutBuildArgs& a, dim3 grid, size_t smem, cudaStream_t s) {
-    lut_build_kernel<V, false><<<grid, kThreads, smem, s>>>(a.centroid, a.weight, nullptr, a.words, nullptr, a.CT, a.v, a.N);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, lut_build_kernel<V, false>, a.centroid, a.weight, static_cast<int8_t*>(nullptr), a.words, static_cast<float*>(nullptr), a.CT, a.v, a.N);
+    if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, lut_build_kernel<V, true>, a.centroid, a.weight, a.lut, a.words, a.scalars, a.CT, a.v, a.N);
+    e = cudaLaunchKernelEx(&cfg, lut_build_kernel<V, true>, a.centroid, a.weight, a.lut, a.words, a.scalars, a.CT, a.v, a.N);
+    // only pass 2 clears the maximum that pass 1 leaves, and the next table would be scaled with it
+    if (e != cudaSuccess) cudaMemsetAsync(a.words, 0, 2 * sizeof(uint32_t), s);
+    return e;
 }
 
 }  // namespace
