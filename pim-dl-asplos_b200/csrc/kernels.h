@@ -90,8 +90,8 @@ cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N,
 size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N);
 // ... of `n` columns of a table that has `pitch`, from column n0 on; chained: nothing the stream still runs writes `lut`
 cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t n, uint32_t n0, uint32_t pitch, bool chained, cudaStream_t s);
-// ... returns the microseconds it expects, launch apart (about 4)
-float sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split);
+// Tile width (`only`, where that is not 0) and split; returns the microseconds it expects, launch apart (about 4)
+float sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split, uint32_t only = 0);
 void sparse_split_scratch(uint32_t M, uint32_t N, uint32_t n_tile, uint32_t split, size_t* partial_bytes, size_t* counter_bytes);
 bool sparse_tile_ok(uint32_t n_tile);
 cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile,

@@ -262,9 +262,9 @@ int run_sparse(lutamm_ctx* c, Layer& L, const LutArgs& a, uint32_t n_tile, uint3
     int r = make_table(c, &L.d_lut_s, sparse_table_bytes(L.CB, L.CT, L.N),
                        [&](int8_t* t) { return launch_sparse_table(L.d_lut, t, L.CB, L.CT, L.N, 0, L.N, false, c->stream); });
     if (r) return r;
-    if (!n_tile) {
+    if (!n_tile || !split) {
         uint32_t s;
-        sparse_default_plan(a.M, a.CB, a.CT, a.N, c->sm_count, &n_tile, &s);
+        sparse_default_plan(a.M, a.CB, a.CT, a.N, c->sm_count, &n_tile, &s, n_tile);
         if (!split) split = s;
     }
     if (split > 1 && (uint64_t)((a.M + 255) / 256) * ((a.N + n_tile - 1) / n_tile) * split > (uint64_t)c->sm_count / 2) split = 1;

@@ -1,0 +1,57 @@
+"""Plans: what a plan leaves at 0 is the library's choice, and tuning does not make a call slower than leaving it alone."""
+import numpy as np
+import pytest
+
+import pim_dl_asplos_b200 as P
+
+pytestmark = pytest.mark.gpu
+
+
+class _Call:
+    """One operator on device buffers; microseconds of a call, calls queued back to back."""
+
+    def __init__(self, ctx, M, K, N, v=2, CT=16):
+        import torch
+        self.ctx, self.torch, self.M = ctx, torch, M
+        rng = np.random.default_rng(K + N)
+        ctx.load_weights(83, rng.standard_normal((K // v, CT, v), dtype=np.float32), rng.integers(-127, 128, (K // v, CT, N), dtype=np.int8),
+                         rng.standard_normal(N, dtype=np.float32), 0.01)
+        self.stream = torch.cuda.Stream()
+        ctx.set_stream(self.stream.cuda_stream)
+        with torch.cuda.stream(self.stream):
+            self.x, self.y = torch.randn(M, K, device="cuda"), torch.empty(M, N, device="cuda")
+        self.stream.synchronize()
+
+    def us(self, calls=100):
+        e = [self.torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        for _ in range(5):
+            self.ctx.amm_host(83, self.x, self.y, flags=P.FLAG_ASYNC)
+        e[0].record(self.stream)
+        for _ in range(calls):
+            self.ctx.amm_host(83, self.x, self.y, flags=P.FLAG_ASYNC)
+        e[1].record(self.stream)
+        self.ctx.sync()
+        return e[0].elapsed_time(e[1]) * 1e3 / calls
+
+    def median(self, *plans, rounds=7):
+        """Median time per plan (None: the layer's own), the plans taken in turn."""
+        times = [[] for _ in plans]
+        for _ in range(rounds):
+            for t, plan in zip(times, plans):
+                self.ctx.set_plan(83, **plan)
+                t.append(self.us())
+        return [sorted(t)[rounds // 2] for t in times]
+
+    def close(self):
+        self.ctx.set_stream(None)
+        self.ctx.unload_weights(83)
+
+
+def test_a_named_tile_splits_by_itself(ctx):
+    """umma_split 0 is the library's choice also where the plan names the sparse form and its tile: 12 tiles of 384 slabs
+    each on 74 pairs (about 12 us split, 21 whole; the bar is half-way)."""
+    call = _Call(ctx, 128, 3072, 768)
+    own, named, whole = call.median({}, dict(variant=P.VARIANT_UMMA, umma_operand=3, umma_n_tile=64),
+                                    dict(variant=P.VARIANT_UMMA, umma_operand=3, umma_n_tile=64, umma_split=1))
+    call.close()
+    assert named < (own + whole) / 2
