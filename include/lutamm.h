@@ -326,8 +326,10 @@ int lutamm_get_plan(lutamm_ctx* ctx, int layer_id, lutamm_plan* plan);
 int lutamm_set_activation(lutamm_ctx* ctx, int layer_id, uint32_t activation);
 
 /* Replaces the auto-tuner's mapping search (src/tuner/auto_tuner.cpp:368-603): times the
- * candidate kernel variants and tile configurations for n_tokens rows with CUDA events
- * and installs the fastest.  best may be NULL. */
+ * candidate kernel variants and tile configurations for n_tokens rows with CUDA events - whole calls, search and
+ * contraction, on activations that select all rows of the table - and installs the fastest.  The library's own choice is the
+ * one to beat: another plan replaces it where it is faster by 2 % and by more than the runs of either differ.
+ * best may be NULL. */
 int lutamm_tune(lutamm_ctx* ctx, int layer_id, uint32_t n_tokens, lutamm_plan* best);
 
 /* Plans found by lutamm_tune are remembered in the context by shape - (n_tokens, K, N, CB, CT, SM count) -

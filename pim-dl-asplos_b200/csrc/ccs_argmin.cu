@@ -725,7 +725,17 @@ cudaError_t run_any(const CcsArgs& a, cudaStream_t s) {
                             cb_per_cta, a.n_stile, a.cb_mtile);
 }
 
+// The instances whose thread walks a run of tokens.
+#define LUTAMM_CCS_RUN_INSTANCES(X) X(2, 8) X(2, 16) X(4, 8)
+
 }  // namespace
+
+// Whether tokens_per_thread changes anything but the choice of the short form.
+bool ccs_reads_tokens_per_thread(uint32_t v, uint32_t CT) {
+#define LUTAMM_CCS_IS(V_, CT_) || (v == V_ && CT == CT_)
+    return false LUTAMM_CCS_RUN_INSTANCES(LUTAMM_CCS_IS);
+#undef LUTAMM_CCS_IS
+}
 
 cudaError_t launch_ccs(const CcsArgs& a, cudaStream_t s, const char** why) {
     *why = nullptr;
@@ -751,9 +761,7 @@ cudaError_t launch_ccs(const CcsArgs& a, cudaStream_t s, const char** why) {
 #undef LUTAMM_CCS_SHORT
 #define LUTAMM_CCS_REG(V_, CT_) \
     if (a.v == V_ && a.CT == CT_) return run_reg<V_, CT_>(a, s);
-        LUTAMM_CCS_REG(2, 8)
-        LUTAMM_CCS_REG(2, 16)
-        LUTAMM_CCS_REG(4, 8)
+        LUTAMM_CCS_RUN_INSTANCES(LUTAMM_CCS_REG)
 #undef LUTAMM_CCS_REG
     }
     switch (a.v) {

@@ -62,7 +62,7 @@ void put_plan(yaml_lite::Doc& doc, const std::string& pre, const GpuPlan& p) {
 }
 
 void print_plan(const char* what, const GpuPlan& best) {
-    std::cout << what << ": variant " << best.variant << " (1 gather, 2 tcgen05), ccs tokens " << best.ccs_tokens << ", gather cfg "
+    std::cout << what << ": variant " << best.variant << " (0 auto, 1 gather, 2 tcgen05), ccs tokens " << best.ccs_tokens << ", gather cfg "
               << best.gather_cfg << ", n tile " << best.umma_n_tile << ", split " << best.umma_split << ", stages " << best.umma_stages
               << ", groups " << best.umma_groups << ", operand " << best.umma_operand << std::endl;
 }

@@ -85,6 +85,25 @@ cudaError_t launch_int8_peak(uint32_t n_tile, uint32_t slabs, uint32_t grid, uns
 }
 
 
+// ---- activations to time an operator on ------------------------------------------------------------
+// Which rows of the table a call reads, and how often the search's filter decides, depend on the activations: with one
+// centroid for all tokens the rows would come from L2.
+namespace {
+__global__ void spread_input_kernel(const float* __restrict__ centroid, float* __restrict__ x, uint64_t count, uint32_t CB, uint32_t CT, uint32_t v) {
+    const uint32_t K = CB * v;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t m = (uint32_t)(i / K), k = (uint32_t)(i % K), cb = k / v;
+        const uint32_t c = (m * 2654435761u + cb * 2246822519u) / 65536u % CT;
+        x[i] = centroid[((size_t)cb * CT + c) * v + k % v];
+    }
+}
+}  // namespace
+
+cudaError_t launch_spread_input(const float* centroid, float* x, uint32_t M, uint32_t CB, uint32_t CT, uint32_t v, cudaStream_t s) {
+    spread_input_kernel<<<1184, 256, 0, s>>>(centroid, x, (uint64_t)M * CB * v, CB, CT, v);
+    return cudaGetLastError();
+}
+
 // ---- self-test of the way out after a wait that runs out -----------------------------------------
 // One CTA sets up what the tcgen05 LUT kernel sets up (tensor memory, an mbarrier), then one thread waits
 // - with the library's own bounded wait, limited to `polls` probes - on a barrier nobody ever arrives at.

@@ -18,6 +18,7 @@ struct CcsArgs {
     uint32_t tokens_per_thread;  // 0 = default
 };
 cudaError_t launch_ccs(const CcsArgs& a, cudaStream_t s, const char** why);
+bool ccs_reads_tokens_per_thread(uint32_t v, uint32_t CT);
 
 // ---- step 2+3: gather-accumulate + dequantise -----------------------------------------
 // Output addressing: row-major [M][N], or the reference's DPU-tiled layout.
@@ -131,6 +132,9 @@ cudaError_t launch_lut_untile(const int8_t* dpu, int8_t* canonical, uint32_t row
 // `slabs` x four 128 x n_tile x 32 instructions per CTA, `grid` CTAs; the cycles CTA 0 took land in *d_cycles.
 cudaError_t launch_int8_peak(uint32_t n_tile, uint32_t slabs, uint32_t grid, unsigned long long* d_cycles, uint32_t* dev_err,
                              cudaStream_t s, const char** why);
+
+// Activations for timing: token m's sub-vector of codebook cb is one of that codebook's centroids, spread evenly over them.
+cudaError_t launch_spread_input(const float* centroid, float* x, uint32_t M, uint32_t CB, uint32_t CT, uint32_t v, cudaStream_t s);
 
 // Self-test: a bounded wait on a barrier nobody arrives at; the kernel reports through *dev_err and returns.
 cudaError_t launch_stalled_wait(uint32_t polls, uint32_t* dev_err, cudaStream_t s);

@@ -7,7 +7,8 @@ loading x tile shapes, and loop order x sub-LUT tile for the "global optimal" pl
 baseline latency; it then marks the auto-tuner's pick against the measured best and worst.  On a GPU the
 mapping space is the execution plan of the library (lutamm_plan), so the same experiment is a sweep of that:
 
-  operand-tile   where the one-hot operand lives (tensor / shared memory) x tile width      (tcgen05 kernel)
+  operand-tile   where the one-hot operand lives (2 / 1: tensor / shared memory, 3: tensor memory in the 2:4 sparse form)
+                 x tile width                                                              (tcgen05 kernels)
   split-ring     split of the codebook axis x depth of the LUT ring                         (tcgen05 kernel)
   builders       one-hot builder groups x tile width                                        (tcgen05 kernel)
   epilogue       how finished tiles leave the SM (transposing stores / copy engine) x width (tcgen05 kernel)
@@ -17,6 +18,7 @@ mapping space is the execution plan of the library (lutamm_plan), so the same ex
     python search_space.py                                        # all explorations -> CSV
     python search_space.py --single_point --experiment_type operand-tile --exploration_value 2-192
     python search_space.py --plot_only                            # re-emit the summary from saved CSVs
+    python search_space.py --tuned_linears                        # tuner's pick against no plan, BERT-base linears by tokens
 
 Results are CSV (no matplotlib here): per point the device time of the whole operator (search + LUT kernel),
 and the speed-up over the library's default plan.
@@ -39,7 +41,7 @@ def points(experiment: str):
     U, G = 2, 1
     if experiment == "operand-tile":
         return [(f"{op}-{nt}", dict(variant=U, umma_operand=op, umma_n_tile=nt, umma_split=1))
-                for op, tiles in ((2, (64, 128, 160, 192)), (1, (64, 128, 256))) for nt in tiles]
+                for op, tiles in ((3, (64, 128, 160)), (2, (64, 128, 160, 192)), (1, (64, 128, 256))) for nt in tiles]
     if experiment == "split-ring":
         return [(f"{sp}-{st}", dict(variant=U, umma_operand=2, umma_n_tile=192, umma_split=sp, umma_stages=st))
                 for sp in (1, 2, 4) for st in (2, 4, 6, 0)]
@@ -71,13 +73,14 @@ def parse_args(argv=None):
     p.add_argument('--exploration_value', type=str, default="2-192")
     p.add_argument('--out_dir', type=str, default=os.path.join(os.getcwd(), "search_space_results"))
     p.add_argument('--tokens', type=int, default=SHAPE["n"])
+    p.add_argument('--tuned_linears', action='store_true', default=False)
     p.add_argument('--dry_run', action='store_true', help='list the points, run nothing')
     p.add_argument('--device', type=int, default=0)
     return p.parse_args(argv)
 
 
 class Bench:
-    def __init__(self, tokens: int, device: int):
+    def __init__(self, tokens: int, device: int, shape: dict = SHAPE):
         import torch
         import pim_dl_asplos_b200 as P
         from pim_dl_asplos_b200 import synth
@@ -86,7 +89,7 @@ class Bench:
         self.ctx = P.LutAmmContext(device)
         self.stream = torch.cuda.Stream()
         self.ctx.set_stream(self.stream.cuda_stream)
-        K, N, CB, CT = SHAPE["K"], SHAPE["N"], SHAPE["CB"], SHAPE["CT"]
+        K, N, CB, CT = (shape[k] for k in ("K", "N", "CB", "CT"))
         cen, lut, bias = synth.make_weights(K, N, K // CB, CT, seed=0)
         self.ctx.load_weights(0, cen, lut, bias, 0.1, 0.2)     # the reference configs' scale / bias
         with torch.cuda.stream(self.stream):
@@ -137,6 +140,21 @@ def run_experiment(bench, experiment: str, out_dir: str):
     return rows
 
 
+def tuned_linears(device: int, tokens=(32, 128, 512, 1024, 12608)):
+    """Each linear of a BERT-base layer by tokens: microseconds without a plan and with the tuner's pick, in turn, the
+    least of five rounds."""
+    rows = []
+    for M in tokens:
+        for name, K, N in (("qkv", 768, 2304), ("o", 768, 768), ("ffn1", 768, 3072), ("ffn2", 3072, 768)):
+            b = Bench(M, device, dict(K=K, N=N, CB=K // 2, CT=16))
+            pick = b.tuned()
+            own, tuned = (1e6 * min(t) for t in zip(*((b.seconds({}, 100), b.seconds(pick, 100)) for _ in range(5))))
+            b.ctx.close()
+            rows.append(dict(tokens=M, linear=name, own_us=own, tuned_us=tuned, plan={k: v for k, v in pick.items() if v}))
+            print(f"{M:6d} tokens, {name:4s}: no plan {own:7.2f} us, tuned {tuned:7.2f} us  {rows[-1]['plan']}")
+    return rows
+
+
 def write_csv(path, rows):
     os.makedirs(os.path.dirname(path), exist_ok=True)
     keys = []
@@ -160,6 +178,8 @@ def main(argv=None):
             if os.path.exists(p):
                 print(open(p).read())
         return None
+    if args.tuned_linears:
+        return tuned_linears(args.device)
     bench = Bench(args.tokens, args.device)
     if args.single_point:
         plan = dict(points(args.experiment_type)).get(args.exploration_value)

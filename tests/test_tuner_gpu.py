@@ -55,3 +55,23 @@ def test_a_named_tile_splits_by_itself(ctx):
                                     dict(variant=P.VARIANT_UMMA, umma_operand=3, umma_n_tile=64, umma_split=1))
     call.close()
     assert named < (own + whole) / 2
+
+
+@pytest.mark.parametrize("M,K,N,v,CT", [(8, 768, 768, 2, 16), (128, 3072, 768, 2, 16), (512, 768, 3072, 2, 16), (1024, 768, 3072, 2, 16), (1024, 3072, 768, 2, 16),
+                                        (200, 1024, 1040, 4, 32), (300, 240, 272, 5, 13)])
+def test_tuned_is_not_slower_than_untuned(ctx, M, K, N, v, CT):
+    """Tuning chooses among what the library does by itself, too.  (The bar leaves room for a host that is interrupted; what a
+    missing form costs is 20 % and more.)"""
+    call = _Call(ctx, M, K, N, v, CT)
+    plan = ctx.tune(83, M)
+    want = call.y.clone()
+    own, tuned = call.median({}, plan)
+    ctx.set_plan(83)
+    ctx.amm_host(83, call.x, want)
+    ctx.set_plan(83, **plan)
+    ctx.amm_host(83, call.x, call.y)
+    same = bool((call.y == want).all())
+    call.close()
+    assert same and tuned < 1.08 * own, plan
+    if (v, CT) not in ((2, 8), (2, 16), (4, 8)):   # no search kernel there that reads it
+        assert plan["ccs_tokens"] == 0
