@@ -336,7 +336,8 @@ int lutamm_tune(lutamm_ctx* ctx, int layer_id, uint32_t n_tokens, lutamm_plan* b
  * and a later lutamm_tune for a shape it knows installs the remembered plan without measuring.  These two
  * calls keep that table in a text file beside the configuration, so that a new process does not re-tune
  * (the reference's tuner writes its result into the YAML, src/tuner/auto_tuner.cpp:552-603; so does the
- * tuner here, and this file is the shape-keyed form of the same thing). */
+ * tuner here, and this file is the shape-keyed form of the same thing).  The file's first line names the version of the
+ * kernels that its plans were measured on; plans of another version are passed over. */
 int lutamm_plan_cache_save(lutamm_ctx* ctx, const char* path);
 int lutamm_plan_cache_load(lutamm_ctx* ctx, const char* path);
 

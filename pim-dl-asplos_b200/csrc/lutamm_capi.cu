@@ -1051,13 +1051,16 @@ int lutamm_tune(lutamm_ctx* c, int layer_id, uint32_t M, lutamm_plan* best_out) 
 }
 
 // Plan cache as a text file: one line per shape, "n K N CB CT SMs : variant ccs_tokens gather_cfg n_tile split
-// stages groups operand sps".  A plan only applies to the GPU it was measured on, hence the SM count in the key.
+// stages groups operand sps".  A plan only applies to the GPU it was measured on, hence the SM count in the key, and to the
+// kernels: a file without the line of this version keeps no shape from being measured anew (the plans of the first version
+// name the dense form, at half the rate of the sparse one).  To be raised when a new kernel form may change the fastest plan.
+constexpr int kPlanVersion = 2;
 int lutamm_plan_cache_save(lutamm_ctx* c, const char* path) {
     if (!c) return fail(nullptr, LUTAMM_EINVAL, "null context");
     if (!path) return fail(c, LUTAMM_EINVAL, "null path");
     FILE* f = std::fopen(path, "w");
     if (!f) return fail(c, LUTAMM_EINVAL, std::string("cannot write ") + path);
-    std::fprintf(f, "# lutamm plan cache: n K N CB CT SMs : variant ccs_tokens gather_cfg n_tile split stages groups operand sps\n");
+    std::fprintf(f, "# lutamm plan cache %d: n K N CB CT SMs : variant ccs_tokens gather_cfg n_tile split stages groups operand sps\n", kPlanVersion);
     for (const auto& kv : c->plan_cache) {
         const lutamm_plan& p = kv.second;
         std::fprintf(f, "%u %u %u %u %u %u : %u %u %u %u %u %u %u %u %u\n", kv.first[0], kv.first[1], kv.first[2], kv.first[3], kv.first[4],
@@ -1074,7 +1077,10 @@ int lutamm_plan_cache_load(lutamm_ctx* c, const char* path) {
     FILE* f = std::fopen(path, "r");
     if (!f) return fail(c, LUTAMM_EINVAL, std::string("cannot read ") + path);
     char line[512];
+    bool current = false;
     while (std::fgets(line, sizeof line, f)) {
+        int version = 0;
+        if (std::sscanf(line, "# lutamm plan cache %d:", &version) == 1) current = version == kPlanVersion;
         if (line[0] == '#' || line[0] == '\n') continue;
         unsigned k[6], v[9];
         if (std::sscanf(line, "%u %u %u %u %u %u : %u %u %u %u %u %u %u %u %u", &k[0], &k[1], &k[2], &k[3], &k[4], &k[5], &v[0], &v[1], &v[2],
@@ -1082,6 +1088,7 @@ int lutamm_plan_cache_load(lutamm_ctx* c, const char* path) {
             std::fclose(f);
             return fail(c, LUTAMM_EINVAL, std::string("malformed plan cache line in ") + path);
         }
+        if (!current) continue;
         lutamm_plan p{};
         p.variant = v[0]; p.ccs_tokens = v[1]; p.gather_cfg = v[2]; p.umma_n_tile = v[3]; p.umma_split = v[4];
         p.umma_stages = v[5]; p.umma_groups = v[6]; p.umma_operand = v[7]; p.umma_sps = v[8];

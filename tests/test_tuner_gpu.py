@@ -75,3 +75,35 @@ def test_tuned_is_not_slower_than_untuned(ctx, M, K, N, v, CT):
     assert same and tuned < 1.08 * own, plan
     if (v, CT) not in ((2, 8), (2, 16), (4, 8)):   # no search kernel there that reads it
         assert plan["ccs_tokens"] == 0
+
+
+def test_plan_files_of_other_kernels_are_not_applied(ctx, tmp_path):
+    """A file names the forms that were fastest among the kernels it was measured on; one without the present version has
+    been written by other kernels and is measured anew."""
+    M, K, N = 96, 256, 256
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    dense = dict(variant=P.VARIANT_UMMA, umma_operand=2, umma_n_tile=64, umma_split=1)
+    line = f"{M} {K} {N} {K // 2} 16 {sms} : 2 0 0 64 1 0 0 2 0\n"
+    old, saved = tmp_path / "old.plans", tmp_path / "saved.plans"
+    old.write_text("# lutamm plan cache: n K N CB CT SMs : variant ccs_tokens gather_cfg n_tile split stages groups operand sps\n" + line)
+    with P.LutAmmContext(0) as other:
+        other.load_weights(0, *_weights(K, N), 0.01)
+        other.plan_cache_load(str(old))
+        measured = other.tune(0, M)
+        assert {k: v for k, v in measured.items() if v} != dense
+        other.plan_cache_save(str(saved))
+    version = saved.read_text().splitlines()[0]
+    saved.write_text(version + "\n" + line)
+    with P.LutAmmContext(0) as other:   # the version it writes it also reads
+        other.load_weights(0, *_weights(K, N), 0.01)
+        other.plan_cache_load(str(saved))
+        assert {k: v for k, v in other.tune(0, M).items() if v} == dense
+        old.write_text("not a plan\n")
+        with pytest.raises(P.LutAmmError):
+            other.plan_cache_load(str(old))
+
+
+def _weights(K, N):
+    rng = np.random.default_rng(0)
+    return rng.standard_normal((K // 2, 16, 2), dtype=np.float32), rng.integers(-127, 128, (K // 2, 16, N), dtype=np.int8), np.zeros(N, np.float32)
