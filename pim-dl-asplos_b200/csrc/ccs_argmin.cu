@@ -725,7 +725,8 @@ cudaError_t run_any(const CcsArgs& a, cudaStream_t s) {
                             cb_per_cta, a.n_stile, a.cb_mtile);
 }
 
-// The instances whose thread walks a run of tokens.
+// The instances with a short form, and those whose thread walks a run of tokens.
+#define LUTAMM_CCS_SHORT_INSTANCES(X) X(2, 8) X(2, 16) X(2, 32) X(4, 8) X(4, 16) X(8, 8) X(8, 16)
 #define LUTAMM_CCS_RUN_INSTANCES(X) X(2, 8) X(2, 16) X(4, 8)
 
 }  // namespace
@@ -734,8 +735,13 @@ cudaError_t run_any(const CcsArgs& a, cudaStream_t s) {
 bool ccs_reads_tokens_per_thread(uint32_t v, uint32_t CT) {
 #define LUTAMM_CCS_IS(V_, CT_) || (v == V_ && CT == CT_)
     return false LUTAMM_CCS_RUN_INSTANCES(LUTAMM_CCS_IS);
-#undef LUTAMM_CCS_IS
 }
+uint32_t ccs_light_ctas(uint32_t M, uint32_t CB, uint32_t CT, uint32_t v) {
+    const bool has = false LUTAMM_CCS_SHORT_INSTANCES(LUTAMM_CCS_IS);
+    const uint64_t ctas = (uint64_t)((CB + 31) / 32) * ((M + 4 * kTok - 1) / (4 * kTok));
+    return has && CT * v <= 64 && ctas < 1u << 30 ? (uint32_t)ctas : 0;
+}
+#undef LUTAMM_CCS_IS
 
 cudaError_t launch_ccs(const CcsArgs& a, cudaStream_t s, const char** why) {
     *why = nullptr;
@@ -751,13 +757,7 @@ cudaError_t launch_ccs(const CcsArgs& a, cudaStream_t s, const char** why) {
         dim3 grid;
 #define LUTAMM_CCS_SHORT(V_, CT_) \
     if (a.v == V_ && a.CT == CT_ && short_fits<V_, CT_>(a, &grid)) return run_reg_grid<V_, CT_, kTok, true>(a, grid, kTok, s);
-        LUTAMM_CCS_SHORT(2, 8)
-        LUTAMM_CCS_SHORT(2, 16)
-        LUTAMM_CCS_SHORT(2, 32)
-        LUTAMM_CCS_SHORT(4, 8)
-        LUTAMM_CCS_SHORT(4, 16)
-        LUTAMM_CCS_SHORT(8, 8)
-        LUTAMM_CCS_SHORT(8, 16)
+        LUTAMM_CCS_SHORT_INSTANCES(LUTAMM_CCS_SHORT)
 #undef LUTAMM_CCS_SHORT
 #define LUTAMM_CCS_REG(V_, CT_) \
     if (a.v == V_ && a.CT == CT_) return run_reg<V_, CT_>(a, s);

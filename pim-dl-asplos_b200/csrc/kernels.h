@@ -19,6 +19,9 @@ struct CcsArgs {
 };
 cudaError_t launch_ccs(const CcsArgs& a, cudaStream_t s, const char** why);
 bool ccs_reads_tokens_per_thread(uint32_t v, uint32_t CT);
+// CTAs of the search in its short form, where their centroids are at most 64 floats a codebook: such CTAs do as well
+// several to an SM as spread out.  0 where the search has another form.
+uint32_t ccs_light_ctas(uint32_t M, uint32_t CB, uint32_t CT, uint32_t v);
 
 // ---- step 2+3: gather-accumulate + dequantise -----------------------------------------
 // Output addressing: row-major [M][N], or the reference's DPU-tiled layout.
@@ -36,6 +39,7 @@ struct LutArgs {
     float scale, lut_bias;
     OutLayout layout;
     uint32_t act;         // LUTAMM_ACT_*: applied after the dequantisation
+    uint32_t search_ctas; // ccs_light_ctas() of the layer
     // Column sharding with the exchange fused into the kernel: the [M][N] block is also stored, by plain
     // st.global over NVLink, at the same offsets of n_peers - 1 other GPUs' buffers (peer_out[g] points at
     // this rank's block inside GPU g's gathered buffer; the entry for this GPU itself equals `out` and is

@@ -847,11 +847,15 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
     // go through the columns with as many row tiles as there are pairs: 13.8 GB of reads become 1.9 GB of table.
     p.group_m = (uint64_t)a.M * a.CB > (48ull << 20) && p.tiles_m > cap ? cap : p.tiles_m;
     p.one_tile = items <= cap;
-    // With one tile per pair all pairs reach the end of their main loops together, and the next kernel of the stream
-    // may as well be launched; with several they finish a tile apart and its early CTAs, which pile up on the SMs that
-    // are free first, would skew it.  A search of many CTAs is skewed by the SMs that one tile per pair leaves idle, too:
-    // four linears of 768 at 256 tokens 53.8 us with the trigger, 55.0 without, at 1024 tokens 78.2 and 76.9.
-    p.early_trigger = p.one_tile && (uint64_t)a.M * a.CB <= 200 * 1024;
+    // With one tile per pair all pairs reach the end of their main loops together, and the next kernel of the stream may as
+    // well be launched then; with several they finish a tile apart and its early CTAs would skew it.  Where they go are the SMs
+    // that the tiles leave idle, as many to an SM as fit: that pays where the next kernel is a light search of up to four
+    // CTAs per idle SM.  What the next kernel is this launch does not know; it goes by its own layer's search, and from
+    // 64 tokens on, where that is hardly the row gather, which needs its CTAs spread out.  Measured on chains of an
+    // encoder layer's four linears, without the trigger / always with it: width 768, v = 2, 16 centroids at 128 tokens 48.7 / 50.7 us,
+    // by this rule 49.3; v = 4 at 128 41.7 / 43.6 / 41.0; 32 centroids at 512 90 / 102 / 90; v = 4, 64 centroids at 320 104 / 123 / 104;
+    // width 1280, v = 4 at 64 54.7 / 50.7 / 50.5; 1024, v = 4 at 384 60.2 / 56.9 / 58.0, at 32 (rows) 36.9 / 42.4 / 36.9.
+    p.early_trigger = p.one_tile && a.M >= 64 && a.search_ctas && a.search_ctas <= 4 * (max_ctas - 2 * pairs);
     p.fresh_table = fresh_table;
     if (accumulators(n_tile) == 1 && !p.one_tile) { *why = "tiles wider than 160 columns of the sparse form take one tile per pair"; return cudaErrorInvalidValue; }
     const size_t smem = sparse_smem(n_tile, lg, p.b_slots);

@@ -1,0 +1,63 @@
+"""What a call launches, by size, type and alignment: the library's objects on a runtime that only logs (fake_cudart.cpp)."""
+import ctypes
+import glob
+import os
+import shutil
+import subprocess
+
+import pytest
+
+import pim_dl_asplos_b200 as P
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "pim-dl-asplos_b200", "csrc")
+OBJECTS = sorted(glob.glob(os.path.join(CSRC, "build", "*.o")))
+INCLUDE = "/usr/local/cuda/include"
+
+pytestmark = pytest.mark.skipif(not (OBJECTS and shutil.which("g++") and os.path.exists(os.path.join(INCLUDE, "cuda_runtime.h"))),
+                                reason="the library's objects or the toolkit's headers are not here")
+
+
+class _Library:
+    def __init__(self, path):
+        self.lib = ctypes.CDLL(path)
+        self.lib.fake_log.restype = ctypes.c_char_p
+        self.ctx = ctypes.c_void_p()
+        assert self.lib.lutamm_create(ctypes.byref(self.ctx), 0) == P.OK
+        self.memory = ctypes.create_string_buffer(1 << 26)   # stands for any buffer of the caller: nothing is run on it
+        self.base = (ctypes.addressof(self.memory) + 255) // 256 * 256
+
+    def log(self):
+        return self.lib.fake_log().decode().splitlines()
+
+    def amm(self, M, K, N, v=2, CT=16, plan=None):
+        """Launches of lutamm_amm on device buffers."""
+        at, L = ctypes.c_void_p(self.base), self.lib
+        ip, lp = P.make_params(M, K, N, K // v, CT, 0.01)
+        assert L.lutamm_load_weights(self.ctx, 0, at, at, at, ctypes.byref(ip), ctypes.byref(lp)) == P.OK
+        if plan:
+            assert L.lutamm_set_plan(self.ctx, 0, ctypes.byref(P.Plan(**plan))) == P.OK
+        for _ in range(2):   # the first call lays the table out
+            self.log()
+            assert L.lutamm_amm(self.ctx, 0, at, at, ctypes.c_uint32(M), ctypes.c_uint32(P.FLAG_ASYNC)) == P.OK
+        return self.log()
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    path = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", CSRC, "-I", INCLUDE, "-o", path,
+                    os.path.join(HERE, "fake_cudart.cpp")] + OBJECTS + ["-ldl"], check=True, timeout=300)
+    return _Library(path)
+
+
+@pytest.mark.parametrize("early,M,K,N,v,CT", [
+    (1, 128, 768, 2304, 2, 16), (1, 256, 768, 3072, 2, 16), (1, 64, 1280, 3840, 4, 16), (1, 128, 768, 2304, 2, 32), (1, 128, 768, 2304, 4, 8),
+    (0, 512, 768, 3072, 2, 16),       # more than four search CTAs per idle SM
+    (0, 320, 768, 2304, 2, 16),       # four idle SMs
+    (0, 320, 768, 3072, 4, 64), (0, 192, 2560, 7680, 10, 16), (0, 256, 768, 3072, 8, 16),   # no light search
+    (0, 48, 1024, 3072, 4, 16),       # the next call may gather rows
+    (0, 12608, 768, 3072, 2, 16)])    # several tiles per pair
+def test_who_launches_the_next_kernel_early(fake, early, M, K, N, v, CT):
+    contraction = [ln for ln in fake.amm(M, K, N, v, CT) if "lut_sparse_kernel" in ln]
+    assert len(contraction) == 1 and contraction[0].endswith(f"early={early}")
