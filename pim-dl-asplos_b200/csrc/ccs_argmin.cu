@@ -736,10 +736,12 @@ bool ccs_reads_tokens_per_thread(uint32_t v, uint32_t CT) {
 #define LUTAMM_CCS_IS(V_, CT_) || (v == V_ && CT == CT_)
     return false LUTAMM_CCS_RUN_INSTANCES(LUTAMM_CCS_IS);
 }
+bool ccs_has_short_form(uint32_t v, uint32_t CT) {
+    return false LUTAMM_CCS_SHORT_INSTANCES(LUTAMM_CCS_IS);
+}
 uint32_t ccs_light_ctas(uint32_t M, uint32_t CB, uint32_t CT, uint32_t v) {
-    const bool has = false LUTAMM_CCS_SHORT_INSTANCES(LUTAMM_CCS_IS);
     const uint64_t ctas = (uint64_t)((CB + 31) / 32) * ((M + 4 * kTok - 1) / (4 * kTok));
-    return has && CT * v <= 64 && ctas < 1u << 30 ? (uint32_t)ctas : 0;
+    return ccs_has_short_form(v, CT) && CT * v <= 64 && ctas < 1u << 30 ? (uint32_t)ctas : 0;
 }
 #undef LUTAMM_CCS_IS
 

@@ -19,6 +19,7 @@ struct CcsArgs {
 };
 cudaError_t launch_ccs(const CcsArgs& a, cudaStream_t s, const char** why);
 bool ccs_reads_tokens_per_thread(uint32_t v, uint32_t CT);
+bool ccs_has_short_form(uint32_t v, uint32_t CT);   // for small calls
 // CTAs of the search in its short form, where their centroids are at most 64 floats a codebook: such CTAs do as well
 // several to an SM as spread out.  0 where the search has another form.
 uint32_t ccs_light_ctas(uint32_t M, uint32_t CB, uint32_t CT, uint32_t v);

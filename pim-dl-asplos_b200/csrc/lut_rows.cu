@@ -182,14 +182,15 @@ float rows_us(uint32_t M, uint32_t CB, uint32_t N, int sm_count) {
     return 4.f + 0.24e-6f * tiles * kTile * CB + (rounds > 1.f ? 1.2f * (rounds - 1.f) : 0.f);
 }
 
-// The same with the search, for centroid sets that a thread reads in a few batches, up to 4.75 MB of them over all CTAs: a
-// lane's 16 bytes come from a line of their own, and a token's centroids are read once per column tile.  768 -> 768, v = 2,
-// 16 centroids, one launch against two: 5.0 us against 6.1 at one token, 5.4 / 6.5 at eight, 6.0 / 6.4 at 16, 7.8 / 6.7 at
-// 32.  Where the search on its own has no quick form (v = 4, 32 centroids: 800 -> 1008 at eight tokens 6.2 / 11.0,
-// 1024 -> 4096 at four 8.5 / 11.0) up to 16 MB.
+// The same with the search, for centroid sets that a thread reads in a few batches: a lane's 16 bytes come from a line of
+// their own, and a token's centroids are read once per column tile, so it goes by those bytes over all CTAs.  One launch
+// over two, K = 256 to 3072, 1 to 48 tokens: where the search alone has a short form 0.8 to 0.9 up to 3 MB and 0.91 to 0.97 at 6 (v = 2,
+// 16 centroids), 0.95 to 1.05 at 7, 1.08 to 1.17 at 9; with 128 floats a codebook (v = 8, 16) 0.97 at 10.6, 1.00 to 1.18 at 14; where it has none
+// (v = 4, 13 centroids) 0.83 at 15, 0.96 to 1.05 at 23, (v = 4, 32) 0.82 to 1.01 at 14, 1.14 at 17.
 bool rows_search_ok(uint32_t M, uint32_t CB, uint32_t CT, uint32_t v, uint32_t N, const float* x) {
     if ((v != 2 && v != 4 && v != 8) || CT * v % 4 || CT * v > 128 || (reinterpret_cast<uintptr_t>(x) & 15u) || (uint64_t)CB * v % 4) return false;
-    return (uint64_t)M * ((N + kTile - 1) / kTile) * CB * CT * v * 4 <= (CT * v > 64 ? 16000000u : 4750000u);
+    const uint64_t most = !ccs_has_short_form(v, CT) ? 16000000 : CT * v > 64 ? 13000000 : 6500000;
+    return (uint64_t)M * ((N + kTile - 1) / kTile) * CB * CT * v * 4 <= most;
 }
 
 template <int V>

@@ -61,3 +61,19 @@ def fake(tmp_path_factory):
 def test_who_launches_the_next_kernel_early(fake, early, M, K, N, v, CT):
     contraction = [ln for ln in fake.amm(M, K, N, v, CT) if "lut_sparse_kernel" in ln]
     assert len(contraction) == 1 and contraction[0].endswith(f"early={early}")
+
+
+def _rows_bytes(M, K, N, CT):
+    return M * ((N + 127) // 128) * K * CT * 4   # centroids read by all CTAs
+
+
+@pytest.mark.parametrize("launches,M,K,N,v,CT", [
+    (1, 1, 768, 768, 2, 16), (1, 20, 768, 768, 2, 16), (2, 24, 768, 768, 2, 16), (2, 4, 1024, 4096, 2, 16),   # 6.5 MB: the search alone has a short form
+    (1, 12, 768, 2304, 8, 16), (2, 48, 768, 768, 8, 16),                                                      # 13 MB: with 128 floats a codebook
+    (1, 24, 768, 768, 4, 13), (1, 12, 768, 768, 2, 64), (2, 4, 1024, 4096, 4, 32),                            # 16 MB: it has none
+    (2, 4, 768, 768, 2, 13), (2, 4, 780, 768, 10, 16)])                                                     # no such instance
+def test_who_searches_in_the_row_gather(fake, launches, M, K, N, v, CT):
+    log = fake.amm(M, K, N, v, CT)
+    assert len(log) == launches and "lut_rows_kernel" in log[-1]
+    if launches == 1:
+        assert _rows_bytes(M, K, N, CT) <= 16e6
