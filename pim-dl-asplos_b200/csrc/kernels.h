@@ -55,8 +55,8 @@ struct GatherPlan {
     uint32_t cfg;  // tile configuration id
 };
 uint32_t gather_num_cfgs();
-// microseconds a gather launch takes at least, by its best configuration
-float gather_us(uint32_t M, uint32_t CB, uint32_t N, int sm_count);
+// microseconds a launch takes
+float gather_us(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, uint32_t cfg, int sm_count);
 // Encodes the tensor map the configuration needs (box sizes depend on it).
 cudaError_t gather_make_tmap(CUtensorMap* out, const int8_t* lut, uint32_t CB, uint32_t CT, uint32_t N, uint32_t cfg,
                              const char** why);
@@ -96,8 +96,10 @@ cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N,
 size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N);
 // ... of `n` columns of a table that has `pitch`, from column n0 on; chained: nothing the stream still runs writes `lut`
 cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t n, uint32_t n0, uint32_t pitch, bool chained, cudaStream_t s);
-// Tile width (`only`, where that is not 0) and split; returns the microseconds it expects, launch apart (about 4)
-float sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split, uint32_t only = 0);
+// Tile width (`only`, where that is not 0) and split (up to most_split); returns the microseconds it expects, launch apart
+// (about 4)
+float sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split, uint32_t only = 0,
+                          uint32_t most_split = 16);
 void sparse_split_scratch(uint32_t M, uint32_t N, uint32_t n_tile, uint32_t split, size_t* partial_bytes, size_t* counter_bytes);
 bool sparse_tile_ok(uint32_t n_tile);
 cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile,
@@ -112,7 +114,7 @@ cudaError_t launch_rows(const LutArgs& a, const int8_t* lut, int sm_count, cudaS
 // ... and the search, in one launch, where rows_search_ok()
 bool rows_search_ok(uint32_t M, uint32_t CB, uint32_t CT, uint32_t v, uint32_t N, const float* x);
 cudaError_t launch_rows_search(const LutArgs& a, const int8_t* lut, const float* x, const float* centroid, uint32_t v, int sm_count, cudaStream_t s);
-float rows_us(uint32_t M, uint32_t CB, uint32_t N, int sm_count);
+float rows_us(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count);
 
 // LUT [CB*CT][N] -> [N][CB*CT]
 cudaError_t launch_transpose_lut(const int8_t* lut, int8_t* lut_t, uint32_t rows, uint32_t cols, cudaStream_t s);

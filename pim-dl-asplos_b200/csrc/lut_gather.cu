@@ -18,6 +18,8 @@
 // HBM traffic: M*CB (indices) + CB*CT*N (LUT, once if it stays in L2 across M tiles)
 //              + 4*N (bias) + 4*M*N (output).
 #include "kernels.h"
+
+#include <algorithm>
 #include "ptx.cuh"
 #include "epilogue.cuh"
 
@@ -299,11 +301,16 @@ cudaError_t launch_gather(const LutArgs& a, const CUtensorMap& lut_map, uint32_t
     }
 }
 
-// By the adds a full GPU sustains or, where the tiles are few, by one CTA's walk over the codebooks.
-float gather_us(uint32_t M, uint32_t CB, uint32_t N, int sm_count) {
-    const float ctas = (float)((M + 31) / 32) * ((N + 127) / 128), sum = (float)M * CB * N / 9.7e6f;
-    const float chain = 0.105f * CB * (ctas > sm_count ? 1.f + ctas / sm_count / 8 : 1.f);
-    return 4.f + (sum > chain ? sum : chain);
+// One CTA's walk over the codebooks - the staging of a codebook's rows, from 16 or 32 centroids on - and, of the wide
+// tiles (cfg 0 to 3), the adds that a full GPU sustains.  Measured at 4 to 256 centroids, 48 to 768 codebooks, 256 to 4096 columns, 1 to
+// 8192 tokens: within 0.8 to 1.3 of it.  (192 codebooks -> 1024 at 128 tokens, cfg 4: 21 us with 16 centroids, 36 with 64, 98 with 256.)
+float gather_us(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, uint32_t cfg, int sm_count) {
+    const bool narrow = cfg == 4;
+    const float centroids = (float)CT;
+    const float step = narrow ? std::max(0.1f, 0.065f + 0.0017f * centroids) : CT > 128 ? 0.61f : std::max(0.225f, 0.165f + 0.004f * centroids);
+    if (!narrow) return 1.8f + std::max(CB * step, (float)M * CB * N / 9.7e6f * std::max(1.f, 0.78f + 0.0085f * centroids));
+    const uint64_t ctas = (uint64_t)((M + 31) / 32) * ((N + 127) / 128), per_sm = (ctas + sm_count - 1) / sm_count;
+    return std::max(6.5f, 1.8f + CB * step * std::max(1.f, 0.8f * per_sm));
 }
 
 }  // namespace lutamm

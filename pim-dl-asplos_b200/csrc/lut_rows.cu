@@ -176,10 +176,14 @@ static uint32_t rows_shares(uint32_t M, uint32_t CB, uint32_t N, int sm_count) {
     return shares;
 }
 
-// What a launch takes, in microseconds: 0.24 per megabyte of rows (whole tiles of columns), and rounds of CTAs.
-float rows_us(uint32_t M, uint32_t CB, uint32_t N, int sm_count) {
+// What a launch takes, in microseconds: 0.24 per megabyte of rows (whole tiles of columns), and rounds of CTAs; from about
+// 30 MB on 0.155 per megabyte (67 MB 13 us, 134 MB 24, 268 MB 46, 537 MB 90) of a table that the half of L2 on an SM's die
+// holds (of 78 MB 0.24, of 107 MB 0.44), but no less than 3 a round of CTAs.
+float rows_us(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count) {
+    if (M > 65535) return 3e38f;   // a token is a block of grid.z
     const float tiles = (float)((N + kTile - 1) / kTile) * (float)M, rounds = tiles * rows_shares(M, CB, N, sm_count) / (4.f * sm_count);
-    return 4.f + 0.24e-6f * tiles * kTile * CB + (rounds > 1.f ? 1.2f * (rounds - 1.f) : 0.f);
+    const float mb = 1e-6f * tiles * kTile * CB, few = 4.f + 0.24f * mb + (rounds > 1.f ? 1.2f * (rounds - 1.f) : 0.f), many = 6.6f + (0.155f * mb > 3.f * rounds ? 0.155f * mb : 3.f * rounds);
+    return few < many || (uint64_t)CB * CT * N > 40000000 ? few : many;
 }
 
 // The same with the search, for centroid sets that a thread reads in a few batches: a lane's 16 bytes come from a line of

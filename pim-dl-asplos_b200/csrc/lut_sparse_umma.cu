@@ -787,8 +787,8 @@ static uint32_t slice_unit(uint32_t CT) { return CT > 16 ? CT / 16 : 1; }
 // two: 384 codebooks of 16 -> 3072 at 1024 tokens 15.8 -> 12.7 us, 1024 codebooks 29.6 -> 21.3 (four LUT slots instead of
 // eight at 256 columns: 27.8 and 15.4).  (Measured at 32 to 16384 tokens; at 96 columns nothing gained.)  Where the tiles leave pairs idle the axis is split over them, one item per pair, which costs 5 to 6 us for the
 // partial sums' way through L2 (1536 codebooks -> 768 at 128 tokens 20.7 -> 12.2 us, at 1024 tokens 21.6 -> 17.6).
-// only: the one tile width to choose the split for, 0 = any.
-float sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split, uint32_t only) {
+// only: the one tile width to choose the split for, 0 = any; most_split: 1 for a caller that has no scratch.
+float sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile, uint32_t* split, uint32_t only, uint32_t most_split) {
     const uint32_t pairs = sm_count >= 2 ? (uint32_t)sm_count / 2 : 1, slabs = sparse_slabs(CB, CT), unit = slice_unit(CT);
     const uint64_t tm = (M + 2 * kRows - 1) / (2 * kRows);
     const struct { uint32_t n; float slab_us, split_us; } tiles[] = {{64, 0.170f, 5.f}, {128, 0.199f, 6.2f}, {160, 0.220f, 0.f}, {192, 0.250f, 0.f}};
@@ -799,7 +799,7 @@ float sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int 
         const uint64_t items = tm * ((N + t.n - 1) / t.n), rounds = (items + pairs - 1) / pairs;
         if (only ? t.n != only : accumulators(t.n) == 1 && rounds > 1) continue;
         const uint32_t most = items < pairs ? (uint32_t)(pairs / items) : 1;
-        for (uint32_t s = 1; s <= most && s <= (t.n >= 160 ? 1u : 16u) && (s == 1 || s * unit <= slabs); ++s) {
+        for (uint32_t s = 1; s <= most && s <= (t.n >= 160 ? 1u : most_split) && (s == 1 || s * unit <= slabs); ++s) {
             const uint32_t per = ((slabs + s - 1) / s + unit - 1) / unit * unit;
             const float main = per * t.slab_us, epi = 0.93f * (t.n / 32);
             const float us = (float)rounds * (rounds > 1 && epi > main ? epi : main) + 0.25f * (t.n / 32) + (s > 1 ? t.split_us : 0.f);

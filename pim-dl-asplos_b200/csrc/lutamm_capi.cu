@@ -303,8 +303,8 @@ bool takes_rows(const lutamm_ctx* c, const Layer& L, uint32_t M, const lutamm_pl
     if (plan.variant != LUTAMM_VARIANT_AUTO || plan.gather_cfg || !umma_plan_open(plan)) return false;
     uint32_t n_tile, split;
     const float other = umma_supported(L.CB, L.CT, L.N) ? 4.f + sparse_default_plan(M, L.CB, L.CT, L.N, c->sm_count, &n_tile, &split)
-                                                        : gather_us(M, L.CB, L.N, c->sm_count);
-    return rows_us(M, L.CB, L.N, c->sm_count) < other;
+                                                        : gather_us(M, L.CB, L.CT, L.N, plan.gather_cfg, c->sm_count);
+    return rows_us(M, L.CB, L.CT, L.N, c->sm_count) < other;
 }
 
 // ... and the search in the same launch.

@@ -72,14 +72,16 @@ uint32_t sm_count_of(int device) {
 }
 
 // By estimated time: the table's used rows, for few tokens; the table laid out for the tcgen05 kernel on every call,
-// `columns` at a time in what the indices leave of the array; or the CUDA-core gather, which reads the table as it is.
+// `columns` at a time in what the indices leave of the array; or the CUDA-core gather, which reads the table as it is: its
+// narrow tiles of few tokens where wide ones would leave SMs without a CTA.
 struct TablePlan {
     bool rows;
-    uint32_t columns;
+    uint32_t columns, gather_cfg;
 };
 TablePlan plan_table(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, bool aligned, uint32_t sms) {
-    const double gather = lutamm::gather_us(M, CB, N, (int)sms), rows = aligned ? lutamm::rows_us(M, CB, N, (int)sms) : 1e30;
-    double table = 1e30;
+    const uint32_t cfg = (uint64_t)((M + 63) / 64) * ((N + 255) / 256) < sms ? 4 : 0;
+    const float gather = lutamm::gather_us(M, CB, CT, N, cfg, (int)sms), rows = aligned ? lutamm::rows_us(M, CB, CT, N, (int)sms) : 3e38f;
+    float table = 3e38f;
     uint32_t columns = 0;
     if (lutamm::umma_supported(CB, CT, N)) {
         const size_t per_column = lutamm::sparse_table_bytes(CB, CT, 1), used = (((size_t)M * CB + 255) / 256) * 256;
@@ -90,12 +92,12 @@ TablePlan plan_table(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, bool alig
             columns = ((N + chunks - 1) / chunks + 63) / 64 * 64;   // near-equal chunks
             if (columns > N) columns = N;
             uint32_t n_tile, split;
-            lutamm::sparse_default_plan(M, CB, CT, columns, (int)sms, &n_tile, &split);
-            const uint64_t tiles = (uint64_t)((M + 255) / 256) * ((columns + n_tile - 1) / n_tile), rounds = (tiles + sms / 2 - 1) / (sms / 2);
-            table = chunks * (5.0 + per_column * (double)columns / 2.5e6 + rounds * per_column / 256 * 0.2);
+            // a piece: two launches, the layout at 2.5 TB/s, the contraction (measured 768 -> 768 to 512 -> 8192, 1 to 5 pieces)
+            const float contraction = lutamm::sparse_default_plan(M, CB, CT, columns, (int)sms, &n_tile, &split, 0, 1);
+            table = 2.6f + chunks * (3.7f + (float)per_column * columns / 2.5e6f + contraction);
         }
     }
-    return {rows < table && rows < gather, table < gather ? columns : 0u};
+    return {rows < table && rows < gather, table < gather ? columns : 0u, cfg};
 }
 
 }  // namespace
@@ -194,7 +196,7 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
             la.bias = bias + n0;
             la.out = output + n0;
             uint32_t n_tile, split;
-            sparse_default_plan(M, CB, CT, la.N, (int)sms, &n_tile, &split);
+            sparse_default_plan(M, CB, CT, la.N, (int)sms, &n_tile, &split, 0, 1);
             CUtensorMap table_map, out_map;
             // (the second table and on: the contraction in front began when all that the caller had queued was complete)
             e = launch_sparse_table(lut, table, CB, CT, la.N, n0, N, n0 > 0, s);
@@ -205,8 +207,8 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
         if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : (std::string("tcgen05 launch: ") + cudaGetErrorString(e)));
     } else {
         // The gather-accumulate kernel reads the LUT in its canonical layout through a tensor map encoded on the host (no
-        // device memory involved).  Narrow tiles of few tokens where wide ones would leave SMs without a CTA.
-        const uint32_t cfg = (uint64_t)((M + 63) / 64) * ((N + 255) / 256) < sms ? 4 : 0;
+        // device memory involved).
+        const uint32_t cfg = plan.gather_cfg;
         CUtensorMap map;
         e = gather_make_tmap(&map, lut, CB, CT, N, cfg, &why);
         if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : cudaGetErrorString(e));

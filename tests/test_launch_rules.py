@@ -77,3 +77,34 @@ def test_who_searches_in_the_row_gather(fake, launches, M, K, N, v, CT):
     assert len(log) == launches and "lut_rows_kernel" in log[-1]
     if launches == 1:
         assert _rows_bytes(M, K, N, CT) <= 16e6
+
+
+def _static(fake, M, K, N, v, CT, offset=0):
+    at, lib = ctypes.c_void_p(fake.base), fake.lib
+    ip, lp = P.make_params(M, K, N, K // v, CT, 0.01)
+    fake.log()
+    rc = lib.lutamm_amm_static_scratch(0, None, at, at, ctypes.c_void_p(fake.base + offset), at, at, ctypes.byref(ip), ctypes.byref(lp))
+    assert rc == P.OK
+    return fake.log()
+
+
+@pytest.mark.parametrize("form,M,K,N,v,CT", [
+    ("rows", 1, 768, 3072, 2, 16), ("rows", 256, 768, 2304, 4, 64), ("rows", 128, 768, 3072, 4, 32), ("rows", 256, 3072, 768, 2, 16),
+    ("table", 256, 768, 3072, 2, 16), ("table", 1024, 768, 2304, 4, 64), ("table", 512, 768, 3072, 4, 32), ("table", 256, 4096, 4096, 8, 16),
+    ("gather", 128, 512, 8192, 2, 16), ("gather", 64, 32, 8192, 2, 13), ("gather", 66000, 16, 16, 2, 200)])
+def test_how_the_static_call_contracts(fake, form, M, K, N, v, CT):
+    """The fastest by measurement of all three at these sizes, and no split of the codebook axis, for which it has no scratch."""
+    log = _static(fake, M, K, N, v, CT)
+    assert {"rows": "lut_rows_kernel", "table": "lut_sparse_kernel", "gather": "lut_gather_kernel"}[form] in log[-1]
+    assert all("split=1" in ln for ln in log if "lut_sparse_kernel" in ln)
+
+
+def test_an_unaligned_table_is_not_gathered_by_rows(fake):
+    assert "lut_rows_kernel" in _static(fake, 1, 768, 768, 2, 16)[-1]
+    assert not any("lut_rows_kernel" in ln for ln in _static(fake, 1, 768, 768, 2, 16, offset=4))
+
+
+@pytest.mark.parametrize("M,K,N,CT,rows", [(600, 1088, 1248, 13, True), (65535, 1024, 128, 200, True), (65536, 1024, 128, 200, False)])
+def test_rows_without_a_tensor_core_form(fake, M, K, N, CT, rows):
+    """13 and 200 centroids have no contraction; a token is a block of the row gather's grid.z."""
+    assert ("lut_rows_kernel" in fake.amm(M, K, N, 2, CT)[-1]) == rows
