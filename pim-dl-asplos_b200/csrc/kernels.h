@@ -40,7 +40,8 @@ struct LutArgs {
     float scale, lut_bias;
     OutLayout layout;
     uint32_t act;         // LUTAMM_ACT_*: applied after the dequantisation
-    uint32_t search_ctas; // ccs_light_ctas() of the layer
+    uint32_t next_ctas, next_per_sm;  // CTAs of the kernel that is expected next in the stream (0: not known, or not to be
+                                      // launched early), and how many of them an SM without a tile takes well
     // Column sharding with the exchange fused into the kernel: the [M][N] block is also stored, by plain
     // st.global over NVLink, at the same offsets of n_peers - 1 other GPUs' buffers (peer_out[g] points at
     // this rank's block inside GPU g's gathered buffer; the entry for this GPU itself equals `out` and is
@@ -94,6 +95,7 @@ cudaError_t make_out_tmap(CUtensorMap* out, float* base, uint32_t M, uint32_t N,
 // The same contraction on CTA pairs with the one-hot operand 2:4 sparse (row-major fp32 output): from its own layout of
 // the table (sparse_table_bytes of it), at twice the rate.
 size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N);
+uint32_t sparse_table_ctas(uint32_t CB, uint32_t CT, uint32_t N);
 // ... of `n` columns of a table that has `pitch`, from column n0 on; chained: nothing the stream still runs writes `lut`
 cudaError_t launch_sparse_table(const int8_t* lut, int8_t* out, uint32_t CB, uint32_t CT, uint32_t n, uint32_t n0, uint32_t pitch, bool chained, cudaStream_t s);
 // Tile width (`only`, where that is not 0) and split (up to most_split); returns the microseconds it expects, launch apart

@@ -683,6 +683,7 @@ cudaError_t run_lg(uint32_t lg, const CUtensorMap& map, const CUtensorMap& idx_m
 
 }  // namespace
 
+uint32_t sparse_table_ctas(uint32_t CB, uint32_t CT, uint32_t N) { return sparse_slabs(CB, CT) * ((N + 63) / 64); }
 size_t sparse_table_bytes(uint32_t CB, uint32_t CT, uint32_t N) { return (size_t)sparse_slabs(CB, CT) * kSlab * N; }
 
 // The table as the kernel above wants it: [N][slabs * 256], row n's slab s holding at position 2 (d * codebooks + c) + h
@@ -850,12 +851,13 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
     // With one tile per pair all pairs reach the end of their main loops together, and the next kernel of the stream may as
     // well be launched then; with several they finish a tile apart and its early CTAs would skew it.  Where they go are the SMs
     // that the tiles leave idle, as many to an SM as fit: that pays where the next kernel is a light search of up to four
-    // CTAs per idle SM.  What the next kernel is this launch does not know; it goes by its own layer's search, and from
-    // 64 tokens on, where that is hardly the row gather, which needs its CTAs spread out.  Measured on chains of an
-    // encoder layer's four linears, without the trigger / always with it: width 768, v = 2, 16 centroids at 128 tokens 48.7 / 50.7 us,
+    // CTAs per idle SM, or the layout of the next piece of a table (256 threads and 16 loads each) of up to eight.  Measured
+    // on chains of an encoder layer's four linears, without the trigger / always with it: width 768, v = 2, 16 centroids at 128 tokens 48.7 / 50.7 us,
     // by this rule 49.3; v = 4 at 128 41.7 / 43.6 / 41.0; 32 centroids at 512 90 / 102 / 90; v = 4, 64 centroids at 320 104 / 123 / 104;
     // width 1280, v = 4 at 64 54.7 / 50.7 / 50.5; 1024, v = 4 at 384 60.2 / 56.9 / 58.0, at 32 (rows) 36.9 / 42.4 / 36.9.
-    p.early_trigger = p.one_tile && a.M >= 64 && a.search_ctas && a.search_ctas <= 4 * (max_ctas - 2 * pairs);
+    // Tables in pieces (never / always): 768 -> 3072 at 512 tokens (4.6 CTAs per idle SM) 53.4 / 50.7 us, at 1024 (19) 55.0 / 59.2; 512 ->
+    // 8192 at 640 (5.9) 76.9 / 73.3, at 384 (9.5) 72.6 / 80.7.
+    p.early_trigger = p.one_tile && a.next_ctas && a.next_ctas <= a.next_per_sm * (max_ctas - 2 * pairs);
     p.fresh_table = fresh_table;
     if (accumulators(n_tile) == 1 && !p.one_tile) { *why = "tiles wider than 160 columns of the sparse form take one tile per pair"; return cudaErrorInvalidValue; }
     const size_t smem = sparse_smem(n_tile, lg, p.b_slots);

@@ -344,7 +344,10 @@ int run_lut(lutamm_ctx* c, Layer& L, const uint8_t* d_idx, float* d_out, int32_t
     a.lut_bias = L.lp.bias;
     a.layout = make_layout(L, flags);
     a.act = L.act;
-    a.search_ctas = ccs_light_ctas(M, L.CB, L.CT, L.v);
+    // What comes next is not known; the layer's own search stands for it, from 64 tokens on, where it is hardly the row
+    // gather, which needs its CTAs spread out.
+    a.next_ctas = M >= 64 ? ccs_light_ctas(M, L.CB, L.CT, L.v) : 0;
+    a.next_per_sm = 4;
     const char* why = nullptr;
     uint32_t variant = plan.variant;
     if (takes_rows(c, L, M, plan) && !a.n_peers && !a.acc_out && !a.layout.tiled) {

@@ -195,6 +195,9 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
             la.N = N - n0 < plan.columns ? N - n0 : plan.columns;
             la.bias = bias + n0;
             la.out = output + n0;
+            const uint32_t left = N - n0 - la.N;
+            la.next_ctas = left ? sparse_table_ctas(CB, CT, left < plan.columns ? left : plan.columns) : 0;   // the next piece's layout
+            la.next_per_sm = 8;
             uint32_t n_tile, split;
             sparse_default_plan(M, CB, CT, la.N, (int)sms, &n_tile, &split, 0, 1);
             CUtensorMap table_map, out_map;

@@ -99,6 +99,14 @@ def test_how_the_static_call_contracts(fake, form, M, K, N, v, CT):
     assert all("split=1" in ln for ln in log if "lut_sparse_kernel" in ln)
 
 
+@pytest.mark.parametrize("early,M,K,N,v,CT", [("110", 512, 768, 3072, 2, 16), ("000", 1024, 768, 3072, 2, 16), ("00000", 384, 512, 8192, 2, 16),
+                                              ("11110", 640, 512, 8192, 2, 16), ("0", 300, 256, 512, 2, 16)])
+def test_who_launches_the_next_pieces_layout_early(fake, early, M, K, N, v, CT):
+    """Up to eight of its CTAs per SM without a tile; nothing behind the last piece."""
+    log = [ln for ln in _static(fake, M, K, N, v, CT) if "lut_sparse_kernel" in ln]
+    assert "".join(ln[-1] for ln in log) == early
+
+
 def test_an_unaligned_table_is_not_gathered_by_rows(fake):
     assert "lut_rows_kernel" in _static(fake, 1, 768, 768, 2, 16)[-1]
     assert not any("lut_rows_kernel" in ln for ln in _static(fake, 1, 768, 768, 2, 16, offset=4))
