@@ -135,3 +135,32 @@ def test_what_the_ordinary_call_refuses_or_autograd_follows_is_not_replayed():
     assert lay._graph_key(x) is None
     with torch.no_grad():
         assert lay._graph_key(x) is not None
+
+
+@pytest.mark.gpu
+def test_replayed_forward_in_and_out_of_inference_mode(ctx):
+    """The layer itself on the GPU: the same bytes in every mode, and its launches counted in each."""
+    S, B, H, D, F = 16, 2, 4, 64, 128
+    cb = {"qkv": 32, "o": 32, "ffn1": 32, "ffn2": 64}
+    stream = torch.cuda.Stream()
+    ctx.set_stream(stream.cuda_stream)
+    lay = L.LutTransformerLayer(ctx, L.random_layer_weights(D, F, cb, {k: 16 for k in cb}, seed=4), S, B, H, first_layer_id=84)
+    x = torch.from_numpy(L.synth.make_input(S * B, D, seed=4)).cuda()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        want = torch.add(*lay._body(x))
+        for mode in (torch.inference_mode, torch.no_grad, torch.enable_grad):
+            lay.forward(x)
+            before = ctx.launch_count
+            lay.forward(x)
+            ordinary = ctx.launch_count - before
+            with mode():
+                for _ in range(5):
+                    before = ctx.launch_count
+                    assert torch.equal(lay.forward(x), want)
+                    assert ctx.launch_count - before == ordinary > 0
+            assert lay._graph is not None
+        stream.synchronize()
+    ctx.set_stream(None)
+    for lid in lay.ids.values():
+        ctx.unload_weights(lid)
