@@ -110,7 +110,8 @@ typedef struct lutamm_plan {
     uint32_t umma_groups;     /* tcgen05 one-hot builder groups of 4 warps (0 = default)  */
     uint32_t umma_operand;    /* where the one-hot operand lives: 0 = default,
                                  1 = shared memory, 2 = tensor memory (TMEM), 3 = tensor memory in the 2:4
-                                 sparse form, on CTA pairs (umma_n_tile 0, 64, 128 or 160, and
+                                 sparse form, on CTA pairs (umma_n_tile 0, 64, 128 or 160 - 192 only
+                                 by the library's own choice, for one tile per pair - and
                                  umma_split where every slice gets a pair of its own; the other umma_
                                  fields are the dense kernel's and ignored).  A plan that leaves
                                  all umma_ fields 0 takes form 3 wherever it applies: row-major output,
@@ -379,7 +380,7 @@ uint64_t lutamm_launch_count(const lutamm_ctx* ctx);
  * every GPU that loads the library holds them (plus 256) until the process exits. */
 #define LUTAMM_STATIC_SCRATCH_BYTES (8u * 1024u * 1024u)
 
-/* The whole AMM (search + gather-accumulate + dequantise, CUDA-core gather variant) without
+/* The whole AMM (search + gather-accumulate + dequantise; which kernels, by the sizes) without
  * any allocation: no cudaMalloc/cudaFree, no pooled allocator, no context.  It has no
  * counterpart in the reference.  It is for hosts that fix their device-memory layout at
  * start-up and forbid allocation afterwards (serving processes with pre-sized arenas,
@@ -387,7 +388,8 @@ uint64_t lutamm_launch_count(const lutamm_ctx* ctx);
  * All five buffers are DEVICE memory of `device`, laid out as for lutamm_load_weights /
  * lutamm_amm; n_tokens = index_params->n.  The index buffer between the two kernels lives in
  * a fixed __device__ array: n * num_codebook > LUTAMM_STATIC_SCRATCH_BYTES is rejected with
- * LUTAMM_EINVAL.  The call is synchronous on `cuda_stream` (a cudaStream_t, NULL = default
+ * LUTAMM_EINVAL.  What the indices leave of the array holds the table, some columns at a time, in the
+ * tensor-core kernel's layout, where that pays.  The call is synchronous on `cuda_stream` (a cudaStream_t, NULL = default
  * stream).  All calls in a process share the array on a device, so calls that overlap on the
  * GPU race: serialise them.  The first call on a device resolves the array's device address
  * (cudaGetSymbolAddress) and should therefore come before any stream capture.

@@ -21,8 +21,8 @@
 // What bounds it: dispatch.  Per centroid v/2 packed multiply-adds, half a packed addition (two dispatch cycles
 // each), half a three-input minimum and a funnel shift that collects the comparison's sign bit, against 3v/2 packed
 // and 4 other instructions of the scan; per (token, codebook) about 25 instructions around that.  v = 2, 16 centroids,
-// 65536 x 4096: 593 -> 484 us, the ALU pipe 53 % and the FMA pipe 45 % busy (they hardly overlap); v = 4, 64
-// centroids, 32768 x 3072: 1267 -> 492 us; v = 10, 16 centroids, 1576 x 2560: 87 -> 12 us.
+// 65536 x 4096: 593 -> 460 us, the ALU pipe 53 % and the FMA pipe 45 % busy (they hardly overlap); v = 4, 64
+// centroids, 32768 x 3072: 1267 -> 472 us; v = 10, 16 centroids, 1576 x 2560: 87 -> 14 us (CUDA events around the launch).
 //
 // Two mappings:
 //   ccs_reg_kernel  thread <-> codebook, the codebook's centroids in registers, the thread walks a run of

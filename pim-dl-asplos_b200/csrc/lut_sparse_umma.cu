@@ -433,8 +433,8 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
         // accumulate into one accumulator, and that is ordered between instructions of one thread only; between threads it takes
         // the tcgen05 fences on either side of a barrier.  So the warps issue in turn, slab after slab, each
         // handing over behind its four instructions (not behind their completion).  Unordered, the four linears of BERT-base at
-        // 1024 tokens take as long (76.4 and 76.8 us), 512 tokens 768 -> 3072 13.4 and 13.7 us; one warp alone, which needs no
-        // hand-over, 81.8 and 15.1 us.  Converged loop, one elected lane issues.
+        // 1024 tokens take 76.4 us, in turn 76.8, 512 tokens 768 -> 3072 13.5 and 13.7, 65536 tokens 4096 -> 16384 12.46 and 12.68 ms; one
+        // warp alone, which needs no hand-over, takes 81.8 and 15.1 us for the first two.  Converged loop, one elected lane issues.
         if (rank == 0) {
             const uint32_t me = warp - kFirstMma;
             uint32_t j = me, pb = 0, t = 0, x0 = 0;   // LUT slot and phases of this warp's next slab; slabs before the item
@@ -870,7 +870,7 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
     LUTAMM_SPARSE_CASE(160, false)
     LUTAMM_SPARSE_CASE(192, false)
 #undef LUTAMM_SPARSE_CASE
-    *why = "tcgen05 variant: the sparse form is built for 64-, 128- and 160-wide tiles";
+    *why = "tcgen05 variant: the sparse form is built for 64-, 128-, 160- and (one tile per pair) 192-wide tiles";
     return cudaErrorInvalidValue;
 }
 

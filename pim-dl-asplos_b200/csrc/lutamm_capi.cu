@@ -364,7 +364,7 @@ int run_lut(lutamm_ctx* c, Layer& L, const uint8_t* d_idx, float* d_out, int32_t
         // name a dense form, take the dense kernel.
         const bool sparse_fits = !a.n_peers && !a.acc_out && !a.layout.tiled;
         if (plan.umma_operand == 3 && plan.umma_n_tile && !sparse_tile_ok(plan.umma_n_tile))
-            return fail(c, LUTAMM_EINVAL, "umma_n_tile must be 64, 128 or 160 for the sparse form");
+            return fail(c, LUTAMM_EINVAL, "umma_n_tile must be 64, 128 or 160 for the sparse form (192 is the library's own choice only)");
         if (sparse_fits && (plan.umma_operand == 3 || umma_plan_open(plan))) return run_sparse(c, L, a, plan.umma_n_tile, plan.umma_split);
         UmmaPlan up;
         const bool dense_plan = plan.umma_operand != 3;   // else: where the sparse form does not fit, the dense default
@@ -867,7 +867,7 @@ int lutamm_set_plan(lutamm_ctx* c, int layer_id, const lutamm_plan* plan) {
     if (plan->gather_cfg >= gather_num_cfgs()) return fail(c, LUTAMM_EINVAL, "unknown gather tile configuration");
     if (plan->umma_operand > 3) return fail(c, LUTAMM_EINVAL, "umma_operand must be 0, 1 (shared memory), 2 (tensor memory) or 3 (2:4 sparse, CTA pairs)");
     if (plan->umma_operand == 3) {
-        if (plan->umma_n_tile && !sparse_tile_ok(plan->umma_n_tile)) return fail(c, LUTAMM_EINVAL, "umma_n_tile must be 0, 64, 128 or 160 for the sparse form");
+        if (plan->umma_n_tile && !sparse_tile_ok(plan->umma_n_tile)) return fail(c, LUTAMM_EINVAL, "umma_n_tile must be 0, 64, 128 or 160 for the sparse form (192 is the library's own choice only)");
     } else if (plan->umma_n_tile && plan->umma_operand && !umma_tile_ok(plan->umma_n_tile, plan->umma_operand == 2))
         return fail(c, LUTAMM_EINVAL, "umma_n_tile must be 0, 64, 128 or 256 with the one-hot operand in shared memory, "
                                       "0, 64, 128, 160 or 192 with it in tensor memory");
