@@ -142,7 +142,7 @@ cudaError_t launch_lut_untile(const int8_t* dpu, int8_t* canonical, uint32_t row
 cudaError_t launch_int8_peak(uint32_t n_tile, uint32_t slabs, uint32_t grid, unsigned long long* d_cycles, uint32_t* dev_err,
                              cudaStream_t s, const char** why);
 
-// Activations for timing: token m's sub-vector of codebook cb is one of that codebook's centroids, spread evenly over them.
+// Activations for timing: token m's sub-vector of codebook cb lies near one of that codebook's centroids, spread evenly over them.
 cudaError_t launch_spread_input(const float* centroid, float* x, uint32_t M, uint32_t CB, uint32_t CT, uint32_t v, cudaStream_t s);
 
 // Self-test: a bounded wait on a barrier nobody arrives at; the kernel reports through *dev_err and returns.
