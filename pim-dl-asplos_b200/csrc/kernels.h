@@ -106,10 +106,13 @@ void sparse_split_scratch(uint32_t M, uint32_t N, uint32_t n_tile, uint32_t spli
 bool sparse_tile_ok(uint32_t n_tile);
 cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile,
                              const char** why);
+// ... and straight from the canonical table (16-byte aligned), in 64- and 128-wide tiles without a split
+float sparse_canonical_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile);
+cudaError_t sparse_make_canonical_tmap(CUtensorMap* out, const int8_t* lut, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile, const char** why);
 cudaError_t sparse_make_idx_tmap(CUtensorMap* out, const uint8_t* idx, uint32_t M, uint32_t CB, uint32_t CT, const char** why);
 cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CUtensorMap& idx_map, const CUtensorMap& out_map, uint32_t n_tile,
                           uint32_t split, void* partial, uint32_t* counters /* zero between launches */, uint32_t max_ctas,
-                          bool fresh_table /* written by a kernel the stream may still run */, uint32_t* dev_err, cudaStream_t s, const char** why);
+                          bool fresh_table /* written by a kernel the stream may still run */, bool canonical /* lut_map: sparse_make_canonical_tmap */, uint32_t* dev_err, cudaStream_t s, const char** why);
 
 // A few tokens: the used rows of the canonical table alone (16-byte aligned), row-major fp32 output.
 cudaError_t launch_rows(const LutArgs& a, const int8_t* lut, int sm_count, cudaStream_t s);

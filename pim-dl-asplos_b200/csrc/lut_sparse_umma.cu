@@ -84,14 +84,15 @@ __device__ __forceinline__ void split2(const uint32_t (&in)[N], uint32_t b1, uin
 // The operand of one row's slab from its 256 / CT index bytes: 128 stored bytes (w) and the metadata of 64 positions of
 // the axis (m), which repeats for all four instructions of the slab.
 //
-// Stored byte p = d * codebooks + codebook, d being the centroid index without its bit 1: bytes of four codebooks share
+// Stored byte p = d * codebooks + codebook, d being the centroid index without its bit H: bytes of four codebooks share
 // a word, so a word is the AND of a few (complemented) bits of four packed indices - one three-input operation - where
 // codebook-major bytes would take two shifts and an extraction per codebook.  Positions 2p and 2p + 1 of the axis belong
-// to byte p: the index's bit 1 chooses, through the metadata nibble of the pair of bytes (2g, 2g + 1): the first stands
-// for position 0 or 1 of four, the second for 2 or 3.  The table is laid out to match (launch_sparse_table).
+// to byte p: the index's bit H chooses, through the metadata nibble of the pair of bytes (2g, 2g + 1): the first stands
+// for position 0 or 1 of four, the second for 2 or 3.  The table is laid out to match (launch_sparse_table, H = 1), or its
+// rows are copied in that order (the highest bit: then the rest of the index counts rows, and four dimensions say it all).
 //
 // An index that is out of range (they may come from a caller) stores nothing.
-template <int LG>
+template <int LG, int H>
 __device__ __forceinline__ void build_row(const uint32_t (&raw)[LG == 3 ? 8 : 4], uint32_t (&w)[32], uint32_t (&m)[2]) {
     constexpr int kCbs = 256 >> LG, kQ = kCbs >= 4 ? kCbs / 4 : 1;   // codebooks, words of packed indices
     constexpr uint32_t kOnes = 0x01010101u, kBeyond = LG == 8 ? 0u : ((0xFFu << LG) & 0xFFu) * kOnes;
@@ -103,8 +104,8 @@ __device__ __forceinline__ void build_row(const uint32_t (&raw)[LG == 3 ? 8 : 4]
         else v[q] = raw[q];
         any |= v[q] & kBeyond;
         valid[q] = kOnes;
-        // bits 0, 2, 4, 6 of the top byte: bit 1 of the four indices
-        top[q] = ((v[q] >> 1) & kOnes) * 0x01041040u;
+        // bits 0, 2, 4, 6 of the top byte: bit H of the four indices
+        top[q] = ((v[q] >> H) & kOnes) * 0x01041040u;
     }
     if (LG < 8 && any) {
         constexpr uint32_t kRange = 1u << (8 - LG);
@@ -114,33 +115,33 @@ __device__ __forceinline__ void build_row(const uint32_t (&raw)[LG == 3 ? 8 : 4]
 #pragma unroll
     for (int q = 0; q < kQ; ++q) {
         const uint32_t x = v[q];
+        auto bit = [x](int i) { return x >> (i >= H ? i + 1 : i); };   // bit i of d at bit 0 of the bytes
         if constexpr (LG == 3) {
             uint32_t in[1] = {valid[q]}, o[4];
-            split2(in, x >> 2, x, o);
+            split2(in, bit(1), bit(0), o);
 #pragma unroll
             for (int d = 0; d < 4; ++d) w[d * kQ + q] = o[d];
         } else if constexpr (LG == 4) {
             uint32_t in[1] = {valid[q]}, t[2], o[8];
-            split1(in, x >> 3, t);
-            split2(t, x >> 2, x, o);
+            split1(in, bit(2), t);
+            split2(t, bit(1), bit(0), o);
 #pragma unroll
             for (int d = 0; d < 8; ++d) w[d * kQ + q] = o[d];
         } else if constexpr (LG == 5) {
             uint32_t in[1] = {valid[q]}, t[4], o[16];
-            split2(in, x >> 4, x >> 3, t);
-            split2(t, x >> 2, x, o);
+            split2(in, bit(3), bit(2), t);
+            split2(t, bit(1), bit(0), o);
 #pragma unroll
             for (int d = 0; d < 16; ++d) w[d * kQ + q] = o[d];
         } else {
             // 32 words of one index word: five bits; what is left of d lies within the word
             uint32_t in[1], t[2], u[8];
-            constexpr int b = LG == 6 ? 0 : LG == 7 ? 2 : 3;   // lowest of the five bits (6: bits 5, 4, 3, 2, 0)
             if constexpr (LG == 6) in[0] = valid[q];
             else if constexpr (LG == 7) in[0] = valid[q] & ~(x ^ 0x01010000u);   // bytes: (d even) cb 0, 1, (d odd) cb 0, 1
-            else in[0] = 1u << (8 * (((x >> 1) & 2u) | (x & 1u)));
-            split1(in, LG == 6 ? x >> 5 : x >> (b + 4), t);
-            split2(t, LG == 6 ? x >> 4 : x >> (b + 3), LG == 6 ? x >> 3 : x >> (b + 2), u);
-            split2(u, LG == 6 ? x >> 2 : x >> (b + 1), x >> b, w);
+            else in[0] = 1u << (8 * (((bit(1) & 1u) << 1) | (x & 1u)));
+            split1(in, bit(LG - 2), t);
+            split2(t, bit(LG - 3), bit(LG - 4), u);
+            split2(u, bit(LG - 5), bit(LG - 6), w);
         }
     }
     uint32_t meta[2];
@@ -268,12 +269,19 @@ __device__ __forceinline__ bool split_finish(const SparseParams& p, const Sparse
 }
 
 // SPLIT: items are slices of a tile's codebook axis, one per pair.
-template <uint32_t N_TILE, int LG, bool SPLIT>
+// CANONICAL: the slabs come from the table as the caller has it, [codebook][centroid][N], columns contiguous: a slab is 256
+// of its rows, in the order of the positions, by a four-dimensional copy (sparse_make_canonical_tmap), and the operand is
+// column-major (MN-major) in shared memory.  For callers who have no room for the other layout, or use a table once: 512
+// tokens, 384 codebooks of 16 -> 3072, the synchronous call 54 -> 25 us.  The copies move rows of 64 or 32 bytes where
+// those of the other layout move 128, which costs nothing while the rows begin on sectors (a slab 0.16-0.2 us in a full
+// round, like there); tiles are powers of two wide, as a row has to be one row of a swizzle pattern.
+template <uint32_t N_TILE, int LG, bool SPLIT, bool CANONICAL>
 __global__ void __launch_bounds__(kThreads, 1)
 lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_constant__ CUtensorMap idx_map,
                   const __grid_constant__ CUtensorMap out_map, const SparseParams p) {
     constexpr uint32_t kHalfN = N_TILE / 2, kBBytes = kHalfN * kSlab;
-    constexpr uint32_t kIdesc = umma_idesc_i8(2 * kRows, N_TILE, 1, 1) | kIdescSparse;
+    constexpr uint32_t kIdesc = umma_idesc_i8(2 * kRows, N_TILE, 1, 1) | kIdescSparse | (CANONICAL ? kIdescColumnMajorB : 0);
+    static_assert(!CANONICAL || kHalfN == 32 || kHalfN == 64, "a row of a slab is one row of a swizzle pattern");
     constexpr uint32_t kASlots = operand_slots(N_TILE);
     constexpr bool kOne = accumulators(N_TILE) == 1;
     constexpr uint32_t kDataBase = accumulators(N_TILE) * N_TILE, kMetaBase = kDataBase + 32 * kASlots;   // tensor-memory columns
@@ -398,8 +406,12 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     ok = mbar_wait<32>(b_empty0 + 8 * j, ph ^ 1, s_abort);
                     if (!ok) break;
                     if (rank == 0) mbar_arrive_expect_tx(b_full0 + 8 * j, 2 * kBBytes);
-                    tma_load_3d_pair(smem_u32(s_b + (size_t)j * kBBytes), &lut_map, full_leader + 8 * j, 0,
-                                     (int32_t)(it.n0 + rank * kHalfN), (int32_t)(2 * (it.begin + i)));
+                    if constexpr (CANONICAL)
+                        tma_load_4d_pair(smem_u32(s_b + (size_t)j * kBBytes), &lut_map, full_leader + 8 * j, (int32_t)(it.n0 + rank * kHalfN),
+                                         (int32_t)((it.begin + i) * (kSlab >> LG)));
+                    else
+                        tma_load_3d_pair(smem_u32(s_b + (size_t)j * kBBytes), &lut_map, full_leader + 8 * j, 0,
+                                         (int32_t)(it.n0 + rank * kHalfN), (int32_t)(2 * (it.begin + i)));
                     j += kCopyWarps;
                     if (j >= SB) { j -= SB; ph ^= 1; }
                 }
@@ -439,8 +451,10 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             const uint32_t me = warp - kFirstMma;
             uint32_t j = me, pb = 0, t = 0, x0 = 0;   // LUT slot and phases of this warp's next slab; slabs before the item
             bool ok = true;
-            const uint32_t b_lo0 = (uint32_t)umma_desc_k_sw128(smem_u32(s_b));
-            const uint32_t desc_hi = (uint32_t)(umma_desc_k_sw128(0) >> 32);
+            const uint64_t b_desc = CANONICAL ? umma_desc_columns(smem_u32(s_b), kHalfN) : umma_desc_k_sw128(smem_u32(s_b));
+            const uint32_t b_lo0 = (uint32_t)b_desc, desc_hi = (uint32_t)(b_desc >> 32);
+            // from one instruction's 64 positions to the next: two per 128-byte swizzle row, or 64 rows on
+            constexpr uint32_t kOdd = CANONICAL ? 64 * kHalfN >> 4 : 4, kEven = CANONICAL ? 128 * kHalfN >> 4 : kHalfN * 128 >> 4;
             for (uint32_t item = first; item < n_items && ok; item += n_pairs, ++t) {
                 const uint32_t ab = t & 1, slabs = sparse_item<SPLIT>(p, item, N_TILE, rank).slabs;
                 ok = mbar_wait(acc_empty0 + 8 * ab, ((t >> 1) & 1) ^ 1, s_abort);
@@ -456,9 +470,9 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     if (elect_one()) {
                         const uint32_t b_lo = b_lo0 + j * (kBBytes >> 4);
 #pragma unroll
-                        for (uint32_t kk = 0; kk < 4; ++kk)   // 64 positions each: two per 128-byte swizzle row
+                        for (uint32_t kk = 0; kk < 4; ++kk)
                             umma_i8_sparse_pair(d_tmem, tmem_base + kDataBase + 32 * k + 8 * kk,
-                                                ((uint64_t)desc_hi << 32) | (b_lo + (kk >> 1) * (kHalfN * 128 >> 4) + (kk & 1) * 4),
+                                                ((uint64_t)desc_hi << 32) | (b_lo + (kk >> 1) * kEven + (kk & 1) * kOdd),
                                                 tmem_base + kMetaBase + 2 * k, kIdesc);
                         tc_fence_before_sync();
                         mbar_arrive(turn0 + 8 * ((me + 1) & (kMmaWarps - 1)));
@@ -512,7 +526,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     const uint32_t x = x0 + i0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
                     uint32_t raw[kRaw], w[32], m[2];
                     load_raw(s_idx + st * kIdxBytes, i, raw);
-                    build_row<LG>(raw, w, m);
+                    build_row<LG, CANONICAL ? LG - 1 : 1>(raw, w, m);
                     // the row is in registers before the slot is waited for (the compiler would sink it behind the wait,
                     // onto the slot's turn-around path)
 #pragma unroll
@@ -646,9 +660,9 @@ size_t sparse_smem(uint32_t n_tile, int lg, uint32_t b_slots) {
            kEpiWarps * n_tile * 4 + kNumBarriers * 8 + 16 + 1024;
 }
 
-template <uint32_t N_TILE, int LG, bool SPLIT>
+template <uint32_t N_TILE, int LG, bool SPLIT, bool CANONICAL>
 cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
-    auto k = lut_sparse_kernel<N_TILE, LG, SPLIT>;
+    auto k = lut_sparse_kernel<N_TILE, LG, SPLIT, CANONICAL>;
     static SmemOptIn memo;
     cudaError_t e = allow_smem(memo, k, (int)smem);
     if (e != cudaSuccess) return e;
@@ -669,15 +683,15 @@ cudaError_t run(const CUtensorMap& map, const CUtensorMap& idx_map, const CUtens
     return cudaLaunchKernelEx(&cfg, k, map, idx_map, out_map, p);
 }
 
-template <uint32_t N_TILE, bool SPLIT>
+template <uint32_t N_TILE, bool SPLIT, bool CANONICAL = false>
 cudaError_t run_lg(uint32_t lg, const CUtensorMap& map, const CUtensorMap& idx_map, const CUtensorMap& out_map, const SparseParams& p, uint32_t pairs, size_t smem, cudaStream_t s) {
     switch (lg) {
-        case 3: return run<N_TILE, 3, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
-        case 4: return run<N_TILE, 4, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
-        case 5: return run<N_TILE, 5, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
-        case 6: return run<N_TILE, 6, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
-        case 7: return run<N_TILE, 7, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
-        default: return run<N_TILE, 8, SPLIT>(map, idx_map, out_map, p, pairs, smem, s);
+        case 3: return run<N_TILE, 3, SPLIT, CANONICAL>(map, idx_map, out_map, p, pairs, smem, s);
+        case 4: return run<N_TILE, 4, SPLIT, CANONICAL>(map, idx_map, out_map, p, pairs, smem, s);
+        case 5: return run<N_TILE, 5, SPLIT, CANONICAL>(map, idx_map, out_map, p, pairs, smem, s);
+        case 6: return run<N_TILE, 6, SPLIT, CANONICAL>(map, idx_map, out_map, p, pairs, smem, s);
+        case 7: return run<N_TILE, 7, SPLIT, CANONICAL>(map, idx_map, out_map, p, pairs, smem, s);
+        default: return run<N_TILE, 8, SPLIT, CANONICAL>(map, idx_map, out_map, p, pairs, smem, s);
     }
 }
 
@@ -762,6 +776,22 @@ cudaError_t sparse_make_tmap(CUtensorMap* out, const int8_t* table, uint32_t CB,
     return cudaSuccess;
 }
 
+// The canonical table [CB][CT][N] as boxes of half a tile's columns of one slab's 256 rows, in the order of the slab's
+// positions 2 (d * codebooks + c) + h: columns, h (the highest bit of the centroid index), codebook, d (the bits below).
+cudaError_t sparse_make_canonical_tmap(CUtensorMap* out, const int8_t* lut, uint32_t CB, uint32_t CT, uint32_t N, uint32_t n_tile, const char** why) {
+    *why = nullptr;
+    EncodeTiledFn enc = get_encode_tiled();
+    if (!enc) { *why = "cuTensorMapEncodeTiled is not available from this driver"; return cudaErrorNotSupported; }
+    cuuint64_t dims[4] = {N, 2, CB, CT / 2};
+    cuuint64_t strides[3] = {(cuuint64_t)CT / 2 * N, (cuuint64_t)CT * N, N};
+    cuuint32_t box[4] = {n_tile / 2, 2, kSlab / CT, CT / 2};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<int8_t*>(lut), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     n_tile == 64 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the canonical table"; return cudaErrorInvalidValue; }
+    return cudaSuccess;
+}
+
 // uint8 indices [M][CB] as 128 rows x idx_width bytes
 cudaError_t sparse_make_idx_tmap(CUtensorMap* out, const uint8_t* idx, uint32_t M, uint32_t CB, uint32_t CT, const char** why) {
     *why = nullptr;
@@ -813,6 +843,23 @@ float sparse_default_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int 
 // Tiles a plan may name; 192 columns suit only launches of one round, which sparse_default_plan() knows.
 bool sparse_tile_ok(uint32_t n_tile) { return n_tile == 64 || n_tile == 128 || n_tile == 160; }
 
+// The same for the canonical table: its tile width, and the time.  A slab takes what it takes above where the rows that
+// the copies fetch, 64 or 32 bytes of 256 table rows, begin on multiples of 64 or 32 bytes, and up to twice that where
+// N makes every other one straddle sectors (2048 codebooks of 16, 64 tokens: N = 3136 44 us a call in 128-wide tiles, 3104 56,
+// 3088 73, in 64-wide ones 57).
+float sparse_canonical_plan(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count, uint32_t* n_tile) {
+    const uint32_t pairs = sm_count >= 2 ? (uint32_t)sm_count / 2 : 1, slabs = sparse_slabs(CB, CT);
+    const uint64_t tm = (M + 2 * kRows - 1) / (2 * kRows);
+    const struct { uint32_t n; float slab_us; } tiles[] = {{64, N % 32 ? 0.29f : 0.17f}, {128, N % 32 ? 0.42f : N % 64 ? 0.27f : 0.2f}};
+    float least = 3e38f;
+    for (const auto& t : tiles) {
+        const uint64_t rounds = (tm * ((N + t.n - 1) / t.n) + pairs - 1) / pairs;
+        const float main = slabs * t.slab_us, epi = 0.93f * (t.n / 32), us = (float)rounds * (rounds > 1 && epi > main ? epi : main) + 0.25f * (t.n / 32);
+        if (us < least) { least = us; *n_tile = t.n; }
+    }
+    return least;
+}
+
 // Scratch of a split launch: partial sums and counter words.
 void sparse_split_scratch(uint32_t M, uint32_t N, uint32_t n_tile, uint32_t split, size_t* partial_bytes, size_t* counter_bytes) {
     const size_t tiles = (size_t)((M + 2 * kRows - 1) / (2 * kRows)) * ((N + n_tile - 1) / n_tile);
@@ -821,7 +868,7 @@ void sparse_split_scratch(uint32_t M, uint32_t N, uint32_t n_tile, uint32_t spli
 }
 
 cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CUtensorMap& idx_map, const CUtensorMap& out_map, uint32_t n_tile,
-                          uint32_t split, void* partial, uint32_t* counters, uint32_t max_ctas, bool fresh_table, uint32_t* dev_err,
+                          uint32_t split, void* partial, uint32_t* counters, uint32_t max_ctas, bool fresh_table, bool canonical, uint32_t* dev_err,
                           cudaStream_t s, const char** why) {
     *why = nullptr;
     if (a.M == 0 || a.N == 0) return cudaSuccess;
@@ -861,6 +908,12 @@ cudaError_t launch_sparse(const LutArgs& a, const CUtensorMap& lut_map, const CU
     p.fresh_table = fresh_table;
     if (accumulators(n_tile) == 1 && !p.one_tile) { *why = "tiles wider than 160 columns of the sparse form take one tile per pair"; return cudaErrorInvalidValue; }
     const size_t smem = sparse_smem(n_tile, lg, p.b_slots);
+    if (canonical) {
+        if (p.split == 1 && n_tile == 64) return run_lg<64, false, true>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
+        if (p.split == 1 && n_tile == 128) return run_lg<128, false, true>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
+        *why = "the canonical table is contracted in 64- and 128-wide tiles, unsplit";
+        return cudaErrorInvalidValue;
+    }
 #define LUTAMM_SPARSE_CASE(NT, SP) \
     if (n_tile == NT && (p.split > 1) == SP) return run_lg<NT, SP>(lg, lut_map, idx_map, out_map, p, pairs, smem, s);
     LUTAMM_SPARSE_CASE(64, false)

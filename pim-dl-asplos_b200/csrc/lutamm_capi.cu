@@ -291,7 +291,7 @@ int run_sparse(lutamm_ctx* c, Layer& L, const LutArgs& a, uint32_t n_tile, uint3
     }
     if (e == cudaSuccess)
         e = launch_sparse(a, L.sparse_maps[slot], L.sparse_idx_map, L.sparse_out_map, n_tile, split, c->d_acc_scratch.p,
-                          static_cast<uint32_t*>(c->d_counters.p), (uint32_t)c->sm_count, false, c->d_err, c->stream, &why);
+                          static_cast<uint32_t*>(c->d_counters.p), (uint32_t)c->sm_count, false, false, c->d_err, c->stream, &why);
     if (e != cudaSuccess) return fail(c, LUTAMM_ECUDA, why ? why : (std::string("tcgen05 launch: ") + cudaGetErrorString(e)));
     ++c->launches;
     return LUTAMM_OK;

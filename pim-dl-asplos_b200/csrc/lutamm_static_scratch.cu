@@ -71,33 +71,41 @@ uint32_t sm_count_of(int device) {
     return n;
 }
 
-// By estimated time: the table's used rows, for few tokens; the table laid out for the tcgen05 kernel on every call,
-// `columns` at a time in what the indices leave of the array; or the CUDA-core gather, which reads the table as it is: its
-// narrow tiles of few tokens where wide ones would leave SMs without a CTA.
+// By estimated time: the table's used rows, for few tokens; the tcgen05 kernel on the table as it is; or the CUDA-core
+// gather, its narrow tiles of few tokens where wide ones would leave SMs without a CTA.  Laying the table out first, as a
+// context does once per layer, was slower at all of 70 sizes (512 tokens 768 -> 3072: 54 us a call against 25; 8192 tokens
+// 1024 -> 4096: 116 against 92), and is left for tables that are not 16-byte aligned, which the copy engine cannot read:
+// `columns` at a time in what the indices leave of the array.  Over those sizes (1 to 8192 tokens) the choice takes 0.6 %
+// more than the fastest form of each, on average.
 struct TablePlan {
     bool rows;
-    uint32_t columns, gather_cfg;
+    uint32_t direct, columns, gather_cfg;   // direct: tile width
 };
 TablePlan plan_table(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, bool aligned, uint32_t sms) {
     const uint32_t cfg = (uint64_t)((M + 63) / 64) * ((N + 255) / 256) < sms ? 4 : 0;
-    const float gather = lutamm::gather_us(M, CB, CT, N, cfg, (int)sms), rows = aligned ? lutamm::rows_us(M, CB, CT, N, (int)sms) : 3e38f;
+    const float gather = 2.f + lutamm::gather_us(M, CB, CT, N, cfg, (int)sms), rows = aligned ? lutamm::rows_us(M, CB, CT, N, (int)sms) : 3e38f;
     float table = 3e38f;
-    uint32_t columns = 0;
+    uint32_t columns = 0, direct = 0;
     if (lutamm::umma_supported(CB, CT, N)) {
-        const size_t per_column = lutamm::sparse_table_bytes(CB, CT, 1), used = (((size_t)M * CB + 255) / 256) * 256;
-        const size_t fit = used < LUTAMM_STATIC_SCRATCH_BYTES ? (LUTAMM_STATIC_SCRATCH_BYTES - used) / per_column : 0;
-        columns = fit < N ? (uint32_t)(fit / 64 * 64) : N;
-        if (columns) {
-            const uint32_t chunks = (N + columns - 1) / columns;
-            columns = ((N + chunks - 1) / chunks + 63) / 64 * 64;   // near-equal chunks
-            if (columns > N) columns = N;
-            uint32_t n_tile, split;
-            // a piece: two launches, the layout at 2.5 TB/s, the contraction (measured 768 -> 768 to 512 -> 8192, 1 to 5 pieces)
-            const float contraction = lutamm::sparse_default_plan(M, CB, CT, columns, (int)sms, &n_tile, &split, 0, 1);
-            table = 2.6f + chunks * (3.7f + (float)per_column * columns / 2.5e6f + contraction);
+        if (aligned) {
+            table = 6.f + lutamm::sparse_canonical_plan(M, CB, CT, N, (int)sms, &direct);
+        } else {
+            const size_t per_column = lutamm::sparse_table_bytes(CB, CT, 1), used = (((size_t)M * CB + 255) / 256) * 256;
+            const size_t fit = used < LUTAMM_STATIC_SCRATCH_BYTES ? (LUTAMM_STATIC_SCRATCH_BYTES - used) / per_column : 0;
+            columns = fit < N ? (uint32_t)(fit / 64 * 64) : N;
+            if (columns) {
+                const uint32_t chunks = (N + columns - 1) / columns;
+                columns = ((N + chunks - 1) / chunks + 63) / 64 * 64;   // near-equal chunks
+                if (columns > N) columns = N;
+                uint32_t n_tile, split;
+                // a piece: two launches, the layout at 2.5 TB/s, the contraction (measured 768 -> 768 to 512 -> 8192, 1 to 5 pieces)
+                const float contraction = lutamm::sparse_default_plan(M, CB, CT, columns, (int)sms, &n_tile, &split, 0, 1);
+                table = 2.6f + chunks * (3.7f + (float)per_column * columns / 2.5e6f + contraction);
+            }
         }
     }
-    return {rows < table && rows < gather, table < gather ? columns : 0u, cfg};
+    const bool contract = table < gather;
+    return {rows < table && rows < gather, contract ? direct : 0u, contract ? columns : 0u, cfg};
 }
 
 }  // namespace
@@ -186,6 +194,14 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
     if (plan.rows) {
         e = launch_rows(la, lut, (int)sms, s);
         if (e != cudaSuccess) return fail(LUTAMM_ECUDA, std::string("row gather launch: ") + cudaGetErrorString(e));
+    } else if (plan.direct) {
+        CUtensorMap idx_map, table_map, out_map;
+        e = sparse_make_idx_tmap(&idx_map, d_idx, M, CB, CT, &why);
+        if (e == cudaSuccess) e = sparse_make_canonical_tmap(&table_map, lut, CB, CT, N, plan.direct, &why);
+        if (e == cudaSuccess) e = make_out_tmap(&out_map, output, M, N, &why);
+        // (the table may be what the caller's last kernel writes: its copies wait for the search, and that for the caller)
+        if (e == cudaSuccess) e = launch_sparse(la, table_map, idx_map, out_map, plan.direct, 1, nullptr, nullptr, sms, true, true, d_err, s, &why);
+        if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : (std::string("tcgen05 launch: ") + cudaGetErrorString(e)));
     } else if (plan.columns) {
         // the tcgen05 kernel on as many columns at a time as the rest of the array holds of its layout of the table
         int8_t* table = reinterpret_cast<int8_t*>(d_idx + (((size_t)M * CB + 255) / 256) * 256);
@@ -205,7 +221,7 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
             e = launch_sparse_table(lut, table, CB, CT, la.N, n0, N, n0 > 0, s);
             if (e == cudaSuccess) e = sparse_make_tmap(&table_map, table, CB, CT, la.N, n_tile, &why);
             if (e == cudaSuccess) e = make_out_tmap(&out_map, la.out, M, la.N, &why, N);
-            if (e == cudaSuccess) e = launch_sparse(la, table_map, idx_map, out_map, n_tile, 1, nullptr, nullptr, sms, true, d_err, s, &why);
+            if (e == cudaSuccess) e = launch_sparse(la, table_map, idx_map, out_map, n_tile, 1, nullptr, nullptr, sms, true, false, d_err, s, &why);
         }
         if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : (std::string("tcgen05 launch: ") + cudaGetErrorString(e)));
     } else {

@@ -257,6 +257,13 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(cluster_bar), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
+// Same for the four dimensions (x, all, z, all).
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap* m, uint32_t cluster_bar, int32_t x, int32_t z) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %5, %4, %5}], [%2];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(cluster_bar), "r"(x), "r"(z), "r"(0)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -282,6 +289,7 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
                  : "memory");
 }
 constexpr uint32_t kIdescSparse = 1u << 2;   // instruction-descriptor bit of the sparse form
+constexpr uint32_t kIdescColumnMajorB = 1u << 16;   // ... of a B operand whose columns, not its contraction axis, are contiguous
 
 // Shared-memory matrix descriptor for a K-major operand tile whose K extent is exactly one
 // 128-byte swizzle row (SWIZZLE_128B): rows 128 B apart, groups of 8 rows 1024 B apart.
@@ -296,6 +304,18 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr) {
     d |= static_cast<uint64_t>(1024u >> 4) << 32;
     d |= static_cast<uint64_t>(1) << 46;
     d |= static_cast<uint64_t>(2) << 61;
+    return d;
+}
+
+// ... for a column-major (MN-major) operand of 8-bit elements whose columns are exactly one swizzle row of 32 or 64 bytes
+// (SWIZZLE_32B / SWIZZLE_64B, bits 61-63 = 6 / 4): positions of the contraction axis `row` bytes apart, eight of them a group.
+__device__ __forceinline__ uint64_t umma_desc_columns(uint32_t smem_addr, uint32_t row) {
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
+    d |= static_cast<uint64_t>(8 * row >> 4) << 16;   // to the next swizzle row of columns: there is none
+    d |= static_cast<uint64_t>(8 * row >> 4) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    d |= static_cast<uint64_t>(row == 32 ? 6 : 4) << 61;
     return d;
 }
 

@@ -89,12 +89,14 @@ def _static(fake, M, K, N, v, CT, offset=0):
 
 
 @pytest.mark.parametrize("form,M,K,N,v,CT", [
-    ("rows", 1, 768, 3072, 2, 16), ("rows", 256, 768, 2304, 4, 64), ("rows", 128, 768, 3072, 4, 32), ("rows", 256, 3072, 768, 2, 16),
+    ("rows", 1, 768, 3072, 2, 16), ("rows", 64, 768, 768, 4, 16), ("rows", 29, 1408, 12464, 4, 128), ("rows", 252, 896, 224, 8, 8),
     ("table", 256, 768, 3072, 2, 16), ("table", 1024, 768, 2304, 4, 64), ("table", 512, 768, 3072, 4, 32), ("table", 256, 4096, 4096, 8, 16),
-    ("gather", 128, 512, 8192, 2, 16), ("gather", 64, 32, 8192, 2, 13), ("gather", 66000, 16, 16, 2, 200)])
+    ("table", 256, 768, 2304, 4, 64), ("table", 128, 768, 3072, 4, 32), ("table", 256, 3072, 768, 2, 16),
+    ("gather", 122, 160, 15440, 10, 16), ("gather", 64, 32, 8192, 2, 13), ("gather", 66000, 16, 16, 2, 200)])
 def test_how_the_static_call_contracts(fake, form, M, K, N, v, CT):
     """The fastest by measurement of all three at these sizes, and no split of the codebook axis, for which it has no scratch."""
     log = _static(fake, M, K, N, v, CT)
+    assert len(log) == 2
     assert {"rows": "lut_rows_kernel", "table": "lut_sparse_kernel", "gather": "lut_gather_kernel"}[form] in log[-1]
     assert all("split=1" in ln for ln in log if "lut_sparse_kernel" in ln)
 
@@ -102,9 +104,17 @@ def test_how_the_static_call_contracts(fake, form, M, K, N, v, CT):
 @pytest.mark.parametrize("early,M,K,N,v,CT", [("110", 512, 768, 3072, 2, 16), ("000", 1024, 768, 3072, 2, 16), ("00000", 384, 512, 8192, 2, 16),
                                               ("11110", 640, 512, 8192, 2, 16), ("0", 300, 256, 512, 2, 16)])
 def test_who_launches_the_next_pieces_layout_early(fake, early, M, K, N, v, CT):
-    """Up to eight of its CTAs per SM without a tile; nothing behind the last piece."""
-    log = [ln for ln in _static(fake, M, K, N, v, CT) if "lut_sparse_kernel" in ln]
+    """An unaligned table is laid out in pieces.  Up to eight CTAs of the next layout per SM without a tile; nothing behind the last piece."""
+    log = [ln for ln in _static(fake, M, K, N, v, CT, offset=4) if "lut_sparse_kernel" in ln]
     assert "".join(ln[-1] for ln in log) == early
+
+
+@pytest.mark.parametrize("tile,M,K,N,v,CT", [(64, 1300, 512, 144, 2, 8), (64, 1000, 1536, 144, 2, 32), (64, 512, 768, 1072, 4, 64), (64, 385, 1024, 2064, 4, 128),
+                                             (128, 385, 512, 4176, 2, 256), (128, 3000, 832, 2064, 4, 16), (128, 512, 768, 3072, 2, 16)])
+def test_an_aligned_table_is_contracted_as_it_is(fake, tile, M, K, N, v, CT):
+    """One launch behind the search, no layout of the table; the tile width by how N lies to the sectors."""
+    log = _static(fake, M, K, N, v, CT)
+    assert len(log) == 2 and f"lut_sparse_kernelILj{tile}E" in log[1]
 
 
 def test_an_unaligned_table_is_not_gathered_by_rows(fake):
