@@ -5,9 +5,11 @@
 // codebooks of 16 -> 1152 are 35 MB instead of 61.
 //
 // A CTA takes one token, 128 columns and a share of the codebooks: 8 lanes per row, 16 bytes each, so a warp reads four
-// rows and every thread has 8 loads in flight.  Bytes are widened to 16 bits, two per register, offset by 128 so that
-// they cannot be negative: 256 rows of at most 255 fit, which is what a CTA reduces before it adds to int32.  The CTAs
-// of a cluster hold the shares of one token and tile and are summed through distributed shared memory.
+// rows and every thread has 8 loads in flight, a chunk of 256 codebooks; the indices of the next chunk are on their way
+// meanwhile.  Bytes are widened to 16 bits, two per register, offset by 128 so that they cannot be negative: 256 rows of at
+// most 255 fit into what four threads of a warp add up, so warps meet and add to int32 once in 8 chunks (once in every
+// chunk 1536 codebooks -> 768 took 10.9 us for one token, and 9.5 now).  The CTAs of a cluster hold the shares of one token and
+// tile and are summed through distributed shared memory.
 //
 // V > 0: the search as well, one launch for the whole operator.  A CTA searches the codebooks of its share, a thread each,
 // by the reference's scan (ccs_argmin.cu) on centroids it reads itself; every column tile of a token repeats that, which
@@ -24,7 +26,7 @@ namespace lutamm {
 
 namespace {
 
-constexpr uint32_t kThreads = 256, kTile = 128, kChunk = 256;   // columns of a CTA, codebooks between int32 sums
+constexpr uint32_t kThreads = 256, kTile = 128, kChunk = 256;   // columns of a CTA, codebooks whose rows are in flight together
 constexpr uint32_t kMaxCluster = 8;
 
 __device__ __forceinline__ int32_t load_cluster(uint32_t addr) {
@@ -70,12 +72,13 @@ __device__ __forceinline__ uint32_t scan(const float (&x)[V], const float* p, fl
     return best;
 }
 
-template <int V>
-__global__ void __launch_bounds__(kThreads, V > 0 ? 3 : 4)
+// LONG: shares of more than one chunk.  (One kernel for both cost calls of one chunk 0.4 us of 3.8.)
+template <int V, bool LONG>
+__global__ void __launch_bounds__(kThreads, V > 0 ? (LONG ? 2 : 3) : 4)
 lut_rows_kernel(const int8_t* __restrict__ lut, const LutArgs a, const SearchArgs sa, uint32_t per) {
     __shared__ uint32_t s_part[8][kTile / 2];
     __shared__ int32_t s_sum[kTile];
-    __shared__ uint8_t s_idx[kChunk];
+    __shared__ uint8_t s_idx[LONG ? 2 : 1][kChunk];
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, shares = gridDim.x, rank = blockIdx.x;
     const uint32_t m = blockIdx.z, n0 = blockIdx.y * kTile;
     const uint32_t begin = rank * per, end = min(a.CB, begin + per);
@@ -86,8 +89,12 @@ lut_rows_kernel(const int8_t* __restrict__ lut, const LutArgs a, const SearchArg
         if (begin + t < end) load_centroids(q, sa.centroid + (size_t)(begin + t) * a.CT * V, a.CT * V);
     pdl_wait_prior_grid();   // activations or indices, and the reader of an output that may be written again
     int32_t sum0 = 0, sum1 = 0;
-    for (uint32_t c0 = begin; c0 < end; c0 += kChunk) {
-        const uint32_t count = min(kChunk, end - c0);
+    uint32_t acc[8] = {}, buf = 0, pending = 0;   // [word][columns 0 and 2, columns 1 and 3]; chunks in it
+    uint8_t ahead = 0;   // this thread's index of the next chunk
+    if (LONG && V == 0 && begin + t < end) ahead = __ldcg(a.idx + (size_t)m * a.CB + begin + t);
+    uint32_t c0 = begin;
+    do {
+        const uint32_t count = c0 < end ? min(kChunk, end - c0) : 0u;
         if constexpr (V > 0) {
             if (t < count) {
                 const float* p = sa.centroid + (size_t)(c0 + t) * a.CT * V;
@@ -103,11 +110,16 @@ lut_rows_kernel(const int8_t* __restrict__ lut, const LutArgs a, const SearchArg
                         x[d] = u.x; x[d + 1] = u.y; x[d + 2] = u.z; x[d + 3] = u.w;
                     }
                 }
-                if (c0 != begin) load_centroids(q, p, a.CT * V);
-                s_idx[t] = (uint8_t)scan<V>(x, p, q, a.CT);
+                if (LONG && c0 != begin) load_centroids(q, p, a.CT * V);
+                s_idx[buf][t] = (uint8_t)scan<V>(x, p, q, a.CT);
             }
         } else {
-            if (t < count) s_idx[t] = __ldcg(a.idx + (size_t)m * a.CB + c0 + t);
+            if constexpr (LONG) {
+                s_idx[buf][t] = ahead;
+                if (c0 + kChunk + t < end) ahead = __ldcg(a.idx + (size_t)m * a.CB + c0 + kChunk + t);
+            } else {
+                if (t < count) s_idx[0][t] = __ldcg(a.idx + (size_t)m * a.CB + c0 + t);
+            }
         }
         __syncthreads();
         uint4 w[8];
@@ -116,11 +128,10 @@ lut_rows_kernel(const int8_t* __restrict__ lut, const LutArgs a, const SearchArg
             const uint32_t c = group + 32 * j;
             w[j] = make_uint4(0, 0, 0, 0);
             if (c < count && n < a.N) {
-                const uint32_t i = s_idx[c];   // one that is out of range adds nothing
+                const uint32_t i = s_idx[buf][c];   // one that is out of range adds nothing
                 if (i < a.CT) w[j] = __ldg(reinterpret_cast<const uint4*>(lut + ((size_t)(c0 + c) * a.CT + i) * a.N + n));
             }
         }
-        uint32_t acc[8] = {};   // [word][columns 0 and 2, columns 1 and 3]
 #pragma unroll
         for (uint32_t j = 0; j < 8; ++j) {
             const uint32_t q[4] = {w[j].x, w[j].y, w[j].z, w[j].w};
@@ -130,6 +141,12 @@ lut_rows_kernel(const int8_t* __restrict__ lut, const LutArgs a, const SearchArg
                 acc[2 * k + 1] += ((q[k] >> 8) ^ 0x00808080u) & 0x00FF00FFu;
             }
         }
+        if constexpr (LONG) {
+            buf ^= 1;
+            c0 += kChunk;
+            if (++pending < 8 && c0 < end) continue;
+        }
+        // 64 rows of a thread at most, over the four threads of a warp that hold the same columns: 256 * 255 < 2^16
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k) {
             acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 8);
@@ -142,13 +159,28 @@ lut_rows_kernel(const int8_t* __restrict__ lut, const LutArgs a, const SearchArg
         }
         __syncthreads();
         if (t < kTile / 2) {
-            uint32_t s = 0;
+            const int32_t none = -128 * (int32_t)((LONG ? pending : 1) * kChunk);   // a row, or the zero in its place, was added with 128 more
+            sum0 += none;
+            sum1 += none;
+            if (!LONG || pending == 1) {   // 8 rows a thread: all 256 fit into the two halves
+                uint32_t s = 0;
 #pragma unroll
-            for (uint32_t k = 0; k < 8; ++k) s += s_part[k][t];
-            sum0 += (int32_t)(s & 0xFFFFu) - 128 * (int32_t)kChunk;   // every thread added 8 rows, some of them zero
-            sum1 += (int32_t)(s >> 16) - 128 * (int32_t)kChunk;
+                for (uint32_t k = 0; k < 8; ++k) s += s_part[k][t];
+                sum0 += (int32_t)(s & 0xFFFFu);
+                sum1 += (int32_t)(s >> 16);
+            } else {
+#pragma unroll
+                for (uint32_t k = 0; k < 8; ++k) {
+                    const uint32_t s = s_part[k][t];
+                    sum0 += (int32_t)(s & 0xFFFFu);
+                    sum1 += (int32_t)(s >> 16);
+                }
+            }
         }
-    }
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) acc[k] = 0;
+        pending = 0;
+    } while (LONG && c0 < end);
     if (t < kTile / 2) {
         const uint32_t col = (t >> 3) * 16 + ((t >> 1) & 3u) * 4 + (t & 1u);
         s_sum[col] = sum0;
@@ -166,24 +198,38 @@ lut_rows_kernel(const int8_t* __restrict__ lut, const LutArgs a, const SearchArg
 
 }  // namespace
 
-// Shares of the codebook axis: until the SMs have a CTA and a half each, at most one cluster, of 32 codebooks at least.
-// (A launch is done in 4.5 us without a cluster and in 5.3 with one; 8 tokens, 1536 codebooks -> 768: 11.9 us whole, 8.8 in
-// halves, 7.9 in quarters, 7.0 in eighths.)
-static uint32_t rows_shares(uint32_t M, uint32_t CB, uint32_t N, int sm_count) {
-    const uint64_t tiles = (uint64_t)M * ((N + kTile - 1) / kTile);
-    uint32_t shares = 1;
-    while (shares < kMaxCluster && 2 * tiles * shares < 3ull * sm_count && shares * 64 <= CB) shares *= 2;
-    return shares;
+// What a call takes, in microseconds, with its codebook axis in `shares`: a cluster is a microsecond, so is every chunk of
+// codebooks after the first (two where they are searched, too), a CTA costs 4 ns and its rows 11 ns per 1000, and a table
+// that the half of L2 on an SM's die does not hold costs more per row.  With the search every CTA also reads and scans the
+// centroids of its share.  Fitted to 870 calls of 1 to 200 tokens, 256 to 8192 features, 5 to 128 centroids, each with 1, 2, 4
+// and 8 shares, to 20 % (11 % with the search).  By the least of these, and of the contraction in lutamm_capi.cu, those calls
+// take 0.7 % more than the fastest form of each; 5.5 % with as many shares as made a CTA and a half for every SM.
+static float rows_call_us(bool search, uint32_t M, uint32_t CB, uint32_t CT, uint32_t v, uint32_t N, uint32_t shares, int sm_count) {
+    const uint32_t per = (CB + shares - 1) / shares;
+    const float tiles = (float)((N + kTile - 1) / kTile) * (float)M, ctas = tiles * shares * (148.f / sm_count), more = (float)((per + kChunk - 1) / kChunk - 1);
+    const float far = (uint64_t)CB * CT * N > 40000000 ? 1e-6f * tiles * kTile * CB : 0.f, cluster = shares > 1 ? 1.f : 0.f;
+    if (search)
+        return 2.1f + cluster * (1.f + 0.00043f * ctas * shares) + 0.0039f * ctas + 12.6e-6f * ctas * per + 0.022f * far +
+               more * (1.9f + 0.0066f * CT * v) + 1.5e-4f * (per < kChunk ? per : kChunk) * CT * v + 5e-7f * tiles * CB * CT * v;
+    return 4.5f + cluster * (1.1f + 0.00032f * ctas * shares) + 0.0003f * per + 0.0038f * ctas + 11.4e-6f * ctas * per + 0.032f * far + 1.1f * more;
 }
 
-// What a launch takes, in microseconds: 0.24 per megabyte of rows (whole tiles of columns), and rounds of CTAs; from about
-// 30 MB on 0.155 per megabyte (67 MB 13 us, 134 MB 24, 268 MB 46, 537 MB 90) of a table that the half of L2 on an SM's die
-// holds (of 78 MB 0.24, of 107 MB 0.44), but no less than 3 a round of CTAs.
+// The split of the codebook axis, at least 32 codebooks a CTA.  8 tokens, 384 codebooks of 16 -> 768 with the search: eighths
+// 5.25 us, halves 4.4, whole 5.8; 32 tokens without: whole 5.9, halves 6.5.
+static uint32_t rows_shares(bool search, uint32_t M, uint32_t CB, uint32_t CT, uint32_t v, uint32_t N, int sm_count) {
+    uint32_t best = 1;
+    float least = rows_call_us(search, M, CB, CT, v, N, 1, sm_count);
+    for (uint32_t s = 2; s <= kMaxCluster && s * 32 <= CB; s *= 2) {
+        const float us = rows_call_us(search, M, CB, CT, v, N, s, sm_count);
+        if (us < least) { least = us; best = s; }
+    }
+    return best;
+}
+
+// Without the search, which the other forms need as well.
 float rows_us(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, int sm_count) {
     if (M > 65535) return 3e38f;   // a token is a block of grid.z
-    const float tiles = (float)((N + kTile - 1) / kTile) * (float)M, rounds = tiles * rows_shares(M, CB, N, sm_count) / (4.f * sm_count);
-    const float mb = 1e-6f * tiles * kTile * CB, few = 4.f + 0.24f * mb + (rounds > 1.f ? 1.2f * (rounds - 1.f) : 0.f), many = 6.6f + (0.155f * mb > 3.f * rounds ? 0.155f * mb : 3.f * rounds);
-    return few < many || (uint64_t)CB * CT * N > 40000000 ? few : many;
+    return rows_call_us(false, M, CB, CT, 0, N, rows_shares(false, M, CB, CT, 0, N, sm_count), sm_count);
 }
 
 // The same with the search, for centroid sets that a thread reads in a few batches: a lane's 16 bytes come from a line of
@@ -199,7 +245,7 @@ bool rows_search_ok(uint32_t M, uint32_t CB, uint32_t CT, uint32_t v, uint32_t N
 
 template <int V>
 static cudaError_t run_rows(const LutArgs& a, const int8_t* lut, const SearchArgs& sa, int sm_count, cudaStream_t s) {
-    const uint32_t shares = rows_shares(a.M, a.CB, a.N, sm_count), per = (a.CB + shares - 1) / shares;
+    const uint32_t shares = rows_shares(V > 0, a.M, a.CB, a.CT, V, a.N, sm_count), per = (a.CB + shares - 1) / shares;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(shares, (a.N + kTile - 1) / kTile, a.M);
     cfg.blockDim = dim3(kThreads);
@@ -213,7 +259,7 @@ static cudaError_t run_rows(const LutArgs& a, const int8_t* lut, const SearchArg
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, lut_rows_kernel<V>, lut, a, sa, per);
+    return cudaLaunchKernelEx(&cfg, per > kChunk ? lut_rows_kernel<V, true> : lut_rows_kernel<V, false>, lut, a, sa, per);
 }
 
 cudaError_t launch_rows(const LutArgs& a, const int8_t* lut, int sm_count, cudaStream_t s) {

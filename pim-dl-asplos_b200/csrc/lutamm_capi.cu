@@ -301,9 +301,14 @@ int run_sparse(lutamm_ctx* c, Layer& L, const LutArgs& a, uint32_t n_tile, uint3
 // contraction (or the gather, where that does not fit) takes to go through the whole table.
 bool takes_rows(const lutamm_ctx* c, const Layer& L, uint32_t M, const lutamm_plan& plan) {
     if (plan.variant != LUTAMM_VARIANT_AUTO || plan.gather_cfg || !umma_plan_open(plan)) return false;
-    uint32_t n_tile, split;
-    const float other = umma_supported(L.CB, L.CT, L.N) ? 4.f + sparse_default_plan(M, L.CB, L.CT, L.N, c->sm_count, &n_tile, &split)
-                                                        : gather_us(M, L.CB, L.CT, L.N, plan.gather_cfg, c->sm_count);
+    float other;
+    if (umma_supported(L.CB, L.CT, L.N)) {   // (fitted to the calls that rows_us() was fitted to, to 14 %)
+        uint32_t n_tile, split;
+        const float us = sparse_default_plan(M, L.CB, L.CT, L.N, c->sm_count, &n_tile, &split);
+        other = 6.1f + 0.91f * us + 0.07e-6f * ((float)L.CB * L.CT * L.N) + (split > 1 ? 1.2f : 0.f);
+    } else {
+        other = gather_us(M, L.CB, L.CT, L.N, plan.gather_cfg, c->sm_count);
+    }
     return rows_us(M, L.CB, L.CT, L.N, c->sm_count) < other;
 }
 

@@ -75,7 +75,7 @@ uint32_t sm_count_of(int device) {
 // gather, its narrow tiles of few tokens where wide ones would leave SMs without a CTA.  Laying the table out first, as a
 // context does once per layer, was slower at all of 70 sizes (512 tokens 768 -> 3072: 54 us a call against 25; 8192 tokens
 // 1024 -> 4096: 116 against 92), and is left for tables that are not 16-byte aligned, which the copy engine cannot read:
-// `columns` at a time in what the indices leave of the array.  Over those sizes (1 to 8192 tokens) the choice takes 0.6 %
+// `columns` at a time in what the indices leave of the array.  Over those sizes (1 to 8192 tokens) the choice takes 0.7 %
 // more than the fastest form of each, on average.
 struct TablePlan {
     bool rows;
@@ -83,12 +83,12 @@ struct TablePlan {
 };
 TablePlan plan_table(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, bool aligned, uint32_t sms) {
     const uint32_t cfg = (uint64_t)((M + 63) / 64) * ((N + 255) / 256) < sms ? 4 : 0;
-    const float gather = 2.f + lutamm::gather_us(M, CB, CT, N, cfg, (int)sms), rows = aligned ? lutamm::rows_us(M, CB, CT, N, (int)sms) : 3e38f;
+    const float gather = 2.5f + lutamm::gather_us(M, CB, CT, N, cfg, (int)sms), rows = aligned ? lutamm::rows_us(M, CB, CT, N, (int)sms) : 3e38f;
     float table = 3e38f;
     uint32_t columns = 0, direct = 0;
     if (lutamm::umma_supported(CB, CT, N)) {
         if (aligned) {
-            table = 6.f + lutamm::sparse_canonical_plan(M, CB, CT, N, (int)sms, &direct);
+            table = 6.5f + lutamm::sparse_canonical_plan(M, CB, CT, N, (int)sms, &direct);
         } else {
             const size_t per_column = lutamm::sparse_table_bytes(CB, CT, 1), used = (((size_t)M * CB + 255) / 256) * 256;
             const size_t fit = used < LUTAMM_STATIC_SCRATCH_BYTES ? (LUTAMM_STATIC_SCRATCH_BYTES - used) / per_column : 0;
@@ -100,7 +100,7 @@ TablePlan plan_table(uint32_t M, uint32_t CB, uint32_t CT, uint32_t N, bool alig
                 uint32_t n_tile, split;
                 // a piece: two launches, the layout at 2.5 TB/s, the contraction (measured 768 -> 768 to 512 -> 8192, 1 to 5 pieces)
                 const float contraction = lutamm::sparse_default_plan(M, CB, CT, columns, (int)sms, &n_tile, &split, 0, 1);
-                table = 2.6f + chunks * (3.7f + (float)per_column * columns / 2.5e6f + contraction);
+                table = 3.1f + chunks * (3.7f + (float)per_column * columns / 2.5e6f + contraction);
             }
         }
     }

@@ -109,8 +109,8 @@ def test_who_launches_the_next_pieces_layout_early(fake, early, M, K, N, v, CT):
     assert "".join(ln[-1] for ln in log) == early
 
 
-@pytest.mark.parametrize("tile,M,K,N,v,CT", [(64, 1300, 512, 144, 2, 8), (64, 1000, 1536, 144, 2, 32), (64, 512, 768, 1072, 4, 64), (64, 385, 1024, 2064, 4, 128),
-                                             (128, 385, 512, 4176, 2, 256), (128, 3000, 832, 2064, 4, 16), (128, 512, 768, 3072, 2, 16)])
+@pytest.mark.parametrize("tile,M,K,N,v,CT", [(64, 1300, 512, 144, 2, 8), (64, 1500, 768, 272, 2, 32), (64, 512, 768, 1072, 4, 64), (64, 385, 1024, 2064, 4, 128),
+                                             (128, 385, 512, 4160, 2, 256), (128, 3000, 832, 2064, 4, 16), (128, 512, 768, 3072, 2, 16)])
 def test_an_aligned_table_is_contracted_as_it_is(fake, tile, M, K, N, v, CT):
     """One launch behind the search, no layout of the table; the tile width by how N lies to the sectors."""
     log = _static(fake, M, K, N, v, CT)
@@ -126,3 +126,11 @@ def test_an_unaligned_table_is_not_gathered_by_rows(fake):
 def test_rows_without_a_tensor_core_form(fake, M, K, N, CT, rows):
     """13 and 200 centroids have no contraction; a token is a block of the row gather's grid.z."""
     assert ("lut_rows_kernel" in fake.amm(M, K, N, 2, CT)[-1]) == rows
+
+
+@pytest.mark.parametrize("shares,M,CB,N", [(2, 600, 4096, 16), (2, 600, 4098, 16), (2, 600, 4610, 32), (8, 2, 17000, 16), (1, 260, 511, 144), (4, 4, 1024, 768), (1, 64, 384, 768)])
+def test_shares_of_the_row_gather(fake, shares, M, CB, N):
+    """The split of the codebook axis, and the instance for shares of more than 256 codebooks."""
+    last = fake.amm(M, 2 * CB, N, 2, 13)[-1]
+    assert "lut_rows_kernel" in last and last.split()[-3] == str(shares)
+    assert f"Lb{int((CB + shares - 1) // shares > 256)}E" in last

@@ -14,7 +14,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M,CB,CT,N", [(1, 1, 16, 16), (1, 1000, 16, 144), (2, 77, 13, 272), (3, 2600, 16, 128), (5, 64, 256, 1040), (16, 96, 16, 2000),
-                                       (33, 384, 16, 96), (40, 48, 200, 3056)])
+                                       (33, 384, 16, 96), (40, 48, 200, 3056),
+                                       # shares of 8 and more chunks of 256 codebooks: sums of 16 bits as full as they get
+                                       (600, 4096, 13, 16), (600, 4098, 13, 16), (600, 4610, 13, 32), (2, 17000, 13, 16), (260, 511, 13, 144)])
 def test_rows(ctx, M, CB, CT, N):
     rng = np.random.default_rng(M + CB + CT + N)
     cen = rng.standard_normal((CB, CT, 2), dtype=np.float32)

@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 
 PIECES = [(300, 256, 512, 2, 16), (520, 768, 1616, 2, 16), (1100, 512, 3088, 4, 64), (2300, 2048, 1040, 2, 8), (9, 1024, 2064, 4, 16)]
-WHOLE = [(1300, 512, 144, 2, 8), (1000, 1536, 144, 2, 32), (512, 768, 1072, 4, 64), (385, 1024, 2064, 4, 128), (385, 512, 4176, 2, 256),
+WHOLE = [(1300, 512, 144, 2, 8), (1500, 768, 272, 2, 32), (512, 768, 1072, 4, 64), (385, 1024, 2064, 4, 128), (385, 512, 4160, 2, 256),
          (3000, 832, 2064, 4, 16), (257, 768, 3104, 4, 64)]
 
 
