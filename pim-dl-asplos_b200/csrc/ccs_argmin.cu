@@ -24,6 +24,8 @@
 // 65536 x 4096: 593 -> 460 us, the ALU pipe 53 % and the FMA pipe 45 % busy (they hardly overlap); v = 4, 64
 // centroids, 32768 x 3072: 1267 -> 472 us; v = 10, 16 centroids, 1576 x 2560: 87 -> 14 us (CUDA events around the launch).
 //
+// Calls of many scores take the filter to the tensor cores: ccs_umma.cu.
+//
 // Two mappings:
 //   ccs_reg_kernel  thread <-> codebook, the codebook's centroids in registers, the thread walks a run of
 //                   tokens; activations load as coalesced float2 / float4.  Small centroid sets.
@@ -33,17 +35,12 @@
 //
 // HBM traffic: 4*M*K (activations) + 4*CB*CT*v (centroids) + M*CB (uint8 indices).
 #include "kernels.h"
+#include "ccs_scan.cuh"
 #include "../../include/lutamm.h"
 
 namespace lutamm {
 
 namespace {
-
-constexpr float kEps = 1e-6f;  // (double)diff > 1e-6  <=>  diff > 1e-6f for fp32 diff
-constexpr float kHuge = 1e30f;  // beyond this the filter's own arithmetic could overflow
-
-__host__ __device__ constexpr float margin_factor(int v) { return (float)(8 * v + 16) * 5.9604644775390625e-08f; }
-constexpr float kMarginBase = 0.51e-6f;
 
 // V floats of shared memory
 template <int V>
@@ -86,73 +83,6 @@ template <int kBytes>
 __device__ __forceinline__ void copy_async(uint32_t dst, const void* src) {
     if constexpr (kBytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
     else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(kBytes) : "memory");
-}
-
-__device__ __forceinline__ float min3(float a, float b, float c) {
-    float r;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-
-// smallest of n values, as a tree of three-input minima
-template <int N>
-__device__ __forceinline__ float min_of(const float (&k)[N]) {
-    if constexpr (N == 1) {
-        return k[0];
-    } else if constexpr (N == 2) {
-        return fminf(k[0], k[1]);
-    } else {
-        float t[(N + 2) / 3];
-#pragma unroll
-        for (int i = 0; i < N / 3; ++i) t[i] = min3(k[3 * i], k[3 * i + 1], k[3 * i + 2]);
-        if constexpr (N % 3 == 1) t[N / 3] = k[N - 1];
-        if constexpr (N % 3 == 2) t[N / 3] = fminf(k[N - 2], k[N - 1]);
-        return min_of(t);
-    }
-}
-
-// One bit per key that lies below the threshold: key i at bit i.  The comparison is the sign of key - threshold;
-// NaN and overflow are excluded by the callers' check of the margin.  (Two scalar multiply-adds per key, the first
-// saturating to 0 or 1, need no integer instruction but measured 4 % slower: a scalar multiply-add holds its pipe
-// as long as a packed one.)
-template <int N>
-__device__ __forceinline__ uint32_t below(const float (&k)[N], float thr) {
-    uint32_t mask = 0;
-    const float2 neg = make_float2(-thr, -thr);
-#pragma unroll
-    for (int i = N - 2; i >= 0; i -= 2) {
-        const float2 e = __fadd2_rn(make_float2(k[i], k[i + 1]), neg);
-        mask = __funnelshift_l(__float_as_uint(e.y), mask, 1);
-        mask = __funnelshift_l(__float_as_uint(e.x), mask, 1);
-    }
-    return mask;
-}
-// position of the highest set bit
-__device__ __forceinline__ uint32_t high_bit(uint32_t v) {
-    uint32_t r;
-    asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(v));
-    return r;
-}
-__device__ __forceinline__ uint32_t all_but_lowest(uint32_t mask) { return mask & (mask - 1); }
-
-// The reference's scan.  cent(c, d) returns the NEGATED component, so x - c is x + (-c): the same IEEE result.
-template <int V, typename F>
-__device__ __forceinline__ uint32_t exact_scan(const float (&x)[V], uint32_t CT, F cent) {
-    float mn = 0.f;
-    uint32_t best = 0;
-#pragma unroll 1
-    for (uint32_t c = 0; c < CT; ++c) {
-        float acc = 0.f;
-#pragma unroll
-        for (int d = 0; d < V; ++d) {
-            const float e = __fadd_rn(x[d], cent(c, d));
-            acc = __fadd_rn(acc, __fmul_rn(e, e));
-        }
-        const bool take = c == 0 || __fsub_rn(mn, acc) > kEps;  // false for NaN: keeps the earlier index
-        mn = take ? acc : mn;
-        best = take ? c : best;
-    }
-    return best;
 }
 
 __device__ __forceinline__ size_t tiled_index_offset(uint32_t m, uint32_t cb, uint32_t CB, uint32_t n_stile,
@@ -752,6 +682,7 @@ cudaError_t launch_ccs(const CcsArgs& a, cudaStream_t s, const char** why) {
         *why = "closest-centroid search: need 1 <= num_centroid <= 256 and input_feature_len == num_codebook*sub_vec_len";
         return cudaErrorInvalidValue;
     }
+    if (ccs_umma_takes(a)) return launch_ccs_umma(a, s);
     // vector loads need the row pitch and the base address aligned to the vector width
     const uintptr_t xa = reinterpret_cast<uintptr_t>(a.x);
     const uint32_t vec_bytes = (a.v % 4 == 0) ? 16u : (a.v % 2 == 0) ? 8u : 4u;

@@ -16,8 +16,12 @@ struct CcsArgs {
     uint32_t format;        // LUTAMM_INDEX_*
     uint32_t n_stile, cb_mtile;  // tiled format only
     uint32_t tokens_per_thread;  // 0 = default
+    uint32_t* dev_err;           // null: without the form on the tensor cores, which has waits that may run out
 };
 cudaError_t launch_ccs(const CcsArgs& a, cudaStream_t s, const char** why);
+// ... on the tensor cores, for many tokens (ccs_umma.cu), and the calls it can take
+bool ccs_umma_takes(const CcsArgs& a);
+cudaError_t launch_ccs_umma(const CcsArgs& a, cudaStream_t s);
 bool ccs_reads_tokens_per_thread(uint32_t v, uint32_t CT);
 bool ccs_has_short_form(uint32_t v, uint32_t CT);   // for small calls
 // CTAs of the search in its short form, where their centroids are at most 64 floats a codebook: such CTAs do as well

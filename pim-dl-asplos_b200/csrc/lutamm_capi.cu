@@ -435,6 +435,7 @@ int run_ccs(lutamm_ctx* c, Layer& L, const float* d_x, void* d_idx, uint32_t M, 
     a.n_stile = L.ip.n_stile_size;
     a.cb_mtile = L.ip.cb_mtile_size;
     a.tokens_per_thread = ccs_tokens >= 0 ? (uint32_t)ccs_tokens : L.plan.ccs_tokens;
+    a.dev_err = c->d_err;
     const char* why = nullptr;
     cudaError_t e = launch_ccs(a, c->stream, &why);
     if (e != cudaSuccess) return fail(c, LUTAMM_ECUDA, why ? why : (std::string("search launch: ") + cudaGetErrorString(e)));

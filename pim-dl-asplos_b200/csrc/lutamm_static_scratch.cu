@@ -182,6 +182,7 @@ extern "C" int lutamm_amm_static_scratch(int device, void* cuda_stream, const fl
     ca.x = input; ca.centroid = centroid; ca.idx_out = d_idx;
     ca.M = M; ca.K = K; ca.v = K / CB; ca.CB = CB; ca.CT = CT;
     ca.format = LUTAMM_INDEX_U8_ROWMAJOR;
+    ca.dev_err = d_err;
     cudaError_t e = launch_ccs(ca, s, &why);
     if (e != cudaSuccess) return fail(LUTAMM_ECUDA, why ? why : (std::string("search launch: ") + cudaGetErrorString(e)));
 

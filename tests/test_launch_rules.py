@@ -134,3 +134,18 @@ def test_shares_of_the_row_gather(fake, shares, M, CB, N):
     last = fake.amm(M, 2 * CB, N, 2, 13)[-1]
     assert "lut_rows_kernel" in last and last.split()[-3] == str(shares)
     assert f"Lb{int((CB + shares - 1) // shares > 256)}E" in last
+
+
+@pytest.mark.parametrize("tensor,M,K,v,CT,offset", [
+    (1, 32768, 768, 4, 64, 0), (1, 8192, 768, 4, 64, 0), (1, 8192, 3072, 2, 32, 0), (1, 4096, 3072, 4, 128, 0), (1, 32768, 768, 8, 32, 0),
+    (0, 7812, 768, 4, 64, 0), (0, 32768, 768, 2, 16, 0), (0, 32768, 768, 4, 16, 0), (0, 32768, 2560, 10, 32, 0),   # too little to save
+    (0, 32768, 768, 4, 64, 4),     # activations that are not 16-byte aligned
+    (0, 65536, 8 * 191, 8, 64, 0)])   # codebooks that do not divide among CTAs
+def test_who_searches_on_the_tensor_cores(fake, tensor, M, K, v, CT, offset):
+    at, L = ctypes.c_void_p(fake.base), fake.lib
+    ip, lp = P.make_params(M, K, 64, K // v, CT, 0.01)
+    assert L.lutamm_load_weights(fake.ctx, 0, at, at, at, ctypes.byref(ip), ctypes.byref(lp)) == P.OK
+    fake.log()
+    assert L.lutamm_index_calculation(fake.ctx, 0, ctypes.c_void_p(fake.base + offset), at, ctypes.c_uint32(M), ctypes.c_uint32(P.INDEX_U8_ROWMAJOR)) == P.OK
+    names = fake.log()
+    assert sum("ccs_umma_kernel" in n for n in names) == tensor, names
