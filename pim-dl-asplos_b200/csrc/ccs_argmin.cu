@@ -104,21 +104,24 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // ------------------------------------------------------------------ thread <-> codebook
 constexpr int kRegThreads = 128;
 
-// SHORT: a thread takes one batch of kTok tokens and no more.  The CTA takes 32 codebooks, its four warps take
-// different tokens and share one staged copy of the centroids (a quarter of the bytes), the activations load
-// straight into registers, and the scan runs as it is: a batch small enough for this is bound by a chain of
-// latencies, which the filter would lengthen (0.3 us of a 15 us call).  Otherwise the CTA takes 128 codebooks, one
-// per thread, and every thread a run of tokens.
-template <int V, int CT, bool TILED, int kTok, bool SHORT>
-__global__ void __launch_bounds__(kRegThreads, SHORT ? (CT * V >= 64 ? 6 : 8) : CT * V >= 32 ? 5 : 7)
+// The CTA takes W codebooks, one per thread, and its kRegThreads / W groups of threads different runs of tokens: they share
+// one staged copy of the centroids.
+// SHORT (W = 32): a thread takes one batch of kTok tokens and no more, the activations load straight into registers, and
+// the scan runs as it is: a batch small enough for this is bound by a chain of latencies, which the filter would lengthen
+// (0.3 us of a 15 us call).  Otherwise every thread takes a run of tokens.
+// With 64 numbers a codebook (v = 4 with 16 centroids, v = 2 with 32) registers hold them for two tokens at a time, against
+// ccs_tile_kernel's copies in shared memory: 32768 x 1024, v = 4, 16 centroids 224 -> 182 us with its contraction, 8192 x
+// 256 30 -> 28; 2048 x 512, v = 2, 32 centroids 28.3 -> 25.8.
+template <int V, int CT, bool TILED, int kTok, bool SHORT, int W>
+__global__ void __launch_bounds__(kRegThreads, SHORT ? (CT * V >= 64 ? 6 : 8) : CT * V >= 64 ? (CT == 32 ? 3 : 4) : CT * V >= 32 ? 5 : 7)
 ccs_reg_kernel(const float* __restrict__ x, const float* __restrict__ cent, void* __restrict__ out, uint32_t M,
                uint32_t K, uint32_t CB, uint32_t tokens_per_cta, uint32_t n_stile, uint32_t cb_mtile) {
     pdl_launch();
     // tokens_per_cta is the run of ONE thread: the CTA's run, or each warp's where the warps take different tokens
-    constexpr uint32_t kCbCta = SHORT ? 32u : (uint32_t)kRegThreads, kTokWarps = SHORT ? (uint32_t)kRegThreads / 32u : 1u;
-    const uint32_t col = kTokWarps > 1 ? (threadIdx.x & 31u) : threadIdx.x;   // codebook of the CTA this thread works on
+    constexpr uint32_t kCbCta = W, kTokWarps = (uint32_t)kRegThreads / W;
+    const uint32_t col = kTokWarps > 1 ? threadIdx.x % W : threadIdx.x;   // codebook of the CTA this thread works on
     const uint32_t cb = blockIdx.x * kCbCta + col;
-    const uint32_t m0 = (blockIdx.y * kTokWarps + (kTokWarps > 1 ? threadIdx.x >> 5 : 0u)) * tokens_per_cta;
+    const uint32_t m0 = (blockIdx.y * kTokWarps + (kTokWarps > 1 ? threadIdx.x / W : 0u)) * tokens_per_cta;
     const uint32_t m1 = min(M, m0 + tokens_per_cta);
     const bool active = cb < CB && m0 < M;
 
@@ -567,45 +570,63 @@ uint32_t sm_count() {
     return n;
 }
 
-template <int V, int CT, int kTok, bool SHORT>
+template <int V, int CT, int kTok, bool SHORT, int W>
 uint32_t resident_ctas() {
     static const uint32_t n = [] {
         int r = 0;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, ccs_reg_kernel<V, CT, false, kTok, SHORT>, kRegThreads, 0) == cudaSuccess && r > 0 ? (uint32_t)r : 4u;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, ccs_reg_kernel<V, CT, false, kTok, SHORT, W>, kRegThreads, 0) == cudaSuccess && r > 0 ? (uint32_t)r : 4u;
     }();
     return n * sm_count();
 }
 
-template <int V, int CT, int kTok, bool SHORT>
+template <int V, int CT, int kTok, bool SHORT, int W>
 cudaError_t run_reg_grid(const CcsArgs& a, dim3 grid, uint32_t run, cudaStream_t s) {
-    auto k = a.format == LUTAMM_INDEX_U16_TILED ? ccs_reg_kernel<V, CT, true, kTok, SHORT> : ccs_reg_kernel<V, CT, false, kTok, SHORT>;
+    auto k = a.format == LUTAMM_INDEX_U16_TILED ? ccs_reg_kernel<V, CT, true, kTok, SHORT, W> : ccs_reg_kernel<V, CT, false, kTok, SHORT, W>;
     return launch_dependent(k, grid, dim3(kRegThreads), 0, s, a.x, a.centroid, a.idx_out, a.M, a.K, a.CB, run, a.n_stile, a.cb_mtile);
 }
 
 constexpr uint32_t kTok = 4;   // tokens whose activations a thread loads together: one round trip to memory instead of four
 
+// tokens of a batch in a run: two where the centroids leave no registers, and no shared memory, for four
+constexpr int run_tok(int v, int CT) { return v * CT >= 64 ? 2 : (int)kTok; }
+
 // One batch of kTok tokens per thread, while the GPU holds all those CTAs at once.
 template <int V, int CT>
 bool short_fits(const CcsArgs& a, dim3* grid) {
     *grid = dim3((a.CB + 31) / 32, (a.M + 4 * kTok - 1) / (4 * kTok));
-    return !a.tokens_per_thread && (uint64_t)grid->x * grid->y <= resident_ctas<V, CT, kTok, true>();
+    return !a.tokens_per_thread && (uint64_t)grid->x * grid->y <= resident_ctas<V, CT, kTok, true, 32>();
+}
+
+template <int V, int CT, int W>
+cudaError_t run_reg_width(const CcsArgs& a, cudaStream_t s) {
+    constexpr int kTok = run_tok(V, CT);
+    constexpr uint64_t kGroups = kRegThreads / W;   // of threads that take different runs
+    const uint64_t cb_blocks = (a.CB + W - 1) / W;
+    uint64_t run = a.tokens_per_thread;
+    if (!run) {
+        // Waves of equal runs of up to 2048 tokens, filled as far as whole runs fill them: a last wave that is a third full
+        // costs as much as a full one, and staging the centroids costs a few microseconds per wave (32 tokens' worth).
+        const uint64_t wave = resident_ctas<V, CT, kTok, false, W>(), cap = 2048 * kGroups;
+        const uint64_t fewest = (cb_blocks * ((a.M + cap - 1) / cap) + wave - 1) / wave;
+        uint64_t least = ~0ull;
+        for (uint64_t waves = fewest; waves < fewest + 4; ++waves) {
+            const uint64_t rows = waves * wave / cb_blocks;   // CTAs of a block of codebooks
+            if (!rows) continue;
+            const uint64_t r = (a.M + rows * kGroups - 1) / (rows * kGroups), cost = waves * (r + 32);
+            if (cost < least) { least = cost; run = r; }
+        }
+        if (!run) run = 2048;
+    }
+    const uint32_t tokens = (uint32_t)((run + kTok - 1) / kTok * kTok);
+    return run_reg_grid<V, CT, kTok, false, W>(a, dim3((uint32_t)cb_blocks, (uint32_t)((a.M + tokens * kGroups - 1) / (tokens * kGroups))), tokens, s);
 }
 
 template <int V, int CT>
 cudaError_t run_reg(const CcsArgs& a, cudaStream_t s) {
-    // One wave of equal runs of up to 2048 tokens: a last wave that is a third full costs as much as a full one,
-    // and staging the centroids costs a few microseconds per wave.
-    const uint64_t cb_blocks = (a.CB + kRegThreads - 1) / kRegThreads;
-    uint64_t run = a.tokens_per_thread;
-    if (!run) {
-        const uint64_t wave = resident_ctas<V, CT, kTok, false>();
-        constexpr uint64_t kCap = 2048;
-        const uint64_t ctas_at_cap = cb_blocks * ((a.M + kCap - 1) / kCap), waves = (ctas_at_cap + wave - 1) / wave;
-        run = ((uint64_t)a.M * cb_blocks + waves * wave - 1) / (waves * wave);
-        if (run > kCap) run = kCap;
-    }
-    const uint32_t tokens = (uint32_t)((run + kTok - 1) / kTok * kTok);
-    return run_reg_grid<V, CT, kTok, false>(a, dim3((uint32_t)cb_blocks, (a.M + tokens - 1) / tokens), tokens, s);
+    // Narrow blocks waste fewer threads (32768 x 192, v = 4, 16 centroids: 62 -> 50 us with its contraction) and make shorter
+    // waves (8192 x 384: 33.1 -> 32.5; 1576 x 1024, v = 2: 24.0 -> 22.9).  Wide ones read 1 to 2 KB of a row at once, which
+    // pays where wide rows come from memory throughout (20000 x 1536, v = 4: 176 -> 170; 8192 x 1536: 92.1 against 93.3).
+    return a.M >= 10000 && a.CB >= 768 && a.CB % 128 == 0 ? run_reg_width<V, CT, 128>(a, s) : run_reg_width<V, CT, 32>(a, s);
 }
 
 template <int V, int G, bool ONE, int kTok>
@@ -657,7 +678,7 @@ cudaError_t run_any(const CcsArgs& a, cudaStream_t s) {
 
 // The instances with a short form, and those whose thread walks a run of tokens.
 #define LUTAMM_CCS_SHORT_INSTANCES(X) X(2, 8) X(2, 16) X(2, 32) X(4, 8) X(4, 16) X(8, 8) X(8, 16)
-#define LUTAMM_CCS_RUN_INSTANCES(X) X(2, 8) X(2, 16) X(4, 8)
+#define LUTAMM_CCS_RUN_INSTANCES(X) X(2, 8) X(2, 16) X(4, 8) X(4, 16) X(2, 32)
 
 }  // namespace
 
@@ -689,7 +710,7 @@ cudaError_t launch_ccs(const CcsArgs& a, cudaStream_t s, const char** why) {
     if (xa % vec_bytes == 0) {
         dim3 grid;
 #define LUTAMM_CCS_SHORT(V_, CT_) \
-    if (a.v == V_ && a.CT == CT_ && short_fits<V_, CT_>(a, &grid)) return run_reg_grid<V_, CT_, kTok, true>(a, grid, kTok, s);
+    if (a.v == V_ && a.CT == CT_ && short_fits<V_, CT_>(a, &grid)) return run_reg_grid<V_, CT_, kTok, true, 32>(a, grid, kTok, s);
         LUTAMM_CCS_SHORT_INSTANCES(LUTAMM_CCS_SHORT)
 #undef LUTAMM_CCS_SHORT
 #define LUTAMM_CCS_REG(V_, CT_) \

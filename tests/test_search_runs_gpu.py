@@ -1,0 +1,38 @@
+"""The search whose threads walk runs of tokens: codebooks that do not fill a CTA, runs that end within a batch and within a
+CTA's group of threads, both widths of a CTA.  Indices are compared exactly."""
+import numpy as np
+import pytest
+
+import oracle
+import pim_dl_asplos_b200 as P  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("data", ["normal", "ties", "nonfinite"])
+@pytest.mark.parametrize("tokens", [0, 6])
+@pytest.mark.parametrize("v,CT,CB,M", [(4, 16, 33, 7201), (4, 16, 1, 300007), (4, 16, 31, 15001), (4, 16, 768, 10001), (2, 32, 45, 7303), (2, 32, 768, 3001),
+                                       (2, 16, 95, 7777), (2, 8, 65, 7301), (4, 8, 130, 4099)])
+def test_indices_equal_the_scan(ctx, v, CT, CB, M, tokens, data):
+    import torch
+    rng = np.random.default_rng(v * 1000 + CT)
+    x = rng.standard_normal((M, CB * v), dtype=np.float32)
+    cen = rng.standard_normal((CB, CT, v), dtype=np.float32)
+    if data == "ties":
+        x, cen = np.round(x * 2) / 2, np.round(cen * 2) / 2
+    elif data == "nonfinite":
+        x[rng.random(x.shape) < 0.002] = np.nan
+        cen[rng.random(cen.shape) < 0.002] = np.inf
+    x, cen = np.ascontiguousarray(x, np.float32), np.ascontiguousarray(cen, np.float32)
+    ctx.load_weights(81, cen, np.zeros((CB, CT, 16), np.int8), np.zeros(16, np.float32), 1.0)
+    ctx.set_plan(81, ccs_tokens=tokens)
+    with np.errstate(all="ignore"):
+        want = oracle.index_calculation(x, cen).astype(np.uint8)
+    idx = torch.full((M + 1, CB), 255, dtype=torch.uint8, device="cuda")
+    xd = torch.from_numpy(x).cuda()
+    torch.cuda.synchronize()
+    ctx.index_calculation(81, xd, idx[:M])
+    got = idx.cpu().numpy()
+    assert np.array_equal(got[:M], want)
+    assert (got[M] == 255).all()
+    ctx.unload_weights(81)
