@@ -359,9 +359,17 @@ ccs_tile_kernel(const float* __restrict__ x, const float* __restrict__ cent, voi
         constexpr uint32_t kW = kCbs * V;
         const uint32_t w = cbs * V;
         if (V % 2 == 0 && kW % 4 == 0 && copy16) {
-            for (uint32_t i = threadIdx.x; i < rows * (kW / 4); i += kTileThreads) {
-                const uint32_t r = i / (kW / 4), q = i % (kW / 4);
-                if (4 * q < w) copy_async<16>(dst + (r * kPitch + 4 * q) * 4, xg + (size_t)(m_base + r) * K + 4 * q);
+            // A thread keeps its column of 16 bytes and walks down the rows, so that a copy costs two additions.  With a
+            // division per copy a warp and codebook took 298 instructions at v = 10, 16 centroids; 250 like this: 8192 x 1024
+            // 137 -> 122 us with its contraction (v = 20 138 -> 123, v = 8 131 -> 125).
+            constexpr uint32_t kQ = kW / 4, kRows = kTileThreads / kQ;   // rows of one turn
+            const uint32_t q = threadIdx.x % kQ;
+            uint32_t r = threadIdx.x / kQ, to = dst + (r * kPitch + 4 * q) * 4;
+            if (r < kRows && 4 * q < w) {
+                const float* from = xg + (size_t)(m_base + r) * K + 4 * q;
+                const size_t step = (size_t)kRows * K;
+#pragma unroll 4
+                for (; r < rows; r += kRows, to += kRows * kPitch * 4, from += step) copy_async<16>(to, from);
             }
         } else {
             for (uint32_t i = threadIdx.x; i < rows * kW; i += kTileThreads) {
