@@ -34,7 +34,9 @@ __device__ __forceinline__ float2 plus(float2 a, float2 b) { return make_float2(
 // store per centroid, so a warp writes 128 contiguous bytes per centroid row).
 // V > 0: compile-time sub-vector length, the thread's weight slice lives in registers.
 // V == 0: run-time length, the slice is re-read (L1 resident) for every kTogether centroids; one at a time the load was
-// most of what a sum took (4160 x 8368, v = 20: 330 -> 191 us a call).
+// most of what a sum took (4160 x 8368, v = 20: 330 -> 191 us a call).  In registers a call is 1.2 to 1.7 times as fast, at 32
+// too, where they leave room for one block an SM: 5120 x 16384, 16 centroids, v = 10 398 -> 241 us, v = 20 359 -> 246, v = 32
+// 352 -> 297; 640 x 2560 34 -> 28, 39 -> 29, 49 -> 31.
 template <int V, bool kWrite>
 __global__ void __launch_bounds__(kThreads)
 lut_build_kernel(const float* __restrict__ centroid, const float* __restrict__ weight, int8_t* __restrict__ lut,
@@ -220,7 +222,10 @@ cudaError_t launch_lut_build(const LutBuildArgs& a, cudaStream_t s, const char**
         case 2: e = launch_both<2>(a, grid, smem, s); break;
         case 4: e = launch_both<4>(a, grid, smem, s); break;
         case 8: e = launch_both<8>(a, grid, smem, s); break;
+        case 10: e = launch_both<10>(a, grid, smem, s); break;
         case 16: e = launch_both<16>(a, grid, smem, s); break;
+        case 20: e = launch_both<20>(a, grid, smem, s); break;
+        case 32: e = launch_both<32>(a, grid, smem, s); break;
         default: e = launch_both<0>(a, grid, smem, s); break;
     }
     return e == cudaSuccess ? cudaGetLastError() : e;
