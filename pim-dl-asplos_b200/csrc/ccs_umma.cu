@@ -514,15 +514,11 @@ uint32_t sm_count() {
     return n;
 }
 
+// Tiles of a CTA: runs of equal length in up to four waves, one more tile standing for what a CTA spends on its centroids.
+// `used`: the part of that time that the GPU's CTAs spend on tokens.
 template <int V, int CT, int CC>
-cudaError_t run(const CcsArgs& a, cudaStream_t s) {
-    using F = Form<V, CT, CC>;
-    auto k = ccs_umma_kernel<V, CT, CC>;
-    static SmemOptIn memo;
-    cudaError_t e = allow_smem(memo, k, (int)F::kSmem);
-    if (e != cudaSuccess) return e;
-    constexpr uint32_t kFit = (uint32_t)(227 * 1024 / (F::kSmem + 1024 + 256)), kPerSm = kFit < 4 ? kFit : 4;   // (1 KB a CTA is the system's)
-    // Runs of equal length; one more tile stands for what a CTA spends on its centroids.
+uint32_t plan_run(const CcsArgs& a, float* used) {
+    constexpr uint32_t kFit = (uint32_t)(227 * 1024 / (Form<V, CT, CC>::kSmem + 1024 + 256)), kPerSm = kFit < 4 ? kFit : 4;   // (1 KB a CTA is the system's)
     const uint32_t groups = a.CB / CC, tiles = (a.M + kThreads - 1) / kThreads;
     const uint64_t resident = (uint64_t)kPerSm * sm_count();
     uint32_t run = tiles;
@@ -533,6 +529,19 @@ cudaError_t run(const CcsArgs& a, cudaStream_t s) {
         const uint64_t ctas = (uint64_t)groups * ((tiles + r - 1) / r), cost = (ctas + resident - 1) / resident * (r + 1);
         if (cost < least) { least = cost; run = r; }
     }
+    *used = (float)groups * (float)a.M / (float)kThreads / ((float)resident * (float)least);
+    return run;
+}
+
+template <int V, int CT, int CC>
+cudaError_t run(const CcsArgs& a, cudaStream_t s) {
+    using F = Form<V, CT, CC>;
+    auto k = ccs_umma_kernel<V, CT, CC>;
+    static SmemOptIn memo;
+    cudaError_t e = allow_smem(memo, k, (int)F::kSmem);
+    if (e != cudaSuccess) return e;
+    float used;
+    const uint32_t run = plan_run<V, CT, CC>(a, &used), groups = a.CB / CC, tiles = (a.M + kThreads - 1) / kThreads;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(groups, (tiles + run - 1) / run);
     if (cfg.gridDim.y > 65535u) return cudaErrorInvalidValue;
@@ -551,6 +560,9 @@ cudaError_t run(const CcsArgs& a, cudaStream_t s) {
 #define LUTAMM_CCS_UMMA_INSTANCES(X) X(2, 32, 8) X(4, 32, 4) X(4, 64, 4) X(4, 128, 4) X(8, 32, 2) X(8, 64, 2)
 // Below about this many scores its prologue (tensor memory, the centroids) costs more than it saves: 100 M 1.01 to 1.2
 // times as fast, 50 M 0.95 to 1.06, 25 M 0.8 to 1.0, over these instances and 48 to 1536 codebooks.
+// The same where few tokens of very many codebooks leave its waves empty: 128 centroids, v = 4, 390 x 2560 0.33 of the time
+// used 0.86, 768 x 2560 0.54 used 0.93, 1400 x 2560 0.59 used 1.01, 512 x 2048 0.69 used 1.05, 1400 x 2048 0.79 used 1.18.
+constexpr float kLeastUsed = 0.6f;
 constexpr uint64_t kFewestScores = 96000000;
 
 }  // namespace
@@ -559,7 +571,11 @@ bool ccs_umma_takes(const CcsArgs& a) {
     if (!a.dev_err || a.format != LUTAMM_INDEX_U8_ROWMAJOR || a.tokens_per_thread) return false;
     if ((uint64_t)a.M * a.CB * a.CT < kFewestScores || reinterpret_cast<uintptr_t>(a.x) % 16 || a.K % 4) return false;
 #define LUTAMM_CCS_UMMA(V_, CT_, CC_) \
-    if (a.v == V_ && a.CT == CT_) return a.CB % CC_ == 0 && reinterpret_cast<uintptr_t>(a.idx_out) % CC_ == 0;
+    if (a.v == V_ && a.CT == CT_) {                                                                                     \
+        float used = 0.f;                                                                                               \
+        if (a.CB % CC_ == 0 && reinterpret_cast<uintptr_t>(a.idx_out) % CC_ == 0) plan_run<V_, CT_, CC_>(a, &used);      \
+        return used >= kLeastUsed;                                                                                      \
+    }
     LUTAMM_CCS_UMMA_INSTANCES(LUTAMM_CCS_UMMA)
 #undef LUTAMM_CCS_UMMA
     return false;

@@ -57,3 +57,18 @@ def test_the_polling_warp_meets_behind_the_fence():
     src = _source("lut_sparse_umma.cu")
     told = src.index("__shfl_sync(0xffffffffu, go, 0);")
     assert "__syncwarp();" in src[told:src.index("} else {", told)]
+
+
+def test_the_search_hands_its_columns_over_in_order():
+    """The warp that reads last has the next columns computed into those all four have read: its lanes' reads, and what they
+    wrote for the next tile, are ordered before the count by lane 0, and the count before the instructions of whichever lane
+    issues them.  The kernel that wants all tensor memory is let in behind the allocation."""
+    src = _source("ccs_umma.cu")
+    release = src[src.index("auto release = "):src.index("auto settle_all = ")]
+    assert re.search(r"tc_fence_before_sync\(\);\s*__syncwarp\(\);.*atom\.acq_rel\.cta.*__shfl_sync\(.*__syncwarp\(\);.*issue\(", release, re.S)
+    issue = src[src.index("auto issue = "):src.index("auto release = ")]
+    assert issue.index("tc_fence_after_sync();") < issue.index("elect_one()")
+    convert = src[src.index("auto convert = "):src.index("auto issue = ")]
+    assert convert.rstrip().endswith("fence_proxy_async_smem();\n    };")
+    kernel = src[src.index("ccs_umma_kernel("):]
+    assert kernel.index("tmem_alloc(") < kernel.index("__syncthreads();") < kernel.index("pdl_launch_dependents();")
