@@ -81,7 +81,10 @@ __device__ __forceinline__ void load_global(const float* __restrict__ p, float (
 
 template <int kBytes>
 __device__ __forceinline__ void copy_async(uint32_t dst, const void* src) {
-    if constexpr (kBytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    if constexpr (kBytes == 32) {
+        copy_async<16>(dst, src);
+        copy_async<16>(dst + 16, static_cast<const char*>(src) + 16);
+    } else if constexpr (kBytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
     else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(kBytes) : "memory");
 }
 
@@ -109,9 +112,10 @@ constexpr int kRegThreads = 128;
 // SHORT (W = 32): a thread takes one batch of kTok tokens and no more, the activations load straight into registers, and
 // the scan runs as it is: a batch small enough for this is bound by a chain of latencies, which the filter would lengthen
 // (0.3 us of a 15 us call).  Otherwise every thread takes a run of tokens.
-// With 64 numbers a codebook (v = 4 with 16 centroids, v = 2 with 32) registers hold them for two tokens at a time, against
+// With 64 numbers a codebook (v = 4 with 16 centroids, v = 2 with 32, v = 8 with 8) registers hold them for two tokens at a time, against
 // ccs_tile_kernel's copies in shared memory: 32768 x 1024, v = 4, 16 centroids 224 -> 182 us with its contraction, 8192 x
-// 256 30 -> 28; 2048 x 512, v = 2, 32 centroids 28.3 -> 25.8.
+// 256 30 -> 28; 2048 x 512, v = 2, 32 centroids 28.3 -> 25.8; 8192 x 1280, v = 8, 8 centroids
+// 95 -> 72, 8192 x 128 18.1 -> 15.2.
 template <int V, int CT, bool TILED, int kTok, bool SHORT, int W>
 __global__ void __launch_bounds__(kRegThreads, SHORT ? (CT * V >= 64 ? 6 : 8) : CT * V >= 64 ? (CT == 32 ? 3 : 4) : CT * V >= 32 ? 5 : 7)
 ccs_reg_kernel(const float* __restrict__ x, const float* __restrict__ cent, void* __restrict__ out, uint32_t M,
@@ -634,7 +638,9 @@ cudaError_t run_reg(const CcsArgs& a, cudaStream_t s) {
     // Narrow blocks waste fewer threads (32768 x 192, v = 4, 16 centroids: 62 -> 50 us with its contraction) and make shorter
     // waves (8192 x 384: 33.1 -> 32.5; 1576 x 1024, v = 2: 24.0 -> 22.9).  Wide ones read 1 to 2 KB of a row at once, which
     // pays where wide rows come from memory throughout (20000 x 1536, v = 4: 176 -> 170; 8192 x 1536: 92.1 against 93.3).
-    return a.M >= 10000 && a.CB >= 768 && a.CB % 128 == 0 ? run_reg_width<V, CT, 128>(a, s) : run_reg_width<V, CT, 32>(a, s);
+    // (at v = 8 a narrow block reads 1 KB, and the wide one's centroids and batches are more shared memory than there is)
+    if constexpr (V == 8) return run_reg_width<V, CT, 32>(a, s);
+    else return a.M >= 10000 && a.CB >= 768 && a.CB % 128 == 0 ? run_reg_width<V, CT, 128>(a, s) : run_reg_width<V, CT, 32>(a, s);
 }
 
 template <int V, int G, bool ONE, int kTok>
@@ -686,7 +692,7 @@ cudaError_t run_any(const CcsArgs& a, cudaStream_t s) {
 
 // The instances with a short form, and those whose thread walks a run of tokens.
 #define LUTAMM_CCS_SHORT_INSTANCES(X) X(2, 8) X(2, 16) X(2, 32) X(4, 8) X(4, 16) X(8, 8) X(8, 16)
-#define LUTAMM_CCS_RUN_INSTANCES(X) X(2, 8) X(2, 16) X(4, 8) X(4, 16) X(2, 32)
+#define LUTAMM_CCS_RUN_INSTANCES(X) X(2, 8) X(2, 16) X(4, 8) X(4, 16) X(2, 32) X(8, 8)
 
 }  // namespace
 

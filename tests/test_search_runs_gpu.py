@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("data", ["normal", "ties", "nonfinite"])
 @pytest.mark.parametrize("tokens", [0, 6])
 @pytest.mark.parametrize("v,CT,CB,M", [(4, 16, 33, 7201), (4, 16, 1, 300007), (4, 16, 31, 15001), (4, 16, 768, 10001), (2, 32, 45, 7303), (2, 32, 768, 3001),
-                                       (2, 16, 95, 7777), (2, 8, 65, 7301), (4, 8, 130, 4099)])
+                                       (2, 16, 95, 7777), (2, 8, 65, 7301), (4, 8, 130, 4099), (8, 8, 33, 7201), (8, 8, 96, 12001)])
 def test_indices_equal_the_scan(ctx, v, CT, CB, M, tokens, data):
     import torch
     rng = np.random.default_rng(v * 1000 + CT)
