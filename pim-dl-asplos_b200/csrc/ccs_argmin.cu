@@ -37,6 +37,7 @@
 #include "kernels.h"
 #include "ccs_scan.cuh"
 #include "../../include/lutamm.h"
+#include <algorithm>
 
 namespace lutamm {
 
@@ -597,6 +598,7 @@ cudaError_t run_reg_grid(const CcsArgs& a, dim3 grid, uint32_t run, cudaStream_t
     return launch_dependent(k, grid, dim3(kRegThreads), 0, s, a.x, a.centroid, a.idx_out, a.M, a.K, a.CB, run, a.n_stile, a.cb_mtile);
 }
 
+constexpr uint64_t kMostGridY = 65535;
 constexpr uint32_t kTok = 4;   // tokens whose activations a thread loads together: one round trip to memory instead of four
 
 // tokens of a batch in a run: two where the centroids leave no registers, and no shared memory, for four
@@ -629,6 +631,7 @@ cudaError_t run_reg_width(const CcsArgs& a, cudaStream_t s) {
         }
         if (!run) run = 2048;
     }
+    run = std::max(run, (a.M + kMostGridY * kGroups - 1) / (kMostGridY * kGroups));   // what a plan names, as far as the grid holds it
     const uint32_t tokens = (uint32_t)((run + kTok - 1) / kTok * kTok);
     return run_reg_grid<V, CT, kTok, false, W>(a, dim3((uint32_t)cb_blocks, (uint32_t)((a.M + tokens * kGroups - 1) / (tokens * kGroups))), tokens, s);
 }

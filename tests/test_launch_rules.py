@@ -150,3 +150,18 @@ def test_who_searches_on_the_tensor_cores(fake, tensor, M, K, v, CT, offset):
     assert L.lutamm_index_calculation(fake.ctx, 0, ctypes.c_void_p(fake.base + offset), at, ctypes.c_uint32(M), ctypes.c_uint32(P.INDEX_U8_ROWMAJOR)) == P.OK
     names = fake.log()
     assert sum("ccs_umma_kernel" in n for n in names) == tensor, names
+
+
+@pytest.mark.parametrize("v,CT", [(2, 8), (2, 16), (4, 8), (4, 16), (2, 32), (8, 8)])
+@pytest.mark.parametrize("M,tokens", [(16 * 65535 + 1, 4), (8 * 65535 + 1, 1), (4 * 65535 * 64 + 1, 64), (1 << 20, 1)])
+def test_a_planned_run_of_the_search_fits_the_grid(fake, v, CT, M, tokens):
+    """More tokens than 65535 CTAs of the planned run walk: the run grows, as the tuner tries 4 tokens at any number."""
+    at, L = ctypes.c_void_p(fake.base), fake.lib
+    ip, lp = P.make_params(M, 8 * v, 64, 8, CT, 0.01)
+    assert L.lutamm_load_weights(fake.ctx, 0, at, at, at, ctypes.byref(ip), ctypes.byref(lp)) == P.OK
+    assert L.lutamm_set_plan(fake.ctx, 0, ctypes.byref(P.Plan(ccs_tokens=tokens))) == P.OK
+    fake.log()
+    assert L.lutamm_index_calculation(fake.ctx, 0, at, at, ctypes.c_uint32(M), ctypes.c_uint32(P.INDEX_U8_ROWMAJOR)) == P.OK
+    (line,) = fake.log()
+    x, y, z = map(int, line.split()[-3:])
+    assert "ccs_reg_kernel" in line and x * z == 1 and 1 <= y <= 65535
