@@ -631,7 +631,8 @@ cudaError_t run_reg_width(const CcsArgs& a, cudaStream_t s) {
         }
         if (!run) run = 2048;
     }
-    run = std::max(run, (a.M + kMostGridY * kGroups - 1) / (kMostGridY * kGroups));   // what a plan names, as far as the grid holds it
+    // what a plan names, as far as the grid holds it and there are tokens (a run of 2^32 - 1 rounds up to none)
+    run = std::clamp(run, (a.M + kMostGridY * kGroups - 1) / (kMostGridY * kGroups), (a.M + kGroups - 1) / kGroups);
     const uint32_t tokens = (uint32_t)((run + kTok - 1) / kTok * kTok);
     return run_reg_grid<V, CT, kTok, false, W>(a, dim3((uint32_t)cb_blocks, (uint32_t)((a.M + tokens * kGroups - 1) / (tokens * kGroups))), tokens, s);
 }

@@ -165,3 +165,18 @@ def test_a_planned_run_of_the_search_fits_the_grid(fake, v, CT, M, tokens):
     (line,) = fake.log()
     x, y, z = map(int, line.split()[-3:])
     assert "ccs_reg_kernel" in line and x * z == 1 and 1 <= y <= 65535
+
+
+@pytest.mark.parametrize("v,CT", [(2, 16), (8, 8)])
+@pytest.mark.parametrize("M", [1, 7, 4099])
+@pytest.mark.parametrize("tokens", [0xFFFFFFFF, 0xFFFFFFFD, 0x80000001, 5000])
+def test_a_planned_run_beyond_the_tokens(fake, v, CT, M, tokens):
+    """Any number is a plan: rounded up to whole batches it stays one, and one row of CTAs takes all tokens."""
+    at, L = ctypes.c_void_p(fake.base), fake.lib
+    ip, lp = P.make_params(M, 8 * v, 64, 8, CT, 0.01)
+    assert L.lutamm_load_weights(fake.ctx, 0, at, at, at, ctypes.byref(ip), ctypes.byref(lp)) == P.OK
+    assert L.lutamm_set_plan(fake.ctx, 0, ctypes.byref(P.Plan(ccs_tokens=tokens))) == P.OK
+    fake.log()
+    assert L.lutamm_index_calculation(fake.ctx, 0, at, at, ctypes.c_uint32(M), ctypes.c_uint32(P.INDEX_U8_ROWMAJOR)) == P.OK
+    (line,) = fake.log()
+    assert "ccs_reg_kernel" in line and line.split()[-2] == "1"
