@@ -377,7 +377,7 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
     __syncthreads();
     if (t0 < t1 && warp == 0) issue(0, 0);
     if (t0 + 1 < t1) fetch(t0 + 1);
-    for (uint32_t tile = t0; tile < t1 && ok; ++tile) {
+    for (uint32_t tile = t0; tile < t1; ++tile) {
         const uint32_t side = (tile - t0) & 1u;
         const bool more = tile + 1 < t1;
         const float* norm = s_norm + side * F::kTile;
@@ -416,10 +416,10 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
         };
 #pragma unroll 1
         for (uint32_t w = 0; w < F::kWindows; ++w) {
-            ok = ok && mbar_wait(bar, phase, abort_word);
+            ok = mbar_wait_warp(bar, phase, abort_word);
+            if (!ok) break;   // a warp that leaves issues nothing more, and the others' waits see the abort word
             phase ^= 1u;
             tc_fence_after_sync();
-            __syncwarp();
             float least[F::kParts];
             uint32_t cand[F::kCbWindow][F::kWords], several = (unsound >> (w * F::kCbWindow)) & ((1u << F::kCbWindow) - 1);
             decltype(word) got = 0;
@@ -487,6 +487,7 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
                 }
             }
         }
+        if (!ok) break;
         if (m < M) {
             uint8_t* o = out + (size_t)m * CB + cb0;
             if constexpr (CC == 8) *reinterpret_cast<uint2*>(o) = make_uint2((uint32_t)word, (uint32_t)((uint64_t)word >> 32));
@@ -498,11 +499,18 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
     if (queued && ok) settle_all(false, 0);
     tc_fence_before_sync();
     __syncthreads();
+    if (s_abort) {
+        if (tid == 0) {   // instructions that may still be in flight have a bounded time to end before their memory is handed back
+            const long long start = clock64();
+            while (clock64() - start < 200000) {}
+            report_error(dev_err, 5u);
+        }
+        __syncthreads();
+    }
     if (warp == 0) {
         tc_fence_after_sync();
         tmem_dealloc(tmem, kTmemColumns);
     }
-    if (tid == 0 && s_abort) report_error(dev_err, 5u);
 }
 
 uint32_t sm_count() {

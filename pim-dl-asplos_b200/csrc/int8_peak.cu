@@ -107,20 +107,25 @@ cudaError_t launch_spread_input(const float* centroid, float* x, uint32_t M, uin
 }
 
 // ---- self-test of the way out after a wait that runs out -----------------------------------------
-// One CTA sets up what the tcgen05 LUT kernel sets up (tensor memory, an mbarrier), then one thread waits
-// - with the library's own bounded wait, limited to `polls` probes - on a barrier nobody ever arrives at.
-// The wait gives up, the abort word is set, the CTA goes through the same tear-down as the LUT kernel
+// One CTA sets up what the tcgen05 LUT kernel sets up (tensor memory, mbarriers), then one warp waits - with the
+// library's own bounded wait, limited to `polls` probes - its even lanes on a barrier nobody ever arrives at, its odd lanes
+// on one that has completed.  The wait gives up with one answer for the warp (another error code says that it has not),
+// the abort word is set, the CTA goes through the same tear-down as the LUT kernel
 // (report in the device error word, everybody meets, tensor memory is freed) and returns.  Nothing traps and
 // nothing spins on: the host reads the error word and the context stays usable.
 namespace {
 __global__ void __launch_bounds__(128, 1) stalled_wait_kernel(uint32_t polls, uint32_t* dev_err) {
     __shared__ uint32_t s_tmem;
     __shared__ uint32_t s_abort;
-    __shared__ uint64_t s_bar;
+    __shared__ uint32_t s_parted;
+    __shared__ uint64_t s_bar[2];
     if (threadIdx.x == 0) {
         s_abort = 0;
-        mbar_init(smem_u32(&s_bar), 1);
+        s_parted = 0;
+        mbar_init(smem_u32(&s_bar[0]), 1);
+        mbar_init(smem_u32(&s_bar[1]), 1);
         fence_barrier_init();
+        mbar_arrive(smem_u32(&s_bar[1]));   // its phase 0 completes
     }
     __syncthreads();
     if (threadIdx.x < 32) { tmem_alloc(smem_u32(&s_tmem), 32); tmem_relinquish(); }
@@ -128,9 +133,12 @@ __global__ void __launch_bounds__(128, 1) stalled_wait_kernel(uint32_t polls, ui
     __syncthreads();
     tc_fence_after_sync();
     volatile uint32_t* abort_word = &s_abort;
-    if (threadIdx.x == 32) (void)mbar_wait_limited(smem_u32(&s_bar), 0, abort_word, polls);   // phase 0 never completes
+    if (threadIdx.x >= 32 && threadIdx.x < 64) {
+        const bool all = mbar_wait_warp_limited(smem_u32(&s_bar[threadIdx.x & 1u]), 0, abort_word, polls);   // phase 0 of the first never completes
+        if (all) s_parted = 1;   // any lane that takes its own answer for the warp's
+    }
     __syncthreads();
-    if (*abort_word && threadIdx.x == 0) report_error(dev_err, 4u);
+    if (*abort_word && threadIdx.x == 0) report_error(dev_err, s_parted ? 6u : 4u);
     __syncthreads();
     if (threadIdx.x < 32) { tc_fence_after_sync(); tmem_dealloc(s_tmem, 32); }
 }

@@ -88,6 +88,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return mbar_wait_limited<kSleepNs>(bar, parity, abort_word, kWaitLimit);
 }
 
+// A whole warp's wait, with one answer: full-mask instructions may follow, and lanes that disagreed would wait for one
+// another there without end.
+__device__ __forceinline__ bool mbar_wait_warp_limited(uint32_t bar, uint32_t parity, volatile uint32_t* abort_word, uint32_t limit) {
+    return __all_sync(0xFFFFFFFFu, mbar_wait_limited(bar, parity, abort_word, limit)) != 0;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_word) {
+    return mbar_wait_warp_limited(bar, parity, abort_word, kWaitLimit);
+}
+
 // The error word is host memory mapped into the device: a kernel touches it only when it gives up.
 __device__ __forceinline__ void report_error(uint32_t* word, uint32_t code) {
     *reinterpret_cast<volatile uint32_t*>(word) = code;

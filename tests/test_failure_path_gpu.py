@@ -22,6 +22,7 @@ def test_a_wait_that_runs_out_reports_and_leaves_the_context_usable(ctx):
     for _ in range(2):
         rc = ctx._L.lutamm_selftest_bounded_wait(ctx._h, 4096)
         assert rc == P.EDEVICE
+        assert b"code 4" in ctx._L.lutamm_last_error(ctx._h)     # 6: the lanes of the waiting warp parted
         assert b"bounded wait" in ctx._L.lutamm_last_error(ctx._h)
         y[:] = 0
         ctx.amm_host(30, c.x, y)                                 # the very next ordinary call

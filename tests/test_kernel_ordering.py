@@ -72,3 +72,16 @@ def test_the_search_hands_its_columns_over_in_order():
     assert convert.rstrip().endswith("fence_proxy_async_smem();\n    };")
     kernel = src[src.index("ccs_umma_kernel("):]
     assert kernel.index("tmem_alloc(") < kernel.index("__syncthreads();") < kernel.index("pdl_launch_dependents();")
+
+
+def test_the_searching_warps_leave_together():
+    """Full-mask instructions follow each wait of the search, so its answer is one for the warp, and a warp whose wait has
+    run out does nothing more; the columns are handed back when what is in flight has had time to end."""
+    src = _source("ccs_umma.cu")
+    assert not re.search(r"\bmbar_(try_)?wait(_limited)?\b", src)
+    waits = list(re.finditer(r"mbar_wait_warp\([^;]*;", src))
+    assert waits
+    for w in waits:
+        assert re.match(r"\s*if \(!ok\) break;", src[w.end():])
+    down = src[src.rindex("__syncthreads();", 0, src.index("tmem_dealloc(")) - 400:src.index("tmem_dealloc(")]
+    assert down.index("if (s_abort)") < down.index("clock64()") < down.index("report_error(")
