@@ -242,19 +242,15 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
             for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++t) {
                 const Item it = decode_item(p, item, N_TILE);
                 const uint32_t ab = t & 1, aph = (t >> 1) & 1;
-                ok = mbar_wait(acc_empty0 + 8 * ab, aph ^ 1, s_abort);  // epilogue drained and cleared this buffer
+                ok = mbar_wait_warp(acc_empty0 + 8 * ab, aph ^ 1, s_abort);  // epilogue drained and cleared this buffer
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + ab * N_TILE;
                 for (uint32_t i = (x0 + me) & 1u; i < it.nslab; i += 2) {
                     const uint32_t x = x0 + i;
                     a_slot(x, k, pa);
-                    if (!ready) {
-                        ok = mbar_wait(b_full0 + 8 * j, pb, s_abort) && mbar_wait(a_full0 + 8 * k, pa, s_abort);
-                        if (!ok) break;
-                    }
-                    ok = mbar_wait(turn0 + 8 * me, ((x >> 1) & 1u) ^ (me == 0 ? 1u : 0u), s_abort);   // slab 0 has its turn
-                    if (!ok) break;
+                    if (!ready) ok = mbar_wait(b_full0 + 8 * j, pb, s_abort) && mbar_wait(a_full0 + 8 * k, pa, s_abort);
+                    ok = ok && mbar_wait(turn0 + 8 * me, ((x >> 1) & 1u) ^ (me == 0 ? 1u : 0u), s_abort);   // slab 0 has its turn
                     uint32_t j2 = j + 2, pb2 = pb;
                     if (j2 >= SB) { j2 -= SB; pb2 ^= 1; }
                     uint32_t k2, pa2;
@@ -281,7 +277,8 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
                         umma_commit(a_empty0 + 8 * k);  // each slot is free once these MMAs have read it
                         umma_commit(b_empty0 + 8 * j);
                     }
-                    __syncwarp();
+                    ok = __all_sync(0xFFFFFFFFu, ok);   // behind the instructions: see ptx.cuh
+                    if (!ok) break;
                     j = j2; pb = pb2;
                     ready = next_ready;
                 }
@@ -388,8 +385,7 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
                     // The row is in registers before the slot is waited for: what follows the wait is on
                     // the slot's turn-around path.  The whole warp polls (one broadcast access), so it
                     // stays converged.
-                    ok = ok && mbar_wait(a_empty0 + 8 * k, pa ^ 1, s_abort);
-                    if (!ok) continue;
+                    ok = mbar_wait(a_empty0 + 8 * k, pa ^ 1, s_abort) && ok;
                     if constexpr (A_TMEM) {
                         tc_fence_after_sync();
                         // the row goes to this warp's lane quadrant of tensor memory, K bytes in column order
@@ -421,6 +417,7 @@ lut_onehot_umma_kernel(const __grid_constant__ CUtensorMap lut_t_map, const Umma
                             mbar_arrive(a_full0 + 8 * (x - div_magic(x, sa_magic) * SA));
                         }
                 }
+                ok = __all_sync(0xFFFFFFFFu, ok);
             }
             ga += it.nslab;
             qb += (it.nslab + kBatch - 1) / kBatch;

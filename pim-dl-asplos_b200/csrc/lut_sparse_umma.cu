@@ -220,7 +220,7 @@ __device__ __forceinline__ bool split_finish(const SparseParams& p, const Sparse
         go = __shfl_sync(0xffffffffu, go, 0);
         __syncwarp();   // ... in this warp too: a shuffle orders no memory
     } else {
-        go = mbar_wait<32>(sums_bar + 8 * quad, 0, s_abort);
+        go = mbar_wait_warp<32>(sums_bar + 8 * quad, 0, s_abort);
     }
     if (!go) return false;
     const float lbcb = lut_bias_times_cb(a.lut_bias, a.CB);
@@ -457,7 +457,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             constexpr uint32_t kOdd = CANONICAL ? 64 * kHalfN >> 4 : 4, kEven = CANONICAL ? 128 * kHalfN >> 4 : kHalfN * 128 >> 4;
             for (uint32_t item = first; item < n_items && ok; item += n_pairs, ++t) {
                 const uint32_t ab = t & 1, slabs = sparse_item<SPLIT>(p, item, N_TILE, rank).slabs;
-                ok = mbar_wait(acc_empty0 + 8 * ab, ((t >> 1) & 1) ^ 1, s_abort);
+                ok = mbar_wait_warp(acc_empty0 + 8 * ab, ((t >> 1) & 1) ^ 1, s_abort);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + ab * N_TILE;
@@ -465,7 +465,6 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                     const uint32_t x = x0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
                     ok = mbar_wait(b_full0 + 8 * j, pb, s_abort) && mbar_wait(a_full0 + 8 * k, pa, s_abort) &&
                          mbar_wait(turn0 + 8 * me, ((x / kMmaWarps) & 1u) ^ (me == 0 ? 1u : 0u), s_abort);   // slab 0 has its turn
-                    if (!ok) break;
                     tc_fence_after_sync();
                     if (elect_one()) {
                         const uint32_t b_lo = b_lo0 + j * (kBBytes >> 4);
@@ -479,7 +478,8 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                         umma_commit_pair(a_empty0 + 8 * k);
                         umma_commit_pair(b_empty0 + 8 * j);
                     }
-                    __syncwarp();
+                    ok = __all_sync(0xFFFFFFFFu, ok);   // behind the instructions: see ptx.cuh
+                    if (!ok) break;
                     j += kMmaWarps;
                     if (j >= SB) { j -= SB; pb ^= 1; }
                 }
@@ -522,7 +522,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
             const uint32_t slabs = sparse_item<SPLIT>(p, item, N_TILE, rank).slabs;
             for (uint32_t i0 = 0; i0 < slabs && ok; i0 += kIdxSlabs) {
                 ok = mbar_wait(i_full0 + 8 * st, ph, s_abort);
-                for (uint32_t i = (grp - (x0 + i0)) & (kGroups - 1); i < kIdxSlabs && i0 + i < slabs && ok; i += kGroups) {
+                for (uint32_t i = (grp - (x0 + i0)) & (kGroups - 1); i < kIdxSlabs && i0 + i < slabs; i += kGroups) {
                     const uint32_t x = x0 + i0 + i, k = x % kASlots, pa = (x / kASlots) & 1u;
                     uint32_t raw[kRaw], w[32], m[2];
                     load_raw(s_idx + st * kIdxBytes, i, raw);
@@ -532,8 +532,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
 #pragma unroll
                     for (int c = 0; c < 32; ++c) asm volatile("" : "+r"(w[c]));
                     asm volatile("" : "+r"(m[0]), "+r"(m[1]));
-                    ok = mbar_wait(a_empty0 + 8 * k, pa ^ 1, s_abort);
-                    if (!ok) break;
+                    ok = mbar_wait(a_empty0 + 8 * k, pa ^ 1, s_abort) && ok;
                     tc_fence_after_sync();
                     tmem_st_32x32b_x32(tmem_base + my_lanes + kDataBase + 32 * k, w);
                     tmem_st_32x32b_x2(tmem_base + my_lanes + kMetaBase + 2 * k, m);
@@ -544,6 +543,7 @@ lut_sparse_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_cons
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(i_empty0 + 8 * st);   // this warp has read its rows of the stage
+                ok = __all_sync(0xFFFFFFFFu, ok);
                 if (++st == kIdxStages) { st = 0; ph ^= 1; }
             }
             x0 += slabs;

@@ -85,3 +85,15 @@ def test_the_searching_warps_leave_together():
         assert re.match(r"\s*if \(!ok\) break;", src[w.end():])
     down = src[src.rindex("__syncthreads();", 0, src.index("tmem_dealloc(")) - 400:src.index("tmem_dealloc(")]
     assert down.index("if (s_abort)") < down.index("clock64()") < down.index("report_error(")
+
+
+@pytest.mark.parametrize("name", ["lut_sparse_umma.cu", "lut_onehot_umma.cu"])
+def test_no_lane_leaves_a_warp_alone(name):
+    """Waits of whole warps: between one whose answer is a lane's own and the vote on it no lane takes another way."""
+    src = _source(name)
+    own = list(re.finditer(r"\bok = (ok && )?mbar_wait\(", src))
+    assert len(own) >= 3
+    for w in own:
+        behind = src[w.end():]
+        assert not re.search(r"\b(break|continue|return)\b", behind[:behind.index("__all_sync(0xFFFFFFFFu, ok)")])
+    assert len(re.findall(r"__all_sync\(0xFFFFFFFFu, ok\)", src)) == 2
