@@ -3,7 +3,7 @@
 //
 // Replaces index_calculation() of the reference (inference-engine/src/host/index_calc_host.cpp:8-53), bit for bit like
 // the other search kernels: a score only decides where it is certain, and every doubtful (token, codebook) goes on to the
-// fp32 filter and from there to the reference's scan (ccs_scan.cuh).
+// reference's scan (ccs_scan.cuh).
 //
 // Every component is split into two f16 numbers, a = hi + lo to 22 bits, and a codebook's contraction axis holds
 //     activations   hi   hi   lo   1   1        centroids   -hi  -lo  -hi   hi(h)  lo(h)      h = |c|^2 / 2
@@ -13,20 +13,33 @@
 // A = |x|^2, B = max |c|^2 and u = 2^-24, |s computed - s| is at most
 //     6u (A+B)             of the split (2^-22 of x, of c, and the missing lo.lo, on sum |x_d c_d| <= (A+B)/2), 3u B of h's,
 //     (v+1) u B            of h itself,
-//     2 (3v+4) u (A+B)     of the accumulation, each of the 3v+2 products off by a whole unit in the last place of the sum,
+//     2 (3v+4) u (A+B)     of the accumulation, each of the 3v+2 products off by a whole unit in the last place of the
+//                          largest, twice (how the unit rounds is not documented),
 //     17v 2^-25            where a component's lo is subnormal,
-// so a margin of that twice and the fp32 filter's own, (22v + 54) u (A+B), would do; (24v + 64) is used.  Measured
-// against 64 bits the scores were off by at most 4 u (A+B) (v = 2, 4, 8 with 32 to 128 centroids: N(0,1), the same in
-// thousandths, a hundred added, rows and centroids at mixed magnitudes).  Rows with |x|^2 beyond 2^29 in scaled numbers,
-// and what is not finite, take the scan.
+// so a margin of that twice and the fp32 filter's own, (22v + 54) u (A+B), would do; (24v + 64) is used, three times the
+// fp32 filter's.  Measured against 64 bits the scores were off by at most 4 u (A+B) (v = 2, 4, 8 with 32 to 128 centroids:
+// N(0,1), the same in thousandths, a hundred added, rows and centroids at mixed magnitudes).  The scores are 22-bit numbers
+// where the other filter's are fp32; no score leaves the kernel, and no index depends on one that the margin does not settle.
+// Rows with |x|^2 beyond 2^29 in scaled numbers, and what is not finite, take the scan.
 //
 // What bounds it: dispatch, like the other kernels.  Per centroid two instructions of selection and half a minimum are
 // left, and nothing is read from shared memory; a token's codebook costs about 70 more (splitting, margin, hand-overs).
-// 64 centroids, v = 4: 289 instructions a warp and codebook against 433 of ccs_tile_kernel, both at 0.6 of the dispatch
-// rate; the tensor pipe is 5 % busy.  Search and a 192-column contraction, us, ccs_tile_kernel -> this one:
-//     32768 x 768 codebooks, v = 4, 64 centroids     584 -> 443         8192 x 768, v = 4, 128     305 -> 236
-//     32768 x 384, v = 8, 32                         262 -> 204         8192 x 1536, v = 2, 32     148 -> 127
-// With 16 centroids or fewer the 70 outweigh what is saved (12608 x 1536, v = 2: 99 -> 110).
+// The tensor pipe is 5 % busy.  With 16 centroids or fewer the 70 outweigh what is saved (12608 x 1536, v = 2: 99 -> 110 us).
+//
+// The scan of undecided pairs is bound by the load/store unit (75 % busy where all are undecided): a centroid that all lanes
+// read costs it as much as 32 different ones.  Undecided pairs wait in a queue of their warp, which holds all of a tile, and
+// are scanned 32 at a time (scanned on the spot they held the other warps up).  Where more than three quarters of a tile's
+// were undecided - centroids that come twice, a common offset large against their spread - the warp scans the next seven
+// tiles without a look at the scores.  (A queue of candidates for the fp32 filter, 64 of them and the whole tile anew when
+// there were more, took up to five times what ccs_tile_kernel takes.)
+//
+// Search and a 192-column contraction, us, ccs_tile_kernel -> this one, N(0,1) and every centroid twice:
+//     32768 x 768 codebooks, v = 4, 64 centroids     583 -> 438     1961 -> 1456
+//      8192 x 768, v = 4, 128                        304 -> 217      997 -> 689
+//     32768 x 384, v = 8, 32                         262 -> 201      826 -> 760
+//     16384 x 96, v = 8, 64                           72 -> 46       222 -> 168
+//      8192 x 1536, v = 2, 32                        148 -> 122      404 -> 299
+//      8192 x 768, v = 4, 32                          91 -> 82       267 -> 218
 //
 // A CTA of four warps takes CC codebooks and a run of tiles of 128 tokens.  A tile is split into f16 in shared memory
 // (K-major core matrices without swizzle, a pitch that spreads the stores over the banks) while the tile before is
@@ -34,8 +47,7 @@
 // thread reads the scores of one token back from tensor memory, 64 at a time, and the warp that reads last has the next
 // columns computed.  No barrier in that loop: warps meet at these counts alone.  128 columns of tensor memory a CTA: four
 // CTAs share an SM, and what one of them waits for the others hide (two buffers of 64 columns cost a hand-over per 64
-// scores: 119 us where this takes 102).  Undecided tokens wait in a queue of their warp and are settled 32 at a time:
-// settled on the spot they held the other warps up (198 us).
+// scores: 119 us where this took 102).
 #include "kernels.h"
 #include "ccs_scan.cuh"
 #include "ptx.cuh"
@@ -49,6 +61,7 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr uint32_t kTmemColumns = 128;
+constexpr uint32_t kBlind = 7;   // tiles scanned without a look at the scores before one that is looked at
 constexpr float kUnit = 5.9604644775390625e-08f;   // 2^-24
 
 template <int V, int CT, int CC>
@@ -65,12 +78,10 @@ struct Form {
     static constexpr int kALead = kThreads * 16 + 16, kBLead = CC * CT * 16;      // bytes from unit to unit
     static constexpr int kABytes = CC * kUnits * kALead, kBBytes = kBUnits * kBLead;
     static constexpr int kNormPitch = kThreads + (kVec <= 4 ? 8 : 4);
-    static constexpr uint32_t kAll = CT < 32 ? (1u << (CT & 31)) - 1 : 0xFFFFFFFFu;
     static constexpr int kWords = (CT + 31) / 32;                                 // of a mask of candidates
-    static constexpr int kQueue = CT > 64 ? 32 : 64;                              // undecided (token, codebook) pairs that a warp keeps
+    static constexpr int kQueue = 32 * CC + 32;                                   // undecided (token, codebook) pairs of a warp: a tile's and fewer than 32 of earlier ones
     static constexpr int kTile = kVec * kNormPitch;                               // norms of a tile
-    static constexpr int kWarpQueue = kQueue * (kWords + 1);
-    static constexpr size_t kSmem = 2 * kABytes + kBBytes + (2 * kTile + 4 * kWarpQueue) * sizeof(float);
+    static constexpr size_t kSmem = 2 * kABytes + kBBytes + (2 * kTile + 4 * kQueue) * sizeof(float);
     static_assert(CC * V % 4 == 0 && CC * CT % kWindow == 0 && kWindow % kN == 0 && kN % 16 == 0 && CC % kShared == 0 && kWindow % kRead == 0, "");
     static_assert(V % 2 == 0 && CC <= 8 && kBLead / 16 < 1 << 14, "");
 };
@@ -130,46 +141,49 @@ __device__ __forceinline__ uint32_t below_both(const float (&k)[N], float thr) {
     else return mask | (__float_as_uint(sum) & (((1u << kHalf) - 1) << kHalf));
 }
 
-// The candidates within the f16 margin (bit c: centroid c; null: all) by the fp32 filter's scores, and by the scan where these do
-// not decide either.
+// The reference's scan (ccs_scan.cuh) with the centroids straight from global memory (L1), 32 numbers in flight, two
+// components per packed instruction.  c - x for x - c: the squares are the same.
 template <int V, int CT>
-__device__ __forceinline__ uint32_t settle(const float* __restrict__ xp, const float* __restrict__ cp, const uint32_t* cand, float top) {
-    float x[V], xx = 0.f;
+__device__ __forceinline__ uint32_t scan(const float* __restrict__ xp, const float* __restrict__ cp) {
+    float x[V];   // negated
+    if constexpr (V == 2) {
+        const float2 q = __ldg(reinterpret_cast<const float2*>(xp));
+        x[0] = -q.x; x[1] = -q.y;
+    } else {
 #pragma unroll
-    for (int d = 0; d < V; ++d) {
-        x[d] = __ldg(xp + d);
-        xx = fmaf(x[d], x[d], xx);
-    }
-    const float T = fmaf(margin_factor(V), xx + top, kMarginBase);
-    constexpr uint32_t all = CT < 32 ? (1u << (CT & 31)) - 1 : 0xFFFFFFFFu;
-    if (T < kHuge) {
-        float m1 = __int_as_float(0x7f800000), m2 = m1;
-        uint32_t best = 0;
-#pragma unroll
-        for (int g = 0; g < (CT + 31) / 32; ++g) {
-#pragma unroll 1
-            for (uint32_t m = cand ? cand[g] : all; m; m &= m - 1) {
-                const uint32_t c = g * 32 + __ffs(m) - 1;
-                float cc = 0.f, s = 0.f;
-#pragma unroll
-                for (int d = 0; d < V; ++d) {
-                    const float n = -__ldg(cp + c * V + d);
-                    cc = fmaf(n, n, cc);
-                    s = fmaf(x[d], n, s);
-                }
-                s = fmaf(0.5f, cc, s);
-                if (s < m1) {
-                    m2 = m1;
-                    m1 = s;
-                    best = c;
-                } else {
-                    m2 = fminf(m2, s);
-                }
-            }
+        for (int d = 0; d < V; d += 4) {
+            const float4 q = __ldg(reinterpret_cast<const float4*>(xp + d));
+            x[d] = -q.x; x[d + 1] = -q.y; x[d + 2] = -q.z; x[d + 3] = -q.w;
         }
-        if (m2 > m1 + T) return best;   // false for NaN
     }
-    return exact_scan<V>(x, CT, [&](uint32_t c, int d) { return -__ldg(cp + c * V + d); });
+    float mn = 0.f;
+    uint32_t best = 0;
+    constexpr int kGroup = 32 / V;
+    static_assert(CT % kGroup == 0 && 32 % V == 0, "");
+#pragma unroll 1
+    for (uint32_t g = 0; g < CT; g += kGroup) {
+        float k[32];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float4 q = __ldg(reinterpret_cast<const float4*>(cp + g * V) + i);
+            k[4 * i] = q.x; k[4 * i + 1] = q.y; k[4 * i + 2] = q.z; k[4 * i + 3] = q.w;
+        }
+#pragma unroll
+        for (int c = 0; c < kGroup; ++c) {
+            float acc = 0.f;
+#pragma unroll
+            for (int d = 0; d < V; d += 2) {
+                const float2 e = __fadd2_rn(make_float2(k[c * V + d], k[c * V + d + 1]), make_float2(x[d], x[d + 1]));
+                const float2 sq = __fmul2_rn(e, e);
+                acc = d == 0 ? sq.x : __fadd_rn(acc, sq.x);   // 0 + sq.x is exact
+                acc = __fadd_rn(acc, sq.y);
+            }
+            const bool take = (c == 0 && g == 0) || __fsub_rn(mn, acc) > kEps;   // false for NaN: keeps the earlier index
+            mn = take ? acc : mn;
+            best = take ? g + c : best;
+        }
+    }
+    return best;
 }
 
 template <int V, int CT, int CC>
@@ -188,7 +202,7 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
     __shared__ uint32_t s_tmem, s_abort, s_read;
     __shared__ __align__(8) uint64_t s_bar;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    uint32_t* queue = reinterpret_cast<uint32_t*>(s_norm + 2 * F::kTile) + warp * F::kWarpQueue;   // [F::kQueue][1 + kWords]
+    uint32_t* queue = reinterpret_cast<uint32_t*>(s_norm + 2 * F::kTile) + warp * F::kQueue;
     const uint32_t cb0 = blockIdx.x * CC;
     const uint32_t t0 = blockIdx.y * tiles_per_cta, t1 = min(tiles, t0 + tiles_per_cta);
 
@@ -218,11 +232,10 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
         atomicMax(&s_largest, __float_as_uint(top));
     }
     __syncthreads();
-    float scale = 1.f, unscale = 1.f;
+    float scale = 1.f;
     if (s_largest) {
         const int e = min(40, max(-40, 3 - ((int)(s_largest >> 23) - 127)));
         scale = __int_as_float((127 + e) << 23);
-        unscale = __int_as_float((127 - e) << 23);
     }
     for (uint32_t r = tid; r < CC * CT; r += kThreads) {
         const uint32_t cb = r / CT;
@@ -351,20 +364,22 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
         if ((n & 3u) == 3u && (w + 1 < F::kWindows || more)) issue(w + 1 < F::kWindows ? side : side ^ 1u, (w + 1) % F::kWindows);
     };
     uint32_t queued = 0;
-    // Settles the queue; `over` (a tile): and all of that tile, which had more undecided pairs than the queue holds.
-    auto settle_all = [&](bool over, uint32_t tile) {
+    // Settles the queue, 32 pairs at a time, until fewer than `least` are left.
+    auto settle_all = [&](uint32_t least) {
         __syncwarp();
-        const uint32_t items = over ? F::kQueue + 32 * CC : queued;
+        uint32_t done = 0;
 #pragma unroll 1
-        for (uint32_t i = lane; i < items; i += 32) {
-            if (i >= queued && i < F::kQueue) continue;
-            const uint32_t* q = i < F::kQueue ? queue + i * (F::kWords + 1) : nullptr;
-            const uint32_t m = q ? t0 * kThreads + q[0] / 8 : tile * kThreads + tid, b = q ? q[0] % 8 : (i - F::kQueue) / 32;
-            if (m < M)
-                out[(size_t)m * CB + cb0 + b] = (uint8_t)settle<V, CT>(x + (size_t)m * K + (cb0 + b) * V, gc + b * (CT * V), q ? q + 1 : nullptr,
-                                                                      __uint_as_float(s_top[b]) * unscale * unscale);
+        for (; done + least <= queued; done += 32) {
+            if (done + lane < queued) {
+                const uint32_t q = queue[done + lane], m = t0 * kThreads + q / 8, b = q % 8;
+                out[(size_t)m * CB + cb0 + b] = (uint8_t)scan<V, CT>(x + (size_t)m * K + (cb0 + b) * V, gc + b * (CT * V));
+            }
         }
-        queued = 0;
+        const uint32_t rest = queued > done ? queued - done : 0;
+        const uint32_t keep = lane < rest ? queue[done + lane] : 0;
+        __syncwarp();
+        if (lane < rest) queue[lane] = keep;
+        queued = rest;
         __syncwarp();
     };
 
@@ -377,6 +392,7 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
     __syncthreads();
     if (t0 < t1 && warp == 0) issue(0, 0);
     if (t0 + 1 < t1) fetch(t0 + 1);
+    uint32_t blind = 0;   // tiles to come for which the scores are not looked at
     for (uint32_t tile = t0; tile < t1; ++tile) {
         const uint32_t side = (tile - t0) & 1u;
         const bool more = tile + 1 < t1;
@@ -387,7 +403,6 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
         }
         __syncwarp();
         const uint32_t m = tile * kThreads + tid;
-        bool over = false;
         float all = 0.f;
 #pragma unroll
         for (int i = 0; i < F::kVec; ++i) all += norm[i * F::kNormPitch + tid];
@@ -400,20 +415,25 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
                 if (b * V / 4 + i <= (b * V + V - 1) / 4) xx += norm[(b * V / 4 + i) * F::kNormPitch + tid];
             return fmaf(kFactor, xx, s_margin[b]);
         };
-        auto defer = [&](uint32_t b, bool undecided, const uint32_t (&cand)[F::kWords]) {   // all lanes
-            const uint32_t who = __ballot_sync(0xFFFFFFFFu, undecided && m < M), n = __popc(who);
-            if (queued + n > F::kQueue) {
-                over = true;
-            } else {
-                if (undecided && m < M) {
-                    uint32_t* q = queue + (queued + __popc(who & ((1u << lane) - 1))) * (F::kWords + 1);
-                    q[0] = ((tile - t0) * kThreads + tid) * 8 + b;
-#pragma unroll
-                    for (int g = 0; g < F::kWords; ++g) q[1 + g] = (unsound >> b) & 1u ? F::kAll : cand[g];
-                }
-                queued += n;
-            }
+        auto defer = [&](uint32_t b, bool undecided) {   // all lanes
+            const uint32_t who = __ballot_sync(0xFFFFFFFFu, undecided && m < M);
+            if (undecided && m < M) queue[queued + __popc(who & ((1u << lane) - 1))] = ((tile - t0) * kThreads + tid) * 8 + b;
+            queued += __popc(who);
         };
+        const uint32_t before = queued;
+        if (blind) {   // most pairs of an earlier tile were undecided: its scan at once
+            --blind;
+#pragma unroll 1
+            for (uint32_t w = 0; w < F::kWindows && ok; ++w) {
+                ok = mbar_wait_warp(bar, phase, abort_word);
+                if (!ok) break;
+                phase ^= 1u;
+                release(side, w, more);
+            }
+#pragma unroll 1
+            for (uint32_t b = 0; b < (m < M && ok ? CC : 0); ++b)
+                word |= (decltype(word))scan<V, CT>(x + (size_t)m * K + (cb0 + b) * V, gc + b * (CT * V)) << (8 * b);
+        } else
 #pragma unroll 1
         for (uint32_t w = 0; w < F::kWindows; ++w) {
             ok = mbar_wait_warp(bar, phase, abort_word);
@@ -483,7 +503,7 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
                         rest |= all_but_lowest(c[g]) | (c[g] ? seen : 0u);
                         seen |= c[g];
                     }
-                    defer(w * F::kCbWindow + j, ((unsound >> (w * F::kCbWindow + j)) & 1u) || rest != 0, c);
+                    defer(w * F::kCbWindow + j, ((unsound >> (w * F::kCbWindow + j)) & 1u) || rest != 0);
                 }
             }
         }
@@ -494,9 +514,10 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
             else if constexpr (CC == 4) *reinterpret_cast<uint32_t*>(o) = (uint32_t)word;
             else *reinterpret_cast<uint16_t*>(o) = (uint16_t)word;
         }
-        if (over || queued >= F::kQueue / 2) settle_all(over, tile);
+        if (queued - before > 24 * CC) blind = kBlind;   // three quarters: from there on the scores cost more than they save
+        if (queued >= 32) settle_all(32);
     }
-    if (queued && ok) settle_all(false, 0);
+    if (queued && ok) settle_all(1);
     tc_fence_before_sync();
     __syncthreads();
     if (s_abort) {
@@ -577,7 +598,7 @@ constexpr uint64_t kFewestScores = 96000000;
 
 bool ccs_umma_takes(const CcsArgs& a) {
     if (!a.dev_err || a.format != LUTAMM_INDEX_U8_ROWMAJOR || a.tokens_per_thread) return false;
-    if ((uint64_t)a.M * a.CB * a.CT < kFewestScores || reinterpret_cast<uintptr_t>(a.x) % 16 || a.K % 4) return false;
+    if ((uint64_t)a.M * a.CB * a.CT < kFewestScores || reinterpret_cast<uintptr_t>(a.x) % 16 || reinterpret_cast<uintptr_t>(a.centroid) % 16 || a.K % 4) return false;
 #define LUTAMM_CCS_UMMA(V_, CT_, CC_) \
     if (a.v == V_ && a.CT == CT_) {                                                                                     \
         float used = 0.f;                                                                                               \

@@ -180,3 +180,13 @@ def test_a_planned_run_beyond_the_tokens(fake, v, CT, M, tokens):
     assert L.lutamm_index_calculation(fake.ctx, 0, at, at, ctypes.c_uint32(M), ctypes.c_uint32(P.INDEX_U8_ROWMAJOR)) == P.OK
     (line,) = fake.log()
     assert "ccs_reg_kernel" in line and line.split()[-2] == "1"
+
+
+@pytest.mark.parametrize("offset,kernel", [(0, "ccs_umma_kernel"), (4, "ccs_tile_kernel")])
+def test_centroids_of_the_static_call_may_lie_anywhere(fake, offset, kernel):
+    """The search on the tensor cores reads them 16 bytes at a time."""
+    at, lib = ctypes.c_void_p(fake.base), fake.lib
+    ip, lp = P.make_params(16384, 768, 64, 192, 64, 0.01)
+    fake.log()
+    assert lib.lutamm_amm_static_scratch(0, None, at, ctypes.c_void_p(fake.base + offset), at, at, at, ctypes.byref(ip), ctypes.byref(lp)) == P.OK
+    assert kernel in fake.log()[0]
