@@ -7,7 +7,7 @@
 //   * the "argmin" is a sequential scan with hysteresis - centroid c replaces the running minimum only
 //     if fl(min - dist[c]) > 1e-6 - so near-ties are decided by the order of the scan.
 //
-// exact_scan() below is that statement, one (token, codebook) in one thread, ~3v + 4 instructions per centroid.
+// exact_scan() (ccs_scan.cuh) is that statement, one (token, codebook) in one thread, ~3v + 4 instructions per centroid.
 // It runs only where it can matter.  Every (token, codebook) first goes through a FILTER that evaluates
 //     s_c = |c|^2 / 2 - x.c      (so that |x - c|^2 = |x|^2 + 2 s_c),   v fused multiply-adds per centroid,
 // and looks for centroids within a margin T of the smallest s_c.  If there is exactly one, the scan ends on it
@@ -18,11 +18,11 @@
 // every other c: the scan takes the winner when it meets it and nothing after it.  Otherwise - two candidates,
 // or anything not finite - the thread runs exact_scan.  For N(0,1) data a few scans in 1e5 do at v = 2.
 //
-// What bounds it: dispatch.  Per centroid v/2 packed multiply-adds, half a packed addition (two dispatch cycles
-// each), half a three-input minimum and a funnel shift that collects the comparison's sign bit, against 3v/2 packed
-// and 4 other instructions of the scan; per (token, codebook) about 25 instructions around that.  v = 2, 16 centroids,
-// 65536 x 4096: 593 -> 460 us, the ALU pipe 53 % and the FMA pipe 45 % busy (they hardly overlap); v = 4, 64
-// centroids, 32768 x 3072: 1267 -> 472 us; v = 10, 16 centroids, 1576 x 2560: 87 -> 14 us (CUDA events around the launch).
+// What bounds it: dispatch, in ccs_reg_kernel.  Per centroid v/2 packed multiply-adds, half a packed addition (two
+// dispatch cycles each), half a three-input minimum and a funnel shift that collects the comparison's sign bit, against
+// 3v/2 packed and 4 other instructions of the scan; per (token, codebook) about 25 instructions around that.
+// 65536 x 2048 codebooks, v = 2, 16 centroids: 442 us (the scan alone 593), the ALU pipe 53 % and the FMA pipe 45 % busy
+// (they hardly overlap).  ccs_tile_kernel issues in 40 to 60 % of the cycles: a CTA stages everything, waits, and computes.
 //
 // Calls of many scores take the filter to the tensor cores: ccs_umma.cu.
 //
@@ -113,10 +113,16 @@ constexpr int kRegThreads = 128;
 // SHORT (W = 32): a thread takes one batch of kTok tokens and no more, the activations load straight into registers, and
 // the scan runs as it is: a batch small enough for this is bound by a chain of latencies, which the filter would lengthen
 // (0.3 us of a 15 us call).  Otherwise every thread takes a run of tokens.
-// With 64 numbers a codebook (v = 4 with 16 centroids, v = 2 with 32, v = 8 with 8) registers hold them for two tokens at a time, against
-// ccs_tile_kernel's copies in shared memory: 32768 x 1024, v = 4, 16 centroids 224 -> 182 us with its contraction, 8192 x
-// 256 30 -> 28; 2048 x 512, v = 2, 32 centroids 28.3 -> 25.8; 8192 x 1280, v = 8, 8 centroids
-// 95 -> 72, 8192 x 128 18.1 -> 15.2.
+//
+// With 64 numbers a codebook registers hold the centroids for two tokens at a time, where ccs_tile_kernel reads them from
+// shared memory.  Search alone, us, that kernel -> this one, N(0,1) and every centroid twice (all pairs undecided):
+//     v = 4, 16 centroids   16384 x 768 codebooks   90 -> 72   256 -> 158        8192 x 256    21 -> 18    51 -> 33
+//     v = 2, 32             4096 x 384              25 -> 17    68 -> 31         2000 x 1280   34 -> 24    96 -> 46
+//     v = 8, 8              8192 x 1280             85 -> 62   191 -> 132        8192 x 384    33 -> 23    66 -> 44
+// Both tokens have a margin of their own: with one for both, from the sum of their norms, half again as many pairs went to the scan
+// (16384 x 768, v = 4, 16 centroids, an offset of 30: 242 us, 140 now, ccs_tile_kernel 218).  Four tokens share one, which saves
+// what it costs.  The scan takes the centroids from the registers, two at a time; with single ones from shared memory,
+// 12608 x 384, v = 2, 16 centroids that come twice took 76 us, 44 like this (and N(0,1) 26.0, 25.0).
 template <int V, int CT, bool TILED, int kTok, bool SHORT, int W>
 __global__ void __launch_bounds__(kRegThreads, SHORT ? (CT * V >= 64 ? 6 : 8) : CT * V >= 64 ? (CT == 32 ? 3 : 4) : CT * V >= 32 ? 5 : 7)
 ccs_reg_kernel(const float* __restrict__ x, const float* __restrict__ cent, void* __restrict__ out, uint32_t M,
@@ -242,17 +248,47 @@ ccs_reg_kernel(const float* __restrict__ x, const float* __restrict__ cent, void
             t_cb = fine ? fmaf(margin_factor(V), top, kMarginBase) : __int_as_float(0x7f800000);
         }
 
+        // The reference's scan, two centroids at a time from the registers that hold them.
+        auto scan = [&](const float (&x)[V]) {
+            float mn = 0.f;
+            uint32_t best = 0;
+#pragma unroll
+            for (int j = 0; j < CT / 2; ++j) {
+                float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int d = 0; d < V; ++d) {
+                    const float2 e = __fadd2_rn(make_float2(x[d], x[d]), nc[j][d]);
+                    const float2 sq = __fmul2_rn(e, e);
+                    // 0 + sq is exact.  Scalar additions: a packed one is contracted with the packed multiplication
+                    acc = d == 0 ? sq : make_float2(__fadd_rn(acc.x, sq.x), __fadd_rn(acc.y, sq.y));
+                }
+                const bool take = j == 0 || __fsub_rn(mn, acc.x) > kEps;  // false for NaN: keeps the earlier index
+                mn = take ? acc.x : mn;
+                best = take ? (uint32_t)(2 * j) : best;
+                const bool next = __fsub_rn(mn, acc.y) > kEps;
+                mn = next ? acc.y : mn;
+                best = next ? (uint32_t)(2 * j + 1) : best;
+            }
+            return best;
+        };
         auto search = [&](uint32_t m) {
-            // one margin for the kTok tokens: that of the sum of their norms
-            float2 xx = make_float2(0.f, 0.f);
+            // one margin for the kTok tokens: that of the sum of their norms.  Of two, each has its own
+            constexpr int kMargins = kTok == 2 ? 2 : 1;
+            float2 xx[kMargins] = {};
 #pragma unroll
             for (int t = 0; t < kTok; ++t)
 #pragma unroll
                 for (int d = 0; d < V; d += 2) {
                     const float2 q = make_float2(cur[t][d], cur[t][d + 1]);
-                    xx = __ffma2_rn(q, q, xx);
+                    xx[t % kMargins] = __ffma2_rn(q, q, xx[t % kMargins]);
                 }
-            const float T = fmaf(margin_factor(V), xx.x + xx.y, t_cb);
+            float T[kTok];
+            bool sound = true;
+#pragma unroll
+            for (int t = 0; t < kTok; ++t) {
+                T[t] = fmaf(margin_factor(V), xx[t % kMargins].x + xx[t % kMargins].y, t_cb);
+                sound = sound && T[t] < kHuge;
+            }
             uint32_t mask[kTok], best[kTok], several = 0;
 #pragma unroll
             for (int t = 0; t < kTok; ++t) {
@@ -265,15 +301,14 @@ ccs_reg_kernel(const float* __restrict__ x, const float* __restrict__ cent, void
                     k[2 * j] = s.x;
                     k[2 * j + 1] = s.y;
                 }
-                mask[t] = below<CT>(k, min_of(k) + T);
+                mask[t] = below<CT>(k, min_of(k) + T[t]);
                 best[t] = high_bit(mask[t]);
                 several |= all_but_lowest(mask[t]);
             }
-            if (several != 0 || !(T < kHuge)) {
+            if (several != 0 || !sound) {
 #pragma unroll
                 for (int t = 0; t < kTok; ++t)
-                    if (!(T < kHuge) || all_but_lowest(mask[t]) != 0)
-                        best[t] = exact_scan<V>(cur[t], CT, [&](uint32_t c, int d) { return my_cent[c * V + d]; });
+                    if (!(T[t] < kHuge) || all_but_lowest(mask[t]) != 0) best[t] = scan(cur[t]);
             }
             store(m, best);
         };
@@ -639,9 +674,9 @@ cudaError_t run_reg_width(const CcsArgs& a, cudaStream_t s) {
 
 template <int V, int CT>
 cudaError_t run_reg(const CcsArgs& a, cudaStream_t s) {
-    // Narrow blocks waste fewer threads (32768 x 192, v = 4, 16 centroids: 62 -> 50 us with its contraction) and make shorter
-    // waves (8192 x 384: 33.1 -> 32.5; 1576 x 1024, v = 2: 24.0 -> 22.9).  Wide ones read 1 to 2 KB of a row at once, which
-    // pays where wide rows come from memory throughout (20000 x 1536, v = 4: 176 -> 170; 8192 x 1536: 92.1 against 93.3).
+    // Search alone, us, blocks of 32 codebooks and of 128.  Narrow ones waste fewer threads (32768 x 192, v = 4, 16 centroids 39
+    // and 51) and make shorter waves (8192 x 256 18.0 and 18.6; 1576 x 1024, v = 2 12.8 and 13.1).  Wide ones read 1 to 2 KB of a row
+    // at once, which pays where wide rows come from memory throughout (32768 x 1024, v = 4 177 and 169; 20000 x 1536 163 and 157).
     // (at v = 8 a narrow block reads 1 KB, and the wide one's centroids and batches are more shared memory than there is)
     if constexpr (V == 8) return run_reg_width<V, CT, 32>(a, s);
     else return a.M >= 10000 && a.CB >= 768 && a.CB % 128 == 0 ? run_reg_width<V, CT, 128>(a, s) : run_reg_width<V, CT, 32>(a, s);

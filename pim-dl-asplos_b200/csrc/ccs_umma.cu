@@ -24,7 +24,9 @@
 //
 // What bounds it: dispatch, like the other kernels.  Per centroid two instructions of selection and half a minimum are
 // left, and nothing is read from shared memory; a token's codebook costs about 70 more (splitting, margin, hand-overs).
-// The tensor pipe is 5 % busy.  With 16 centroids or fewer the 70 outweigh what is saved (12608 x 1536, v = 2: 99 -> 110 us).
+// The tensor pipe is 5 % busy.  Where ccs_reg_kernel has the centroids in registers the 70 outweigh what is saved (search and a
+// 192-column contraction, that one and this one, us: 12608 x 1536, v = 2, 16 centroids 99 and 110; 32768 x 1536, v = 2, 32 433 and 452,
+// 4096 x 768 43 and 48, 16384 x 384 61 and 64).
 //
 // The scan of undecided pairs is bound by the load/store unit (75 % busy where all are undecided): a centroid that all lanes
 // read costs it as much as 32 different ones.  Undecided pairs wait in a queue of their warp, which holds all of a tile, and
@@ -38,7 +40,6 @@
 //      8192 x 768, v = 4, 128                        304 -> 217      997 -> 689
 //     32768 x 384, v = 8, 32                         262 -> 201      826 -> 760
 //     16384 x 96, v = 8, 64                           72 -> 46       222 -> 168
-//      8192 x 1536, v = 2, 32                        148 -> 122      404 -> 299
 //      8192 x 768, v = 4, 32                          91 -> 82       267 -> 218
 //
 // A CTA of four warps takes CC codebooks and a run of tiles of 128 tokens.  A tile is split into f16 in shared memory
@@ -586,7 +587,7 @@ cudaError_t run(const CcsArgs& a, cudaStream_t s) {
 }
 
 // (sub-vector length, centroids, codebooks of a CTA)
-#define LUTAMM_CCS_UMMA_INSTANCES(X) X(2, 32, 8) X(4, 32, 4) X(4, 64, 4) X(4, 128, 4) X(8, 32, 2) X(8, 64, 2)
+#define LUTAMM_CCS_UMMA_INSTANCES(X) X(4, 32, 4) X(4, 64, 4) X(4, 128, 4) X(8, 32, 2) X(8, 64, 2)
 // Below about this many scores its prologue (tensor memory, the centroids) costs more than it saves: 100 M 1.01 to 1.2
 // times as fast, 50 M 0.95 to 1.06, 25 M 0.8 to 1.0, over these instances and 48 to 1536 codebooks.
 // The same where few tokens of very many codebooks leave its waves empty: 128 centroids, v = 4, 390 x 2560 0.33 of the time

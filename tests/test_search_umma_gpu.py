@@ -83,7 +83,7 @@ def _undecided(v, CT, CB, M, data):
     return np.ascontiguousarray(x.reshape(M, CB * v)), np.ascontiguousarray(cen)
 
 
-INSTANCES = [(2, 32, 8), (4, 32, 16), (4, 64, 8), (4, 128, 8), (8, 32, 6), (8, 64, 6)]
+INSTANCES = [(4, 32, 16), (4, 64, 8), (4, 128, 8), (8, 32, 6), (8, 64, 6)]
 
 
 @pytest.mark.parametrize("data", ["offset", "all", "most", "stretches"])
