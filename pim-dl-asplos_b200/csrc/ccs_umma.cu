@@ -7,8 +7,7 @@
 //
 // Every component is split into two f16 numbers, a = hi + lo to 22 bits, and a codebook's contraction axis holds
 //     activations   hi   hi   lo   1   1        centroids   -hi  -lo  -hi   hi(h)  lo(h)      h = |c|^2 / 2
-// 3v + 2 positions rounded up to 16 (v = 2: 8, two codebooks share an instruction, each column zero where the other
-// codebook's activations stand).  A CTA scales its activations and centroids by the power of two that brings the largest
+// 3v + 2 positions rounded up to 16.  A CTA scales its activations and centroids by the power of two that brings the largest
 // centroid component to 8..16, so nothing leaves f16's range that an ordinary table holds.  In scaled numbers, with
 // A = |x|^2, B = max |c|^2 and u = 2^-24, |s computed - s| is at most
 //     6u (A+B)             of the split (2^-22 of x, of c, and the missing lo.lo, on sum |x_d c_d| <= (A+B)/2), 3u B of h's,
@@ -54,7 +53,6 @@
 #include "ptx.cuh"
 #include "../../include/lutamm.h"
 #include <cuda_fp16.h>
-#include <type_traits>
 
 namespace lutamm {
 
@@ -67,24 +65,21 @@ constexpr float kUnit = 5.9604644775390625e-08f;   // 2^-24
 
 template <int V, int CT, int CC>
 struct Form {
-    static constexpr int kShared = V == 2 ? 2 : 1;                                // codebooks of one instruction
-    static constexpr int kUnits = V == 2 ? 1 : (3 * V + 2 + 15) / 16 * 2;         // 16-byte units of a codebook's axis
-    static constexpr int kBUnits = kUnits * kShared;
+    static constexpr int kUnits = (3 * V + 2 + 15) / 16 * 2;                      // 16-byte units of a codebook's axis
     static constexpr int kVec = CC * V / 4;                                       // float4 of a token; items of a thread
-    static constexpr int kSpan = (V + 3) / 4 + (V > 4 && V % 4 ? 1 : 0);             // float4 a codebook reaches into
+    static constexpr int kSpan = V / 4;                                           // ... of a codebook
     static constexpr int kWindow = CC * CT < 128 ? CC * CT : 128;                 // columns computed at once
     static constexpr int kRead = 64, kParts = kWindow / kRead, kCbPart = CT < kRead ? kRead / CT : 1;   // ... and read at once
     static constexpr int kWindows = CC * CT / kWindow, kCbWindow = kWindow / CT;
-    static constexpr int kN = CT * kShared;
     static constexpr int kALead = kThreads * 16 + 16, kBLead = CC * CT * 16;      // bytes from unit to unit
-    static constexpr int kABytes = CC * kUnits * kALead, kBBytes = kBUnits * kBLead;
-    static constexpr int kNormPitch = kThreads + (kVec <= 4 ? 8 : 4);
+    static constexpr int kABytes = CC * kUnits * kALead, kBBytes = kUnits * kBLead;
+    static constexpr int kNormPitch = kThreads + 8;
     static constexpr int kWords = (CT + 31) / 32;                                 // of a mask of candidates
     static constexpr int kQueue = 32 * CC + 32;                                   // undecided (token, codebook) pairs of a warp: a tile's and fewer than 32 of earlier ones
     static constexpr int kTile = kVec * kNormPitch;                               // norms of a tile
     static constexpr size_t kSmem = 2 * kABytes + kBBytes + (2 * kTile + 4 * kQueue) * sizeof(float);
-    static_assert(CC * V % 4 == 0 && CC * CT % kWindow == 0 && kWindow % kN == 0 && kN % 16 == 0 && CC % kShared == 0 && kWindow % kRead == 0, "");
-    static_assert(V % 2 == 0 && CC <= 8 && kBLead / 16 < 1 << 14, "");
+    static_assert(V % 4 == 0 && kVec == 4 && CC <= 4 && CT >= 32 && CC * CT % kWindow == 0 && kWindow % CT == 0 && CT % 16 == 0 && kWindow % kRead == 0, "");
+    static_assert(kBLead / 16 < 1 << 14, "");
 };
 
 __device__ __forceinline__ uint64_t plain_desc(uint32_t addr, uint32_t lead) {   // K-major, no swizzle: 8 rows x 16 bytes are contiguous
@@ -123,23 +118,19 @@ constexpr uint32_t kOnes = 0x3C003C00u;
 // One bit per key that lies below the threshold, like below(): the upper half of the keys by saturating multiply-adds, 1
 // or 0 each, that a second one weighs and sums in the mantissa of 2^23, so that they share the ALU's work with the FMA
 // pipe.  (2^100 (thr - key) is 0 or beyond 1: both are multiples of 2^-60, and below 2^26.)
-template <int N>
-__device__ __forceinline__ uint32_t below_both(const float (&k)[N], float thr) {
-    constexpr int kHalf = N / 2;
-    float lo[kHalf];
+__device__ __forceinline__ uint32_t below_both(const float (&k)[32], float thr) {
+    float lo[16];
 #pragma unroll
-    for (int i = 0; i < kHalf; ++i) lo[i] = k[i];
+    for (int i = 0; i < 16; ++i) lo[i] = k[i];
     const float big = __int_as_float((127 + 100) << 23), far = thr * big;
     float sum = 8388608.f;
 #pragma unroll
-    for (int i = 0; i < kHalf; ++i) {
+    for (int i = 0; i < 16; ++i) {
         float t;
-        asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(t) : "f"(k[kHalf + i]), "f"(-big), "f"(far));
-        sum = fmaf(t, (float)(N == 32 ? 1 << i : 1 << (kHalf + i)), sum);
+        asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(t) : "f"(k[16 + i]), "f"(-big), "f"(far));
+        sum = fmaf(t, (float)(1 << i), sum);
     }
-    const uint32_t mask = below<kHalf>(lo, thr);
-    if constexpr (N == 32) return __byte_perm(mask, __float_as_uint(sum), 0x5410);
-    else return mask | (__float_as_uint(sum) & (((1u << kHalf) - 1) << kHalf));
+    return __byte_perm(below<16>(lo, thr), __float_as_uint(sum), 0x5410);
 }
 
 // The reference's scan (ccs_scan.cuh) with the centroids straight from global memory (L1), 32 numbers in flight, two
@@ -147,15 +138,10 @@ __device__ __forceinline__ uint32_t below_both(const float (&k)[N], float thr) {
 template <int V, int CT>
 __device__ __forceinline__ uint32_t scan(const float* __restrict__ xp, const float* __restrict__ cp) {
     float x[V];   // negated
-    if constexpr (V == 2) {
-        const float2 q = __ldg(reinterpret_cast<const float2*>(xp));
-        x[0] = -q.x; x[1] = -q.y;
-    } else {
 #pragma unroll
-        for (int d = 0; d < V; d += 4) {
-            const float4 q = __ldg(reinterpret_cast<const float4*>(xp + d));
-            x[d] = -q.x; x[d + 1] = -q.y; x[d + 2] = -q.z; x[d + 3] = -q.w;
-        }
+    for (int d = 0; d < V; d += 4) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(xp + d));
+        x[d] = -q.x; x[d + 1] = -q.y; x[d + 2] = -q.z; x[d + 3] = -q.w;
     }
     float mn = 0.f;
     uint32_t best = 0;
@@ -241,9 +227,9 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
     for (uint32_t r = tid; r < CC * CT; r += kThreads) {
         const uint32_t cb = r / CT;
         unsigned char* row = s_b + r * 16;
-        uint32_t w[F::kBUnits * 4];
+        uint32_t w[F::kUnits * 4];
 #pragma unroll
-        for (int i = 0; i < F::kBUnits * 4; ++i) w[i] = 0;
+        for (int i = 0; i < F::kUnits * 4; ++i) w[i] = 0;
         float cc = 0.f;
 #pragma unroll
         for (int d = 0; d < V; d += 2) {
@@ -258,11 +244,8 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
         }
         w[3 * V / 2] = split_half(0.5f * cc);
 #pragma unroll
-        for (int u = 0; u < F::kBUnits; ++u) {
-            uint4 q = make_uint4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
-            if constexpr (F::kShared == 2) q = (cb & 1u) == (uint32_t)u ? make_uint4(w[0], w[1], w[2], w[3]) : make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4*>(row + u * F::kBLead) = q;
-        }
+        for (int u = 0; u < F::kUnits; ++u)
+            *reinterpret_cast<uint4*>(row + u * F::kBLead) = make_uint4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
         atomicMax(&s_top[cb], __float_as_uint(cc));
     }
     if constexpr (V > 4) {   // what no activation overwrites: the ones behind the components, and zeros
@@ -311,27 +294,15 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
             split(p, ph, pl);
             split(q, qh, ql);
             unsigned char* dst = a + row * 16;
-            if constexpr (V == 2) {
-                *reinterpret_cast<uint4*>(dst + 2 * col * F::kALead) = make_uint4(ph, ph, pl, kOnes);
-                *reinterpret_cast<uint4*>(dst + (2 * col + 1) * F::kALead) = make_uint4(qh, qh, ql, kOnes);
-            } else if constexpr (V == 4) {
+            if constexpr (V == 4) {
                 *reinterpret_cast<uint4*>(dst + 2 * col * F::kALead) = make_uint4(ph, qh, ph, qh);
                 *reinterpret_cast<uint4*>(dst + (2 * col + 1) * F::kALead) = make_uint4(pl, ql, kOnes, 0);
-            } else if constexpr (V % 4 == 0) {
+            } else {
                 const uint32_t cb = col / (V / 4), j = col % (V / 4);
                 auto at = [&](uint32_t k) { return dst + (cb * F::kUnits + k / 4) * F::kALead + (k % 4) * 4; };   // k: 32-bit word of the axis
                 *reinterpret_cast<uint2*>(at(2 * j)) = make_uint2(ph, qh);
                 *reinterpret_cast<uint2*>(at(V / 2 + 2 * j)) = make_uint2(ph, qh);
                 *reinterpret_cast<uint2*>(at(V + 2 * j)) = make_uint2(pl, ql);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const uint32_t pair = 2 * col + e, cb = pair / (V / 2), j = pair % (V / 2);
-                    auto at = [&](uint32_t k) { return dst + (cb * F::kUnits + k / 4) * F::kALead + (k % 4) * 4; };
-                    *reinterpret_cast<uint32_t*>(at(j)) = e ? qh : ph;
-                    *reinterpret_cast<uint32_t*>(at(V / 2 + j)) = e ? qh : ph;
-                    *reinterpret_cast<uint32_t*>(at(V + j)) = e ? ql : pl;
-                }
             }
         }
         fence_proxy_async_smem();
@@ -340,13 +311,13 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
         tc_fence_after_sync();
         if (elect_one()) {
 #pragma unroll
-            for (int g = 0; g < F::kWindow / F::kN; ++g) {
-                const uint32_t n = w * (F::kWindow / F::kN) + g;
-                const uint64_t a = plain_desc(a_addr + side * F::kABytes + n * F::kBUnits * F::kALead, F::kALead);
-                const uint64_t b = plain_desc(b_addr + n * F::kN * 16, F::kBLead);
+            for (int g = 0; g < F::kWindow / CT; ++g) {
+                const uint32_t n = w * (F::kWindow / CT) + g;
+                const uint64_t a = plain_desc(a_addr + side * F::kABytes + n * F::kUnits * F::kALead, F::kALead);
+                const uint64_t b = plain_desc(b_addr + n * CT * 16, F::kBLead);
 #pragma unroll
-                for (int k = 0; k < F::kBUnits / 2; ++k)
-                    umma_f16(tmem + g * F::kN, a + k * (2 * F::kALead >> 4), b + k * (2 * F::kBLead >> 4), f16_idesc(F::kN), k > 0);
+                for (int k = 0; k < F::kUnits / 2; ++k)
+                    umma_f16(tmem + g * CT, a + k * (2 * F::kALead >> 4), b + k * (2 * F::kBLead >> 4), f16_idesc(CT), k > 0);
             }
             umma_commit(bar);
         }
@@ -408,12 +379,12 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
 #pragma unroll
         for (int i = 0; i < F::kVec; ++i) all += norm[i * F::kNormPitch + tid];
         const uint32_t unsound = m >= M ? 0u : all < (float)(1 << 29) ? s_unsound : 0xFFu;
-        typename std::conditional<(CC > 4), uint64_t, uint32_t>::type word = 0;
+        uint32_t word = 0;
         auto margin = [&](uint32_t b) {
             float xx = 0.f;
 #pragma unroll
             for (int i = 0; i < F::kSpan; ++i)
-                if (b * V / 4 + i <= (b * V + V - 1) / 4) xx += norm[(b * V / 4 + i) * F::kNormPitch + tid];
+                xx += norm[(b * F::kSpan + i) * F::kNormPitch + tid];
             return fmaf(kFactor, xx, s_margin[b]);
         };
         auto defer = [&](uint32_t b, bool undecided) {   // all lanes
@@ -433,7 +404,7 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
             }
 #pragma unroll 1
             for (uint32_t b = 0; b < (m < M && ok ? CC : 0); ++b)
-                word |= (decltype(word))scan<V, CT>(x + (size_t)m * K + (cb0 + b) * V, gc + b * (CT * V)) << (8 * b);
+                word |= scan<V, CT>(x + (size_t)m * K + (cb0 + b) * V, gc + b * (CT * V)) << (8 * b);
         } else
 #pragma unroll 1
         for (uint32_t w = 0; w < F::kWindows; ++w) {
@@ -443,7 +414,7 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
             tc_fence_after_sync();
             float least[F::kParts];
             uint32_t cand[F::kCbWindow][F::kWords], several = (unsound >> (w * F::kCbWindow)) & ((1u << F::kCbWindow) - 1);
-            decltype(word) got = 0;
+            uint32_t got = 0;
 #pragma unroll
             for (int part = 0; part < F::kParts; ++part) {
                 uint32_t raw[2][32];
@@ -461,17 +432,17 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
                     for (int c = 0; c < kG; ++c) k[c] = __uint_as_float(raw[(i * CT + c) / 32][(i * CT + c) % 32]);
                     least[part] = min_of(k);
                     const float thr = least[part] + margin(w * F::kCbWindow + j);
-                    if constexpr (CT <= 32) {
-                        cand[j][0] = below_both<CT>(k, thr);
+                    if constexpr (CT == 32) {
+                        cand[j][0] = below_both(k, thr);
                         several |= all_but_lowest(cand[j][0]);
-                        got |= (decltype(word))(high_bit(cand[j][0]) & (CT - 1)) << (8 * j);
+                        got |= (high_bit(cand[j][0]) & 31u) << (8 * j);
                     } else {
                         constexpr int kAt = CT == 64 ? 0 : 2;
                         float lo[32], hi[32];
 #pragma unroll
                         for (int c = 0; c < 32; ++c) { lo[c] = k[c]; hi[c] = k[32 + c]; }
-                        cand[j][kAt * part] = below_both<32>(lo, thr);
-                        cand[j][kAt * part + 1] = below_both<32>(hi, thr);
+                        cand[j][kAt * part] = below_both(lo, thr);
+                        cand[j][kAt * part + 1] = below_both(hi, thr);
                         if constexpr (CT == 64) {
                             const uint32_t l = cand[j][0], h = cand[j][1];
                             several |= all_but_lowest(l) | all_but_lowest(h) | (l ? h : 0u);
@@ -511,8 +482,7 @@ ccs_umma_kernel(const float* __restrict__ x, const float* __restrict__ cent, uin
         if (!ok) break;
         if (m < M) {
             uint8_t* o = out + (size_t)m * CB + cb0;
-            if constexpr (CC == 8) *reinterpret_cast<uint2*>(o) = make_uint2((uint32_t)word, (uint32_t)((uint64_t)word >> 32));
-            else if constexpr (CC == 4) *reinterpret_cast<uint32_t*>(o) = (uint32_t)word;
+            if constexpr (CC == 4) *reinterpret_cast<uint32_t*>(o) = word;
             else *reinterpret_cast<uint16_t*>(o) = (uint16_t)word;
         }
         if (queued - before > 24 * CC) blind = kBlind;   // three quarters: from there on the scores cost more than they save
