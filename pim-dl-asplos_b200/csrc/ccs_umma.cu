@@ -558,10 +558,15 @@ cudaError_t run(const CcsArgs& a, cudaStream_t s) {
 
 // (sub-vector length, centroids, codebooks of a CTA)
 #define LUTAMM_CCS_UMMA_INSTANCES(X) X(4, 32, 4) X(4, 64, 4) X(4, 128, 4) X(8, 32, 2) X(8, 64, 2)
-// Below about this many scores its prologue (tensor memory, the centroids) costs more than it saves: 100 M 1.01 to 1.2
-// times as fast, 50 M 0.95 to 1.06, 25 M 0.8 to 1.0, over these instances and 48 to 1536 codebooks.
-// The same where few tokens of very many codebooks leave its waves empty: 128 centroids, v = 4, 390 x 2560 0.33 of the time
-// used 0.86, 768 x 2560 0.54 used 0.93, 1400 x 2560 0.59 used 1.01, 512 x 2048 0.69 used 1.05, 1400 x 2048 0.79 used 1.18.
+// In calls of few scores the prologue (tensor memory, the centroids) costs as much as it saves, and so do the empty waves
+// of few tokens of very many codebooks.  Times of ccs_tile_kernel over those of this one, with a 192-column contraction, over
+// 48 to 1536 codebooks:
+//     scores             100 M           50 M            25 M            12 M
+//     32 centroids       1.01 to 1.23    1.00 to 1.21    0.97 to 1.10    0.92 to 1.06
+//     64 and 128         1.15 to 1.54    1.09 to 1.42    1.06 to 1.37    1.04 to 1.50
+//     128, v = 4, 390 x 2560, 0.37 of the time used 1.14; 768 x 2560, 0.54 1.07; 512 x 2048, 0.69 1.30; 1400 x 2048, 0.79 1.32
+// Both lines were drawn for this kernel when it settled undecided pairs centroid by centroid (0.95 at 50 M, 0.86 and 0.93 in
+// the first two of the last row); for 64 centroids and more they now lie higher than they need.
 constexpr float kLeastUsed = 0.6f;
 constexpr uint64_t kFewestScores = 96000000;
 

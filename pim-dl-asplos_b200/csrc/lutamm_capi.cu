@@ -1064,7 +1064,7 @@ int lutamm_tune(lutamm_ctx* c, int layer_id, uint32_t M, lutamm_plan* best_out) 
 // stages groups operand sps".  A plan only applies to the GPU it was measured on, hence the SM count in the key, and to the
 // kernels: a file without the line of this version keeps no shape from being measured anew (the plans of the first version
 // name the dense form, at half the rate of the sparse one).  To be raised when a new kernel form may change the fastest plan.
-constexpr int kPlanVersion = 3;   // 2: searches of 128 codebooks a CTA, and v = 4 with 16 or 64 centroids through one kernel
+constexpr int kPlanVersion = 4;   // 3: the scan in ccs_reg_kernel from shared memory, 32 centroids of two on the tensor cores
 int lutamm_plan_cache_save(lutamm_ctx* c, const char* path) {
     if (!c) return fail(nullptr, LUTAMM_EINVAL, "null context");
     if (!path) return fail(c, LUTAMM_EINVAL, "null path");
