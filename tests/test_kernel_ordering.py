@@ -1,5 +1,6 @@
 """Orderings inside the tcgen05 kernels that no run shows to be missing: read in the source.  What one thread writes and
-another reads needs a barrier between them that orders memory."""
+another reads needs a barrier between them that orders memory.  The checks are of the text as it stands: they show that a line that
+was found missing once is there, not that the order is right, and a rename has to be followed here."""
 import os
 import re
 
