@@ -190,3 +190,16 @@ def test_centroids_of_the_static_call_may_lie_anywhere(fake, offset, kernel):
     fake.log()
     assert lib.lutamm_amm_static_scratch(0, None, at, ctypes.c_void_p(fake.base + offset), at, at, at, ctypes.byref(ip), ctypes.byref(lp)) == P.OK
     assert kernel in fake.log()[0]
+
+
+def test_the_tuner_launches_what_the_grid_holds(fake):
+    """It tries runs of 4 tokens at any number of them, and a launch that fails would end it."""
+    at, L = ctypes.c_void_p(fake.base), fake.lib
+    M, K, N = (1 << 20) + 16, 16, 16
+    ip, lp = P.make_params(M, K, N, 4, 16, 0.01)
+    assert L.lutamm_load_weights(fake.ctx, 0, at, at, at, ctypes.byref(ip), ctypes.byref(lp)) == P.OK
+    fake.log()
+    assert L.lutamm_tune(fake.ctx, 0, ctypes.c_uint32(M), None) == P.OK
+    searches = [ln for ln in fake.log() if "ccs_" in ln]
+    assert len({ln for ln in searches if "ccs_reg_kernel" in ln}) > 1
+    assert all(int(n) <= 65535 for ln in searches for n in ln.split()[-2:])
