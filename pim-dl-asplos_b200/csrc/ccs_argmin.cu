@@ -633,7 +633,7 @@ cudaError_t run_reg_grid(const CcsArgs& a, dim3 grid, uint32_t run, cudaStream_t
     return launch_dependent(k, grid, dim3(kRegThreads), 0, s, a.x, a.centroid, a.idx_out, a.M, a.K, a.CB, run, a.n_stile, a.cb_mtile);
 }
 
-constexpr uint64_t kMostGridY = 65535;
+constexpr uint64_t kMostGridY = 65535, kLongestRun = 192;
 constexpr uint32_t kTok = 4;   // tokens whose activations a thread loads together: one round trip to memory instead of four
 
 // tokens of a batch in a run: two where the centroids leave no registers, and no shared memory, for four
@@ -653,9 +653,12 @@ cudaError_t run_reg_width(const CcsArgs& a, cudaStream_t s) {
     const uint64_t cb_blocks = (a.CB + W - 1) / W;
     uint64_t run = a.tokens_per_thread;
     if (!run) {
-        // Waves of equal runs of up to 2048 tokens, filled as far as whole runs fill them: a last wave that is a third full
+        // Waves of equal runs of up to 192 tokens, filled as far as whole runs fill them: a last wave that is a third full
         // costs as much as a full one, and staging the centroids costs a few microseconds per wave (32 tokens' worth).
-        const uint64_t wave = resident_ctas<V, CT, kTok, false, W>(), cap = 2048 * kGroups;
+        // In longer runs CTAs that read the same rows drift apart (65536 x 784 codebooks, v = 2, 32 centroids: a wave of 964 tokens
+        // 351 us, 384 tokens 365, 96 to 256 335 to 343; v = 4, 16 centroids: a wave of 712 273, 384 285, 96 to 256 256 to 264).  A cap of
+        // 128 or 256 does the same within 1 % on average over 140 calls.
+        const uint64_t wave = resident_ctas<V, CT, kTok, false, W>(), cap = kLongestRun * kGroups;
         const uint64_t fewest = (cb_blocks * ((a.M + cap - 1) / cap) + wave - 1) / wave;
         uint64_t least = ~0ull;
         for (uint64_t waves = fewest; waves < fewest + 4; ++waves) {
@@ -664,7 +667,7 @@ cudaError_t run_reg_width(const CcsArgs& a, cudaStream_t s) {
             const uint64_t r = (a.M + rows * kGroups - 1) / (rows * kGroups), cost = waves * (r + 32);
             if (cost < least) { least = cost; run = r; }
         }
-        if (!run) run = 2048;
+        if (!run) run = kLongestRun;
     }
     // what a plan names, as far as the grid holds it and there are tokens (a run of 2^32 - 1 rounds up to none)
     run = std::clamp(run, (a.M + kMostGridY * kGroups - 1) / (kMostGridY * kGroups), (a.M + kGroups - 1) / kGroups);
